@@ -11,12 +11,15 @@
 // Semantics follow the reference's src/kernels.cu; every device function
 // cites the lines it restates.  Two launch forms share these functions:
 //   plain : one kernel per reference kernel, in the reference's order;
-//   fused : one persistent kernel per step, a warp per env.
+//   fused : two kernels per step, the agents (a thread per env) and the
+//           images (a persistent grid; a warp or a team of warps per env).
 #pragma once
 #include <cuda_runtime.h>
 #include <cuda_fp16.h>
 #include <stdint.h>
+#include <algorithm>
 #include <type_traits>
+#include <utility>
 #include "mc_internal.h"
 #include "mc_ieee_math.h"
 #include "mc_philox.h"
@@ -176,19 +179,6 @@ __device__ __forceinline__ void load_action_from(const ActionSrc& a, float look_
     }
 }
 
-__device__ __forceinline__ void load_action(const mc_kp& p, long long i, int8_t b[8], float& l0, float& l1) {
-    if (p.actions) {
-        float lk[2];
-        mc_discrete_to_buttons(p.actions[i], p.look_delta, b, lk);
-        l0 = lk[0];
-        l1 = lk[1];
-    } else {
-#pragma unroll
-        for (int k = 0; k < 8; ++k) b[k] = p.buttons[i * 8 + k];
-        l0 = p.look[i * 2 + 0];
-        l1 = p.look[i * 2 + 1];
-    }
-}
 
 struct Agent {
     float x, y, z, vx, vy, vz, yaw, pitch;
@@ -226,12 +216,12 @@ __device__ __forceinline__ void store_agent(const mc_kp& p, long long i, const A
 //   move_x = ((sin*fwd)*speed)*dt + ((cos*str)*walk)*dt   (the build fuses the strafe product)
 //   move_z = ((cos*fwd)*speed)*dt - ((sin*str)*walk)*dt   (the build fuses the forward product)
 //   vel_y += gravity*dt;  y += vel_y*dt                   (both fused)
-__device__ __forceinline__ void physics(Agent& a, const Dec& d, const mc_kp& p) {
+__device__ __forceinline__ void physics(Agent& a, const Dec& d, const mc_kp& p, float& sin_yaw, float& cos_yaw) {
     a.yaw = N::add(a.yaw, d.dyaw);
     float new_pitch = N::add(a.pitch, d.dpitch);
     a.pitch = fminf(fmaxf(new_pitch, -1.56f), 1.56f);
-    float cos_yaw = N::cos(a.yaw);
-    float sin_yaw = N::sin(a.yaw);
+    cos_yaw = N::cos(a.yaw);  // of the new yaw: the interaction's and the camera's too
+    sin_yaw = N::sin(a.yaw);
     float fwd = d.fwd, str = d.strafe;
     float speed = N::mul(p.walk_speed, d.speed);
     float fx_ = N::mul(N::mul(N::mul(sin_yaw, fwd), speed), p.dt);
@@ -350,40 +340,43 @@ __device__ __forceinline__ int interact_seq(int8_t* w, const Agent& a, bool brk,
     return -1;
 }
 
-// The same interaction with the 32 samples spread over the 32 lanes of a
-// warp: the first in-bounds solid sample is the lowest set bit of a ballot
-// and the placement voxel is the highest in-bounds sample below it, which is
-// exactly what the reference's sequential loop selects.  Must be called by
-// all 32 lanes.  Returns the in-env index written (-1 if none), uniform
-// across the warp; *mod_val gets the value written.
-__device__ __forceinline__ int interact_warp(int8_t* w, const Agent& a, bool brk, bool place,
-                                             const mc_kp& p, int lane, float* reward, int8_t* mod_val) {
-    *reward = 0.0f;
-    *mod_val = 0;
-    if (!brk && !place) return -1;  // warp-uniform
-    float dx, dy, dz;
-    interact_dir(a, dx, dy, dz);
-    Sample s = interact_sample(lane, a.x, N::add(a.y, 1.6f), a.z, dx, dy, dz, p.wx, p.wy, p.wz);
-    int8_t blk = (s.inb && in_bounds(s.idx, (long long)p.wx * p.wy * p.wz, MC_SITE_INTERACT)) ? w[s.idx] : AIR;
-    unsigned solid = __ballot_sync(0xffffffffu, s.inb && blk >= 0);
-    unsigned inbm = __ballot_sync(0xffffffffu, s.inb);
-    if (solid == 0u) return -1;
-    int first = __ffs(solid) - 1;
-    if (brk) {
-        int8_t hb = (int8_t)__shfl_sync(0xffffffffu, (int)blk, first);
-        int hidx = __shfl_sync(0xffffffffu, s.idx, first);
-        if (reward_hit(p, hb)) *reward = p.reward_value;
-        if (lane == first) w[s.idx] = AIR;
-        *mod_val = AIR;
-        return hidx;
+// The same interaction for the agent kernel, one thread per env, in two parts:
+// all 32 samples are loaded at once (independent loads: one memory latency
+// instead of one per sample the sequential loop looks at), then judged.  The
+// first in-bounds solid sample is the lowest set bit of `solid` and the
+// placement voxel the highest in-bounds sample below it, which is what the
+// sequential loop selects.
+struct Look {
+    float ex, ey, ez, dx, dy, dz;
+    unsigned inb, solid;
+};
+__device__ __forceinline__ void look_samples(Look& l, const int8_t* w, const mc_kp& p) {
+    int8_t blk[32];
+    l.inb = 0;
+    l.solid = 0;
+#pragma unroll
+    for (int k = 0; k < 32; ++k) {
+        const Sample s = interact_sample(k, l.ex, l.ey, l.ez, l.dx, l.dy, l.dz, p.wx, p.wy, p.wz);
+        const bool in = s.inb && in_bounds(s.idx, (long long)p.wx * p.wy * p.wz, MC_SITE_INTERACT);
+        l.inb |= in ? 1u << k : 0u;
+        blk[k] = in ? w[s.idx] : AIR;
     }
-    unsigned before = inbm & ((1u << first) - 1u);
-    if (before == 0u) return -1;
-    int pl = 31 - __clz(before);
-    int pidx = __shfl_sync(0xffffffffu, s.idx, pl);
-    if (lane == pl) w[s.idx] = DIRT;
-    *mod_val = DIRT;
-    return pidx;
+#pragma unroll
+    for (int k = 0; k < 32; ++k) l.solid |= blk[k] >= 0 ? 1u << k : 0u;
+}
+// Returns the in-env index written (-1 if none), *val the value written there.
+__device__ __forceinline__ int interact_judge(const Look& l, int8_t* w, bool brk, const mc_kp& p, float* reward,
+                                              int* val) {
+    if (l.solid == 0u) return -1;
+    const int first = __ffs(l.solid) - 1;
+    const unsigned before = l.inb & ((1u << first) - 1u);
+    if (!brk && before == 0u) return -1;
+    const int k = brk ? first : 31 - __clz(before);
+    const int idx = interact_sample(k, l.ex, l.ey, l.ez, l.dx, l.dy, l.dz, p.wx, p.wy, p.wz).idx;
+    if (brk && reward_hit(p, w[idx])) *reward = p.reward_value;
+    *val = brk ? AIR : DIRT;
+    w[idx] = (int8_t)*val;
+    return idx;
 }
 
 // ---------------------------------------------------------------------------
@@ -565,17 +558,6 @@ struct VoxShared {
         return in_bounds(idx, n, MC_SITE_MARCH_SHARED) ? w[idx] : (int8_t)-1;
     }
 };
-// Either source behind one generic pointer (one call site for both), with a
-// per-env flag telling whether it points into shared memory.
-struct VoxEither {
-    const int8_t* w;
-    bool smem;
-    __device__ __forceinline__ int8_t operator()(int idx) const { return w[idx]; }
-    __device__ __forceinline__ int8_t at(int idx, int n) const {
-        return in_bounds(idx, n, smem ? MC_SITE_MARCH_SHARED : MC_SITE_MARCH_GLOBAL) ? w[idx] : (int8_t)-1;
-    }
-};
-
 struct Hit {
     int blk;    // block id, -1 for sky
     int face;   // -1 none, 0 x, 1 y, 2 z
@@ -914,8 +896,6 @@ template <class V>
 __device__ __forceinline__ bool staged_source(const V& vox, int wx, int wy, int wz) {
     if constexpr (std::is_same<V, VoxShared>::value) {
         return wx <= 64 && wy <= 64 && wz <= 64;
-    } else if constexpr (std::is_same<V, VoxEither>::value) {
-        return vox.smem && wx <= 64 && wy <= 64 && wz <= 64;
     } else {
         (void)vox; (void)wx; (void)wy; (void)wz;
         return false;
@@ -925,7 +905,7 @@ __device__ __forceinline__ bool staged_source(const V& vox, int wx, int wy, int 
 // staged_source turns away).
 template <class V>
 __device__ __forceinline__ uint32_t staged_base(const V& vox) {
-    if constexpr (std::is_same<V, VoxShared>::value || std::is_same<V, VoxEither>::value) {
+    if constexpr (std::is_same<V, VoxShared>::value) {
         return (uint32_t)__cvta_generic_to_shared(vox.w);
     } else {
         (void)vox;
@@ -967,17 +947,11 @@ __device__ __forceinline__ float aabb_exit(float ix, float iy, float iz, float l
 // entered closer than view_distance) the march has no distance test.  In
 // both, `ytop` (per env: no solid voxel above this layer) ends rays going up
 // once they pass it, as sky.
-// VDLIM = false leaves out the branch-free march for view-limited worlds
-// (those then take the reference-shaped loop), for callers whose register
-// budget is better spent elsewhere.
-// TAB: the caller passes `start`, the packed march's start values for the
-// eight sign combinations of the ray (packed_starts), whenever the packed
-// march applies to the env (nullptr otherwise).
-template <bool FASTG, class V, bool VDLIM = true, bool TAB = false>
+template <bool FASTG, class V>
 __device__ __forceinline__ Hit shade_ray(const Cam& c, const Dda0& d0, float u, float v, const V& vox, int wx, int wy,
                                          int wz, int max_steps, float vd, int gh, bool inside,
                                          bool skip_first = false, bool sky_exit = false, bool vd_safe = false,
-                                         int ytop = 1 << 20, const int4* start = nullptr) {
+                                         int ytop = 1 << 20) {
     float ray_x, ray_y, ray_z;
     ray_dir<true>(c, u, v, ray_x, ray_y, ray_z);
     float ray_len = N::sqrt(len2(ray_x, ray_y, ray_z));
@@ -1022,10 +996,8 @@ __device__ __forceinline__ Hit shade_ray(const Cam& c, const Dda0& d0, float u, 
     int idx = vy * wxz + vx * wz + vz;
     const int dix = sx * wz, diy = sy * wxz, diz = sz;
     int step = 0;
-    if constexpr (std::is_same<V, VoxShared>::value || std::is_same<V, VoxEither>::value) {
-        bool staged = true;
-        if constexpr (std::is_same<V, VoxEither>::value) staged = vox.smem;
-        if (!FASTG && sky_exit && staged && max_steps > 0 && wx <= 64 && wy <= 64 && wz <= 64) {
+    if constexpr (std::is_same<V, VoxShared>::value) {
+        if (!FASTG && sky_exit && max_steps > 0 && wx <= 64 && wy <= 64 && wz <= 64) {
             // A staged world and the eye inside the box: the PTX marches.
             // They test view_distance once, at the hit: t never decreases
             // along the ray, so a first hit closer than view_distance is the
@@ -1039,12 +1011,7 @@ __device__ __forceinline__ Hit shade_ray(const Cam& c, const Dda0& d0, float u, 
                       cz = (sz > 0) ? wz - 1 - vz : vz;
             if (b < 0) {
                 const uint32_t base = (uint32_t)__cvta_generic_to_shared(vox.w);
-                if (TAB && start) {
-                    // the env's start values for this ray's signs
-                    const int4 e = start[(ray_x >= 0.0f ? 1 : 0) | (ray_y >= 0.0f ? 2 : 0) | (ray_z >= 0.0f ? 4 : 0)];
-                    b = march_packed_shared(base, e.x, e.y, e.z, e.w, tmx, tmy, tmz, tdx, tdy, tdz,
-                                            staged_range(base, wxz, nvox));
-                } else if (vd_safe && max_steps > wx + wy + wz && wx <= 31 && wy <= 31 && wz <= 31 &&
+                if (vd_safe && max_steps > wx + wy + wz && wx <= 31 && wy <= 31 && wz <= 31 &&
                            wx * wy * wz < 8192) {
                     // index and in-box counts in one register (march_packed_shared)
                     const int packed = (idx << 18) | ((31 - cx) << 12) | ((31 - max(cy, -32)) << 6) | (31 - cz);
@@ -1137,7 +1104,7 @@ __device__ __forceinline__ Hit shade_ray(const Cam& c, const Dda0& d0, float u, 
         h.t = t;
         return h;
     }
-    if (VDLIM && !FASTG && sky_exit && max_steps > 0) {
+    if (!FASTG && sky_exit && max_steps > 0) {
         // the same branch-free march with the distance test and the step
         // count in its single exit test (worlds whose far corners lie beyond
         // view_distance)
@@ -1284,13 +1251,10 @@ __device__ __forceinline__ uint32_t to_u8(float x) {
 // caller needs only the colour of sky pixels) the march stops when the ray
 // leaves the box, where the reference keeps stepping out-of-box voxels until
 // max_steps: a ray that left never re-enters, so both end as sky.
-// TAB: `start` holds the packed march's start values per ray sign
-// combination (packed_start) whenever every ray of the env takes the packed
-// march, else nullptr.
-template <bool TRIG, class V, bool TAB = false>
+template <bool TRIG, class V>
 __device__ __forceinline__ Hit flat_ray(const Cam& c, const Dda0& d0, float u, float v, const V& vox, int wx, int wy,
                                         int wz, int max_steps, bool skip_first = false, bool sky_exit = false,
-                                        int ytop = 1 << 20, const int4* start = nullptr) {
+                                        int ytop = 1 << 20) {
     float ray_x, ray_y, ray_z;
     ray_dir<TRIG>(c, u, v, ray_x, ray_y, ray_z);
     float ray_len = N::rsqrt(len2(ray_x, ray_y, ray_z));
@@ -1325,14 +1289,8 @@ __device__ __forceinline__ Hit flat_ray(const Cam& c, const Dda0& d0, float u, f
             // a ray going up stops above ytop (no solid voxel lies higher): it ends as sky
             const int cx = (sx > 0) ? wx - 1 - vx : vx, cy = (sy > 0) ? min(wy - 1, ytop) - vy : vy,
                       cz = (sz > 0) ? wz - 1 - vz : vz;
-            if (TAB && start) {
-                const int4 e = start[(ray_x >= 0.0f ? 1 : 0) | (ray_y >= 0.0f ? 2 : 0) | (ray_z >= 0.0f ? 4 : 0)];
-                b = march_packed_shared(staged_base(vox), e.x, e.y, e.z, e.w, tmx, tmy, tmz, tdx, tdy, tdz,
-                                        staged_range(staged_base(vox), wxz, nvox));
-            } else {
-                b = march_staged(staged_base(vox), idx, cx, cy, cz, dix, diy, diz, wx, wy, wz, max_steps, tmx, tmy,
+            b = march_staged(staged_base(vox), idx, cx, cy, cz, dix, diy, diz, wx, wy, wz, max_steps, tmx, tmy,
                                  tmz, tdx, tdy, tdz);
-            }
             if (b >= 0) {
                 const bool bx = tmx < tmy && tmx < tmz;
                 face = bx ? 0 : ((tmy < tmz) ? 1 : 2);
@@ -1465,7 +1423,7 @@ __global__ void k_decode(mc_kp p) {
     if (i >= p.B) return;
     int8_t b[8];
     float l0, l1;
-    load_action(p, i, b, l0, l1);
+    load_action_from(ActionSrc{p.actions, p.buttons, p.look}, p.look_delta, i, b, l0, l1);
     Dec d = decode_buttons(b, l0, l1, p.sprint_mult);
     p.s_fwd[i] = d.fwd;
     p.s_strafe[i] = d.strafe;
@@ -1494,7 +1452,8 @@ __global__ void k_physics(mc_kp p) {
     long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= p.B) return;
     Agent a = load_agent(p, i);
-    physics(a, load_dec(p, i), p);
+    float sy, cy;
+    physics(a, load_dec(p, i), p, sy, cy);
     p.positions[i * 3 + 0] = a.x;
     p.positions[i * 3 + 1] = a.y;
     p.positions[i * 3 + 2] = a.z;
@@ -1660,7 +1619,7 @@ __global__ void __launch_bounds__(128) k_render_coalesced(const int8_t* vox, con
 }
 
 // ---------------------------------------------------------------------------
-// Fused form: one persistent kernel per step, one warp per env
+// Fused form: shared-memory layout and helpers of the image kernels
 // ---------------------------------------------------------------------------
 // Shared memory layout (per CTA): u/v tables, colour tables, then per warp a
 // pixel staging buffer, an mbarrier and (stage=1) one world.  A warp marches
@@ -1727,25 +1686,13 @@ __device__ __forceinline__ bool mbar_wait(uint32_t mbar, uint32_t phase, int pol
     return false;
 }
 
-// Write `bytes` of a repeating 48-byte pattern (p0 p1 p2) to dst, lanes
-// strided.  dst must be 16-byte aligned and bytes a multiple of 16.
-__device__ __forceinline__ void fill_pattern16(uint8_t* dst, int bytes, uint4 p0, uint4 p1, uint4 p2, int lane) {
-    uint4* d = reinterpret_cast<uint4*>(dst);
-    int n = bytes >> 4;
-    int m = lane % 3;  // (lane + 32 k) mod 3 advances by 2 per iteration
-    for (int k = lane; k < n; k += 32) {
-        d[k] = (m == 0) ? p0 : ((m == 1) ? p1 : p2);
-        m = (m + 2 >= 3) ? m - 1 : m + 2;
-    }
-}
-
-// Next env for this warp: claimed from a device counter (dynamic schedule,
+// Next unit of this warp: claimed from a device counter (flag word `counter`; dynamic schedule,
 // balances the uneven per-env work) or by static striding.
-__device__ __forceinline__ long long next_env(const mc_kp& p, long long cur, long long total_warps, int lane) {
+__device__ __forceinline__ int next_unit(const mc_kp& p, int counter, int cur, int total_warps, int lane) {
     if (!p.sched_dynamic) return cur + total_warps;
     unsigned v = 0;
-    if (lane == 0) v = atomicAdd(reinterpret_cast<unsigned*>(&p.flags[MC_FLAG_WORK]), 1u);
-    return (long long)__shfl_sync(0xffffffffu, v, 0);
+    if (lane == 0) v = atomicAdd(reinterpret_cast<unsigned*>(&p.flags[counter]), 1u);
+    return (int)__shfl_sync(0xffffffffu, v, 0);
 }
 
 // Per-warp view of the shared-memory tables and buffers used by one env.
@@ -1757,7 +1704,7 @@ struct FusedCtx {
     const uint8_t (*s_rgb8)[3];
     const uint8_t* s_sky8;
     uint8_t* stage;              // staging band of this warp
-    int8_t* sworld;              // staged world of this warp
+    uint8_t* colours;            // the colour tables' start
     uint32_t mbar_a;             // mbarrier of this warp
     float rcp_vd;                // reciprocal of the env's view distance
     const float4* s_cs;          // colour x shade table of the common-case loop (fast_band)
@@ -1783,23 +1730,26 @@ __device__ __forceinline__ void build_fast_tables(float4* s_cs, uint32_t* s_rgbp
 constexpr int kColourTableBytes = 13 * 3 * 4 + 16 + 13 * 3 + 3;
 static_assert(kColourTableBytes <= MC_COLOUR_TABLE_BYTES, "colour tables");
 
+__device__ __forceinline__ void colour_tables(uint8_t* base, FusedCtx& cx) {
+    cx.colours = base;
+    cx.s_rgb = reinterpret_cast<const float (*)[3]>(base);
+    cx.s_sky = reinterpret_cast<const float*>(base + 13 * 3 * 4);
+    cx.s_rgb8 = reinterpret_cast<const uint8_t (*)[3]>(base + 13 * 3 * 4 + 16);
+    cx.s_sky8 = base + 13 * 3 * 4 + 16 + 13 * 3;
+}
+
 __device__ __forceinline__ void load_colour_tables(uint8_t* base, FusedCtx& cx) {
-    float (*s_rgb)[3] = reinterpret_cast<float (*)[3]>(base);
-    float* s_sky = reinterpret_cast<float*>(s_rgb + 13);
-    uint8_t (*s_rgb8)[3] = reinterpret_cast<uint8_t (*)[3]>(s_sky + 4);
-    uint8_t* s_sky8 = reinterpret_cast<uint8_t*>(s_rgb8 + 13);
+    colour_tables(base, cx);
+    float* rgb = reinterpret_cast<float*>(base);
+    uint8_t* rgb8 = base + 13 * 3 * 4 + 16;
     for (int k = threadIdx.x; k < 39; k += blockDim.x) {
-        s_rgb[k / 3][k % 3] = c_rgb[k / 3][k % 3];
-        s_rgb8[k / 3][k % 3] = c_rgb8[k / 3][k % 3];
+        rgb[k] = c_rgb[k / 3][k % 3];
+        rgb8[k] = c_rgb8[k / 3][k % 3];
     }
     if (threadIdx.x < 3) {
-        s_sky[threadIdx.x] = c_sky[threadIdx.x];
-        s_sky8[threadIdx.x] = c_sky8[threadIdx.x];
+        rgb[39 + threadIdx.x] = c_sky[threadIdx.x];
+        rgb8[39 + threadIdx.x] = c_sky8[threadIdx.x];
     }
-    cx.s_rgb = s_rgb;
-    cx.s_sky = s_sky;
-    cx.s_rgb8 = s_rgb8;
-    cx.s_sky8 = s_sky8;
 }
 
 // u/v tables of one image size (threads of the CTA cooperate).
@@ -1837,13 +1787,12 @@ __device__ __forceinline__ RayPar ray_par(const mc_kp& p) {
 }
 
 // One pixel's ray through one of the two voxel sources.
-// VDLIM = false: view-limited worlds take the reference-shaped loop (fewer registers).
-template <int FAM, class V, bool VDLIM = true>
+template <int FAM, class V>
 __device__ __forceinline__ Hit march_pixel(const RayPar& p, const Cam& c, const Dda0& d0, float u, float v,
                                            const V& vox, bool inside, bool skip_first, bool sky_exit = false,
                                            bool vd_safe = false, int ytop = 1 << 20) {
     if (FAM == MC_FAM_SHADED || FAM == MC_FAM_SHADED_FAST)
-        return shade_ray<FAM == MC_FAM_SHADED_FAST, V, VDLIM>(c, d0, u, v, vox, p.wx, p.wy, p.wz, p.max_steps, p.vd,
+        return shade_ray<FAM == MC_FAM_SHADED_FAST, V>(c, d0, u, v, vox, p.wx, p.wy, p.wz, p.max_steps, p.vd,
                                                               p.gh, inside, skip_first, sky_exit, vd_safe, ytop);
     if (FAM == MC_FAM_FP16) return fp16_ray(c, d0, u, v, vox, p.wx, p.wy, p.wz, p.max_steps);
     return flat_ray<FAM != MC_FAM_PREBASIS>(c, d0, u, v, vox, p.wx, p.wy, p.wz, p.max_steps, skip_first, sky_exit,
@@ -1857,13 +1806,19 @@ __device__ __forceinline__ void mbar_init_warp(uint32_t mbar_a, int lane) {
     }
 }
 
-// Last warp of a dynamically scheduled launch resets the work counters.
-__device__ __forceinline__ void finish_dynamic(int32_t* flags, long long total_warps) {
+// The last warp (or team) of a dynamically scheduled launch resets the work
+// counters and, for each of the groups, the any-done flag that the launch's
+// regeneration has answered.  Every other one has read what it needs by then.
+template <class Groups>
+__device__ __forceinline__ void finish_dynamic(int32_t* flags, long long total, Groups clear_done) {
     __threadfence();
     unsigned prev = atomicAdd(reinterpret_cast<unsigned*>(&flags[MC_FLAG_WARPS_DONE]), 1u);
-    if (prev == (unsigned)(total_warps - 1)) {
+    if (prev == (unsigned)(total - 1)) {
         flags[MC_FLAG_WORK] = 0;
+        flags[MC_FLAG_SLOW_WORK] = 0;
         flags[MC_FLAG_WARPS_DONE] = 0;
+        flags[MC_FLAG_ANY_SLOW] = 0;
+        clear_done();
         __threadfence();
     }
 }
@@ -1999,13 +1954,8 @@ __device__ __forceinline__ UpBounds staged_up_bounds(const int8_t* world, int wx
 }
 
 // ---------------------------------------------------------------------------
-// Fused step, one warp per env (one env group per launch)
+// Rendering one env
 // ---------------------------------------------------------------------------
-// The per-env body below does what agent_step + fill_env + render_env of the
-// team kernel do, written out in one piece: built from those helpers, the
-// same kernel needed spill slots at its 64-register budget (4 CTAs of 8 warps
-// per SM) and ran 8% slower on B=32768, 16^3, 32x32, so it keeps its own
-// copy; the parity tests hold the two kernels to the same bits.
 // The common-case render of one band of an env's image (both step
 // kernels): the world is staged, the eye is inside the box with air in its
 // voxel (every ray starts one DDA step in, and ends as sky when it leaves
@@ -2127,15 +2077,11 @@ __device__ __forceinline__ int4 split_start(int k, int vx, int vy, int vz, int w
     return make_int4(split_counts(cx, cy, cz, max_steps, wx, wy, wz), sx * wz, sy * wx * wz, sz);
 }
 
-// Whether an env takes the common-case loop, and which march: 0 no, 1
-// packed, 2 split.  `eye_air_inside`: the eye is strictly inside the box
-// (view distance > 0 for the shaded family) and its voxel holds air.
+// Which march an env on the common path takes: 1 packed (small worlds where
+// every ray leaves the box before max_steps; for the shaded family the whole
+// box within view distance), 2 split.
 template <int FAM>
-__device__ __forceinline__ int fast_kind(bool staged, bool eye_air_inside, bool dbg, bool vd_safe, int max_steps,
-                                         int wx, int wy, int wz, int W, int H, int TW, int bpp, bool vec_ok) {
-    if (!(FAM == MC_FAM_SHADED || FAM == MC_FAM_MINIMAL || FAM == MC_FAM_PREBASIS)) return 0;
-    if (!staged || !eye_air_inside || dbg || max_steps <= 0 || wx > 64 || wy > 64 || wz > 64) return 0;
-    if (W % TW || H % (32 / TW) || !vec_ok || ((W * (32 / TW) * bpp) & 15)) return 0;
+__device__ __forceinline__ int fast_kind(bool vd_safe, int max_steps, int wx, int wy, int wz) {
     const bool packed = (FAM == MC_FAM_SHADED ? vd_safe : true) && max_steps > wx + wy + wz && wx <= 31 &&
                         wy <= 31 && wz <= 31 && wx * wy * wz < 8192;
     return packed ? 1 : 2;
@@ -2150,460 +2096,292 @@ __device__ __forceinline__ void build_fast_start(int4* sstart, int kind, const D
     __syncwarp();
 }
 
-// Per-env facts of a render (EnvRender::bits).
-// MC_ER_TSCAN: the up bounds are scanned by the whole team after its barrier.
-enum { MC_ER_DONE = 1, MC_ER_BURIED = 2, MC_ER_INSIDE = 4, MC_ER_SKIP = 8, MC_ER_STAGED = 16, MC_ER_TSCAN = 32 };
+// Per-env facts of a render (EnvRec::bits, EnvRender::bits).
+// MC_ER_SLOW: a marching env that needs the general path (render_slow_from).
+enum { MC_ER_DONE = 1, MC_ER_BURIED = 2, MC_ER_INSIDE = 4, MC_ER_SKIP = 8, MC_ER_SLOW = 16 };
 
-// The rest of a per-warp launch for a warp whose bulk copy timed out
-// (defined after render_env): env e, already stepped, then `claimed` (the
-// env a depth-2 warp has already claimed, or -1 for none), then every env
-// the warp claims after them, rendered from the worlds in global memory.
-// Called after the main loop and out of line, so the staged path keeps its
-// registers.  Returns whether any of those envs was done.
-template <int FAM, bool F32>
-__device__ __noinline__ bool fused_finish_from_global(const mc_kp& p, long long e, long long claimed,
-                                                      long long total_warps, int tile_w, int lane, FusedCtx cx);
+// ---------------------------------------------------------------------------
+// The agents: one thread per env
+// ---------------------------------------------------------------------------
+// What the image of one env needs from its agent step: the eye, sin and cos of
+// yaw and pitch (the same calls the reference makes per pixel), and the facts
+// settled by the eye's voxel.  48 bytes, read as three 16-byte loads.
+struct __align__(16) EnvRec {
+    float ex, ey, ez;
+    int env;             // the env's index in its group
+    float sy, cy, sp, cp;
+    int bits;            // MC_ER_*
+    int fill_blk;        // block of the uniform fill of a buried camera
+    int arrived;         // slices of the image that are done (last_slice)
+    int pad;
+};
+static_assert(sizeof(EnvRec) == MC_REC_BYTES, "env record");
 
-#ifndef MC_FUSED_MIN_BLOCKS
-#define MC_FUSED_MIN_BLOCKS 4
-#endif
-// DEPTH: 0 worlds read from global memory, 1 staged, 2 staged with the next
-// env claimed ahead and its world prefetched into L2.
-template <int FAM, bool F32, int DEPTH>
-__global__ void __launch_bounds__(256, MC_FUSED_MIN_BLOCKS) k_step_fused(const __grid_constant__ mc_kp p, int tile_w) {
-    constexpr bool STAGE = DEPTH > 0;
-    constexpr bool prefetch = DEPTH == 2;
-    extern __shared__ __align__(16) uint8_t smem[];
-    const int lane = threadIdx.x & 31;
-    const int warp = threadIdx.x >> 5;
-    const int nwarps = blockDim.x >> 5;
-    const int W = p.W, H = p.H;
-    const int HW = W * H;
-    const int wxz = p.wx * p.wz;
-    const int wxyz = wxz * p.wy;
-    FusedLayout L = fused_layout(W, H, wxyz, p.wx * p.wz, F32, STAGE, tile_w);
+__device__ __forceinline__ EnvRec load_rec(const void* rec, long long i) {
+    const float4* q = reinterpret_cast<const float4*>(rec) + i * 3;
+    const float4 a = q[0], b = q[1];
+    const int4 c = reinterpret_cast<const int4*>(q)[2];
+    EnvRec r;
+    r.ex = a.x; r.ey = a.y; r.ez = a.z;
+    r.env = __float_as_int(a.w);
+    r.sy = b.x; r.cy = b.y; r.sp = b.z; r.cp = b.w;
+    r.bits = c.x;
+    r.fill_blk = c.y;
+    return r;
+}
+__device__ __forceinline__ void store_rec(void* rec, long long i, const EnvRec& r) {
+    float4* q = reinterpret_cast<float4*>(rec) + i * 3;
+    q[0] = make_float4(r.ex, r.ey, r.ez, __int_as_float(r.env));
+    q[1] = make_float4(r.sy, r.cy, r.sp, r.cp);
+    reinterpret_cast<int4*>(q)[2] = make_int4(r.bits, r.fill_blk, 0, 0);
+}
 
-    // --- tables -------------------------------------------------------------
-    float4* s_cs = reinterpret_cast<float4*>(smem);                           // [13][4]
-    uint32_t* s_rgbp = reinterpret_cast<uint32_t*>(smem + kShadeTableBytes);  // [13]
-    build_fast_tables(s_cs, s_rgbp);
-    float* s_u = reinterpret_cast<float*>(smem + kFastTableBytes);
-    float* s_v = s_u + W;
-    float (*s_rgb)[3] = reinterpret_cast<float (*)[3]>(s_v + H);
-    float* s_sky = reinterpret_cast<float*>(s_rgb + 13);
-    uint8_t (*s_rgb8)[3] = reinterpret_cast<uint8_t (*)[3]>(s_sky + 4);
-    uint8_t* s_sky8 = reinterpret_cast<uint8_t*>(s_rgb8 + 13);
-    float pb_su = 0.0f, pb_sv = 0.0f;
-    if (FAM == MC_FAM_PREBASIS) prebasis_scales(W, H, p.fov, &pb_su, &pb_sv);
-    for (int k = threadIdx.x; k < W; k += blockDim.x) {
-        if (FAM == MC_FAM_SHADED || FAM == MC_FAM_SHADED_FAST) s_u[k] = u_shaded(k, W, H, p.fov);
-        else if (FAM == MC_FAM_MINIMAL || FAM == MC_FAM_FP16) s_u[k] = u_minimal(k, W, H, p.fov);
-        else s_u[k] = u_prebasis(k, W, pb_su);
-    }
-    for (int k = threadIdx.x; k < H; k += blockDim.x) {
-        if (FAM == MC_FAM_SHADED || FAM == MC_FAM_SHADED_FAST) s_v[k] = v_shaded(k, H, p.fov);
-        else if (FAM == MC_FAM_MINIMAL || FAM == MC_FAM_FP16) s_v[k] = v_minimal(k, H, p.fov);
-        else s_v[k] = v_prebasis(k, H, pb_sv);
-    }
-    for (int k = threadIdx.x; k < 39; k += blockDim.x) {
-        s_rgb[k / 3][k % 3] = c_rgb[k / 3][k % 3];
-        s_rgb8[k / 3][k % 3] = c_rgb8[k / 3][k % 3];
-    }
-    if (threadIdx.x < 3) {
-        s_sky[threadIdx.x] = c_sky[threadIdx.x];
-        s_sky8[threadIdx.x] = c_sky8[threadIdx.x];
-    }
-    uint8_t* wbase = smem + L.head_bytes + warp * L.warp_bytes;
-    uint64_t* mbar = reinterpret_cast<uint64_t*>(wbase);
-    int4* sstart = reinterpret_cast<int4*>(wbase + 16);
-    uint8_t* stage = wbase + 16 + 128;
-    int8_t* sworld = reinterpret_cast<int8_t*>(wbase + 16 + 128 + L.stage_bytes);
-    uint32_t mbar_a = smem_u32(mbar);
-    if (STAGE && lane == 0) {
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(mbar_a) : "memory");
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    __syncthreads();
-    uint32_t phase = 0;
-    bool no_stage = false;        // a copy timed out: this warp renders from global memory from now on
-    bool pending = false;         // ... and that copy may still be in flight
-    uint32_t pending_phase = 0;   // its phase, waited for before the warp leaves
-    // The kernel runs at its 64-register budget: values that would stay live
-    // across the env loop are recomputed where they are used (1 / vd, the
-    // env sizes) or not kept at all (the any-done flag goes straight to the
-    // flag word), and env indices are 32-bit (fewer spills, measured faster).
+// The camera of a record: the products of cam_trig / basis_compute.
+__device__ __forceinline__ Cam cam_of_rec(const EnvRec& r) {
+    Cam c;
+    c.eye_x = r.ex; c.eye_y = r.ey; c.eye_z = r.ez;
+    c.fx = N::mul(r.sy, r.cp);
+    c.fy = r.sp;
+    c.fz = N::mul(r.cy, r.cp);
+    c.rx = r.cy;
+    c.rz = -r.sy;
+    c.ux = N::mul(-r.sy, r.sp);
+    c.uy = r.cp;
+    c.uz = N::mul(-r.cy, r.sp);
+    c.sy = r.sy;
+    c.cy = r.cy;
+    c.cp = r.cp;
+    return c;
+}
 
-    const int obs_env_bytes = HW * 3 * (F32 ? 4 : 1);
-    const int total_warps = gridDim.x * nwarps;
-    const int first = p.sched_dynamic ? (int)next_env(p, 0, total_warps, lane) : blockIdx.x * nwarps + warp;
-    int e = first;
-    // staging depth 2 (prefetch): the warp claims its next env one ahead and,
-    // while it steps and renders this one, prefetches that env's world (and
-    // the state the step reads) into L2, so the next bulk copy reads L2
-    int ahead = (prefetch && e < p.B) ? (int)next_env(p, e, total_warps, lane) : p.B;
-    auto advance = [&]() -> int {
-        if (!prefetch) return (int)next_env(p, e, total_warps, lane);
-        const int r = ahead;
-        ahead = r < p.B ? (int)next_env(p, r, total_warps, lane) : r;
-        return r;
-    };
-    for (; e < p.B; e = advance()) {
-        if (prefetch && ahead < p.B) {
-            if (lane == 0)
-                asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p.voxels + ahead * (long long)wxyz),
-                             "r"(wxyz)
-                             : "memory");
-            const void* st = lane == 1 ? (const void*)(p.positions + ahead * 3)
-                           : lane == 2 ? (const void*)(p.velocities + ahead * 3)
-                           : lane == 3 ? (const void*)(p.yaws + ahead)
-                           : lane == 4 ? (const void*)(p.pitches + ahead)
-                           : lane == 5 ? (const void*)(p.on_ground + ahead)
-                           : lane == 6 && p.actions ? (const void*)(p.actions + ahead)
-                                                    : nullptr;
-            if (st) asm volatile("prefetch.global.L2 [%0];" ::"l"(st));
-        }
-        // ---- agent step (every lane computes the same values) --------------
-        int8_t btn[8];
-        float l0, l1;
-        load_action(p, e, btn, l0, l1);
-        Dec d = decode_buttons(btn, l0, l1, p.sprint_mult);
-        int32_t cnt = p.ext_done ? 0 : p.step_count[e];
-        bool done = p.ext_done ? (p.do_reset[e] != 0) : episode_done(p, cnt);
-        Agent a = load_agent(p, e);
-        physics(a, d, p);
-        int8_t* gw = p.voxels + e * (long long)wxyz;
-        float reward;
-        int8_t mod_val;
-        int mod_idx = interact_warp(gw, a, d.brk, d.place, p, lane, &reward, &mod_val);
-        if (done) reset_agent(a, p);
-        if (done && lane == 0) atomicOr(&p.flags[MC_FLAG_ANY_DONE], 1);  // rare: no per-warp accumulator
-        if (lane == 0) {
-            store_agent(p, e, a);
-            if (!p.ext_done) {
-                p.step_count[e] = done ? 1 : cnt + 1;
-                p.do_reset[e] = done ? 1 : 0;
-            }
-            p.rewards[e] = reward;
-            if (p.res_rewards) {
-                p.res_rewards[e] = reward;
-                p.res_dones[e] = done ? 1 : 0;
-            }
-            p.cameras[e * 5 + 0] = a.x;
-            p.cameras[e * 5 + 1] = a.y;
-            p.cameras[e * 5 + 2] = a.z;
-            p.cameras[e * 5 + 3] = a.yaw;
-            p.cameras[e * 5 + 4] = a.pitch;
-            if (p.dbg_interact) p.dbg_interact[e] = mod_idx;
-        }
-        // ---- per-env render constants -------------------------------------
-        Cam c;
-        float bas[13];
-        if (FAM == MC_FAM_PREBASIS) {
-            basis_compute(a.x, a.y, a.z, a.yaw, a.pitch, W, H, p.fov, bas);
-            c = cam_from_basis(bas);
-            if (p.basis && lane == 0) {
-#pragma unroll
-                for (int k = 0; k < 13; ++k) p.basis[e * 14 + k] = bas[k];
-            }
-        } else {
-            c = cam_trig(a.x, a.y, a.z, a.yaw, a.pitch);
-        }
-        // Every ray starts in the eye's voxel.  If the first DDA step already
-        // hits (the eye is inside a solid voxel, or below ground for the
-        // ground-shortcut family), every pixel of the env gets the same
-        // colour, so the env is filled without marching.
-        const int ex = (int)floorf(c.eye_x), ey = (int)floorf(c.eye_y), ez = (int)floorf(c.eye_z);
-        bool eye_inb = (unsigned)ex < (unsigned)p.wx && (unsigned)ey < (unsigned)p.wy && (unsigned)ez < (unsigned)p.wz;
-        int eye_idx = ey * wxz + ex * p.wz + ez;
-        int8_t eye_blk = AIR;
-        __syncwarp();
-        if (eye_inb && in_bounds(eye_idx, wxyz, MC_SITE_EYE)) eye_blk = gw[eye_idx];
-        bool inside = false;
-        bool buried;
-        int fill_blk = eye_blk;
-        if (FAM == MC_FAM_SHADED || FAM == MC_FAM_SHADED_FAST) {
-            inside = eye_inside(c, p.wx, p.wy, p.wz, p.vd);
-            bool start_hit = eye_blk >= 0;
-            if (FAM == MC_FAM_SHADED_FAST && ey < p.gh) {
-                start_hit = true;
-                fill_blk = (ey == p.gh - 1) ? GRASS : DIRT;
-            }
-            buried = inside && p.vd > 0.0f && p.max_steps > 0 && start_hit;
-        } else {
-            buried = p.max_steps > 0 && eye_inb && eye_blk >= 0;
-        }
-        // not buried: the first DDA step of every ray tests the eye voxel and
-        // advances; when that test is known to fail, rays start advanced
-        bool skip_first;
-        if (FAM == MC_FAM_SHADED || FAM == MC_FAM_SHADED_FAST)
-            skip_first = inside && p.vd > 0.0f && p.max_steps > 0 && eye_blk < 0 &&
-                         !(FAM == MC_FAM_SHADED_FAST && ey < p.gh);
-        else
-            skip_first = p.max_steps > 0 && !(eye_inb && eye_blk >= 0);
-        uint8_t* oenv = (uint8_t*)p.obs + (long long)e * obs_env_bytes;
-        const bool vec_ok = ((obs_env_bytes & 15) == 0) && ((((uintptr_t)oenv) & 15) == 0);
-        if (buried) {
-            Hit h;
-            h.blk = fill_blk;
-            h.face = -1;
-            h.t = 0.0f;
-            h.step_y = 1;
-            uint8_t bytes[12];
-            if (F32 || FAM == MC_FAM_SHADED || FAM == MC_FAM_SHADED_FAST) {
-                float rgb[3];
-                shade_rgb<F32 ? MC_COL_F32 : (FAM == MC_FAM_SHADED_FAST ? MC_COL_U8FAST : MC_COL_U8)>(
-                    h, p.vd, N::rcp_of(p.vd), s_rgb, s_sky, rgb);
-                if (F32) {
-                    // pattern period 12 bytes
-#pragma unroll
-                    for (int k = 0; k < 3; ++k) {
-                        uint32_t w32 = __float_as_uint(rgb[k]);
-                        bytes[4 * k + 0] = (uint8_t)(w32);
-                        bytes[4 * k + 1] = (uint8_t)(w32 >> 8);
-                        bytes[4 * k + 2] = (uint8_t)(w32 >> 16);
-                        bytes[4 * k + 3] = (uint8_t)(w32 >> 24);
-                    }
-                } else {
-                    bytes[0] = (uint8_t)to_u8(rgb[0]);
-                    bytes[1] = (uint8_t)to_u8(rgb[1]);
-                    bytes[2] = (uint8_t)to_u8(rgb[2]);
-                }
-            } else {
-                bytes[0] = s_rgb8[fill_blk][0];
-                bytes[1] = s_rgb8[fill_blk][1];
-                bytes[2] = s_rgb8[fill_blk][2];
-            }
-            const int period = F32 ? 12 : 3;
-            if (vec_ok) {
-                uint32_t w[12];
-#pragma unroll
-                for (int k = 0; k < 12; ++k) {
-                    w[k] = (uint32_t)bytes[(4 * k + 0) % period] | ((uint32_t)bytes[(4 * k + 1) % period] << 8) |
-                           ((uint32_t)bytes[(4 * k + 2) % period] << 16) | ((uint32_t)bytes[(4 * k + 3) % period] << 24);
-                }
-                fill_pattern16(oenv, (int)obs_env_bytes, make_uint4(w[0], w[1], w[2], w[3]),
-                               make_uint4(w[4], w[5], w[6], w[7]), make_uint4(w[8], w[9], w[10], w[11]), lane);
-            } else {
-                for (int k = lane; k < obs_env_bytes; k += 32) oenv[k] = bytes[k % period];
-            }
-            if (p.dbg_pixel) {
-                int16_t code = dbg_code(h);
-                for (int k = lane; k < HW; k += 32) p.dbg_pixel[(long long)e * HW + k] = code;
-            }
-            continue;
-        }
-        // ---- stage the world into shared memory ----------------------------
-        const int8_t* wsrc = gw;
-        int ytop = p.wy - 1;  // highest layer with a solid voxel (all layers unless measured)
-        UpBounds ub = up_none(ytop);
-        if (STAGE) {
-#if MC_CHECK_BOUNDS
-            {
-                const SmemRange dyn = dyn_smem_range();
-                const long long off = (long long)smem_u32(sworld) - dyn.lo;
-                if (!in_bounds(off, dyn.span, MC_SITE_STAGE) || !in_bounds(off + wxyz - 1, dyn.span, MC_SITE_STAGE)) {
-                    no_stage = true;  // no copy issued: render from global memory
-                    break;
-                }
-            }
-#endif
-            if (lane == 0) {
-                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(mbar_a), "r"(wxyz)
-                             : "memory");
-                asm volatile(
-                    "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                        smem_u32(sworld)),
-                    "l"(gw), "r"(wxyz), "r"(mbar_a)
-                    : "memory");
-            }
-            if (!mbar_wait(mbar_a, phase, p.wait_polls)) {
-                if (lane == 0) atomicExch(&p.flags[MC_FLAG_ERROR], MC_KERR_TMA_TIMEOUT);
-                no_stage = true;  // the copy may still land in this warp's buffer: never read it again
-                pending = true;
-                pending_phase = phase;
-                break;            // env e and the rest: fused_finish_from_global below
-            }
-            phase ^= 1u;
-            // the interaction may have written after the copy read the byte
-            if (lane == 0 && mod_idx >= 0 && in_bounds(mod_idx, wxyz, MC_SITE_PATCH)) sworld[mod_idx] = mod_val;
-            __syncwarp();
-            wsrc = sworld;
-            if (eye_inb && up_scan_shape(p.wx, p.wy, p.wz)) {
-                ub = staged_up_bounds(sworld, p.wx, p.wy, p.wz, ex, ey, ez, lane);
-                ytop = up_top(ub);  // the same cut for rays going up from the eye
-            } else {
-                ytop = staged_top_layer(sworld, p.wx, p.wy, p.wz, lane);
-                ub = up_none(ytop);
-            }
-        }
-        // ---- march every pixel ---------------------------------------------
-        const Dda0 d0 = dda0(c);
-        // per-env facts that let the march stop early (debug output needs the
-        // reference's face and distance of sky pixels too)
-        const bool sky_exit = (FAM == MC_FAM_SHADED) ? (inside && p.vd > 0.0f && !p.dbg_pixel)
-                                                     : (eye_inb && !p.dbg_pixel);
-        const bool vd_safe = sky_exit && box_within_view(c, p.wx, p.wy, p.wz, p.vd);
-        // where every ray takes the packed march, its start values per sign
-        // combination, built once for the env
-        const int4* start = nullptr;
-        const bool flat_fam = FAM == MC_FAM_MINIMAL || FAM == MC_FAM_PREBASIS;
-        if (STAGE && (FAM == MC_FAM_SHADED ? vd_safe : (flat_fam && sky_exit)) &&
-            p.max_steps > p.wx + p.wy + p.wz && p.wx <= 31 && p.wy <= 31 && p.wz <= 31 && wxyz < 8192) {
-            if (lane < 8) sstart[lane] = packed_start(lane, d0.vx, d0.vy, d0.vz, p.wx, p.wy, p.wz, ub);
-            __syncwarp();
-            start = sstart;
-        }
-        const int TW = L.tile_w, TH = L.tile_h;
-        if constexpr (STAGE && (FAM == MC_FAM_SHADED || FAM == MC_FAM_MINIMAL || FAM == MC_FAM_PREBASIS)) {
-            // the common case (fast_band): staged world, eye inside with air in
-            // its voxel, no debug output, whole tiles
-            const int fk = fast_kind<FAM>(true, sky_exit && skip_first, p.dbg_pixel != nullptr, vd_safe,
-                                          p.max_steps, p.wx, p.wy, p.wz, W, H, TW, 3 * (F32 ? 4 : 1), vec_ok);
-            if (fk) {
-                if (fk == 2 || !start) build_fast_start(sstart, fk, d0, p.wx, p.wy, p.wz, ub, p.max_steps, lane);
-                const uint32_t wb = smem_u32(sworld);
-                FastEnv fe;
-                fe.start = sstart;
-                fe.base = fk == 1 ? wb : wb + (uint32_t)(d0.vy * wxz + d0.vx * p.wz + d0.vz);
-                fe.chk = staged_range(wb, wxz, wxyz);
-                fe.vd = p.vd;
-                fe.rcp_vd = N::rcp_of(p.vd);
-                for (int row0 = 0; row0 < H; row0 += TH) {
-                    uint8_t* dst = oenv + (long long)row0 * W * (3 * (F32 ? 4 : 1));
-                    if (fk == 1)
-                        fast_band<FAM, F32, false>(c, d0, fe, W, TW, row0, lane, s_u, s_v, s_cs, s_rgbp, stage, dst);
-                    else
-                        fast_band<FAM, F32, true>(c, d0, fe, W, TW, row0, lane, s_u, s_v, s_cs, s_rgbp, stage, dst);
-                }
-                continue;
-            }
-        }
-        const int lx = lane % TW, ly = lane / TW;
-        const int bpp = 3 * (F32 ? 4 : 1);  // bytes per pixel
-        for (int row0 = 0; row0 < H; row0 += TH) {
-            const int py = row0 + ly;
-            const float v = (py < H && in_bounds(py, H, MC_SITE_TABLE)) ? s_v[py] : 0.0f;
-            for (int tx0 = 0; tx0 < W; tx0 += TW) {
-                const int px = tx0 + lx;
-                if (px < W && py < H && in_bounds(px, W, MC_SITE_TABLE)) {
-                    Hit h;
-                    const float u = s_u[px];
-                    if (FAM == MC_FAM_SHADED || FAM == MC_FAM_SHADED_FAST) {
-                        // the one-warp-per-env kernel keeps its 64-register budget: the
-                        // branch-free march only where the whole box is within view
-                        if (STAGE) h = shade_ray<FAM == MC_FAM_SHADED_FAST, VoxShared, false, true>(c, d0, u, v, VoxShared{wsrc}, p.wx, p.wy, p.wz, p.max_steps, p.vd, p.gh, inside, skip_first, sky_exit, vd_safe, ytop, start);
-                        else h = shade_ray<FAM == MC_FAM_SHADED_FAST, VoxGlobal, false>(c, d0, u, v, VoxGlobal{wsrc}, p.wx, p.wy, p.wz, p.max_steps, p.vd, p.gh, inside, skip_first, sky_exit, vd_safe);
-                    } else if (FAM == MC_FAM_FP16) {
-                        if (STAGE) h = fp16_ray(c, d0, u, v, VoxShared{wsrc}, p.wx, p.wy, p.wz, p.max_steps);
-                        else h = fp16_ray(c, d0, u, v, VoxGlobal{wsrc}, p.wx, p.wy, p.wz, p.max_steps);
-                    } else {
-                        constexpr bool TRIG = (FAM != MC_FAM_PREBASIS);
-                        if (STAGE) h = flat_ray<TRIG, VoxShared, true>(c, d0, u, v, VoxShared{wsrc}, p.wx, p.wy, p.wz, p.max_steps, skip_first, sky_exit, ytop, start);
-                        else h = flat_ray<TRIG>(c, d0, u, v, VoxGlobal{wsrc}, p.wx, p.wy, p.wz, p.max_steps, skip_first, sky_exit);
-                    }
-                    const int so = ly * W + px;  // pixel within the staged band
-                    if (!in_bounds((long long)(so + 1) * bpp - 1, L.stage_bytes, MC_SITE_BAND)) continue;
-                    if (FAM == MC_FAM_SHADED || FAM == MC_FAM_SHADED_FAST) {
-                        float rgb[3];
-                        shade_rgb<F32 ? MC_COL_F32 : (FAM == MC_FAM_SHADED_FAST ? MC_COL_U8FAST : MC_COL_U8)>(
-                            h, p.vd, N::rcp_of(p.vd), s_rgb, s_sky, rgb);
-                        if (F32) {
-                            float* sf = reinterpret_cast<float*>(stage) + so * 3;
-                            sf[0] = rgb[0]; sf[1] = rgb[1]; sf[2] = rgb[2];
-                        } else {
-                            uint8_t* sb = stage + so * 3;
-                            sb[0] = (uint8_t)to_u8(rgb[0]);
-                            sb[1] = (uint8_t)to_u8(rgb[1]);
-                            sb[2] = (uint8_t)to_u8(rgb[2]);
-                        }
-                    } else {
-                        const uint8_t* col = (h.blk >= 0 && in_bounds(h.blk, 13, MC_SITE_TABLE)) ? s_rgb8[h.blk] : s_sky8;
-                        uint8_t* sb = stage + so * 3;
-                        sb[0] = col[0]; sb[1] = col[1]; sb[2] = col[2];
-                    }
-                    if (p.dbg_pixel && in_bounds(py * W + px, HW, MC_SITE_DEBUG))
-                        p.dbg_pixel[(long long)e * HW + py * W + px] = dbg_code(h);
-                }
-            }
-            __syncwarp();
-            // copy the band (rows row0 .. row0+TH-1) out
-            const int nbytes = min(TH, H - row0) * W * bpp;
-            uint8_t* dst = oenv + (long long)row0 * W * bpp;
-            if (!in_bounds((long long)row0 * W * bpp + nbytes - 1, obs_env_bytes, MC_SITE_COPY_OUT) ||
-                !in_bounds(nbytes - 1, L.stage_bytes, MC_SITE_BAND)) {
-                __syncwarp();
-                continue;
-            }
-            if (vec_ok && (nbytes & 15) == 0 && (((long long)row0 * W * bpp) & 15) == 0) {
-                const uint4* s4 = reinterpret_cast<const uint4*>(stage);
-                uint4* d4 = reinterpret_cast<uint4*>(dst);
-                for (int k = lane; k < (nbytes >> 4); k += 32) d4[k] = s4[k];
-            } else {
-                for (int k = lane; k < nbytes; k += 32) dst[k] = stage[k];
-            }
-            __syncwarp();
-        }
-    }
-    if (STAGE && no_stage) {
-        FusedCtx cx;
-        cx.s_u = s_u;
-        cx.s_v = s_v;
-        cx.s_rgb = s_rgb;
-        cx.s_sky = s_sky;
-        cx.s_rgb8 = s_rgb8;
-        cx.s_sky8 = s_sky8;
-        cx.stage = stage;
-        cx.rcp_vd = N::rcp_of(p.vd);
-        if (fused_finish_from_global<FAM, F32>(p, e, prefetch ? ahead : -1, total_warps, tile_w, lane, cx) && lane == 0)
-            atomicOr(&p.flags[MC_FLAG_ANY_DONE], 1);
-        // the timed-out copy may still be in flight: let it land (bounded, with
-        // the default budget) before this warp's part of shared memory can be released
-        if (pending) mbar_wait(mbar_a, pending_phase);
-    }
-    // No CTA barrier here: warps leave as soon as their last env is done.
-    if (lane == 0) {
-        bounds_to_flags(p.flags);
-        if (p.sched_dynamic) {
-            // every claim of this warp has returned (the last one >= B); the
-            // last warp to get here resets the counters for the next launch
-            __threadfence();
-            unsigned prev = atomicAdd(reinterpret_cast<unsigned*>(&p.flags[MC_FLAG_WARPS_DONE]), 1u);
-            if (prev == (unsigned)(total_warps - 1)) {
-                p.flags[MC_FLAG_WORK] = 0;
-                p.flags[MC_FLAG_WARPS_DONE] = 0;
-                __threadfence();
-            }
-        }
+// The eye's voxel: its index in the world, -1 outside the box.
+__device__ __forceinline__ int eye_index(const EnvRec& r, const mc_kp& p) {
+    const int ex = (int)floorf(r.ex), ey = (int)floorf(r.ey), ez = (int)floorf(r.ez);
+    const bool inb = (unsigned)ex < (unsigned)p.wx && (unsigned)ey < (unsigned)p.wy && (unsigned)ez < (unsigned)p.wz;
+    return inb ? ey * (p.wx * p.wz) + ex * p.wz + ez : -1;
+}
+
+// sin and cos of the camera's angles, as the family's render computes them.
+template <int FAM>
+__device__ __forceinline__ void rec_trig(EnvRec& r, float yaw, float pitch) {
+    if (FAM == MC_FAM_PREBASIS) {
+        N::sincos_i(yaw, &r.sy, &r.cy);
+        N::sincos_i(pitch, &r.sp, &r.cp);
+    } else {
+        r.cy = N::cos(yaw);
+        r.sy = N::sin(yaw);
+        r.cp = N::cos(pitch);
+        r.sp = N::sin(pitch);
     }
 }
 
+// The facts of a record whose eye is set; eye_blk: the block there (AIR outside
+// the box).  Every ray starts in the eye's voxel: if the first DDA step
+// already hits (the eye is inside a solid voxel, or below ground for the
+// ground-shortcut family), every pixel of the env gets the same colour
+// (MC_ER_BURIED); if that test is known to fail, rays start advanced by one
+// step (MC_ER_SKIP).
+template <int FAM>
+__device__ __forceinline__ void rec_facts(EnvRec& r, const mc_kp& p, bool eye_inb, int eye_blk, bool done) {
+    bool inside = false, buried, skip_first;
+    r.fill_blk = eye_blk;
+    if (FAM == MC_FAM_SHADED || FAM == MC_FAM_SHADED_FAST) {
+        Cam c;
+        c.eye_x = r.ex; c.eye_y = r.ey; c.eye_z = r.ez;
+        inside = eye_inside(c, p.wx, p.wy, p.wz, p.vd);
+        const int ey = (int)floorf(r.ey);
+        const bool below = FAM == MC_FAM_SHADED_FAST && ey < p.gh;
+        if (below) r.fill_blk = (ey == p.gh - 1) ? GRASS : DIRT;
+        const bool can = inside && p.vd > 0.0f && p.max_steps > 0;
+        buried = can && (eye_blk >= 0 || below);
+        skip_first = can && eye_blk < 0 && !below;
+    } else {
+        buried = p.max_steps > 0 && eye_inb && eye_blk >= 0;
+        skip_first = p.max_steps > 0 && !(eye_inb && eye_blk >= 0);
+    }
+    // the common case: the launch allows it, and the eye is inside the box with air in its voxel
+    const bool fast = p.fast_ok && skip_first && (FAM == MC_FAM_SHADED || eye_inb);
+    r.bits = (done ? MC_ER_DONE : 0) | (buried ? MC_ER_BURIED : 0) | (inside ? MC_ER_INSIDE : 0) |
+             (skip_first ? MC_ER_SKIP : 0) | (!buried && !fast ? MC_ER_SLOW : 0);
+}
+
+// Decode, episode rule, physics, interaction, reset, counters, camera (and
+// basis) of env e, by one thread.  Its loads come in two waves: the action and
+// state, then the eye's voxel and the interaction's samples.
+template <int FAM>
+__device__ __forceinline__ EnvRec agent_step(const mc_kp& p, const ActionSrc& act, long long e, float* res_rewards,
+                                             uint8_t* res_dones) {
+    const long long wxyz = (long long)p.wx * p.wy * p.wz;
+    int8_t btn[8];
+    float l0, l1;
+    load_action_from(act, p.look_delta, e, btn, l0, l1);
+    const Dec d = decode_buttons(btn, l0, l1, p.sprint_mult);
+    const int32_t cnt = p.ext_done ? 0 : p.step_count[e];
+    const bool done = p.ext_done ? (p.do_reset[e] != 0) : episode_done(p, cnt);
+    Agent a = load_agent(p, e);
+    float sy, cy;
+    physics(a, d, p, sy, cy);
+    int8_t* w = p.voxels + e * wxyz;
+    Look l;
+    l.ex = a.x;
+    l.ey = N::add(a.y, 1.6f);
+    l.ez = a.z;
+    const float cp = N::cos(a.pitch), sp = N::sin(a.pitch);
+    l.dx = N::mul(sy, cp);
+    l.dy = sp;
+    l.dz = N::mul(cy, cp);
+    if (done) reset_agent(a, p);
+    EnvRec r;
+    r.env = (int)e;
+    r.ex = a.x;
+    r.ey = N::add(a.y, 1.6f);
+    r.ez = a.z;
+    r.sy = sy; r.cy = cy; r.sp = sp; r.cp = cp;
+    if (FAM == MC_FAM_PREBASIS || done) rec_trig<FAM>(r, a.yaw, a.pitch);
+    const int eye = eye_index(r, p);
+    int eye_blk = AIR;
+    if (eye >= 0 && in_bounds(eye, wxyz, MC_SITE_EYE)) eye_blk = w[eye];
+    float reward = 0.0f;
+    int mod_idx = -1, mod_val = 0;
+    if (d.brk || d.place) {
+        look_samples(l, w, p);
+        mod_idx = interact_judge(l, w, d.brk, p, &reward, &mod_val);
+        if (mod_idx >= 0 && mod_idx == eye) eye_blk = mod_val;
+    }
+    rec_facts<FAM>(r, p, eye >= 0, eye_blk, done);
+    store_agent(p, e, a);
+    if (!p.ext_done) {
+        p.step_count[e] = done ? 1 : cnt + 1;
+        p.do_reset[e] = done ? 1 : 0;
+    }
+    p.rewards[e] = reward;
+    if (res_rewards) res_rewards[e] = reward;
+    if (res_dones) res_dones[e] = done ? 1 : 0;
+    p.cameras[e * 5 + 0] = a.x;
+    p.cameras[e * 5 + 1] = a.y;
+    p.cameras[e * 5 + 2] = a.z;
+    p.cameras[e * 5 + 3] = a.yaw;
+    p.cameras[e * 5 + 4] = a.pitch;
+    if (p.dbg_interact) p.dbg_interact[e] = mod_idx;
+    if (FAM == MC_FAM_PREBASIS && p.basis) {
+        float bas[13];
+        basis_compute(a.x, a.y, a.z, a.yaw, a.pitch, p.W, p.H, p.fov, bas);
+#pragma unroll
+        for (int k = 0; k < 13; ++k) p.basis[e * 14 + k] = bas[k];
+    }
+    return r;
+}
+
+constexpr int kAgentThreads = MC_AGENT_THREADS;
+
+// File the block's records (called by all its threads): record e at e, or,
+// with more envs than the image kernel has warps (`compact`), the records of the envs on the common path fill the group's record
+// array from the front and those of the others (buried, or left to the
+// general pass) from the back, so the image kernel's warps claim the costly
+// envs first and the cheap uniform fills even out the end of the launch.  One 64-bit counter holds both fill counts;
+// the block that brings their sum to the group's size clears it for the next
+// launch (every env is filed exactly once, so no other block adds after it).
+__device__ __forceinline__ void file_recs(void* rec, int32_t* flags, int32_t* any_slow, long long B, bool compact,
+                                          const EnvRec& r, long long e, bool valid) {
+    __shared__ unsigned s_m[kAgentThreads / 32], s_b[kAgentThreads / 32];
+    __shared__ unsigned long long s_base;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const bool march = valid && !(r.bits & (MC_ER_BURIED | MC_ER_SLOW)), fill = valid && !march;
+    if (valid && (r.bits & MC_ER_SLOW)) *any_slow = 1;
+    const unsigned done = __ballot_sync(0xffffffffu, valid && (r.bits & MC_ER_DONE));
+    if (done && lane == 0) atomicOr(&flags[MC_FLAG_ANY_DONE], 1);
+    if (!compact) {
+        if (valid) store_rec(rec, e, r);
+        return;
+    }
+    const unsigned mm = __ballot_sync(0xffffffffu, march), mb = __ballot_sync(0xffffffffu, fill);
+    if (lane == 0) {
+        s_m[warp] = __popc(mm);
+        s_b[warp] = __popc(mb);
+    }
+    __syncthreads();
+    unsigned pm = 0, pb = 0, tm = 0, tb = 0;
+#pragma unroll
+    for (int w = 0; w < kAgentThreads / 32; ++w) {
+        if (w == warp) { pm = tm; pb = tb; }
+        tm += s_m[w];
+        tb += s_b[w];
+    }
+    if (threadIdx.x == 0) {
+        unsigned long long* ctr = reinterpret_cast<unsigned long long*>(&flags[MC_FLAG_FILED]);
+        const unsigned long long old = atomicAdd(ctr, ((unsigned long long)tb << 32) | tm);
+        s_base = old;
+        if ((long long)((old & 0xffffffffu) + tm) + (long long)((old >> 32) + tb) == B) *ctr = 0ull;
+    }
+    __syncthreads();
+    const unsigned below = (1u << lane) - 1u;
+    if (march) store_rec(rec, (long long)(unsigned)s_base + pm + __popc(mm & below), r);
+    if (fill) store_rec(rec, B - 1 - ((long long)(s_base >> 32) + pb + __popc(mb & below)), r);
+}
+
+// Programmatic dependent launch: a kernel of the step may be scheduled while
+// its predecessor in the stream still runs; it waits here before it touches
+// anything the predecessor writes.  pdl_trigger lets the successor be scheduled.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+// What bounds it: the latency of its dependent loads (action and state,
+// interaction samples, eye voxel), overlapped over 32 envs per warp, where
+// a warp per env repeated every instruction 32 times.
+template <int FAM>
+__global__ void __launch_bounds__(kAgentThreads) k_agent(const __grid_constant__ mc_kp p) {
+    pdl_trigger();
+    pdl_wait();
+    const long long e = (long long)blockIdx.x * kAgentThreads + threadIdx.x;
+    const bool valid = e < p.B;
+    EnvRec r{};
+    if (valid) r = agent_step<FAM>(p, ActionSrc{p.actions, p.buttons, p.look}, e, p.res_rewards, p.res_dones);
+    file_recs(p.rec, p.flags, &p.flags[MC_FLAG_ANY_SLOW], p.B, p.compact, r, e, valid);
+    if (threadIdx.x == 0) bounds_to_flags(p.flags);
+}
+
+// The same for the groups of a ragged launch: blocks ablock[g] .. ablock[g+1]-1 hold group g's envs.
+template <int FAM>
+__global__ void __launch_bounds__(kAgentThreads) k_agent_groups(const __grid_constant__ mc_ragged_kp rk) {
+    pdl_trigger();
+    pdl_wait();
+    int g = 0;
+    while (g + 1 < rk.ngroups && (int)blockIdx.x >= rk.ablock[g + 1]) ++g;
+    const mc_kp& p = rk.groups[g];
+    const long long e = (long long)((int)blockIdx.x - rk.ablock[g]) * kAgentThreads + threadIdx.x, s0 = rk.start[g];
+    const bool valid = e < p.B;
+    EnvRec r{};
+    if (valid) {
+        const ActionSrc act{rk.actions ? rk.actions + s0 : nullptr, rk.actions ? nullptr : rk.buttons + 8 * s0,
+                            rk.actions ? nullptr : rk.look + 2 * s0};
+        r = agent_step<FAM>(p, act, e, rk.rewards_cat ? rk.rewards_cat + s0 : nullptr,
+                            rk.dones_cat ? rk.dones_cat + s0 : nullptr);
+    }
+    file_recs(reinterpret_cast<EnvRec*>(rk.rec) + s0, p.flags, &rk.flags[MC_FLAG_ANY_SLOW], p.B, p.compact, r, e, valid);
+    if (threadIdx.x == 0) bounds_to_flags(p.flags);
+}
 
 // ---------------------------------------------------------------------------
-// Team kernel: env groups of any size, stepped by teams of warps
+// The images
 // ---------------------------------------------------------------------------
-// A CTA of warps_per_cta warps is split into teams of team_warps warps.  A
-// team claims one work unit at a time from a device counter:
-//  * a cooperative group's unit is ONE env: the team's first warp steps the
-//    agent, then all warps of the team march row bands of its image (bands
-//    claimed from a shared counter), reading the world from one shared-memory
-//    copy per team when staged.  Big images over big worlds then keep an
-//    SM's L1 and shared memory on few worlds, like a per-pixel kernel;
-//  * a per-warp group's unit is team_warps envs, one per warp, each stepped
-//    and rendered by its warp alone.
-// Units are ordered by decreasing per-env cost across groups, so the most
-// expensive envs are claimed first and do not straggle at the end.
-
-// What the render of one env needs from its agent step.
+// What the render of one env needs.
 struct EnvRender {
     Cam c;
     int bits;      // MC_ER_*
     int fill_blk;  // block of the uniform fill of a buried camera
-    int mod_idx;   // voxel index the interaction wrote, -1 if none
-    int mod_val;
     int ytop;      // no solid voxel above this layer (wy - 1 unless measured)
     UpBounds ub;   // bounds of the rays going up (up_none(ytop) unless measured)
 };
+
+__device__ __forceinline__ EnvRender render_of_rec(const EnvRec& q, int wy) {
+    EnvRender r;
+    r.c = cam_of_rec(q);
+    r.bits = q.bits;
+    r.fill_blk = q.fill_blk;
+    r.ytop = wy - 1;
+    r.ub = up_none(r.ytop);
+    return r;
+}
 
 // Whether the eye's voxel lies in the box.
 __device__ __forceinline__ bool eye_in_box(const Cam& c, int wx, int wy, int wz) {
@@ -2625,6 +2403,7 @@ __device__ __forceinline__ void measure_staged(EnvRender& r, const int8_t* world
 }
 
 
+
 // Barrier of one team (named barrier `bar`, nthreads threads).
 __device__ __forceinline__ void team_sync(int bar, int nthreads) {
     if (nthreads == 32)
@@ -2633,150 +2412,32 @@ __device__ __forceinline__ void team_sync(int bar, int nthreads) {
         asm volatile("bar.sync %0, %1;" ::"r"(bar), "r"(nthreads) : "memory");
 }
 
-struct TeamShared {
-    unsigned unit[2];  // claimed units, alternating slots
-    int band_ctr;      // next row band of the cooperative env
-    int pad;
-    EnvRender r;       // the cooperative env
-    // the cooperative env's up bounds, combined over the team's warps (UpPart)
-    int uxa[4], uya[4];
-    unsigned long long ump, umm;
-};
-static_assert(sizeof(TeamShared) <= MC_TEAM_HEAD_BYTES, "team head");
 
-// Reset the team's up-bound words (the stepping warp's lane 0, before the
-// barrier that publishes the env).
-__device__ __forceinline__ void team_up_reset(TeamShared* ts) {
-    ts->uxa[0] = 255; ts->uxa[1] = 0; ts->uxa[2] = 255; ts->uxa[3] = 0;
-    ts->uya[0] = ts->uya[1] = ts->uya[2] = ts->uya[3] = 0;
-    ts->ump = ts->umm = 0ull;
-}
-
-// The up bounds of a cooperative env, scanned by all nw warps of its team
-// (warp w sweeps its share of the layers, staged_up_part) and combined in
-// the team's shared words with shared-memory atomics, so every warp holds
-// the same bounds after the team barrier.  Called by every warp of the team.
-template <typename M>
-__device__ __forceinline__ UpBounds team_up_bounds_t(const int8_t* world, int wx, int wy, int wz, int vx, int vy,
-                                                     int vz, int lane, int w, int nw, TeamShared* ts, int bar) {
-    const UpPart<M> r = staged_up_part<M>(world, wx, wy, wz, vx, vy, vz, lane, w, nw);
+// Start the bulk copy of one world into shared memory (lane 0 issues it).
+__device__ __forceinline__ void issue_world_copy(uint32_t mbar_a, int8_t* dst, const int8_t* src, int bytes, int lane) {
     if (lane == 0) {
-        atomicMin(&ts->uxa[0], r.xa0);
-        atomicMax(&ts->uxa[1], r.xa1);
-        atomicMin(&ts->uxa[2], r.xa2);
-        atomicMax(&ts->uxa[3], r.xa3);
-        atomicMax(&ts->uya[0], r.ya0);
-        atomicMax(&ts->uya[1], r.ya1);
-        atomicMax(&ts->uya[2], r.ya2);
-        atomicMax(&ts->uya[3], r.ya3);
-        atomicOr(&ts->ump, (unsigned long long)r.mp);
-        atomicOr(&ts->umm, (unsigned long long)r.mm);
+        // generic-proxy reads of the previous world must precede the copy
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(mbar_a), "r"(bytes) : "memory");
+        asm volatile(
+            "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                smem_u32(dst)),
+            "l"(src), "r"(bytes), "r"(mbar_a)
+            : "memory");
     }
-    team_sync(bar, nw * 32);
-    UpPart<M> t;
-    t.xa0 = ts->uxa[0];
-    t.xa1 = ts->uxa[1];
-    t.xa2 = ts->uxa[2];
-    t.xa3 = ts->uxa[3];
-    t.ya0 = ts->uya[0];
-    t.ya1 = ts->uya[1];
-    t.ya2 = ts->uya[2];
-    t.ya3 = ts->uya[3];
-    t.mp = (M)ts->ump;
-    t.mm = (M)ts->umm;
-    return up_bounds_of(t);
-}
-__device__ __forceinline__ UpBounds team_up_bounds(const int8_t* world, int wx, int wy, int wz, int vx, int vy, int vz,
-                                                   int lane, int w, int nw, TeamShared* ts, int bar) {
-    return wz > 32 ? team_up_bounds_t<unsigned long long>(world, wx, wy, wz, vx, vy, vz, lane, w, nw, ts, bar)
-                   : team_up_bounds_t<uint32_t>(world, wx, wy, wz, vx, vy, vz, lane, w, nw, ts, bar);
 }
 
-// Decode, episode rule, physics, interaction, reset, counters and camera of
-// env e, run by one whole warp: every lane computes the same values, lane 0
-// writes the state.
-template <int FAM>
-__device__ __forceinline__ EnvRender agent_step(const mc_kp& p, const ActionSrc& act, long long e, int lane) {
-    const int wxz = p.wx * p.wz;
-    const int wxyz = wxz * p.wy;
-    int8_t btn[8];
-    float l0, l1;
-    load_action_from(act, p.look_delta, e, btn, l0, l1);
-    Dec d = decode_buttons(btn, l0, l1, p.sprint_mult);
-    int32_t cnt = p.ext_done ? 0 : p.step_count[e];
-    bool done = p.ext_done ? (p.do_reset[e] != 0) : episode_done(p, cnt);
-    Agent a = load_agent(p, e);
-    physics(a, d, p);
-    int8_t* gw = p.voxels + e * (long long)wxyz;
-    float reward;
-    int8_t mod_val;
-    int mod_idx = interact_warp(gw, a, d.brk, d.place, p, lane, &reward, &mod_val);
-    if (done) reset_agent(a, p);
-    if (lane == 0) {
-        store_agent(p, e, a);
-        if (!p.ext_done) {
-            p.step_count[e] = done ? 1 : cnt + 1;
-            p.do_reset[e] = done ? 1 : 0;
-        }
-        p.rewards[e] = reward;
-        if (p.res_rewards) {
-            p.res_rewards[e] = reward;
-            p.res_dones[e] = done ? 1 : 0;
-        }
-        p.cameras[e * 5 + 0] = a.x;
-        p.cameras[e * 5 + 1] = a.y;
-        p.cameras[e * 5 + 2] = a.z;
-        p.cameras[e * 5 + 3] = a.yaw;
-        p.cameras[e * 5 + 4] = a.pitch;
-        if (p.dbg_interact) p.dbg_interact[e] = mod_idx;
-    }
-    EnvRender r;
-    if (FAM == MC_FAM_PREBASIS) {
-        float bas[13];
-        basis_compute(a.x, a.y, a.z, a.yaw, a.pitch, p.W, p.H, p.fov, bas);
-        r.c = cam_from_basis(bas);
-        if (p.basis && lane == 0) {
-#pragma unroll
-            for (int k = 0; k < 13; ++k) p.basis[e * 14 + k] = bas[k];
-        }
-    } else {
-        r.c = cam_trig(a.x, a.y, a.z, a.yaw, a.pitch);
-    }
-    // Every ray starts in the eye's voxel.  If the first DDA step already
-    // hits (the eye is inside a solid voxel, or below ground for the
-    // ground-shortcut family), every pixel of the env gets the same colour.
-    const Cam& c = r.c;
-    const int ex = (int)floorf(c.eye_x), ey = (int)floorf(c.eye_y), ez = (int)floorf(c.eye_z);
-    bool eye_inb = (unsigned)ex < (unsigned)p.wx && (unsigned)ey < (unsigned)p.wy && (unsigned)ez < (unsigned)p.wz;
-    int8_t eye_blk = AIR;
-    __syncwarp();
-    if (eye_inb && in_bounds(ey * wxz + ex * p.wz + ez, wxyz, MC_SITE_EYE)) eye_blk = gw[ey * wxz + ex * p.wz + ez];
-    bool inside = false, buried, skip_first;
-    int fill_blk = eye_blk;
-    if (FAM == MC_FAM_SHADED || FAM == MC_FAM_SHADED_FAST) {
-        inside = eye_inside(c, p.wx, p.wy, p.wz, p.vd);
-        bool start_hit = eye_blk >= 0;
-        if (FAM == MC_FAM_SHADED_FAST && ey < p.gh) {
-            start_hit = true;
-            fill_blk = (ey == p.gh - 1) ? GRASS : DIRT;
-        }
-        buried = inside && p.vd > 0.0f && p.max_steps > 0 && start_hit;
-        // not buried: the first DDA step of every ray tests the eye voxel
-        // and advances; when that test is known to fail, rays start advanced
-        skip_first = inside && p.vd > 0.0f && p.max_steps > 0 && eye_blk < 0 &&
-                     !(FAM == MC_FAM_SHADED_FAST && ey < p.gh);
-    } else {
-        buried = p.max_steps > 0 && eye_inb && eye_blk >= 0;
-        skip_first = p.max_steps > 0 && !(eye_inb && eye_blk >= 0);
-    }
-    r.bits = (done ? MC_ER_DONE : 0) | (buried ? MC_ER_BURIED : 0) | (inside ? MC_ER_INSIDE : 0) |
-             (skip_first ? MC_ER_SKIP : 0);
-    r.fill_blk = fill_blk;
-    r.mod_idx = mod_idx;
-    r.mod_val = mod_val;
-    r.ytop = p.wy - 1;
-    r.ub = up_none(r.ytop);
-    return r;
+// Debug build: whether a staged world of `bytes` at dst lies in the CTA's
+// dynamic shared memory (the same answer for every warp of a team).
+__device__ __forceinline__ bool stage_fits(const int8_t* dst, int bytes) {
+#if MC_CHECK_BOUNDS
+    const SmemRange dyn = dyn_smem_range();
+    const long long off = (long long)smem_u32(dst) - dyn.lo;
+    return in_bounds(off, dyn.span, MC_SITE_STAGE) && in_bounds(off + bytes - 1, dyn.span, MC_SITE_STAGE);
+#else
+    (void)dst; (void)bytes;
+    return true;
+#endif
 }
 
 // Repeating 48-byte pattern written with 16-byte stores by nt threads.
@@ -2794,14 +2455,13 @@ __device__ __forceinline__ void fill_pattern16_n(uint8_t* dst, int bytes, uint4 
 
 // The uniform observation of a buried camera, written by nt threads.
 template <int FAM, bool F32>
-__device__ __forceinline__ void fill_env(const mc_kp& p, long long e, const EnvRender& r, const FusedCtx& cx, int t,
-                                         int nt) {
+__device__ __forceinline__ void fill_env(const mc_kp& p, int e, int fill_blk, const FusedCtx& cx, int t, int nt) {
     const int HW = p.W * p.H;
     const long long obs_env_bytes = (long long)HW * 3 * (F32 ? 4 : 1);
     uint8_t* oenv = (uint8_t*)p.obs + e * obs_env_bytes;
     const bool vec_ok = ((obs_env_bytes & 15) == 0) && ((((uintptr_t)oenv) & 15) == 0);
     Hit h;
-    h.blk = r.fill_blk;
+    h.blk = fill_blk;
     h.face = -1;
     h.t = 0.0f;
     h.step_y = 1;
@@ -2825,9 +2485,9 @@ __device__ __forceinline__ void fill_env(const mc_kp& p, long long e, const EnvR
             bytes[2] = (uint8_t)to_u8(rgb[2]);
         }
     } else {
-        bytes[0] = cx.s_rgb8[r.fill_blk][0];
-        bytes[1] = cx.s_rgb8[r.fill_blk][1];
-        bytes[2] = cx.s_rgb8[r.fill_blk][2];
+        bytes[0] = cx.s_rgb8[fill_blk][0];
+        bytes[1] = cx.s_rgb8[fill_blk][1];
+        bytes[2] = cx.s_rgb8[fill_blk][2];
     }
     const int period = F32 ? 12 : 3;
     if (vec_ok) {
@@ -2848,13 +2508,34 @@ __device__ __forceinline__ void fill_env(const mc_kp& p, long long e, const EnvR
     }
 }
 
-// March row bands of env e's image with one warp: every band when band_ctr is
-// null, else the bands this warp claims from the team's shared counter.
-template <int FAM, bool F32, class V, bool VDLIM = true>
-__device__ __forceinline__ void render_env(const mc_kp& p, long long e, const EnvRender& r, const FusedCtx& cx,
-                                           const V& vox, int tile_w, int lane, int* band_ctr) {
-    // parameters in registers: p may live in shared memory, which the band
-    // stores below would otherwise force to be re-read per pixel
+// Per-env facts that let the march stop early (see shade_ray / flat_ray).
+struct MarchFacts {
+    bool sky_exit, vd_safe;
+};
+template <int FAM>
+__device__ __forceinline__ MarchFacts march_facts(const mc_kp& p, const EnvRender& r) {
+    MarchFacts m;
+    m.sky_exit = (FAM == MC_FAM_SHADED) ? ((r.bits & MC_ER_INSIDE) != 0 && p.vd > 0.0f && !p.dbg_pixel)
+                                        : (eye_in_box(r.c, p.wx, p.wy, p.wz) && !p.dbg_pixel);
+    m.vd_safe = m.sky_exit && box_within_view(r.c, p.wx, p.wy, p.wz, p.vd);
+    return m;
+}
+
+// The next row band of this warp: the bands in turn when band_ctr is null,
+// else those it claims from the team's shared counter.
+__device__ __forceinline__ int next_band(int* band_ctr, int prev, int lane) {
+    if (!band_ctr) return prev + 1;
+    int v = 0;
+    if (lane == 0) v = atomicAdd(band_ctr, 1);
+    return __shfl_sync(0xffffffffu, v, 0);
+}
+
+// The general path, a pixel's ray at a time as in the reference's kernels:
+// worlds that are not staged, debug outputs, eyes outside the box or out of
+// view, families without a fast march, images that are no whole tiles.
+template <int FAM, bool F32, class V>
+__device__ __forceinline__ void render_slow_from(const mc_kp& p, int e, const EnvRender& r, const FusedCtx& cx,
+                                                 const V& vox, int tile_w, int lane, int* band_ctr) {
     const int W = p.W, H = p.H;
     const RayPar rp = ray_par(p);
     int16_t* const dbg_pixel = p.dbg_pixel;
@@ -2863,52 +2544,13 @@ __device__ __forceinline__ void render_env(const mc_kp& p, long long e, const En
     uint8_t* oenv = (uint8_t*)p.obs + e * obs_env_bytes;
     const bool vec_ok = ((obs_env_bytes & 15) == 0) && ((((uintptr_t)oenv) & 15) == 0);
     const bool inside = (r.bits & MC_ER_INSIDE) != 0, skip_first = (r.bits & MC_ER_SKIP) != 0;
-    // per-env facts that let the march stop early (see shade_ray / flat_ray)
-    const bool eye_inb = (unsigned)(int)floorf(r.c.eye_x) < (unsigned)rp.wx &&
-                         (unsigned)(int)floorf(r.c.eye_y) < (unsigned)rp.wy &&
-                         (unsigned)(int)floorf(r.c.eye_z) < (unsigned)rp.wz;
-    const bool sky_exit = (FAM == MC_FAM_SHADED) ? (inside && rp.vd > 0.0f && !dbg_pixel) : (eye_inb && !dbg_pixel);
-    const bool vd_safe = sky_exit && box_within_view(r.c, rp.wx, rp.wy, rp.wz, rp.vd);
+    const MarchFacts mf = march_facts<FAM>(p, r);
     const Dda0 d0 = dda0(r.c);
     const int TW = tile_w, TH = 32 / tile_w;
     const int lx = lane % TW, ly = lane / TW;
     const int bpp = 3 * (F32 ? 4 : 1);
     const int nbands = (H + TH - 1) / TH;
-    auto claim = [&]() -> int {
-        int v = 0;
-        if (lane == 0) v = atomicAdd(band_ctr, 1);
-        return __shfl_sync(0xffffffffu, v, 0);
-    };
-    if constexpr (std::is_same<V, VoxEither>::value &&
-                  (FAM == MC_FAM_SHADED || FAM == MC_FAM_MINIMAL || FAM == MC_FAM_PREBASIS)) {
-        // the common case (fast_band): staged world, eye inside with air in
-        // its voxel, no debug output, whole tiles
-        const int fk = fast_kind<FAM>(vox.smem, sky_exit && skip_first, dbg_pixel != nullptr, vd_safe, rp.max_steps,
-                                      rp.wx, rp.wy, rp.wz, W, H, TW, bpp, vec_ok);
-        if (fk) {
-            build_fast_start(cx.sstart, fk, d0, rp.wx, rp.wy, rp.wz, r.ub, rp.max_steps, lane);
-            const uint32_t wb = staged_base(vox);
-            const int wxz = rp.wx * rp.wz;
-            FastEnv fe;
-            fe.start = cx.sstart;
-            fe.base = fk == 1 ? wb : wb + (uint32_t)(d0.vy * wxz + d0.vx * rp.wz + d0.vz);
-            fe.chk = staged_range(wb, wxz, wxz * rp.wy);
-            fe.vd = vd;
-            fe.rcp_vd = cx.rcp_vd;
-            for (int b = band_ctr ? claim() : 0; b < nbands; b = band_ctr ? claim() : b + 1) {
-                const int row0 = b * TH;
-                uint8_t* dst = oenv + (long long)row0 * W * bpp;
-                if (fk == 1)
-                    fast_band<FAM, F32, false>(r.c, d0, fe, W, TW, row0, lane, cx.s_u, cx.s_v, cx.s_cs, cx.s_rgbp,
-                                               cx.stage, dst);
-                else
-                    fast_band<FAM, F32, true>(r.c, d0, fe, W, TW, row0, lane, cx.s_u, cx.s_v, cx.s_cs, cx.s_rgbp,
-                                              cx.stage, dst);
-            }
-            return;
-        }
-    }
-    for (int b = band_ctr ? claim() : 0; b < nbands; b = band_ctr ? claim() : b + 1) {
+    for (int b = next_band(band_ctr, -1, lane); b < nbands; b = next_band(band_ctr, b, lane)) {
         const int row0 = b * TH;
         const int py = row0 + ly;
         const float v = (py < H && in_bounds(py, H, MC_SITE_TABLE)) ? cx.s_v[py] : 0.0f;
@@ -2916,8 +2558,7 @@ __device__ __forceinline__ void render_env(const mc_kp& p, long long e, const En
             const int px = tx0 + lx;
             if (px < W && py < H && in_bounds(px, W, MC_SITE_TABLE)) {
                 const float u = cx.s_u[px];
-                Hit h = march_pixel<FAM, V, VDLIM>(rp, r.c, d0, u, v, vox, inside, skip_first, sky_exit, vd_safe,
-                                                   r.ytop);
+                Hit h = march_pixel<FAM, V>(rp, r.c, d0, u, v, vox, inside, skip_first, mf.sky_exit, mf.vd_safe, r.ytop);
                 const int so = ly * W + px;  // pixel within the staged band
                 if (!in_bounds((long long)(so + 1) * bpp - 1, (long long)TH * W * bpp, MC_SITE_BAND)) continue;
                 if (FAM == MC_FAM_SHADED || FAM == MC_FAM_SHADED_FAST) {
@@ -2943,7 +2584,7 @@ __device__ __forceinline__ void render_env(const mc_kp& p, long long e, const En
                     sb[2] = col[2];
                 }
                 if (dbg_pixel && in_bounds(py * W + px, W * H, MC_SITE_DEBUG))
-                    dbg_pixel[e * W * H + py * W + px] = dbg_code(h);
+                    dbg_pixel[(long long)e * W * H + py * W + px] = dbg_code(h);
             }
         }
         __syncwarp();
@@ -2966,82 +2607,334 @@ __device__ __forceinline__ void render_env(const mc_kp& p, long long e, const En
 }
 
 template <int FAM, bool F32>
-__device__ __noinline__ bool fused_finish_from_global(const mc_kp& p, long long e, long long claimed,
-                                                      long long total_warps, int tile_w, int lane, FusedCtx cx) {
-    const long long wxyz = (long long)p.wx * p.wy * p.wz;
-    if (e < p.B) {
-        // env e was stepped and found not buried: its camera, as stored by the
-        // step, gives the same render constants bit for bit
-        EnvRender r;
-        const float* cam = p.cameras + e * 5;
-        __syncwarp();
-        if (FAM == MC_FAM_PREBASIS) {
-            float bas[13];
-            basis_compute(cam[0], cam[1], cam[2], cam[3], cam[4], p.W, p.H, p.fov, bas);
-            r.c = cam_from_basis(bas);
-        } else {
-            r.c = cam_trig(cam[0], cam[1], cam[2], cam[3], cam[4]);
-        }
-        const int ey = (int)floorf(r.c.eye_y);
-        bool inside = false, skip_first;
-        if (FAM == MC_FAM_SHADED || FAM == MC_FAM_SHADED_FAST) {
-            inside = eye_inside(r.c, p.wx, p.wy, p.wz, p.vd);
-            skip_first = inside && p.vd > 0.0f && p.max_steps > 0 && !(FAM == MC_FAM_SHADED_FAST && ey < p.gh);
-        } else {
-            skip_first = p.max_steps > 0;  // not buried: the eye's voxel holds air or lies outside the world
-        }
-        r.bits = (inside ? MC_ER_INSIDE : 0) | (skip_first ? MC_ER_SKIP : 0);
-        r.fill_blk = AIR;
-        r.mod_idx = -1;
-        r.mod_val = 0;
-        r.ytop = p.wy - 1;
-        r.ub = up_none(r.ytop);
-        render_env<FAM, F32, VoxGlobal, false>(p, e, r, cx, VoxGlobal{p.voxels + e * wxyz}, tile_w, lane, nullptr);
-        // a depth-2 warp's next env is the one it claimed already
-        e = claimed >= 0 ? claimed : next_env(p, e, total_warps, lane);
-    }
-    bool any_done = false;
-    const ActionSrc act{p.actions, p.buttons, p.look};
-    for (; e < p.B; e = next_env(p, e, total_warps, lane)) {
-        EnvRender r = agent_step<FAM>(p, act, e, lane);
-        any_done |= (r.bits & MC_ER_DONE) != 0;
-        if (r.bits & MC_ER_BURIED)
-            fill_env<FAM, F32>(p, e, r, cx, lane, 32);
+__device__ __forceinline__ void render_slow(const mc_kp& p, const EnvRec& q, int ytop, const FusedCtx& cx,
+                                            const int8_t* staged, int tile_w, int lane, int* band_ctr) {
+    EnvRender r = render_of_rec(q, p.wy);
+    r.ytop = ytop;
+    if (staged)
+        render_slow_from<FAM, F32>(p, q.env, r, cx, VoxShared{staged}, tile_w, lane, band_ctr);
+    else
+        render_slow_from<FAM, F32>(p, q.env, r, cx, VoxGlobal{p.voxels + q.env * (long long)p.wx * p.wy * p.wz},
+                                   tile_w, lane, band_ctr);
+}
+
+// Whether a family has the common-case loop (fast_band).
+__host__ __device__ constexpr bool fast_family(int fam) {
+    return fam == MC_FAM_SHADED || fam == MC_FAM_MINIMAL || fam == MC_FAM_PREBASIS;
+}
+
+// Row bands of slice `part` of `slices` of env e's image by one warp
+// (next_band) in the common case: the launch allows it (mc_fast_launch), the
+// world is staged, the eye is inside the box with air in its voxel.
+template <int FAM, bool F32>
+__device__ __forceinline__ void render_fast(const mc_kp& p, int e, const EnvRender& r, const FusedCtx& cx,
+                                            const int8_t* staged, int tile_w, int lane, int* band_ctr, int part,
+                                            int slices) {
+    const int W = p.W, TW = tile_w, TH = 32 / tile_w;
+    constexpr int bpp = 3 * (F32 ? 4 : 1);
+    uint8_t* oenv = (uint8_t*)p.obs + e * ((long long)W * p.H * bpp);
+    const bool vd_safe = box_within_view(r.c, p.wx, p.wy, p.wz, p.vd);
+    const int fk = fast_kind<FAM>(vd_safe, p.max_steps, p.wx, p.wy, p.wz);
+    const Dda0 d0 = dda0(r.c);
+    build_fast_start(cx.sstart, fk, d0, p.wx, p.wy, p.wz, r.ub, p.max_steps, lane);
+    const uint32_t wb = smem_u32(staged);
+    const int wxz = p.wx * p.wz;
+    FastEnv fe;
+    fe.start = cx.sstart;
+    fe.base = fk == 1 ? wb : wb + (uint32_t)(d0.vy * wxz + d0.vx * p.wz + d0.vz);
+    fe.chk = staged_range(wb, wxz, wxz * p.wy);
+    fe.vd = p.vd;
+    fe.rcp_vd = N::rcp_of(p.vd);
+    const int nb = p.H / TH, b0 = part * nb / slices, nbands = (part + 1) * nb / slices - b0;
+    for (int b = next_band(band_ctr, -1, lane); b < nbands; b = next_band(band_ctr, b, lane)) {
+        const int row0 = (b0 + b) * TH;
+        uint8_t* dst = oenv + row0 * W * bpp;
+        if (fk == 1)
+            fast_band<FAM, F32, false>(r.c, d0, fe, W, TW, row0, lane, cx.s_u, cx.s_v, cx.s_cs, cx.s_rgbp, cx.stage,
+                                       dst);
         else
-            render_env<FAM, F32, VoxGlobal, false>(p, e, r, cx, VoxGlobal{p.voxels + e * wxyz}, tile_w, lane,
-                                                   nullptr);
+            fast_band<FAM, F32, true>(r.c, d0, fe, W, TW, row0, lane, cx.s_u, cx.s_v, cx.s_cs, cx.s_rgbp, cx.stage,
+                                      dst);
     }
-    return any_done;
 }
 
-// Start the bulk copy of one world into shared memory (lane 0 issues it).
-__device__ __forceinline__ void issue_world_copy(uint32_t mbar_a, int8_t* dst, const int8_t* src, int bytes, int lane) {
+// ---- regeneration -----------------------------------------------------------
+// The step's regeneration is done by whoever rendered the env last: its world
+// is not read again in this step, so the template's bytes go over it right
+// after its image, with no pass over all worlds and no kernel of its own.
+// Which worlds (p.regen): none, all of them when any env of the group is done
+// (MC_KREGEN_ALL; the agent kernel has settled that), or the done envs' own.
+__device__ __forceinline__ int regen_any(const mc_kp& p, int lane) {
+    (void)lane;
+    return p.regen == MC_KREGEN_ALL
+               ? __shfl_sync(0xffffffffu, *(volatile int32_t*)&p.flags[MC_FLAG_ANY_DONE], 0) : 0;
+}
+__device__ __forceinline__ bool regen_env(const mc_kp& p, int bits, int any_done) {
+    return any_done || (p.regen == MC_KREGEN_PER_ENV && (bits & MC_ER_DONE));
+}
+__device__ __forceinline__ void regen_world(const mc_kp& p, int e, int t, int nt) {
+    const int wxyz = p.wx * p.wy * p.wz;
+    int8_t* d = p.voxels + e * (long long)wxyz;
+    // 16-byte stores only when every world starts on a 16-byte boundary
+    // (a voxels view may start at any byte offset)
+    if ((wxyz & 15) == 0 && ((((uintptr_t)p.voxels) | ((uintptr_t)p.world_template)) & 15) == 0) {
+        uint4* d4 = reinterpret_cast<uint4*>(d);
+        const uint4* t4 = reinterpret_cast<const uint4*>(p.world_template);
+        for (int k = t; k < (wxyz >> 4); k += nt) d4[k] = __ldg(t4 + k);
+    } else {
+        for (int k = t; k < wxyz; k += nt) d[k] = p.world_template[k];
+    }
+}
+// Whether this warp is the last of its env's slices to get here (all of them
+// are then done reading the env's world).
+__device__ __forceinline__ bool last_slice(const EnvRec* recs, int i, int slices, int lane) {
+    if (slices == 1) return true;
+    int prev = 0;
+    __syncwarp();
     if (lane == 0) {
-        // generic-proxy reads of the previous world must precede the copy
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(mbar_a), "r"(bytes) : "memory");
-        asm volatile(
-            "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                smem_u32(dst)),
-            "l"(src), "r"(bytes), "r"(mbar_a)
-            : "memory");
+        __threadfence();
+        prev = atomicAdd(const_cast<int*>(&recs[i].arrived), 1);
+    }
+    return __shfl_sync(0xffffffffu, prev, 0) == slices - 1;
+}
+
+#ifndef MC_FUSED_MIN_BLOCKS
+#define MC_FUSED_MIN_BLOCKS 4
+#endif
+// One warp per env: a persistent grid whose warps claim records, fill the
+// buried envs and march the others over their world, staged in shared memory
+// (STAGE) or in global memory.  Bound by instruction issue in the march; at
+// its 64-register budget 4 CTAs of 8 warps share an SM.
+//
+// A small batch would leave most of the GPU's warps without an env: its images
+// are cut into `slices` row ranges (slice_rows), each a unit of its own that stages
+// the env's world again (a few KB from L2).
+template <int FAM, bool F32, bool STAGE>
+__global__ void __launch_bounds__(256, MC_FUSED_MIN_BLOCKS)
+    k_render_warp(const __grid_constant__ mc_kp p, int tile_w, int slices) {
+    extern __shared__ __align__(16) uint8_t smem[];
+    const int lane = threadIdx.x & 31;
+    const int warp = threadIdx.x >> 5;
+    const int nwarps = blockDim.x >> 5;
+    const int W = p.W, H = p.H;
+    const int wxz = p.wx * p.wz;
+    const int wxyz = wxz * p.wy;
+    FusedLayout L = fused_layout(W, H, wxyz, wxz, F32, STAGE, tile_w);
+
+    FusedCtx cx;
+    build_fast_tables(reinterpret_cast<float4*>(smem), reinterpret_cast<uint32_t*>(smem + kShadeTableBytes));
+    cx.s_cs = reinterpret_cast<const float4*>(smem);
+    cx.s_rgbp = reinterpret_cast<const uint32_t*>(smem + kShadeTableBytes);
+    float* s_u = reinterpret_cast<float*>(smem + kFastTableBytes);
+    build_uv_tables<FAM>(p, s_u, s_u + W);
+    cx.s_u = s_u;
+    cx.s_v = s_u + W;
+    load_colour_tables(reinterpret_cast<uint8_t*>(s_u + W + H), cx);
+    uint8_t* wbase = smem + L.head_bytes + warp * L.warp_bytes;
+    cx.mbar_a = smem_u32(wbase);
+    cx.sstart = reinterpret_cast<int4*>(wbase + 16);
+    cx.stage = wbase + 16 + 128;
+    int8_t* sworld = reinterpret_cast<int8_t*>(wbase + 16 + 128 + L.stage_bytes);
+    cx.rcp_vd = N::rcp_of(p.vd);
+    if (STAGE) mbar_init_warp(cx.mbar_a, lane);
+    __syncthreads();
+    pdl_trigger();
+    pdl_wait();
+
+    uint32_t phase = 0;
+    bool no_stage = false;  // a copy timed out: this warp renders from global memory from now on
+    bool pending = false;   // ... and that copy may still land
+    const int total_warps = gridDim.x * nwarps;
+    const EnvRec* recs = reinterpret_cast<const EnvRec*>(p.rec);
+    const int first = blockIdx.x * nwarps + warp;
+    const int any_done = regen_any(p, lane);
+    if constexpr (STAGE && fast_family(FAM)) {
+        const int units = p.B * slices;
+        int u = p.sched_dynamic ? next_unit(p, MC_FLAG_WORK, 0, total_warps, lane) : first;
+        for (; u < units; u = next_unit(p, MC_FLAG_WORK, u, total_warps, lane)) {
+            const int i = u / slices, part = u - i * slices;
+            const EnvRec q = load_rec(recs, i);
+            if (q.bits & MC_ER_SLOW) continue;
+            if (q.bits & MC_ER_BURIED) {
+                if (part == 0) fill_env<FAM, F32>(p, q.env, q.fill_blk, cx, lane, 32);
+            } else {
+                if (!stage_fits(sworld, wxyz)) {
+                    no_stage = true;
+                    break;
+                }
+                issue_world_copy(cx.mbar_a, sworld, p.voxels + q.env * (long long)wxyz, wxyz, lane);
+                EnvRender r = render_of_rec(q, p.wy);
+                if (!mbar_wait(cx.mbar_a, phase, p.wait_polls)) {
+                    if (lane == 0) atomicExch(&p.flags[MC_FLAG_ERROR], MC_KERR_TMA_TIMEOUT);
+                    no_stage = pending = true;
+                    break;
+                }
+                phase ^= 1u;
+                measure_staged(r, sworld, p.wx, p.wy, p.wz, lane);
+                render_fast<FAM, F32>(p, q.env, r, cx, sworld, tile_w, lane, nullptr, part, slices);
+            }
+            if (regen_env(p, q.bits, any_done) && last_slice(recs, i, slices, lane)) regen_world(p, q.env, lane, 32);
+        }
+        // a copy that timed out: this unit and the rest of the warp's, from
+        // global memory (a slice's warp renders the whole image: the others'
+        // pixels come out the same)
+        for (; no_stage && u < units; u = next_unit(p, MC_FLAG_WORK, u, total_warps, lane)) {
+            const int i = u / slices, part = u - i * slices;
+            const EnvRec q = load_rec(recs, i);
+            if (q.bits & MC_ER_SLOW) continue;
+            if (!(q.bits & MC_ER_BURIED))
+                render_slow<FAM, F32>(p, q, p.wy - 1, cx, nullptr, tile_w, lane, nullptr);
+            else if (part == 0)
+                fill_env<FAM, F32>(p, q.env, q.fill_blk, cx, lane, 32);
+            if (regen_env(p, q.bits, any_done) && last_slice(recs, i, slices, lane)) regen_world(p, q.env, lane, 32);
+        }
+    }
+    // the general pass: the envs that the common path left (every env of a
+    // launch that has no common path)
+    constexpr bool all = !(STAGE && fast_family(FAM));
+    const int any_slow = __shfl_sync(0xffffffffu, *(volatile int32_t*)&p.flags[MC_FLAG_ANY_SLOW], 0);
+    if (all || !p.sched_dynamic || any_slow) {
+        int u = p.sched_dynamic ? next_unit(p, MC_FLAG_SLOW_WORK, 0, total_warps, lane) : first;
+        for (; u < p.B; u = next_unit(p, MC_FLAG_SLOW_WORK, u, total_warps, lane)) {
+            const EnvRec q = load_rec(recs, u);
+            if (!all && !(q.bits & MC_ER_SLOW)) continue;
+            if (q.bits & MC_ER_BURIED) {
+                fill_env<FAM, F32>(p, q.env, q.fill_blk, cx, lane, 32);
+            } else {
+                bool staged = STAGE && !no_stage && stage_fits(sworld, wxyz);
+                int ytop = p.wy - 1;
+                if (staged) {
+                    issue_world_copy(cx.mbar_a, sworld, p.voxels + q.env * (long long)wxyz, wxyz, lane);
+                    if (mbar_wait(cx.mbar_a, phase, p.wait_polls)) {
+                        phase ^= 1u;
+                        EnvRender r = render_of_rec(q, p.wy);
+                        measure_staged(r, sworld, p.wx, p.wy, p.wz, lane);
+                        ytop = r.ytop;
+                    } else {
+                        if (lane == 0) atomicExch(&p.flags[MC_FLAG_ERROR], MC_KERR_TMA_TIMEOUT);
+                        no_stage = pending = true;
+                        staged = false;
+                    }
+                }
+                render_slow<FAM, F32>(p, q, ytop, cx, staged ? sworld : nullptr, tile_w, lane, nullptr);
+            }
+            if (regen_env(p, q.bits, any_done)) regen_world(p, q.env, lane, 32);
+        }
+    }
+    // a timed-out copy may still be in flight: let it land (bounded, with the
+    // default budget) before this warp's part of shared memory can be released
+    if (STAGE && pending) mbar_wait(cx.mbar_a, phase);
+    // No CTA barrier here: warps leave as soon as their last env is done.
+    if (lane == 0) {
+        bounds_to_flags(p.flags);
+        // every claim of this warp has returned (the last one >= B)
+        if (p.sched_dynamic) finish_dynamic(p.flags, total_warps, [&] { p.flags[MC_FLAG_ANY_DONE] = 0; });
     }
 }
 
-// Bulk copy of one world into shared memory, waited for with a bound.
-__device__ __forceinline__ bool stage_world(uint32_t mbar_a, uint32_t& phase, int8_t* dst, const int8_t* src,
-                                            int bytes, int lane, int polls) {
-    issue_world_copy(mbar_a, dst, src, bytes, lane);
-    const bool ok = mbar_wait(mbar_a, phase, polls);
-    phase ^= 1u;
-    return ok;
+// ---------------------------------------------------------------------------
+// Team kernel: the images of env groups of any size, by teams of warps
+// ---------------------------------------------------------------------------
+// A CTA of warps_per_cta warps is split into teams of team_warps warps.  A
+// team claims one work unit at a time from a device counter:
+//  * a cooperative group's unit is ONE env: all warps of the team march row
+//    bands of its image (bands claimed from a shared counter), reading the
+//    world from one shared-memory copy per team when staged.  Big images over
+//    big worlds then keep an SM's L1 and shared memory on few worlds, like a
+//    per-pixel kernel;
+//  * a per-warp group's unit is team_warps envs, one per warp, each rendered
+//    by its warp alone.
+// Units are ordered by decreasing per-env cost across groups, so the most
+// expensive envs are claimed first and do not straggle at the end.
+//
+// DEPTH 1: one world buffer per team (or warp); the unit's copy starts when
+// its record is read.  DEPTH 2: two buffers; unit k+1's record is read and its
+// copy started before unit k is rendered, so it overlaps that render (one
+// claim further ahead, twice the shared memory).
+//
+// A warp whose wait for a copy runs out records the timeout, never reads a
+// staged world again and renders its bands from global memory; in the shared
+// scan it stands in for its share of the layers with bounds that cut
+// nothing, so the others' results stay exact.
+struct TeamShared {
+    unsigned unit[4];      // claimed units, unit k's number at k & 3
+    int band_ctr[2];       // next row band of the cooperative env of unit k & 1
+    unsigned long long mbar[2];
+    int timed_out;         // a wait for a copy ran out: no further copies, render from global memory
+    int may_stage[2];      // general pass: whether unit k & 1 may be staged
+    unsigned sunit[2];     // general pass: claimed units, alternating slots
+    int any_done;          // bit g: every world of group g is to be regenerated
+    int last;              // the team rendered its env's last slice
+    int pad;
+    // up bounds of the cooperative env of unit k & 1, combined over the team's warps (UpPart)
+    int uxa[2][4], uya[2][4];
+    unsigned long long ump[2], umm[2];
+};
+static_assert(sizeof(TeamShared) <= MC_TEAM_HEAD_BYTES, "team head");
+
+__device__ __forceinline__ void team_unit_reset(TeamShared* ts, int d) {
+    ts->band_ctr[d] = 0;
+    ts->uxa[d][0] = 255; ts->uxa[d][1] = 0; ts->uxa[d][2] = 255; ts->uxa[d][3] = 0;
+    ts->uya[d][0] = ts->uya[d][1] = ts->uya[d][2] = ts->uya[d][3] = 0;
+    ts->ump[d] = ts->umm[d] = 0ull;
+}
+
+// The up bounds of a cooperative env, scanned by all nw warps of its team
+// (warp w sweeps its share of the layers, staged_up_part) and combined in
+// the team's shared words with shared-memory atomics, so every warp holds
+// the same bounds after the team barrier.  Called by every warp of the team;
+// `have` false: this warp may not read the world and adds bounds that cut nothing.
+template <typename M>
+__device__ __forceinline__ UpBounds team_up_bounds_t(bool have, const int8_t* world, int wx, int wy, int wz, int vx,
+                                                     int vy, int vz, int lane, int w, int nw, TeamShared* ts, int d,
+                                                     int bar) {
+    UpPart<M> r;
+    if (have) {
+        r = staged_up_part<M>(world, wx, wy, wz, vx, vy, vz, lane, w, nw);
+    } else {
+        r.xa0 = 0; r.xa1 = wx - 1; r.xa2 = 0; r.xa3 = wx - 1;
+        r.ya0 = r.ya1 = r.ya2 = r.ya3 = wy;
+        r.mp = r.mm = (M(1) << (wz - 1)) | M(1);
+    }
+    if (lane == 0) {
+        atomicMin(&ts->uxa[d][0], r.xa0);
+        atomicMax(&ts->uxa[d][1], r.xa1);
+        atomicMin(&ts->uxa[d][2], r.xa2);
+        atomicMax(&ts->uxa[d][3], r.xa3);
+        atomicMax(&ts->uya[d][0], r.ya0);
+        atomicMax(&ts->uya[d][1], r.ya1);
+        atomicMax(&ts->uya[d][2], r.ya2);
+        atomicMax(&ts->uya[d][3], r.ya3);
+        atomicOr(&ts->ump[d], (unsigned long long)r.mp);
+        atomicOr(&ts->umm[d], (unsigned long long)r.mm);
+    }
+    team_sync(bar, nw * 32);
+    UpPart<M> t;
+    t.xa0 = ts->uxa[d][0];
+    t.xa1 = ts->uxa[d][1];
+    t.xa2 = ts->uxa[d][2];
+    t.xa3 = ts->uxa[d][3];
+    t.ya0 = ts->uya[d][0];
+    t.ya1 = ts->uya[d][1];
+    t.ya2 = ts->uya[d][2];
+    t.ya3 = ts->uya[d][3];
+    t.mp = (M)ts->ump[d];
+    t.mm = (M)ts->umm[d];
+    return up_bounds_of(t);
+}
+__device__ __forceinline__ UpBounds team_up_bounds(bool have, const int8_t* world, int wx, int wy, int wz, int vx,
+                                                   int vy, int vz, int lane, int w, int nw, TeamShared* ts, int d,
+                                                   int bar) {
+    return wz > 32
+               ? team_up_bounds_t<unsigned long long>(have, world, wx, wy, wz, vx, vy, vz, lane, w, nw, ts, d, bar)
+               : team_up_bounds_t<uint32_t>(have, world, wx, wy, wz, vx, vy, vz, lane, w, nw, ts, d, bar);
 }
 
 #ifndef MC_TEAM_MIN_BLOCKS
 #define MC_TEAM_MIN_BLOCKS 3  // 80 registers: the render path without spills
 #endif
-template <int FAM, bool F32>
-__global__ void __launch_bounds__(256, MC_TEAM_MIN_BLOCKS) k_step_team(const __grid_constant__ mc_ragged_kp rk) {
+template <int FAM, bool F32, int DEPTH>
+__global__ void __launch_bounds__(256, MC_TEAM_MIN_BLOCKS) k_render_team(const __grid_constant__ mc_ragged_kp rk) {
     extern __shared__ __align__(16) uint8_t smem[];
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
@@ -3064,326 +2957,255 @@ __global__ void __launch_bounds__(256, MC_TEAM_MIN_BLOCKS) k_step_team(const __g
     TeamShared* ts = reinterpret_cast<TeamShared*>(smem + rk.teams_off + team * rk.team_bytes);
     int8_t* tworld = reinterpret_cast<int8_t*>(ts) + MC_TEAM_HEAD_BYTES;
     uint8_t* wbase = smem + rk.warps_off + warp * rk.warp_bytes;
-    cx.mbar_a = smem_u32(wbase);
+    cx.mbar_a = smem_u32(wbase);  // this warp's mbarriers (per-warp groups), depth slot d's at + 8 d
+    const uint32_t tmbar = smem_u32(ts->mbar);
     cx.sstart = reinterpret_cast<int4*>(wbase + 16);
     cx.stage = wbase + 16 + 128;
-    if (rk.stage_mask) mbar_init_warp(cx.mbar_a, lane);
     const bool claimer = (wt == 0 && lane == 0);
-    const long long total_teams = (long long)gridDim.x * teams_per_cta;
-    const long long my_team = (long long)blockIdx.x * teams_per_cta + team;
-    const unsigned total_units = (unsigned)rk.ustart[G];
-    auto claim = [&](int k) -> unsigned {
-        if (rk.sched_dynamic) return atomicAdd(reinterpret_cast<unsigned*>(&rk.flags[MC_FLAG_WORK]), 1u);
-        const long long u = my_team + (long long)k * total_teams;
-        return u < (long long)total_units ? (unsigned)u : total_units;
-    };
-    if (claimer) ts->unit[0] = claim(0);
-    __syncthreads();
-    const int bar = 1 + team, nthr = TWN * 32;
-    uint32_t phase = 0;
-    bool warp_no_stage = false;   // a copy of this warp timed out: it renders from global memory from now on
-    uint32_t pending_phase = 0;   // that copy's phase, waited for before the warp leaves
-    for (int k = 0;; ++k) {
-        const unsigned u = ts->unit[k & 1];
-        if (u >= total_units) break;
-        int vg = 0;
-        while (vg + 1 < G && (long long)u >= rk.ustart[vg + 1]) ++vg;
-        const int g = rk.order[vg];
-        const mc_kp& p = rk.groups[g];
-        cx.s_u = tables + rk.uv_off[g];
-        cx.s_v = cx.s_u + p.W;
-        cx.rcp_vd = N::rcp_of(p.vd);
-        const long long local = (long long)u - rk.ustart[vg];
-        const int wxyz = p.wx * p.wy * p.wz;
-        const bool coop = (rk.coop_mask >> g) & 1;
-        // coop: warp 0 steps the env and the team renders it; else each warp
-        // steps and renders its own env of the unit
-        const long long e = coop ? local : local * TWN + wt;
-        const bool stepper = coop ? (wt == 0) : (e < p.B);
-        const int8_t* gw = p.voxels + e * (long long)wxyz;
-        int8_t* world = coop ? tworld : tworld + wt * rk.slot_bytes;
-        EnvRender r;
-        bool staged = false;
-        if (stepper) {
-            const long long s0 = rk.start[g];
-            const ActionSrc act{rk.actions ? rk.actions + s0 : nullptr, rk.actions ? nullptr : rk.buttons + 8 * s0,
-                                rk.actions ? nullptr : rk.look + 2 * s0};
-            // the world's bulk copy starts before the agent step, which it
-            // overlaps (the voxel the interaction changes is patched in after it
-            // lands); a buried env's copy is waited for and not used
-            bool copying = ((rk.stage_mask >> g) & 1) && !warp_no_stage;
-#if MC_CHECK_BOUNDS
-            if (copying) {
-                const SmemRange dyn = dyn_smem_range();
-                const long long off = (long long)smem_u32(world) - dyn.lo;
-                if (!in_bounds(off, dyn.span, MC_SITE_STAGE) || !in_bounds(off + wxyz - 1, dyn.span, MC_SITE_STAGE))
-                    copying = false;  // no copy issued: render from global memory
-            }
-#endif
-            if (copying) issue_world_copy(cx.mbar_a, world, gw, wxyz, lane);
-            r = agent_step<FAM>(p, act, e, lane);
-            if (lane == 0) {
-                // rare: set as the env ends (a per-team mask of groups would
-                // stay live across the loop and spill)
-                if (r.bits & MC_ER_DONE) atomicOr(&p.flags[MC_FLAG_ANY_DONE], 1);
-                if (rk.rewards_cat) {
-                    rk.rewards_cat[rk.start[g] + e] = p.rewards[e];
-                    rk.dones_cat[rk.start[g] + e] = (uint8_t)(r.bits & MC_ER_DONE);
-                }
-            }
-            staged = copying && !(r.bits & MC_ER_BURIED);
-            if (copying) {
-                const uint32_t ph = phase;
-                const bool landed = mbar_wait(cx.mbar_a, phase, p.wait_polls);
-                phase ^= 1u;
-                if (!landed) {
-                    if (lane == 0) atomicExch(&p.flags[MC_FLAG_ERROR], MC_KERR_TMA_TIMEOUT);
-                    warp_no_stage = true;  // the copy may still land: render from global memory from now on
-                    pending_phase = ph;
-                    staged = false;
-                } else if (staged) {
-                    // the interaction may have written after the copy read the byte
-                    if (lane == 0 && r.mod_idx >= 0 && in_bounds(r.mod_idx, wxyz, MC_SITE_PATCH))
-                        world[r.mod_idx] = (int8_t)r.mod_val;
-                    __syncwarp();
-                    if (coop && TWN > 1 && eye_in_box(r.c, p.wx, p.wy, p.wz) && up_scan_shape(p.wx, p.wy, p.wz))
-                        r.bits |= MC_ER_TSCAN;  // the whole team scans, after the barrier
-                    else
-                        measure_staged(r, world, p.wx, p.wy, p.wz, lane);
-                }
-            }
-            if (coop && lane == 0) {
-                r.bits |= staged ? MC_ER_STAGED : 0;
-                ts->r = r;
-                ts->band_ctr = 0;
-                if (r.bits & MC_ER_TSCAN) team_up_reset(ts);
-            }
-            __syncwarp();
-        }
-        if (coop) {
-            team_sync(bar, nthr);
-            r = ts->r;
-            staged = (r.bits & MC_ER_STAGED) != 0;
-            if (r.bits & MC_ER_TSCAN) {  // team-uniform
-                r.ub = team_up_bounds(world, p.wx, p.wy, p.wz, (int)floorf(r.c.eye_x), (int)floorf(r.c.eye_y),
-                                      (int)floorf(r.c.eye_z), lane, wt, TWN, ts, bar);
-                r.ytop = up_top(r.ub);
-            }
-        }
-        if (coop || stepper) {
-            if (r.bits & MC_ER_BURIED)
-                fill_env<FAM, F32>(p, e, r, cx, coop ? wt * 32 + lane : lane, coop ? nthr : 32);
-            else
-                render_env<FAM, F32>(p, e, r, cx, VoxEither{staged ? world : gw, staged}, rk.tile_w[g], lane,
-                                     coop ? &ts->band_ctr : nullptr);
-        }
-        if (claimer) ts->unit[(k + 1) & 1] = claim(k + 1);
-        team_sync(bar, nthr);
-    }
-    // a timed-out copy may still be in flight: let it land (bounded) before
-    // this warp's part of shared memory can be released
-    if (warp_no_stage) mbar_wait(cx.mbar_a, pending_phase);
     if (lane == 0) {
-        for (int g = 0; g < G; ++g) bounds_to_flags(rk.groups[g].flags);
-    }
-    if (claimer && rk.sched_dynamic) finish_dynamic(rk.flags, total_teams);
-}
-
-// ---------------------------------------------------------------------------
-// Team kernel with staging depth 2
-// ---------------------------------------------------------------------------
-// The same work as k_step_team, pipelined one unit deep: each team holds two
-// claimed units.  Before a team renders unit k, the warp(s) that step unit
-// k+1 run its agent step and start its world's bulk copy into the second
-// world buffer (and the second mbarrier) of their slot, so the copy and the
-// agent step overlap the render of unit k; the copy is waited for only when
-// unit k+1 is rendered.  The env's render constants wait in a per-warp
-// shared-memory stash between the two.
-static_assert(sizeof(EnvRender) <= MC_ENV_STASH_BYTES, "env stash");
-
-template <int FAM, bool F32>
-__global__ void __launch_bounds__(256, MC_TEAM_MIN_BLOCKS) k_step_team2(const __grid_constant__ mc_ragged_kp rk) {
-    extern __shared__ __align__(16) uint8_t smem[];
-    const int lane = threadIdx.x & 31;
-    const int warp = threadIdx.x >> 5;
-    const int nwarps = blockDim.x >> 5;
-    const int TWN = rk.team_warps;
-    const int team = warp / TWN, wt = warp % TWN;
-    const int teams_per_cta = nwarps / TWN;
-    const int G = rk.ngroups;
-    FusedCtx cx;
-    load_colour_tables(smem, cx);
-    build_fast_tables(reinterpret_cast<float4*>(smem + MC_COLOUR_TABLE_BYTES),
-                      reinterpret_cast<uint32_t*>(smem + MC_COLOUR_TABLE_BYTES + kShadeTableBytes));
-    cx.s_cs = reinterpret_cast<const float4*>(smem + MC_COLOUR_TABLE_BYTES);
-    cx.s_rgbp = reinterpret_cast<const uint32_t*>(smem + MC_COLOUR_TABLE_BYTES + kShadeTableBytes);
-    float* tables = reinterpret_cast<float*>(smem + rk.tables_off);
-    for (int g = 0; g < G; ++g)
-        build_uv_tables<FAM>(rk.groups[g], tables + rk.uv_off[g], tables + rk.uv_off[g] + rk.groups[g].W);
-    TeamShared* ts = reinterpret_cast<TeamShared*>(smem + rk.teams_off + team * rk.team_bytes);
-    int8_t* tworld = reinterpret_cast<int8_t*>(ts) + MC_TEAM_HEAD_BYTES;
-    uint8_t* wbase = smem + rk.warps_off + warp * rk.warp_bytes;
-    const uint32_t mbar0 = smem_u32(wbase);  // depth slot d's mbarrier at mbar0 + 8 d
-    cx.sstart = reinterpret_cast<int4*>(wbase + 16);
-    EnvRender* stash = reinterpret_cast<EnvRender*>(wbase + 16 + 128);  // depth slot d's env at + 96 d
-    cx.stage = wbase + 16 + 128 + 2 * MC_ENV_STASH_BYTES;
-    if (lane == 0) {
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(mbar0) : "memory");
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(mbar0 + 8) : "memory");
+        for (int d = 0; d < DEPTH; ++d) {
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(cx.mbar_a + 8 * d) : "memory");
+            if (wt == 0) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(tmbar + 8 * d) : "memory");
+        }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    const bool claimer = (wt == 0 && lane == 0);
     const long long total_teams = (long long)gridDim.x * teams_per_cta;
-    const long long my_team = (long long)blockIdx.x * teams_per_cta + team;
     const unsigned total_units = (unsigned)rk.ustart[G];
-    auto claim = [&](int k) -> unsigned {
-        if (rk.sched_dynamic) return atomicAdd(reinterpret_cast<unsigned*>(&rk.flags[MC_FLAG_WORK]), 1u);
-        const long long u = my_team + (long long)k * total_teams;
-        return u < (long long)total_units ? (unsigned)u : total_units;
+    auto claim = [&](int counter) -> unsigned {
+        return atomicAdd(reinterpret_cast<unsigned*>(&rk.flags[counter]), 1u);
     };
+    pdl_trigger();
+    pdl_wait();
     if (claimer) {
-        ts->unit[0] = claim(0);
-        ts->unit[1] = claim(1);
+        for (int k = 0; k < DEPTH; ++k) ts->unit[k] = claim(MC_FLAG_WORK);
+        ts->timed_out = 0;
+        int any = 0;
+        for (int g = 0; g < G; ++g)
+            if (rk.groups[g].regen == MC_KREGEN_ALL && *(volatile int32_t*)&rk.groups[g].flags[MC_FLAG_ANY_DONE])
+                any |= 1 << g;
+        ts->any_done = any;
+        team_unit_reset(ts, 0);
     }
     __syncthreads();
     const int bar = 1 + team, nthr = TWN * 32;
-    uint32_t phases = 0;          // bit d: parity of depth slot d's next wait
-    bool warp_no_stage = false;   // a copy of this warp timed out: no more copies, render from global memory
-    uint32_t pending = 0;         // bit d: a timed-out copy into slot d may still be in flight
-    uint32_t pending_phases = 0;  // bit d: its parity
+    uint32_t tphase = 0;     // bit d: parity of the team's next wait on depth slot d
+    uint32_t wphase = 0;     // ... of this warp's own
+    uint32_t tlive = 0, wlive = 0;  // bit d: a copy this warp issued into slot d that it has not seen land
 
-    // Where unit u lies: its group, env, and whether this warp steps it.
+    // Where unit u lies: its group and record, and whether this warp renders it.
     struct Unit {
-        int g;
-        long long e;
-        bool coop, stepper;
+        int g, i, part;
+        bool coop, mine;
     };
     auto locate = [&](unsigned u) -> Unit {
         int vg = 0;
         while (vg + 1 < G && (long long)u >= rk.ustart[vg + 1]) ++vg;
         Unit t;
         t.g = rk.order[vg];
-        const long long local = (long long)u - rk.ustart[vg];
+        const int local = (int)((long long)u - rk.ustart[vg]);
         t.coop = (rk.coop_mask >> t.g) & 1;
-        t.e = t.coop ? local : local * TWN + wt;
-        t.stepper = t.coop ? (wt == 0) : (t.e < rk.groups[t.g].B);
+        t.i = t.coop ? local / rk.slices[t.g] : local * TWN + wt;
+        t.part = t.coop ? local - t.i * rk.slices[t.g] : 0;
+        t.mine = t.coop || t.i < rk.groups[t.g].B;
         return t;
     };
     auto slot_world = [&](int d, bool coop) -> int8_t* {
-        return tworld + d * rk.world_stride + (coop ? 0 : wt * rk.slot_bytes);
+        return tworld + (DEPTH > 1 ? d * rk.world_stride : 0) + (coop ? 0 : wt * rk.slot_bytes);
     };
-    // The stepper of unit u steps its env and starts its world's copy into depth slot d.
-    auto prepare = [&](unsigned u, int d) {
-        const Unit t = locate(u);
-        if (!t.stepper) return;
+    auto recs_of = [&](int g) { return reinterpret_cast<const EnvRec*>(rk.rec) + rk.start[g]; };
+    auto use_group = [&](int g) {
+        cx.s_u = tables + rk.uv_off[g];
+        cx.s_v = cx.s_u + rk.groups[g].W;
+        cx.rcp_vd = N::rcp_of(rk.groups[g].vd);
+    };
+    // Start the copy of unit t's world into depth slot d when its env is one
+    // of `kind` (its MC_ER_BURIED | MC_ER_SLOW bits): the team's first warp
+    // for a cooperative env, every warp for its own env otherwise.
+    auto issue = [&](const Unit& t, int d, int kind) {
+        if (!((rk.stage_mask >> t.g) & 1) || (t.coop && wt != 0) || !t.mine) return;
+        const EnvRec q = load_rec(recs_of(t.g), t.i);
+        if ((q.bits & (MC_ER_BURIED | MC_ER_SLOW)) != kind) return;
         const mc_kp& p = rk.groups[t.g];
         const int wxyz = p.wx * p.wy * p.wz;
-        const long long s0 = rk.start[t.g];
-        const ActionSrc act{rk.actions ? rk.actions + s0 : nullptr, rk.actions ? nullptr : rk.buttons + 8 * s0,
-                            rk.actions ? nullptr : rk.look + 2 * s0};
-        EnvRender r = agent_step<FAM>(p, act, t.e, lane);
-        if (lane == 0) {
-            if (r.bits & MC_ER_DONE) atomicOr(&p.flags[MC_FLAG_ANY_DONE], 1);  // rare: set as the env ends
-            if (rk.rewards_cat) {
-                rk.rewards_cat[s0 + t.e] = p.rewards[t.e];
-                rk.dones_cat[s0 + t.e] = (uint8_t)(r.bits & MC_ER_DONE);
-            }
-        }
-        bool staged = ((rk.stage_mask >> t.g) & 1) && !(r.bits & MC_ER_BURIED) && !warp_no_stage;
         int8_t* world = slot_world(d, t.coop);
-#if MC_CHECK_BOUNDS
-        if (staged) {
-            const SmemRange dyn = dyn_smem_range();
-            const long long off = (long long)smem_u32(world) - dyn.lo;
-            if (!in_bounds(off, dyn.span, MC_SITE_STAGE) || !in_bounds(off + wxyz - 1, dyn.span, MC_SITE_STAGE))
-                staged = false;  // no copy issued: render from global memory
-        }
-#endif
-        if (staged && lane == 0) {
-            const uint32_t mb = mbar0 + 8 * d;
-            // generic-proxy reads of the slot's previous world must precede the copy
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(mb), "r"(wxyz) : "memory");
-            asm volatile(
-                "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                    smem_u32(world)),
-                "l"(p.voxels + t.e * (long long)wxyz), "r"(wxyz), "r"(mb)
-                : "memory");
-        }
-        r.bits |= staged ? MC_ER_STAGED : 0;
-        if (lane == 0) stash[d] = r;
-        __syncwarp();
+        if (!stage_fits(world, wxyz)) return;
+        issue_world_copy((t.coop ? tmbar : cx.mbar_a) + 8 * d, world, p.voxels + q.env * (long long)wxyz, wxyz, lane);
+        if (t.coop) tlive |= 1u << d;
+        else wlive |= 1u << d;
     };
-    // The stepper of unit u (slot d): wait for the world, patch and measure it.
-    auto finish = [&](const Unit& t, int d) {
+    // Wait for the copy of unit t into depth slot d.
+    auto landed = [&](const Unit& t, int d) -> bool {
         const mc_kp& p = rk.groups[t.g];
-        const int wxyz = p.wx * p.wy * p.wz;
-        EnvRender r = stash[d];
-        if (r.bits & MC_ER_STAGED) {
-            int8_t* world = slot_world(d, t.coop);
-            const uint32_t ph = (phases >> d) & 1u;
-            if (mbar_wait(mbar0 + 8 * d, ph, p.wait_polls)) {
-                // the interaction may have written after the copy read the byte
-                if (lane == 0 && r.mod_idx >= 0 && in_bounds(r.mod_idx, wxyz, MC_SITE_PATCH))
-                    world[r.mod_idx] = (int8_t)r.mod_val;
-                __syncwarp();
-                measure_staged(r, world, p.wx, p.wy, p.wz, lane);
-            } else {
-                if (lane == 0) atomicExch(&p.flags[MC_FLAG_ERROR], MC_KERR_TMA_TIMEOUT);
-                warp_no_stage = true;  // the copy may still land: render from global memory from now on
-                pending |= 1u << d;
-                pending_phases = (pending_phases & ~(1u << d)) | (ph << d);
-                r.bits &= ~MC_ER_STAGED;
-            }
-            phases ^= 1u << d;
+        if (!stage_fits(slot_world(d, t.coop), p.wx * p.wy * p.wz)) {
+            *(volatile int*)&ts->timed_out = 1;
+            return false;
         }
-        if (lane == 0) {
-            if (t.coop) {
-                ts->r = r;
-                ts->band_ctr = 0;
-            } else {
-                stash[d] = r;
-            }
+        uint32_t& ph = t.coop ? tphase : wphase;
+        if (!mbar_wait((t.coop ? tmbar : cx.mbar_a) + 8 * d, (ph >> d) & 1u, p.wait_polls)) {
+            if (lane == 0) atomicExch(&p.flags[MC_FLAG_ERROR], MC_KERR_TMA_TIMEOUT);
+            *(volatile int*)&ts->timed_out = 1;
+            return false;
         }
-        __syncwarp();
+        ph ^= 1u << d;
+        if (t.coop) tlive &= ~(1u << d);
+        else wlive &= ~(1u << d);
+        return true;
+    };
+    // After the unit's barrier: regenerate its env's world (see regen_world).
+    auto regen = [&](const Unit& t, int bits, int e, bool sliced) {
+        if (!t.mine || !regen_env(rk.groups[t.g], bits, (ts->any_done >> t.g) & 1)) return;
+        const mc_kp& p = rk.groups[t.g];
+        if (!t.coop) {
+            regen_world(p, e, lane, 32);
+            return;
+        }
+        if (sliced && rk.slices[t.g] > 1) {  // team-uniform
+            if (wt == 0) {
+                const bool last = last_slice(recs_of(t.g), t.i, rk.slices[t.g], lane);
+                if (lane == 0) ts->last = last;
+            }
+            team_sync(bar, nthr);
+            if (!ts->last) return;
+        }
+        regen_world(p, e, wt * 32 + lane, nthr);
     };
 
-    if (ts->unit[0] < total_units) prepare(ts->unit[0], 0);
+    if constexpr (fast_family(FAM)) {
+        int k = 0;
+        bool redo = false;
+        if (DEPTH > 1 && ts->unit[0] < total_units) issue(locate(ts->unit[0]), 0, 0);
+        for (;; ++k) {
+            const int d = DEPTH > 1 ? (k & 1) : 0;  // world slot and mbarrier of this unit
+            const unsigned u = ts->unit[k & 3];
+            if (u >= total_units) break;
+            const Unit t = locate(u);
+            if (DEPTH > 1) {
+                const unsigned u1 = ts->unit[(k + 1) & 3];
+                if (u1 < total_units) issue(locate(u1), d ^ 1, 0);
+            } else {
+                issue(t, d, 0);
+            }
+            if (claimer) team_unit_reset(ts, (k + 1) & 1);
+            const mc_kp& p = rk.groups[t.g];
+            int bits = MC_ER_SLOW, env = 0;
+            if (t.mine) {
+                const EnvRec q = load_rec(recs_of(t.g), t.i);
+                bits = q.bits;
+                env = q.env;
+                use_group(t.g);
+                if (q.bits & MC_ER_BURIED) {
+                    if (t.part == 0)
+                        fill_env<FAM, F32>(p, q.env, q.fill_blk, cx, t.coop ? wt * 32 + lane : lane,
+                                           t.coop ? nthr : 32);
+                } else if (!(q.bits & MC_ER_SLOW)) {
+                    const bool ok = landed(t, d);
+                    const int8_t* world = slot_world(d, t.coop);
+                    EnvRender r = render_of_rec(q, p.wy);
+                    if (t.coop && TWN > 1 && up_scan_shape(p.wx, p.wy, p.wz))  // team-uniform; the eye is in the box
+                        r.ub = team_up_bounds(ok, world, p.wx, p.wy, p.wz, (int)floorf(r.c.eye_x),
+                                              (int)floorf(r.c.eye_y), (int)floorf(r.c.eye_z), lane, wt, TWN, ts, k & 1,
+                                              bar);
+                    else if (ok)
+                        measure_staged(r, world, p.wx, p.wy, p.wz, lane);
+                    if (ok)
+                        render_fast<FAM, F32>(p, q.env, r, cx, world, rk.tile_w[t.g], lane,
+                                              t.coop ? &ts->band_ctr[k & 1] : nullptr, t.part, rk.slices[t.g]);
+                }
+            }
+            if (claimer) ts->unit[(k + DEPTH) & 3] = claim(MC_FLAG_WORK);
+            team_sync(bar, nthr);
+            if (*(volatile int*)&ts->timed_out) {  // set before the barrier: the same for the whole team
+                redo = true;
+                break;
+            }
+            if (!(bits & MC_ER_SLOW)) regen(t, bits, env, true);
+        }
+        // a copy timed out: this unit again and the rest of the team's, from global memory
+        if (redo) {
+            const int k0 = k;
+            if (claimer) team_unit_reset(ts, k & 1);
+            team_sync(bar, nthr);
+            for (;; ++k) {
+                const unsigned u = ts->unit[k & 3];
+                if (u >= total_units) break;
+                const Unit t = locate(u);
+                if (claimer) team_unit_reset(ts, (k + 1) & 1);
+                const mc_kp& p = rk.groups[t.g];
+                int bits = MC_ER_SLOW, env = 0;
+                if (t.mine) {
+                    const EnvRec q = load_rec(recs_of(t.g), t.i);
+                    bits = q.bits;
+                    env = q.env;
+                    use_group(t.g);
+                    if (q.bits & MC_ER_BURIED)
+                        fill_env<FAM, F32>(p, q.env, q.fill_blk, cx, t.coop ? wt * 32 + lane : lane, t.coop ? nthr : 32);
+                    else if (!(q.bits & MC_ER_SLOW))
+                        render_slow<FAM, F32>(p, q, p.wy - 1, cx, nullptr, rk.tile_w[t.g], lane,
+                                              t.coop ? &ts->band_ctr[k & 1] : nullptr);
+                }
+                if (claimer && k > k0) ts->unit[(k + DEPTH) & 3] = claim(MC_FLAG_WORK);
+                team_sync(bar, nthr);
+                if (!(bits & MC_ER_SLOW)) regen(t, bits, env, true);
+            }
+        }
+    }
+    // the general pass: the envs that the common path left (every env of a
+    // family that has no common path)
+    constexpr bool all = !fast_family(FAM);
+    if (claimer) {
+        ts->sunit[0] = all || *(volatile int32_t*)&rk.flags[MC_FLAG_ANY_SLOW] ? claim(MC_FLAG_SLOW_WORK) : total_units;
+        ts->may_stage[0] = !*(volatile int*)&ts->timed_out;
+        team_unit_reset(ts, 0);
+    }
+    team_sync(bar, nthr);
     for (int k = 0;; ++k) {
-        const int d = k & 1;
-        const unsigned u = ts->unit[d];
+        const unsigned u = ts->sunit[k & 1];
         if (u >= total_units) break;
         const Unit t = locate(u);
-        if (t.stepper) finish(t, d);
-        if (t.coop) team_sync(bar, nthr);
-        // step the next unit and start its copy, then render this one
-        const unsigned u1 = ts->unit[d ^ 1];
-        if (u1 < total_units) prepare(u1, d ^ 1);
         const mc_kp& p = rk.groups[t.g];
-        if (t.coop || t.stepper) {
-            const EnvRender r = t.coop ? ts->r : stash[d];
-            cx.s_u = tables + rk.uv_off[t.g];
-            cx.s_v = cx.s_u + p.W;
-            cx.rcp_vd = N::rcp_of(p.vd);
-            const bool staged = (r.bits & MC_ER_STAGED) != 0;
-            const int8_t* gw = p.voxels + t.e * (long long)p.wx * p.wy * p.wz;
-            if (r.bits & MC_ER_BURIED)
-                fill_env<FAM, F32>(p, t.e, r, cx, t.coop ? wt * 32 + lane : lane, t.coop ? nthr : 32);
-            else
-                render_env<FAM, F32>(p, t.e, r, cx, VoxEither{staged ? slot_world(d, t.coop) : gw, staged},
-                                     rk.tile_w[t.g], lane, t.coop ? &ts->band_ctr : nullptr);
+        const bool may_stage = ((rk.stage_mask >> t.g) & 1) && ts->may_stage[k & 1];  // team-uniform
+        if (may_stage && t.part == 0) issue(t, 0, MC_ER_SLOW);
+        if (claimer) team_unit_reset(ts, (k + 1) & 1);
+        int bits = 0, env = 0;
+        bool here = false;  // this unit's env is rendered in this pass (the first slice's unit renders all of it)
+        if (t.mine) {
+            const EnvRec q = load_rec(recs_of(t.g), t.i);
+            bits = q.bits;
+            env = q.env;
+            here = t.part == 0 && (all || (q.bits & MC_ER_SLOW));
+            use_group(t.g);
+            if (!here) {
+                // another pass's env
+            } else if (q.bits & MC_ER_SLOW) {
+                const int8_t* world = slot_world(0, t.coop);
+                const bool staged = may_stage && landed(t, 0);
+                const int ytop = staged ? staged_top_layer(world, p.wx, p.wy, p.wz, lane) : p.wy - 1;
+                render_slow<FAM, F32>(p, q, ytop, cx, staged ? world : nullptr, rk.tile_w[t.g], lane,
+                                      t.coop ? &ts->band_ctr[k & 1] : nullptr);
+            } else {
+                fill_env<FAM, F32>(p, q.env, q.fill_blk, cx, t.coop ? wt * 32 + lane : lane, t.coop ? nthr : 32);
+            }
         }
-        if (claimer) ts->unit[d] = claim(k + 2);
+        if (claimer) {
+            ts->sunit[(k + 1) & 1] = claim(MC_FLAG_SLOW_WORK);
+            ts->may_stage[(k + 1) & 1] = !*(volatile int*)&ts->timed_out;
+        }
         team_sync(bar, nthr);
+        if (here) regen(t, bits, env, false);
     }
-    // timed-out copies may still be in flight: let them land (bounded)
-    // before this warp's part of shared memory can be released
-    for (int d = 0; d < 2; ++d)
-        if ((pending >> d) & 1u) mbar_wait(mbar0 + 8 * d, (pending_phases >> d) & 1u);
+    // timed-out copies may still be in flight: let them land (bounded) before
+    // this warp's part of shared memory can be released
+    for (int d = 0; d < DEPTH; ++d) {
+        if ((tlive >> d) & 1u) mbar_wait(tmbar + 8 * d, (tphase >> d) & 1u);
+        if ((wlive >> d) & 1u) mbar_wait(cx.mbar_a + 8 * d, (wphase >> d) & 1u);
+    }
     if (lane == 0) {
         for (int g = 0; g < G; ++g) bounds_to_flags(rk.groups[g].flags);
     }
-    if (claimer && rk.sched_dynamic) finish_dynamic(rk.flags, total_teams);
+    if (claimer)
+        finish_dynamic(rk.flags, total_teams, [&] {
+            for (int g = 0; g < G; ++g) rk.groups[g].flags[MC_FLAG_ANY_DONE] = 0;
+        });
 }
 
 // ---------------------------------------------------------------------------
@@ -3442,35 +3264,71 @@ static size_t fused_smem(const mc_kp* p, const mc_fused_cfg* cfg) {
     return (size_t)L.head_bytes + (size_t)cfg->warps_per_cta * L.warp_bytes + (size_t)L.pad_bytes;
 }
 
-template <int FAM, bool F32, int DEPTH>
-static int launch_fused_t(const mc_kp* p, const mc_fused_cfg* cfg, int num_sms, cudaStream_t s) {
-    auto kern = k_step_fused<FAM, F32, DEPTH>;
-    size_t smem = fused_smem(p, cfg);
+// A launch whose kernel waits for its predecessor itself (pdl_wait), so that
+// its own set-up overlaps the predecessor's end.
+template <class... P, class... A>
+static int launch_pdl(void (*kern)(P...), long long grid, int threads, size_t smem, cudaStream_t s, A&&... args) {
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t lc{};
+    lc.gridDim = dim3((unsigned)grid);
+    lc.blockDim = dim3((unsigned)threads);
+    lc.dynamicSmemBytes = smem;
+    lc.stream = s;
+    lc.attrs = &at;
+    lc.numAttrs = 1;
+    return (int)cudaLaunchKernelEx(&lc, kern, std::forward<A>(args)...);
+}
+
+// Row ranges each image of the per-warp kernel is cut into: up to two units
+// per warp of the grid.  Measured at 16^3, 32x32 images, in units per warp
+// (4736 warps): 4096 envs 64.6 us a step at 0.9, 54.9 at 1.7, 61.8 at 3.5 (a
+// slice stages and scans its world again); 32768 envs 163.9 at 6.9, 183.7 at 13.8;
+// 64 envs 34.6 whole, 20.8 in 4 slices.
+static int slices_of(long long B, int bands, long long warps) {
+    int n = 1;
+    while (n * 2 <= bands && B * n * 2 <= 2 * warps) n *= 2;
+    return n;
+}
+
+template <int FAM, bool F32, bool STAGE>
+static int launch_warp_t(const mc_kp* p, const mc_fused_cfg* cfg, int slices, long long grid, cudaStream_t s) {
+    auto kern = k_render_warp<FAM, F32, STAGE>;
+    const size_t smem = fused_smem(p, cfg);
     static size_t attr_set = 0;  // per instantiation
     if (smem > 48 * 1024 && smem > attr_set) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return (int)e;
         attr_set = smem;
     }
-    int threads = 32 * cfg->warps_per_cta;
-    long long ctas_needed = ((long long)p->B + cfg->warps_per_cta - 1) / cfg->warps_per_cta;
-    long long grid = (long long)num_sms * (cfg->ctas_per_sm > 0 ? cfg->ctas_per_sm : 1);
-    if (grid > ctas_needed) grid = ctas_needed;
-    if (grid < 1) grid = 1;
-    kern<<<(unsigned)grid, threads, smem, s>>>(*p, cfg->tile_w);
-    return (int)cudaGetLastError();
+    return launch_pdl(kern, grid, 32 * cfg->warps_per_cta, smem, s, *p, cfg->tile_w, slices);
 }
 
+// The agents, then the images: one warp per env, or per slice of its image.
 template <int FAM, bool F32>
-static int launch_fused_f(const mc_kp* p, const mc_fused_cfg* cfg, int num_sms, cudaStream_t s) {
-    if (cfg->stage == 2) return launch_fused_t<FAM, F32, 2>(p, cfg, num_sms, s);
-    return cfg->stage ? launch_fused_t<FAM, F32, 1>(p, cfg, num_sms, s) : launch_fused_t<FAM, F32, 0>(p, cfg, num_sms, s);
+static int launch_fused_f(const mc_kp* kp, const mc_fused_cfg* cfg, int num_sms, cudaStream_t s) {
+    mc_kp p = *kp;
+    p.fast_ok = mc_fast_launch(p, cfg->stage, cfg->tile_w);
+    const int wpc = cfg->warps_per_cta;
+    long long grid = (long long)num_sms * (cfg->ctas_per_sm > 0 ? cfg->ctas_per_sm : 1);
+    const int slices = p.fast_ok && p.sched_dynamic ? slices_of(p.B, p.H / (32 / cfg->tile_w), grid * wpc) : 1;
+    const long long units = (long long)p.B * slices;
+    p.compact = p.sched_dynamic && units > grid * wpc;
+    grid = std::max(1LL, std::min(grid, (units + wpc - 1) / wpc));
+    const int rc = launch_pdl(k_agent<FAM>, grid_1d(p.B, kAgentThreads), kAgentThreads, 0, s, p);
+    if (rc) return rc;
+    return cfg->stage ? launch_warp_t<FAM, F32, true>(&p, cfg, slices, grid, s)
+                      : launch_warp_t<FAM, F32, false>(&p, cfg, slices, grid, s);
 }
 
 template <int FAM, bool F32>
 static int launch_team_t(const mc_ragged_kp* rk, int warps_per_cta, int ctas_per_sm, int num_sms, cudaStream_t s) {
+    const int G = rk->ngroups;
+    const int rc = launch_pdl(k_agent_groups<FAM>, rk->ablock[G], kAgentThreads, 0, s, *rk);
+    if (rc) return rc;
     const bool deep = rk->depth == 2;
-    auto kern = deep ? k_step_team2<FAM, F32> : k_step_team<FAM, F32>;
+    auto kern = deep ? k_render_team<FAM, F32, 2> : k_render_team<FAM, F32, 1>;
     size_t smem = (size_t)rk->warps_off + (size_t)warps_per_cta * rk->warp_bytes + (size_t)rk->tail_bytes;
     static size_t attr_set[2] = {0, 0};  // per kernel of this instantiation
     if (smem > 48 * 1024 && smem > attr_set[deep]) {
@@ -3483,8 +3341,7 @@ static int launch_team_t(const mc_ragged_kp* rk, int warps_per_cta, int ctas_per
     long long grid = (long long)num_sms * (ctas_per_sm > 0 ? ctas_per_sm : 1);
     if (grid > ctas_needed) grid = ctas_needed;
     if (grid < 1) grid = 1;
-    kern<<<(unsigned)grid, 32 * warps_per_cta, smem, s>>>(*rk);
-    return (int)cudaGetLastError();
+    return launch_pdl(kern, grid, 32 * warps_per_cta, smem, s, *rk);
 }
 
 static int step_team(const mc_ragged_kp* rk, int family, int obs_f32, int warps_per_cta, int ctas_per_sm,

@@ -52,6 +52,7 @@ struct mc_env {
     mc_fused_cfg fcfg;
     int32_t* flags;
     int8_t* tmpl;
+    uint8_t* rec;      // render records of the fused form (MC_REC_BYTES per env)
     uint8_t* scratch;  // plain-form decode buffers
     cudaStream_t cap_stream;
     std::vector<RolloutGraph> graphs;

@@ -18,9 +18,12 @@ enum {
     MC_FLAG_ANY_DONE = 0,    // set by a step when any env is done
     MC_FLAG_REGEN_CTR = 1,   // CTAs of the regeneration kernel that finished
     MC_FLAG_ERROR = 2,       // MC_KERR_* recorded by a kernel
-    MC_FLAG_WORK = 3,        // next env to claim (fused kernel, dynamic schedule)
+    MC_FLAG_WORK = 3,        // next unit to claim (image kernels, dynamic schedule)
     MC_FLAG_WARPS_DONE = 4,  // warps of the fused kernel that finished
-    MC_FLAG_WORDS = 8
+    MC_FLAG_SLOW_WORK = 5,   // next unit to claim in the general pass
+    MC_FLAG_FILED = 6,       // two words, one 64-bit counter: records filed by the agent kernel (marching, buried)
+    MC_FLAG_ANY_SLOW = 8,    // some env of the step needs the general pass
+    MC_FLAG_WORDS = 12
 };
 
 // Error codes a kernel can record in flags[MC_FLAG_ERROR] (never a trap).
@@ -102,11 +105,20 @@ struct mc_kp {
     float* s_speed;
     int32_t* flags;               // MC_FLAG_* words
     const int8_t* world_template; // one generated world (wx*wy*wz bytes)
-    // optional (per-warp fused kernel only): every env's reward and done also
+    // optional (fused form of one env): every env's reward and done also
     // written here, in env order (the host-buffer step's read-back buffer)
     float* res_rewards;
     uint8_t* res_dones;
+    void* rec;    // fused form: the agent kernel's render records, MC_REC_BYTES each
+    int fast_ok;  // fused form: the launch has the images' common path (set per launch)
+    int compact;  // fused form: records filed marching envs first (set per launch)
+    int regen;    // fused form: MC_KREGEN_*, worlds the step's images regenerate (set per launch)
 };
+
+// Worlds regenerated at the end of a fused step.
+enum { MC_KREGEN_NONE = 0, MC_KREGEN_ALL = 1, MC_KREGEN_PER_ENV = 2 };
+
+enum { MC_REC_BYTES = 48 };  // one env's render record (EnvRec)
 
 // Launch shape of the fused step kernel (chosen by the autotuner).
 struct mc_fused_cfg {
@@ -125,13 +137,15 @@ enum { MC_COLOUR_TABLE_BYTES = 224 };  // shared colour tables of the fused kern
 // flat colours: 13 uint32 padded to 64 bytes), after the colour tables
 enum { MC_FAST_TABLE_BYTES = 13 * 4 * 16 + 64 };
 enum { MC_TEAM_HEAD_BYTES = 256 };     // per-team shared words ahead of the team's world buffer
-enum { MC_ENV_STASH_BYTES = 96 };      // one env's render constants, kept in shared memory (depth 2)
+enum { MC_AGENT_THREADS = 128 };       // envs per block of the agent kernels
 struct mc_ragged_kp {
     mc_kp groups[MC_MAX_GROUPS];    // the groups' parameter blocks (kernel parameter space)
     // optional: every env's reward and done flag also written at its global
     // index (one contiguous read-back for a batch of jobs)
     float* rewards_cat;
     uint8_t* dones_cat;
+    void* rec;                           // render records of all groups, in group order (MC_REC_BYTES each)
+    int ablock[MC_MAX_GROUPS + 1];       // first block of each group in the agent kernel
     // actions of all groups, concatenated in group order: discrete actions, or buttons + look
     const uint8_t* actions;
     const int8_t* buttons;
@@ -147,6 +161,7 @@ struct mc_ragged_kp {
     int coop_mask;                  // bit g: a whole team renders each env of group g
     int stage_mask;                 // bit g: group g's worlds are bulk-copied into shared memory
     int tile_w[MC_MAX_GROUPS];
+    int slices[MC_MAX_GROUPS];      // row ranges each image of a cooperative group is cut into (units per env)
     int uv_off[MC_MAX_GROUPS];      // float offset of each group's u table (v follows)
     int sched_dynamic;              // 1: teams claim units from flags[MC_FLAG_WORK]
     // shared-memory layout (bytes): colour tables at 0, then
@@ -156,10 +171,22 @@ struct mc_ragged_kp {
     int depth;                      // staging depth: 0 none, 1 one world buffer per stepper, 2 two (the
                                     // next unit's world is copied while the current one renders)
     int world_stride;               // bytes of one depth slot of a team's world region
-    int warp_bytes;                 // 16 (two mbarriers) + 128 (march start values) [+ depth 2: two env
-                                    // stashes] + one band of observation bytes
+    int warp_bytes;                 // 16 (two mbarriers) + 128 (march start values) + one band of observation bytes
     int tail_bytes;                 // allocated after the warps: the march may read one world layer past the last world
 };
+
+// Whether a launch that stages its worlds (stage) has the images' common path
+// for this env's configuration: a family with a common-case loop, no debug
+// output, worlds within the marches' 64-voxel counts, and images of whole
+// tile_w x (32 / tile_w) tiles whose bands are whole 16-byte pieces.
+static inline int mc_fast_launch(const mc_kp& k, int stage, int tile_w) {
+    const int bpp = 3 * (k.obs_f32 ? 4 : 1), th = 32 / tile_w;
+    if (!(k.family == MC_FAM_SHADED || k.family == MC_FAM_MINIMAL || k.family == MC_FAM_PREBASIS)) return 0;
+    if (!stage || k.dbg_pixel || k.max_steps <= 0 || k.wx > 64 || k.wy > 64 || k.wz > 64) return 0;
+    if (k.family == MC_FAM_SHADED && !(k.vd > 0.0f)) return 0;
+    if (k.W % tile_w || k.H % th || ((k.W * th * bpp) & 15) || (((uintptr_t)k.obs) & 15)) return 0;
+    return 1;
+}
 
 // One numerics back end (ref_fast or ieee).
 struct mc_backend {
@@ -192,11 +219,6 @@ extern "C" const mc_backend* mc_backend_ieee();
 int mc_launch_reset_agents(const mc_kp* p, const uint8_t* mask, cudaStream_t s);
 int mc_launch_regen(const mc_kp* p, int conditional, cudaStream_t s);
 int mc_launch_regen_if(const mc_kp* p, const uint8_t* flag, cudaStream_t s);
-// The conditional regeneration of up to MC_MAX_GROUPS groups in one launch
-// (groups that cannot end an episode are skipped; no launch when none can);
-// ctr is a counter word no other launch uses concurrently.
-int mc_launch_regen_groups(const mc_kp* const* kps, int G, int32_t* ctr, cudaStream_t s);
-
 // Record an error message for mc_last_error() and return `code`.
 int mc_set_error(int code, const char* msg);
 // mc_step_stateless with the flag words supplied by the caller (no lazy

@@ -297,88 +297,6 @@ int mc_launch_regen(const mc_kp* p, int conditional, cudaStream_t s) {
     return (int)cudaGetLastError();
 }
 
-// The conditional regeneration of several env groups in one launch (a
-// ragged step, a server launch): each group whose any-done flag its step set
-// gets its worlds back (every world under the all-world rule, the worlds of
-// its done envs under the per-env rule), as mc_launch_regen would for that
-// group alone; one launch instead of one per group.
-namespace {
-struct RegenGroups {
-    int8_t* vox[MC_MAX_GROUPS];
-    const int8_t* tmpl[MC_MAX_GROUPS];
-    const uint8_t* do_reset[MC_MAX_GROUPS];
-    int32_t* flags[MC_MAX_GROUPS];
-    int B[MC_MAX_GROUPS];
-    int wxyz[MC_MAX_GROUPS];
-    int per_env[MC_MAX_GROUPS];
-    int G;
-    int32_t* ctr;  // finished CTAs of the launch (cleared by the last one)
-};
-
-__global__ void k_regen_groups(const __grid_constant__ RegenGroups rg) {
-    __shared__ int go[MC_MAX_GROUPS];
-    __shared__ int any;
-    if (threadIdx.x == 0) any = 0;
-    __syncthreads();
-    if (threadIdx.x < rg.G) {
-        go[threadIdx.x] = *(volatile int32_t*)&rg.flags[threadIdx.x][MC_FLAG_ANY_DONE] != 0;
-        if (go[threadIdx.x]) atomicOr(&any, 1);
-    }
-    __syncthreads();
-    // The flags were set before this launch and only its last CTA clears
-    // them: every CTA reads the same values, so when none is set none of them
-    // has anything to write, count or clear.
-    if (!any) return;
-    for (int g = 0; g < rg.G; ++g) {
-        if (!go[g]) continue;
-        const int wxyz = rg.wxyz[g];
-        const bool vec = (wxyz & 15) == 0 && ((((uintptr_t)rg.vox[g]) | ((uintptr_t)rg.tmpl[g])) & 15) == 0;
-        for (long long b = blockIdx.x; b < rg.B[g]; b += gridDim.x) {
-            if (rg.per_env[g] && !rg.do_reset[g][b]) continue;  // the same for every thread of the CTA
-            int8_t* d = rg.vox[g] + b * (long long)wxyz;
-            if (vec) {
-                uint4* d4 = reinterpret_cast<uint4*>(d);
-                const uint4* t4 = reinterpret_cast<const uint4*>(rg.tmpl[g]);
-                for (int k = threadIdx.x; k < (wxyz >> 4); k += blockDim.x) d4[k] = __ldg(t4 + k);
-            } else {
-                for (int k = threadIdx.x; k < wxyz; k += blockDim.x) d[k] = rg.tmpl[g][k];
-            }
-        }
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        __threadfence();
-        const unsigned prev = atomicAdd(reinterpret_cast<unsigned*>(rg.ctr), 1u);
-        if (prev == gridDim.x - 1) {
-            for (int g = 0; g < rg.G; ++g)
-                if (go[g]) rg.flags[g][MC_FLAG_ANY_DONE] = 0;
-            *rg.ctr = 0;
-            __threadfence();
-        }
-    }
-}
-}  // namespace
-
-int mc_launch_regen_groups(const mc_kp* const* kps, int G, int32_t* ctr, cudaStream_t s) {
-    RegenGroups rg{};
-    for (int g = 0; g < G; ++g) {
-        const mc_kp& k = *kps[g];
-        if (k.B == 0 || !dones_possible(k)) continue;
-        const int i = rg.G++;
-        rg.vox[i] = k.voxels;
-        rg.tmpl[i] = k.world_template;
-        rg.do_reset[i] = k.do_reset;
-        rg.flags[i] = k.flags;
-        rg.B[i] = k.B;
-        rg.wxyz[i] = k.wx * k.wy * k.wz;
-        rg.per_env[i] = k.regen_per_env;
-    }
-    if (rg.G == 0) return 0;
-    rg.ctr = ctr;
-    k_regen_groups<<<1184, 256, 0, s>>>(rg);  // 148 SMs x 8
-    return (int)cudaGetLastError();
-}
-
 namespace {
 __global__ void k_flag_from_byte(int32_t* flags, const uint8_t* flag) {
     flags[MC_FLAG_ANY_DONE] = *flag ? 1 : 0;
@@ -532,6 +450,12 @@ bool dones_possible(const mc_kp& k) {
     return k.episode_length > 0;
 }
 
+// Worlds that a fused step of these parameters regenerates (MC_KREGEN_*).
+static int step_regen(const mc_kp& k) {
+    if (!dones_possible(k)) return MC_KREGEN_NONE;
+    return k.regen_per_env ? MC_KREGEN_PER_ENV : MC_KREGEN_ALL;
+}
+
 static inline int align16i(long long x) { return (int)((x + 15) & ~15LL); }
 
 void team_layout(const mc_kp* const* kps, int G, const int* stage, const int* tile_w, const int* coop,
@@ -547,6 +471,9 @@ void team_layout(const mc_kp* const* kps, int G, const int* stage, const int* ti
         const mc_kp& k = *kps[g];
         const long long wxyz = (long long)k.wx * k.wy * k.wz;
         rk->groups[g] = k;
+        rk->groups[g].fast_ok = mc_fast_launch(k, stage[g], tile_w[g]);
+        rk->groups[g].regen = step_regen(k);
+        rk->slices[g] = 1;
         rk->start[g] = start;
         start += k.B;
         rk->uv_off[g] = uv;
@@ -573,13 +500,32 @@ void team_layout(const mc_kp* const* kps, int G, const int* stage, const int* ti
         return (double)k.W * k.H * (k.wx + k.wy + k.wz);
     };
     std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return cost(a) > cost(b); });
+    // few envs: the images of cooperative groups are cut into row ranges, each a
+    // unit of its own, until the units fill a grid's teams (every range keeps a
+    // band per warp of its team)
+    long long units = 0;
+    for (int g = 0; g < G; ++g) units += coop[g] ? kps[g]->B : (kps[g]->B + team_warps - 1) / team_warps;
+    for (bool more = true; more;) {
+        more = false;
+        for (int g = 0; g < G; ++g) {
+            const int bands = kps[g]->H / (32 / tile_w[g]);
+            const long long add = (long long)kps[g]->B * rk->slices[g];
+            if (!coop[g] || !rk->groups[g].fast_ok || add == 0 || units + add > 888 ||
+                rk->slices[g] * 2 * team_warps > bands)
+                continue;
+            units += add;
+            rk->slices[g] *= 2;
+            more = true;
+        }
+    }
     rk->ustart[0] = 0;
     for (int v = 0; v < G; ++v) {
         const int g = order[v];
         rk->order[v] = g;
         const long long B = kps[g]->B;
-        rk->ustart[v + 1] = rk->ustart[v] + (coop[g] ? B : (B + team_warps - 1) / team_warps);
+        rk->ustart[v + 1] = rk->ustart[v] + (coop[g] ? B * rk->slices[g] : (B + team_warps - 1) / team_warps);
     }
+    for (int g = 0; g < G; ++g) rk->groups[g].compact = rk->ustart[G] > 512;  // more units than a grid's teams
     rk->slot_bytes = slot;
     rk->tables_off = MC_COLOUR_TABLE_BYTES + MC_FAST_TABLE_BYTES;
     rk->teams_off = rk->tables_off + align16i((long long)uv * 4);
@@ -591,8 +537,10 @@ void team_layout(const mc_kp* const* kps, int G, const int* stage, const int* ti
     rk->world_stride = std::max(coop_world, team_warps * slot);
     rk->team_bytes = MC_TEAM_HEAD_BYTES + std::max(depth, 1) * rk->world_stride;
     rk->warps_off = rk->teams_off + (warps_per_cta / team_warps) * rk->team_bytes;
-    // per warp: two mbarriers, a table of march start values, [depth 2: two env stashes], one band
-    rk->warp_bytes = 16 + 128 + (depth == 2 ? 2 * MC_ENV_STASH_BYTES : 0) + band;
+    rk->ablock[0] = 0;
+    for (int g = 0; g < G; ++g) rk->ablock[g + 1] = rk->ablock[g] + (kps[g]->B + MC_AGENT_THREADS - 1) / MC_AGENT_THREADS;
+    // per warp: two mbarriers, a table of march start values, one band
+    rk->warp_bytes = 16 + 128 + band;
     const int after = warps_per_cta * rk->warp_bytes;
     rk->tail_bytes = after < pad ? pad - after : 0;
 }
@@ -760,6 +708,7 @@ extern "C" int mc_env_create(const mc_env_config* cfg, const mc_env_state* state
     if (ce == cudaSuccess) ce = cudaMalloc(&e->flags, MC_FLAG_WORDS * sizeof(int32_t));
     if (ce == cudaSuccess) ce = cudaMemset(e->flags, 0, MC_FLAG_WORDS * sizeof(int32_t));
     if (ce == cudaSuccess) ce = cudaMalloc(&e->tmpl, (size_t)((wxyz + 15) & ~15LL));
+    if (ce == cudaSuccess) ce = cudaMalloc(&e->rec, (size_t)cfg->batch_size * MC_REC_BYTES + 16);
     if (ce == cudaSuccess) ce = cudaStreamCreateWithFlags(&e->cap_stream, cudaStreamNonBlocking);
     if (ce == cudaSuccess) {
         // the template world: generate + tree + house on one env
@@ -780,6 +729,7 @@ extern "C" int mc_env_create(const mc_env_config* cfg, const mc_env_state* state
     }
     e->kp.flags = e->flags;
     e->kp.world_template = e->tmpl;
+    e->kp.rec = e->rec;
     e->kp.sched_dynamic = 1;  // the handle's flag block is used by one launch at a time
     default_fused(e);
     *out = e;
@@ -815,6 +765,7 @@ extern "C" int mc_env_destroy(mc_env* e) {
     drop_graphs(e);
     if (e->flags) cudaFree(e->flags);
     if (e->tmpl) cudaFree(e->tmpl);
+    if (e->rec) cudaFree(e->rec);
     if (e->scratch) cudaFree(e->scratch);
     if (e->cap_stream) cudaStreamDestroy(e->cap_stream);
     delete e;
@@ -832,6 +783,7 @@ extern "C" int mc_env_set_state(mc_env* e, const mc_env_state* s) {
     fill_kp(&e->kp, &e->cfg, s);
     e->kp.flags = flags;
     e->kp.world_template = tmpl;
+    e->kp.rec = e->rec;
     e->kp.wait_polls = polls;
     e->kp.regen_per_env = e->regen_mode == MC_REGEN_PER_ENV;
     e->kp.sched_dynamic = 1;
@@ -883,9 +835,9 @@ extern "C" int mc_env_reset(mc_env* e, const uint8_t* mask, void* stream) {
     return render_obs(e, s);
 }
 
-// res_rewards / res_dones: where the per-warp fused kernel also writes every
-// env's reward and done (the host-buffer step's read-back buffer); the other
-// launch forms ignore them.
+// res_rewards / res_dones: where the fused form's agent kernel also writes
+// every env's reward and done (the host-buffer step's read-back buffer); the
+// plain form ignores them.
 static int do_step(mc_env* e, const int8_t* buttons, const float* look, const uint8_t* actions, int form,
                    cudaStream_t s, float* res_rewards = nullptr, uint8_t* res_dones = nullptr) {
     if (e->cfg.batch_size == 0) return MC_OK;
@@ -908,6 +860,9 @@ static int do_step(mc_env* e, const int8_t* buttons, const float* look, const ui
         mc_ragged_kp rk;
         team_layout(kps, 1, &f.stage, &f.tile_w, &f.coop, f.team_warps, f.warps_per_cta, &rk);
         rk.flags = e->flags;
+        rk.rec = e->rec;
+        rk.rewards_cat = res_rewards;
+        rk.dones_cat = res_dones;
         rk.actions = actions;
         rk.buttons = buttons;
         rk.look = look;
@@ -916,12 +871,14 @@ static int do_step(mc_env* e, const int8_t* buttons, const float* look, const ui
     } else if (form == MC_FORM_FUSED) {
         k.res_rewards = res_rewards;
         k.res_dones = res_dones;
+        k.regen = step_regen(k);
         rc = backend_rc(e->be->step_fused(&k, &e->fcfg, e->num_sms, s), "step_fused");
     } else {
         return fail(MC_ERR_INVALID, "unknown form %d", form);
     }
     if (rc) return rc;
-    if (dones_possible(k)) return backend_rc(mc_launch_regen(&k, 1, s), "regen");
+    // the fused forms' images regenerate the worlds themselves
+    if (form == MC_FORM_PLAIN && dones_possible(k)) return backend_rc(mc_launch_regen(&k, 1, s), "regen");
     return MC_OK;
 }
 
@@ -1019,10 +976,10 @@ extern "C" int mc_env_step_host(mc_env* e, const uint8_t* host_actions, float* h
     rc = hostio_upload(h, i, host_actions, B, s);
     if (rc) return rc;
     // results go into this call's buffer once the read-back two calls back
-    // is done with it; the per-warp fused kernel writes them there itself,
-    // the other forms through a copy kernel after the step
+    // is done with it; the fused form writes them there itself, the plain
+    // form through a copy kernel after the step
     MC_CK(cudaStreamWaitEvent(s, h->res_free[i], 0));
-    const bool direct = form == MC_FORM_FUSED && !team_mode(e->fcfg);
+    const bool direct = form == MC_FORM_FUSED;
     float* res_rew = reinterpret_cast<float*>(h->d_res[i]);
     uint8_t* res_done = h->d_res[i] + 4 * B;
     rc = do_step(e, nullptr, nullptr, h->d_act[i], form, s, direct ? res_rew : nullptr, direct ? res_done : nullptr);
@@ -1251,6 +1208,7 @@ struct mc_ragged {
     mc_ragged_config cfg{};
     std::vector<mc_kp> uploaded;  // group parameter blocks the cached graphs were captured with
     int32_t* flags = nullptr;     // the launch's work counter
+    uint8_t* rec = nullptr;       // render records of every env
     mc_ragged_kp rk{};
     long long version = 1;
     cudaStream_t cap_stream = nullptr;
@@ -1272,6 +1230,7 @@ static void ragged_layout(const mc_ragged* r, const mc_ragged_config* c, mc_ragg
     ragged_kps(r, &kps);
     team_layout(kps.data(), (int)kps.size(), c->stage, c->tile_w, c->coop, c->team_warps, c->warps_per_cta, rk);
     rk->flags = r->flags;
+    rk->rec = r->rec;
 }
 
 static int ragged_validate(const mc_ragged* r, const mc_ragged_config* c) {
@@ -1350,6 +1309,7 @@ extern "C" int mc_ragged_create(mc_env* const* groups, int32_t ngroups, mc_ragge
     r->num_sms = groups[0]->num_sms;
     cudaError_t ce = cudaMalloc(&r->flags, MC_FLAG_WORDS * sizeof(int32_t));
     if (ce == cudaSuccess) ce = cudaMemset(r->flags, 0, MC_FLAG_WORDS * sizeof(int32_t));
+    if (ce == cudaSuccess) ce = cudaMalloc(&r->rec, (size_t)total * MC_REC_BYTES + 16);
     if (ce == cudaSuccess) ce = cudaStreamCreateWithFlags(&r->cap_stream, cudaStreamNonBlocking);
     if (ce != cudaSuccess) {
         int rc = cuda_fail(ce, "mc_ragged_create");
@@ -1370,6 +1330,7 @@ extern "C" int mc_ragged_destroy(mc_ragged* r) {
     hostio_close(&r->hio);
     ragged_drop_graphs(r);
     if (r->flags) cudaFree(r->flags);
+    if (r->rec) cudaFree(r->rec);
     if (r->cap_stream) cudaStreamDestroy(r->cap_stream);
     delete r;
     return MC_OK;
@@ -1417,14 +1378,9 @@ static int ragged_do_step(mc_ragged* r, const int8_t* buttons, const float* look
     rk.actions = actions;
     rk.buttons = buttons;
     rk.look = look;
-    rc = backend_rc(r->be->step_team(&rk, r->family, r->obs_f32, r->cfg.warps_per_cta, r->cfg.ctas_per_sm,
-                                     r->num_sms, s),
-                    "step_team");
-    if (rc) return rc;
-    std::vector<const mc_kp*> kps;
-    for (auto* e : r->envs) kps.push_back(&e->kp);
-    return backend_rc(mc_launch_regen_groups(kps.data(), (int)kps.size(), r->flags + MC_FLAG_REGEN_CTR, s),
-                      "regen");
+    return backend_rc(r->be->step_team(&rk, r->family, r->obs_f32, r->cfg.warps_per_cta, r->cfg.ctas_per_sm,
+                                       r->num_sms, s),
+                      "step_team");
 }
 
 extern "C" int mc_ragged_step(mc_ragged* r, const int8_t* buttons, const float* look, void* stream) {
@@ -1707,7 +1663,11 @@ extern "C" int mc_step_stateless(const mc_env_config* cfg, const mc_env_state* s
         f.tile_w = 4;
         f.team_warps = 1;
         f.coop = 0;
-        return backend_rc(be->step_fused(&k, &f, sms, (cudaStream_t)stream), "step_fused");
+        // the render records live for this call only (stream-ordered, so calls on other streams have their own)
+        MC_CK(cudaMallocAsync(&k.rec, (size_t)k.B * MC_REC_BYTES, (cudaStream_t)stream));
+        rc = backend_rc(be->step_fused(&k, &f, sms, (cudaStream_t)stream), "step_fused");
+        MC_CK(cudaFreeAsync(k.rec, (cudaStream_t)stream));
+        return rc;
     }
     return fail(MC_ERR_INVALID, "unknown form %d", form);
 }

@@ -191,6 +191,7 @@ struct mc_server {
     cudaStream_t stream = nullptr, admit_stream = nullptr;
     cudaStream_t up = nullptr, down = nullptr;  // actions uploads, results read-backs
     int32_t* flags = nullptr;  // work counter of the team launches
+    uint8_t* rec = nullptr;    // render records of one team launch (cap envs)
     Slot slots[kMaxSlots];
     int nslots = 0;
     std::deque<int> flight;  // busy slots in launch order
@@ -368,14 +369,13 @@ int run_round(mc_server* s, Slot& sl, const std::vector<Req*>& reqs, const std::
             mc_ragged_kp rk;
             team_layout(kps.data(), G, stage, tile_w, coop, team, 8, &rk);
             rk.flags = s->flags;
+            rk.rec = s->rec;
             rk.actions = d_act;
             rk.rewards_cat = d_rew;
             rk.dones_cat = d_done;
             const mc_kp& k0 = *kps[0];
             rc = s->be->step_team(&rk, k0.family, k0.obs_f32, 8, cps, s->num_sms, st);
             if (rc) return mc_cuda_fail((cudaError_t)rc, "server: step launch");
-            rc = mc_launch_regen_groups(kps.data(), G, s->flags + MC_FLAG_REGEN_CTR, st);
-            if (rc) return mc_cuda_fail((cudaError_t)rc, "server: regeneration");
         } else {
             Req* r = reqs[steps[0]];
             rc = mc_env_step_discrete(r->job->env, d_act, MC_FORM_PLAIN, st);
@@ -603,6 +603,7 @@ extern "C" int mc_server_create(const mc_server_config* cfg, mc_server** out) {
     if (ce == cudaSuccess) ce = cudaStreamCreateWithFlags(&s->down, cudaStreamNonBlocking);
     if (ce == cudaSuccess) ce = cudaMalloc(&s->flags, MC_FLAG_WORDS * sizeof(int32_t));
     if (ce == cudaSuccess) ce = cudaMemset(s->flags, 0, MC_FLAG_WORDS * sizeof(int32_t));
+    if (ce == cudaSuccess) ce = cudaMalloc(&s->rec, (size_t)s->cap * MC_REC_BYTES + 16);
     for (int i = 0; i < s->nslots && ce == cudaSuccess; ++i) {
         Slot& sl = s->slots[i];
         ce = cudaEventCreateWithFlags(&sl.ev, cudaEventDisableTiming);
@@ -663,6 +664,7 @@ extern "C" int mc_server_destroy(mc_server* s) {
         if (sl.d_res) cudaFree(sl.d_res);
     }
     if (s->flags) cudaFree(s->flags);
+    if (s->rec) cudaFree(s->rec);
     if (s->stream) cudaStreamDestroy(s->stream);
     if (s->up) cudaStreamDestroy(s->up);
     if (s->down) cudaStreamDestroy(s->down);
