@@ -2272,6 +2272,26 @@ __device__ __forceinline__ EnvRec agent_step(const mc_kp& p, const ActionSrc& ac
     return r;
 }
 
+// ---- regeneration -----------------------------------------------------------
+// The step's regeneration is done by whoever rendered the env last: its world
+// is not read again in this step, so the template's bytes go over it right
+// after its image, with no pass over all worlds and no kernel of its own.
+// Which worlds (p.regen): none, all of them when any env of the group is done
+// (MC_KREGEN_ALL; the agent kernel has settled that), or the done envs' own.
+__device__ __forceinline__ int regen_any(const mc_kp& p) {
+    return p.regen == MC_KREGEN_ALL
+               ? __shfl_sync(0xffffffffu, *(volatile int32_t*)&p.flags[MC_FLAG_ANY_DONE], 0) : 0;
+}
+__device__ __forceinline__ bool regen_env(const mc_kp& p, int bits, int any_done) {
+    return any_done || (p.regen == MC_KREGEN_PER_ENV && (bits & MC_ER_DONE));
+}
+// The world an env's image shows: its own, or the template where a reset (not
+// a step: `fresh`) regenerates it in this launch.
+__device__ __forceinline__ const int8_t* world_of(const mc_kp& p, int e, int bits, int any_done) {
+    return p.fresh && regen_env(p, bits, any_done) ? p.world_template
+                                                   : p.voxels + e * (long long)p.wx * p.wy * p.wz;
+}
+
 constexpr int kAgentThreads = MC_AGENT_THREADS;
 
 // File the block's records (called by all its threads): record e at e, or,
@@ -2282,13 +2302,13 @@ constexpr int kAgentThreads = MC_AGENT_THREADS;
 // the block that brings their sum to the group's size clears it for the next
 // launch (every env is filed exactly once, so no other block adds after it).
 __device__ __forceinline__ void file_recs(void* rec, int32_t* flags, int32_t* any_slow, long long B, bool compact,
-                                          const EnvRec& r, long long e, bool valid) {
+                                          const EnvRec& r, long long e, bool valid, bool step = true) {
     __shared__ unsigned s_m[kAgentThreads / 32], s_b[kAgentThreads / 32];
     __shared__ unsigned long long s_base;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const bool march = valid && !(r.bits & (MC_ER_BURIED | MC_ER_SLOW)), fill = valid && !march;
     if (valid && (r.bits & MC_ER_SLOW)) *any_slow = 1;
-    const unsigned done = __ballot_sync(0xffffffffu, valid && (r.bits & MC_ER_DONE));
+    const unsigned done = __ballot_sync(0xffffffffu, step && valid && (r.bits & MC_ER_DONE));
     if (done && lane == 0) atomicOr(&flags[MC_FLAG_ANY_DONE], 1);
     if (!compact) {
         if (valid) store_rec(rec, e, r);
@@ -2340,7 +2360,41 @@ __global__ void __launch_bounds__(kAgentThreads) k_agent(const __grid_constant__
     if (threadIdx.x == 0) bounds_to_flags(p.flags);
 }
 
-// The same for the groups of a ragged launch: blocks ablock[g] .. ablock[g+1]-1 hold group g's envs.
+// Cameras and records without a step (reset, get_obs: always the shaded
+// family), one thread per env.  An env whose world this launch regenerates
+// (fresh) looks into the template.
+__global__ void __launch_bounds__(kAgentThreads) k_look(const __grid_constant__ mc_kp p) {
+    pdl_trigger();
+    pdl_wait();
+    const long long e = (long long)blockIdx.x * kAgentThreads + threadIdx.x;
+    const bool valid = e < p.B;
+    const int any_done = regen_any(p);
+    EnvRec r{};
+    if (valid) {
+        const float x = p.positions[e * 3 + 0], y = p.positions[e * 3 + 1], z = p.positions[e * 3 + 2];
+        const float yaw = p.yaws[e], pitch = p.pitches[e];
+        const bool done = p.regen != MC_KREGEN_NONE && p.do_reset[e] != 0;
+        p.cameras[e * 5 + 0] = x;
+        p.cameras[e * 5 + 1] = y;
+        p.cameras[e * 5 + 2] = z;
+        p.cameras[e * 5 + 3] = yaw;
+        p.cameras[e * 5 + 4] = pitch;
+        r.env = (int)e;
+        r.ex = x;
+        r.ey = N::add(y, 1.6f);
+        r.ez = z;
+        rec_trig<MC_FAM_SHADED>(r, yaw, pitch);
+        const long long wxyz = (long long)p.wx * p.wy * p.wz;
+        const int eye = eye_index(r, p);
+        int eye_blk = AIR;
+        if (eye >= 0 && in_bounds(eye, wxyz, MC_SITE_EYE)) eye_blk = world_of(p, (int)e, done ? MC_ER_DONE : 0, any_done)[eye];
+        rec_facts<MC_FAM_SHADED>(r, p, eye >= 0, eye_blk, done);
+    }
+    file_recs(p.rec, p.flags, &p.flags[MC_FLAG_ANY_SLOW], p.B, p.compact, r, e, valid, false);
+    if (threadIdx.x == 0) bounds_to_flags(p.flags);
+}
+
+// The same as k_agent for the groups of a ragged launch: blocks ablock[g] .. ablock[g+1]-1 hold group g's envs.
 template <int FAM>
 __global__ void __launch_bounds__(kAgentThreads) k_agent_groups(const __grid_constant__ mc_ragged_kp rk) {
     pdl_trigger();
@@ -2608,14 +2662,14 @@ __device__ __forceinline__ void render_slow_from(const mc_kp& p, int e, const En
 
 template <int FAM, bool F32>
 __device__ __forceinline__ void render_slow(const mc_kp& p, const EnvRec& q, int ytop, const FusedCtx& cx,
-                                            const int8_t* staged, int tile_w, int lane, int* band_ctr) {
+                                            const int8_t* staged, const int8_t* world, int tile_w, int lane,
+                                            int* band_ctr) {
     EnvRender r = render_of_rec(q, p.wy);
     r.ytop = ytop;
     if (staged)
         render_slow_from<FAM, F32>(p, q.env, r, cx, VoxShared{staged}, tile_w, lane, band_ctr);
     else
-        render_slow_from<FAM, F32>(p, q.env, r, cx, VoxGlobal{p.voxels + q.env * (long long)p.wx * p.wy * p.wz},
-                                   tile_w, lane, band_ctr);
+        render_slow_from<FAM, F32>(p, q.env, r, cx, VoxGlobal{world}, tile_w, lane, band_ctr);
 }
 
 // Whether a family has the common-case loop (fast_band).
@@ -2658,20 +2712,7 @@ __device__ __forceinline__ void render_fast(const mc_kp& p, int e, const EnvRend
     }
 }
 
-// ---- regeneration -----------------------------------------------------------
-// The step's regeneration is done by whoever rendered the env last: its world
-// is not read again in this step, so the template's bytes go over it right
-// after its image, with no pass over all worlds and no kernel of its own.
-// Which worlds (p.regen): none, all of them when any env of the group is done
-// (MC_KREGEN_ALL; the agent kernel has settled that), or the done envs' own.
-__device__ __forceinline__ int regen_any(const mc_kp& p, int lane) {
-    (void)lane;
-    return p.regen == MC_KREGEN_ALL
-               ? __shfl_sync(0xffffffffu, *(volatile int32_t*)&p.flags[MC_FLAG_ANY_DONE], 0) : 0;
-}
-__device__ __forceinline__ bool regen_env(const mc_kp& p, int bits, int any_done) {
-    return any_done || (p.regen == MC_KREGEN_PER_ENV && (bits & MC_ER_DONE));
-}
+// The template's bytes over env e's world, by nt threads.
 __device__ __forceinline__ void regen_world(const mc_kp& p, int e, int t, int nt) {
     const int wxyz = p.wx * p.wy * p.wz;
     int8_t* d = p.voxels + e * (long long)wxyz;
@@ -2747,7 +2788,7 @@ __global__ void __launch_bounds__(256, MC_FUSED_MIN_BLOCKS)
     const int total_warps = gridDim.x * nwarps;
     const EnvRec* recs = reinterpret_cast<const EnvRec*>(p.rec);
     const int first = blockIdx.x * nwarps + warp;
-    const int any_done = regen_any(p, lane);
+    const int any_done = regen_any(p);
     if constexpr (STAGE && fast_family(FAM)) {
         const int units = p.B * slices;
         int u = p.sched_dynamic ? next_unit(p, MC_FLAG_WORK, 0, total_warps, lane) : first;
@@ -2762,7 +2803,7 @@ __global__ void __launch_bounds__(256, MC_FUSED_MIN_BLOCKS)
                     no_stage = true;
                     break;
                 }
-                issue_world_copy(cx.mbar_a, sworld, p.voxels + q.env * (long long)wxyz, wxyz, lane);
+                issue_world_copy(cx.mbar_a, sworld, world_of(p, q.env, q.bits, any_done), wxyz, lane);
                 EnvRender r = render_of_rec(q, p.wy);
                 if (!mbar_wait(cx.mbar_a, phase, p.wait_polls)) {
                     if (lane == 0) atomicExch(&p.flags[MC_FLAG_ERROR], MC_KERR_TMA_TIMEOUT);
@@ -2783,7 +2824,8 @@ __global__ void __launch_bounds__(256, MC_FUSED_MIN_BLOCKS)
             const EnvRec q = load_rec(recs, i);
             if (q.bits & MC_ER_SLOW) continue;
             if (!(q.bits & MC_ER_BURIED))
-                render_slow<FAM, F32>(p, q, p.wy - 1, cx, nullptr, tile_w, lane, nullptr);
+                render_slow<FAM, F32>(p, q, p.wy - 1, cx, nullptr, world_of(p, q.env, q.bits, any_done), tile_w, lane,
+                                      nullptr);
             else if (part == 0)
                 fill_env<FAM, F32>(p, q.env, q.fill_blk, cx, lane, 32);
             if (regen_env(p, q.bits, any_done) && last_slice(recs, i, slices, lane)) regen_world(p, q.env, lane, 32);
@@ -2801,10 +2843,11 @@ __global__ void __launch_bounds__(256, MC_FUSED_MIN_BLOCKS)
             if (q.bits & MC_ER_BURIED) {
                 fill_env<FAM, F32>(p, q.env, q.fill_blk, cx, lane, 32);
             } else {
+                const int8_t* world = world_of(p, q.env, q.bits, any_done);
                 bool staged = STAGE && !no_stage && stage_fits(sworld, wxyz);
                 int ytop = p.wy - 1;
                 if (staged) {
-                    issue_world_copy(cx.mbar_a, sworld, p.voxels + q.env * (long long)wxyz, wxyz, lane);
+                    issue_world_copy(cx.mbar_a, sworld, world, wxyz, lane);
                     if (mbar_wait(cx.mbar_a, phase, p.wait_polls)) {
                         phase ^= 1u;
                         EnvRender r = render_of_rec(q, p.wy);
@@ -2816,7 +2859,7 @@ __global__ void __launch_bounds__(256, MC_FUSED_MIN_BLOCKS)
                         staged = false;
                     }
                 }
-                render_slow<FAM, F32>(p, q, ytop, cx, staged ? sworld : nullptr, tile_w, lane, nullptr);
+                render_slow<FAM, F32>(p, q, ytop, cx, staged ? sworld : nullptr, world, tile_w, lane, nullptr);
             }
             if (regen_env(p, q.bits, any_done)) regen_world(p, q.env, lane, 32);
         }
@@ -3029,7 +3072,8 @@ __global__ void __launch_bounds__(256, MC_TEAM_MIN_BLOCKS) k_render_team(const _
         const int wxyz = p.wx * p.wy * p.wz;
         int8_t* world = slot_world(d, t.coop);
         if (!stage_fits(world, wxyz)) return;
-        issue_world_copy((t.coop ? tmbar : cx.mbar_a) + 8 * d, world, p.voxels + q.env * (long long)wxyz, wxyz, lane);
+        issue_world_copy((t.coop ? tmbar : cx.mbar_a) + 8 * d, world,
+                         world_of(p, q.env, q.bits, (ts->any_done >> t.g) & 1), wxyz, lane);
         if (t.coop) tlive |= 1u << d;
         else wlive |= 1u << d;
     };
@@ -3140,8 +3184,9 @@ __global__ void __launch_bounds__(256, MC_TEAM_MIN_BLOCKS) k_render_team(const _
                     if (q.bits & MC_ER_BURIED)
                         fill_env<FAM, F32>(p, q.env, q.fill_blk, cx, t.coop ? wt * 32 + lane : lane, t.coop ? nthr : 32);
                     else if (!(q.bits & MC_ER_SLOW))
-                        render_slow<FAM, F32>(p, q, p.wy - 1, cx, nullptr, rk.tile_w[t.g], lane,
-                                              t.coop ? &ts->band_ctr[k & 1] : nullptr);
+                        render_slow<FAM, F32>(p, q, p.wy - 1, cx, nullptr,
+                                              world_of(p, q.env, q.bits, (ts->any_done >> t.g) & 1), rk.tile_w[t.g],
+                                              lane, t.coop ? &ts->band_ctr[k & 1] : nullptr);
                 }
                 if (claimer && k > k0) ts->unit[(k + DEPTH) & 3] = claim(MC_FLAG_WORK);
                 team_sync(bar, nthr);
@@ -3180,7 +3225,8 @@ __global__ void __launch_bounds__(256, MC_TEAM_MIN_BLOCKS) k_render_team(const _
                 const int8_t* world = slot_world(0, t.coop);
                 const bool staged = may_stage && landed(t, 0);
                 const int ytop = staged ? staged_top_layer(world, p.wx, p.wy, p.wz, lane) : p.wy - 1;
-                render_slow<FAM, F32>(p, q, ytop, cx, staged ? world : nullptr, rk.tile_w[t.g], lane,
+                render_slow<FAM, F32>(p, q, ytop, cx, staged ? world : nullptr,
+                                      world_of(p, q.env, q.bits, (ts->any_done >> t.g) & 1), rk.tile_w[t.g], lane,
                                       t.coop ? &ts->band_ctr[k & 1] : nullptr);
             } else {
                 fill_env<FAM, F32>(p, q.env, q.fill_blk, cx, t.coop ? wt * 32 + lane : lane, t.coop ? nthr : 32);
@@ -3316,7 +3362,11 @@ static int launch_fused_f(const mc_kp* kp, const mc_fused_cfg* cfg, int num_sms,
     const long long units = (long long)p.B * slices;
     p.compact = p.sched_dynamic && units > grid * wpc;
     grid = std::max(1LL, std::min(grid, (units + wpc - 1) / wpc));
-    const int rc = launch_pdl(k_agent<FAM>, grid_1d(p.B, kAgentThreads), kAgentThreads, 0, s, p);
+    int rc;
+    if (FAM == MC_FAM_SHADED && p.look_only)
+        rc = launch_pdl(k_look, grid_1d(p.B, kAgentThreads), kAgentThreads, 0, s, p);
+    else
+        rc = launch_pdl(k_agent<FAM>, grid_1d(p.B, kAgentThreads), kAgentThreads, 0, s, p);
     if (rc) return rc;
     return cfg->stage ? launch_warp_t<FAM, F32, true>(&p, cfg, slices, grid, s)
                       : launch_warp_t<FAM, F32, false>(&p, cfg, slices, grid, s);
@@ -3325,7 +3375,11 @@ static int launch_fused_f(const mc_kp* kp, const mc_fused_cfg* cfg, int num_sms,
 template <int FAM, bool F32>
 static int launch_team_t(const mc_ragged_kp* rk, int warps_per_cta, int ctas_per_sm, int num_sms, cudaStream_t s) {
     const int G = rk->ngroups;
-    const int rc = launch_pdl(k_agent_groups<FAM>, rk->ablock[G], kAgentThreads, 0, s, *rk);
+    int rc;
+    if (FAM == MC_FAM_SHADED && rk->groups[0].look_only)  // one group
+        rc = launch_pdl(k_look, rk->ablock[G], kAgentThreads, 0, s, rk->groups[0]);
+    else
+        rc = launch_pdl(k_agent_groups<FAM>, rk->ablock[G], kAgentThreads, 0, s, *rk);
     if (rc) return rc;
     const bool deep = rk->depth == 2;
     auto kern = deep ? k_render_team<FAM, F32, 2> : k_render_team<FAM, F32, 1>;

@@ -112,10 +112,12 @@ struct mc_kp {
     void* rec;    // fused form: the agent kernel's render records, MC_REC_BYTES each
     int fast_ok;  // fused form: the launch has the images' common path (set per launch)
     int compact;  // fused form: records filed marching envs first (set per launch)
-    int regen;    // fused form: MC_KREGEN_*, worlds the step's images regenerate (set per launch)
+    int regen;    // fused form: MC_KREGEN_*, worlds the launch's images regenerate (set per launch)
+    int fresh;    // ... and show regenerated (a reset; a step's images show the worlds before it)
+    int look_only;  // fused form: images without a step (reset, get_obs)
 };
 
-// Worlds regenerated at the end of a fused step.
+// Worlds that a fused launch regenerates.
 enum { MC_KREGEN_NONE = 0, MC_KREGEN_ALL = 1, MC_KREGEN_PER_ENV = 2 };
 
 enum { MC_REC_BYTES = 48 };  // one env's render record (EnvRec)

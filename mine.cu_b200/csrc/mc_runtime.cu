@@ -224,17 +224,6 @@ __global__ void k_reset_agents(float* pos, float* vel, float* yaw, float* pitch,
     og[i] = 0;
 }
 
-// update_cameras_kernel (kernels.cu:2320-2335)
-__global__ void k_cameras_rt(mc_kp p) {
-    long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= p.B) return;
-    p.cameras[i * 5 + 0] = p.positions[i * 3 + 0];
-    p.cameras[i * 5 + 1] = p.positions[i * 3 + 1];
-    p.cameras[i * 5 + 2] = p.positions[i * 3 + 2];
-    p.cameras[i * 5 + 3] = p.yaws[i];
-    p.cameras[i * 5 + 4] = p.pitches[i];
-}
-
 __global__ void k_philox(uint8_t* actions, int B, int K, int env_offset, int step0, uint64_t seed, int break_half) {
     long long n = (long long)B * K;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
@@ -813,14 +802,39 @@ extern "C" int mc_env_generate_world(mc_env* e, void* stream) {
     return backend_rc(mc_launch_regen(&e->kp, 0, (cudaStream_t)stream), "regen");
 }
 
-static int render_obs(mc_env* e, cudaStream_t s) {
+// One launch of the fused form over the env's batch: k holds what differs
+// from e->kp (actions, result buffers, regeneration, family).
+static int launch_fused(mc_env* e, const mc_kp& k, cudaStream_t s, const char* what) {
+    const mc_fused_cfg& f = e->fcfg;
+    if (!team_mode(f)) return backend_rc(e->be->step_fused(&k, &f, e->num_sms, s), what);
+    const mc_kp* kps[1] = {&k};
+    mc_ragged_kp rk;
+    team_layout(kps, 1, &f.stage, &f.tile_w, &f.coop, f.team_warps, f.warps_per_cta, &rk);
+    rk.groups[0].regen = k.regen;
+    rk.flags = e->flags;
+    rk.rec = e->rec;
+    rk.rewards_cat = k.res_rewards;
+    rk.dones_cat = k.res_dones;
+    rk.actions = k.actions;
+    rk.buttons = k.buttons;
+    rk.look = k.look;
+    return backend_rc(e->be->step_team(&rk, k.family, k.obs_f32, f.warps_per_cta, f.ctas_per_sm, e->num_sms, s), what);
+}
+
+// Cameras and images without a step; regen: the worlds regenerated first.
+// MineEnv._render always uses the shaded kernel: float32 for "float32",
+// render_uint8 for every uint8 mode (minecu/__init__.py:455-464).  The images
+// come from the step's image kernels: at 4096 envs, 16^3, 64x64 a step, a
+// masked reset and the policy's input take 233 us, with the per-pixel kernel
+// 448.
+static int render_obs(mc_env* e, cudaStream_t s, int regen) {
     mc_kp k = e->kp;
     if (k.B == 0) return MC_OK;
-    k_cameras_rt<<<blocks(k.B, 256), 256, 0, s>>>(k);
-    MC_CK(cudaGetLastError());
-    // MineEnv._render always uses the shaded kernel: float32 for "float32",
-    // render_uint8 for every uint8 mode (minecu/__init__.py:455-464).
-    return backend_rc(e->be->render(&k, MC_FAM_SHADED, s), "render");
+    k.family = MC_FAM_SHADED;
+    k.look_only = 1;
+    k.regen = regen;
+    k.fresh = 1;
+    return launch_fused(e, k, s, "render");
 }
 
 extern "C" int mc_env_reset(mc_env* e, const uint8_t* mask, void* stream) {
@@ -830,9 +844,7 @@ extern "C" int mc_env_reset(mc_env* e, const uint8_t* mask, void* stream) {
     if (e->cfg.batch_size == 0) return MC_OK;
     int rc = backend_rc(mc_launch_reset_agents(&e->kp, mask, s), "reset");
     if (rc) return rc;
-    rc = backend_rc(mc_launch_regen(&e->kp, 1, s), "regen");
-    if (rc) return rc;
-    return render_obs(e, s);
+    return render_obs(e, s, e->kp.regen_per_env ? MC_KREGEN_PER_ENV : MC_KREGEN_ALL);
 }
 
 // res_rewards / res_dones: where the fused form's agent kernel also writes
@@ -854,25 +866,11 @@ static int do_step(mc_env* e, const int8_t* buttons, const float* look, const ui
         k.look = look;
         k.actions = actions;
         rc = backend_rc(e->be->step_plain(&k, s), "step_plain");
-    } else if (form == MC_FORM_FUSED && team_mode(e->fcfg)) {
-        const mc_fused_cfg& f = e->fcfg;
-        const mc_kp* kps[1] = {&e->kp};
-        mc_ragged_kp rk;
-        team_layout(kps, 1, &f.stage, &f.tile_w, &f.coop, f.team_warps, f.warps_per_cta, &rk);
-        rk.flags = e->flags;
-        rk.rec = e->rec;
-        rk.rewards_cat = res_rewards;
-        rk.dones_cat = res_dones;
-        rk.actions = actions;
-        rk.buttons = buttons;
-        rk.look = look;
-        rc = backend_rc(e->be->step_team(&rk, k.family, k.obs_f32, f.warps_per_cta, f.ctas_per_sm, e->num_sms, s),
-                        "step_team");
     } else if (form == MC_FORM_FUSED) {
         k.res_rewards = res_rewards;
         k.res_dones = res_dones;
         k.regen = step_regen(k);
-        rc = backend_rc(e->be->step_fused(&k, &e->fcfg, e->num_sms, s), "step_fused");
+        rc = launch_fused(e, k, s, "step_fused");
     } else {
         return fail(MC_ERR_INVALID, "unknown form %d", form);
     }
@@ -1029,7 +1027,7 @@ extern "C" int mc_env_regenerate_if(mc_env* e, const uint8_t* flag, void* stream
 extern "C" int mc_env_render(mc_env* e, void* stream) {
     NvtxRange nvtx("mc_env_render");
     if (!e) return fail(MC_ERR_INVALID, "env is NULL");
-    return render_obs(e, (cudaStream_t)stream);
+    return render_obs(e, (cudaStream_t)stream, MC_KREGEN_NONE);
 }
 
 static bool same_fcfg(const mc_fused_cfg& a, const mc_fused_cfg& b) {

@@ -1,0 +1,74 @@
+"""The fused form's agent and image kernels at the edges of their dispatch,
+against the CPU oracle (ieee numerics, no tolerance): batches around the agent
+kernel's block size, images cut into slices, more units than the grid has
+warps (records filed marching envs first), worlds regenerated by the image
+warps under both rules, and the images of resets, which come from the same
+kernels."""
+import numpy as np
+import pytest
+
+from minecu import capi
+import oracle as O
+from mc_harness import GpuEnv, actions_for, diff_report, oracle_state
+
+pytestmark = pytest.mark.gpu
+
+
+def run(cuda, B, steps, seed, world=(16, 16, 16), res=(32, 32), regen="all", cfg=None, reset_every=3, break_half=True,
+        **kw):
+    g = GpuEnv(cuda, B, world_x=world[0], world_y=world[1], world_z=world[2], render_width=res[0],
+               render_height=res[1], debug=False, **kw)
+    if cfg:
+        g.set_fused(*cfg)
+    if regen != "all":
+        g.set_regen(True)
+    o = O.OracleEnv(batch_size=B, world_x=world[0], world_y=world[1], world_z=world[2], render_width=res[0],
+                    render_height=res[1], regen=regen, **kw)
+    g.reset()
+    o.reset()
+    rng = np.random.default_rng(seed)
+
+    def same(what):
+        d = diff_report(g.state(), oracle_state(o))
+        assert not d, f"{what}: {d}"
+
+    same("reset")
+    for s in range(steps):
+        _, btn, look = actions_for(B, s, seed, 0.1, break_half)
+        btn[:, 6] = rng.random(B) < 0.1
+        g.step(btn, look, capi.FORM_FUSED)
+        o.step(btn, look)
+        same(f"step {s}")
+        if reset_every and s % reset_every == reset_every - 1:
+            mask = rng.random(B) < (0.3 if B > 1 else 1.0)
+            g.reset(mask)
+            o.reset(mask)
+            same(f"masked reset after step {s}")
+    g.check_error()
+    g.close()
+
+
+@pytest.mark.parametrize("regen", ["all", "per_env"])
+@pytest.mark.parametrize("B", [1, 2, 127, 128, 129, 300])
+def test_batch_edges(cuda, B, regen):
+    run(cuda, B, 12, 40 + B, regen=regen, obs_dtype="uint8", episode_length=5)
+
+
+@pytest.mark.parametrize("mode", ["float32", "uint8_minimal", "uint8_prebasis_full", "uint8_fp16", "uint8_fast"])
+def test_reset_images_of_every_mode(cuda, mode):
+    run(cuda, 33, 9, 51, obs_dtype=mode, episode_length=4)
+    run(cuda, 5, 4, 52, world=(32, 32, 32), res=(64, 64), obs_dtype=mode, episode_length=3, regen="per_env")
+
+
+@pytest.mark.parametrize("regen", ["all", "per_env"])
+def test_records_filed_by_cost(cuda, regen):
+    """More units than warps: marching envs from the front, buried ones from the back."""
+    run(cuda, 10007, 16, 53, res=(8, 8), regen=regen, obs_dtype="uint8", episode_length=13, reset_every=7)
+
+
+@pytest.mark.parametrize("cfg", [(1, 8, 3, 8, 4, 1), (2, 8, 2, 8, 4, 1), (1, 8, 3, 16, 8, 1), (1, 8, 3, 8, 2, 0)],
+                         ids=["team", "team_depth2", "team8", "per_warp_groups"])
+@pytest.mark.parametrize("regen", ["all", "per_env"])
+def test_team_images(cuda, cfg, regen):
+    run(cuda, 3, 8, 54, res=(64, 64), regen=regen, cfg=cfg, obs_dtype="uint8", episode_length=4)
+    run(cuda, 41, 8, 55, world=(32, 16, 32), res=(32, 32), regen=regen, cfg=cfg, obs_dtype="uint8", episode_length=4)
