@@ -1652,7 +1652,7 @@ __host__ __device__ inline FusedLayout fused_layout(int W, int H, int wxyz, int 
     L.H = H;
     L.tile_w = tile_w;
     L.tile_h = 32 / tile_w;
-    L.stage_bytes = mc_align16(W * L.tile_h * 3 * (obs_f32 ? 4 : 1));
+    L.stage_bytes = mc_band_bytes(W, H, obs_f32, tile_w);
     L.world_bytes = stage ? mc_align16(wxyz) : 0;
     L.warp_bytes = 16 + 128 + L.stage_bytes + L.world_bytes;  // 16: mbarrier, 128: packed_start table
     L.head_bytes = kFastTableBytes + mc_align16((W + H) * 4 + 13 * 3 * 4 + 16 + 13 * 3 + 3);
@@ -1959,9 +1959,8 @@ __device__ __forceinline__ UpBounds staged_up_bounds(const int8_t* world, int wx
 // The common-case render of one band of an env's image (both step
 // kernels): the world is staged, the eye is inside the box with air in its
 // voxel (every ray starts one DDA step in, and ends as sky when it leaves
-// the box), no debug output is asked for, and the image is a whole number of
-// tile_w x (32/tile_w) tiles.  Every ray's march start values come from a
-// per-env table of the eight ray sign combinations (packed_start for the
+// the box) and no debug output is asked for.  Every ray's march start values
+// come from a per-env table of the eight ray sign combinations (packed_start for the
 // packed march, split_start for the split march).  Every per-env fact is
 // settled before the loop, so the per-ray code has no branch but the
 // march's: the same operations in the same order as shade_ray / flat_ray
@@ -1970,6 +1969,11 @@ __device__ __forceinline__ UpBounds staged_up_bounds(const int8_t* world, int wx
 // shade read from s_cs (built with the same N::mul), and the band address
 // stepped incrementally.  The band goes to `stage`, then to `dst` with
 // 16-byte stores.
+// ODD: the image is no whole number of tile_w x (32/tile_w) tiles, or its
+// bands no whole 16-byte pieces: lanes beyond the image march the nearest
+// pixel's ray again and store nothing, and the band is staged at dst's offset
+// from a 16-byte boundary, so that all but its first and last bytes still go
+// out in 16-byte stores (`stage` has 16 bytes to spare).
 struct FastEnv {
     const int4* start;  // per sign combination: packed (index|counts, dx, dy, dz) or split (counts, dax, day, daz)
     uint32_t base;      // staged world (packed) / the eye voxel's address in it (split)
@@ -1977,9 +1981,9 @@ struct FastEnv {
     float vd, rcp_vd;
 };
 
-template <int FAM, bool F32, bool SPLIT>
-__device__ __forceinline__ void fast_band(const Cam& c, const Dda0& d0, const FastEnv& fe, int W, int TW, int row0,
-                                          int lane, const float* s_u, const float* s_v, const float4* s_cs,
+template <int FAM, bool F32, bool SPLIT, bool ODD>
+__device__ __forceinline__ void fast_band(const Cam& c, const Dda0& d0, const FastEnv& fe, int W, int H, int TW,
+                                          int row0, int lane, const float* s_u, const float* s_v, const float4* s_cs,
                                           const uint32_t* s_rgbp, uint8_t* stage, uint8_t* dst) {
     constexpr bool SHADED = FAM == MC_FAM_SHADED;
     constexpr bool TRIG = FAM != MC_FAM_PREBASIS;
@@ -1988,11 +1992,14 @@ __device__ __forceinline__ void fast_band(const Cam& c, const Dda0& d0, const Fa
     const float sky0 = 0.53f, sky1 = 0.81f, sky2 = 0.92f;  // SKY_COLOR (c_sky)
     const int TH = 32 / TW;
     const int lx = lane % TW, ly = lane / TW;
-    const float v = s_v[row0 + ly];
+    const bool in_y = !ODD || row0 + ly < H;
+    const float v = s_v[ODD ? min(row0 + ly, H - 1) : row0 + ly];
     const float yraw = N::mad(v, c.uy, c.fy);
+    if (ODD) stage += (uint32_t)(uintptr_t)dst & 15u;
     uint8_t* sp = stage + (ly * W + lx) * bpp;
     for (int tx0 = 0; tx0 < W; tx0 += TW, sp += TW * bpp) {
-        const float u = s_u[tx0 + lx];
+        const bool in = !ODD || (in_y && tx0 + lx < W);
+        const float u = s_u[ODD ? min(tx0 + lx, W - 1) : tx0 + lx];
         float x, y = yraw, z;
         if (TRIG) {
             x = N::mad(v, c.ux, N::mad(c.sy, c.cp, N::mul(u, c.rx)));
@@ -2040,7 +2047,8 @@ __device__ __forceinline__ void fast_band(const Cam& c, const Dda0& d0, const Fa
             const float c1 = (m & 2) ? N::mad(sky1, fog, N::mul(cs.y, omf)) : N::mad(cs.y, omf, N::mul(sky1, fog));
             const float c2 = (m & 4) ? N::mad(sky2, fog, N::mul(cs.z, omf)) : N::mad(cs.z, omf, N::mul(sky2, fog));
             const float o0 = hit ? c0 : sky0, o1 = hit ? c1 : sky1, o2 = hit ? c2 : sky2;
-            if (F32) {
+            if (ODD && !in) {
+            } else if (F32) {
                 float* sf = reinterpret_cast<float*>(sp);
                 sf[0] = o0;
                 sf[1] = o1;
@@ -2053,16 +2061,29 @@ __device__ __forceinline__ void fast_band(const Cam& c, const Dda0& d0, const Fa
         } else {
             // SKY_COLOR_U8 (135, 206, 235) packed
             const uint32_t col = b >= 0 ? s_rgbp[b] : (135u | (206u << 8) | (235u << 16));
-            sp[0] = (uint8_t)col;
-            sp[1] = (uint8_t)(col >> 8);
-            sp[2] = (uint8_t)(col >> 16);
+            if (in) {
+                sp[0] = (uint8_t)col;
+                sp[1] = (uint8_t)(col >> 8);
+                sp[2] = (uint8_t)(col >> 16);
+            }
         }
     }
     __syncwarp();
     // copy the band (rows row0 .. row0+TH-1) out with 16-byte stores
+    int bytes = W * TH * bpp;
+    if (ODD) {
+        bytes = W * min(TH, H - row0) * bpp;
+        const int head = min((int)(-(uint32_t)(uintptr_t)dst & 15u), bytes);
+        const int tail = (bytes - head) & 15;
+        if (lane < head) dst[lane] = stage[lane];
+        if (lane < tail) dst[bytes - tail + lane] = stage[bytes - tail + lane];
+        stage += head;
+        dst += head;
+        bytes -= head + tail;
+    }
     const uint4* s4 = reinterpret_cast<const uint4*>(stage);
     uint4* d4 = reinterpret_cast<uint4*>(dst);
-    for (int k = lane; k < ((W * TH * bpp) >> 4); k += 32) d4[k] = s4[k];
+    for (int k = lane; k < (bytes >> 4); k += 32) d4[k] = s4[k];
     __syncwarp();
 }
 
@@ -2586,7 +2607,7 @@ __device__ __forceinline__ int next_band(int* band_ctr, int prev, int lane) {
 
 // The general path, a pixel's ray at a time as in the reference's kernels:
 // worlds that are not staged, debug outputs, eyes outside the box or out of
-// view, families without a fast march, images that are no whole tiles.
+// view, families without a fast march.
 template <int FAM, bool F32, class V>
 __device__ __forceinline__ void render_slow_from(const mc_kp& p, int e, const EnvRender& r, const FusedCtx& cx,
                                                  const V& vox, int tile_w, int lane, int* band_ctr) {
@@ -2699,16 +2720,25 @@ __device__ __forceinline__ void render_fast(const mc_kp& p, int e, const EnvRend
     fe.chk = staged_range(wb, wxz, wxz * p.wy);
     fe.vd = p.vd;
     fe.rcp_vd = N::rcp_of(p.vd);
-    const int nb = p.H / TH, b0 = part * nb / slices, nbands = (part + 1) * nb / slices - b0;
+    const int H = p.H, nb = (H + TH - 1) / TH, b0 = part * nb / slices, nbands = (part + 1) * nb / slices - b0;
+    const bool odd = p.fast_ok == 2;
     for (int b = next_band(band_ctr, -1, lane); b < nbands; b = next_band(band_ctr, b, lane)) {
         const int row0 = (b0 + b) * TH;
         uint8_t* dst = oenv + row0 * W * bpp;
-        if (fk == 1)
-            fast_band<FAM, F32, false>(r.c, d0, fe, W, TW, row0, lane, cx.s_u, cx.s_v, cx.s_cs, cx.s_rgbp, cx.stage,
-                                       dst);
-        else
-            fast_band<FAM, F32, true>(r.c, d0, fe, W, TW, row0, lane, cx.s_u, cx.s_v, cx.s_cs, cx.s_rgbp, cx.stage,
-                                      dst);
+        if (odd) {
+            if (fk == 1)
+                fast_band<FAM, F32, false, true>(r.c, d0, fe, W, H, TW, row0, lane, cx.s_u, cx.s_v, cx.s_cs,
+                                                 cx.s_rgbp, cx.stage, dst);
+            else
+                fast_band<FAM, F32, true, true>(r.c, d0, fe, W, H, TW, row0, lane, cx.s_u, cx.s_v, cx.s_cs,
+                                                cx.s_rgbp, cx.stage, dst);
+        } else if (fk == 1) {
+            fast_band<FAM, F32, false, false>(r.c, d0, fe, W, H, TW, row0, lane, cx.s_u, cx.s_v, cx.s_cs, cx.s_rgbp,
+                                              cx.stage, dst);
+        } else {
+            fast_band<FAM, F32, true, false>(r.c, d0, fe, W, H, TW, row0, lane, cx.s_u, cx.s_v, cx.s_cs, cx.s_rgbp,
+                                             cx.stage, dst);
+        }
     }
 }
 
@@ -3358,7 +3388,7 @@ static int launch_fused_f(const mc_kp* kp, const mc_fused_cfg* cfg, int num_sms,
     p.fast_ok = mc_fast_launch(p, cfg->stage, cfg->tile_w);
     const int wpc = cfg->warps_per_cta;
     long long grid = (long long)num_sms * (cfg->ctas_per_sm > 0 ? cfg->ctas_per_sm : 1);
-    const int slices = p.fast_ok && p.sched_dynamic ? slices_of(p.B, p.H / (32 / cfg->tile_w), grid * wpc) : 1;
+    const int slices = p.fast_ok && p.sched_dynamic ? slices_of(p.B, (p.H * cfg->tile_w + 31) / 32, grid * wpc) : 1;
     const long long units = (long long)p.B * slices;
     p.compact = p.sched_dynamic && units > grid * wpc;
     grid = std::max(1LL, std::min(grid, (units + wpc - 1) / wpc));

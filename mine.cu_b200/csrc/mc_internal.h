@@ -177,17 +177,35 @@ struct mc_ragged_kp {
     int tail_bytes;                 // allocated after the warps: the march may read one world layer past the last world
 };
 
+// Whether images are whole tile_w x (32 / tile_w) tiles whose bands (the rows
+// of one tile) are whole 16-byte pieces.
+#ifdef __CUDACC__
+__host__ __device__
+#endif
+static inline int mc_whole_tiles(int W, int H, int obs_f32, int tile_w) {
+    const int th = 32 / tile_w;
+    return W % tile_w == 0 && H % th == 0 && (W * th * (obs_f32 ? 12 : 3)) % 16 == 0;
+}
+// Shared-memory bytes of one staged band: 16 to spare where bands start at any byte.
+#ifdef __CUDACC__
+__host__ __device__
+#endif
+static inline int mc_band_bytes(int W, int H, int obs_f32, int tile_w) {
+    const int n = W * (32 / tile_w) * (obs_f32 ? 12 : 3);
+    return ((n + 15) & ~15) + (mc_whole_tiles(W, H, obs_f32, tile_w) ? 0 : 16);
+}
+
 // Whether a launch that stages its worlds (stage) has the images' common path
 // for this env's configuration: a family with a common-case loop, no debug
-// output, worlds within the marches' 64-voxel counts, and images of whole
-// tile_w x (32 / tile_w) tiles whose bands are whole 16-byte pieces.
+// output, worlds within the marches' 64-voxel counts.  1: images of whole
+// tiles in 16-byte pieces; 2: any others (fast_band<ODD>).
 static inline int mc_fast_launch(const mc_kp& k, int stage, int tile_w) {
-    const int bpp = 3 * (k.obs_f32 ? 4 : 1), th = 32 / tile_w;
     if (!(k.family == MC_FAM_SHADED || k.family == MC_FAM_MINIMAL || k.family == MC_FAM_PREBASIS)) return 0;
     if (!stage || k.dbg_pixel || k.max_steps <= 0 || k.wx > 64 || k.wy > 64 || k.wz > 64) return 0;
     if (k.family == MC_FAM_SHADED && !(k.vd > 0.0f)) return 0;
-    if (k.W % tile_w || k.H % th || ((k.W * th * bpp) & 15) || (((uintptr_t)k.obs) & 15)) return 0;
-    return 1;
+    if (k.obs_f32 && (((uintptr_t)k.obs) & 3)) return 0;
+    if (!mc_whole_tiles(k.W, k.H, k.obs_f32, tile_w)) return 2;
+    return (((uintptr_t)k.obs) & 15) ? 0 : 1;
 }
 
 // One numerics back end (ref_fast or ieee).

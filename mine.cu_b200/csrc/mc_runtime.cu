@@ -453,7 +453,6 @@ void team_layout(const mc_kp* const* kps, int G, const int* stage, const int* ti
     rk->ngroups = G;
     rk->team_warps = team_warps;
     rk->sched_dynamic = 1;
-    const int bpp = 3 * (kps[0]->obs_f32 ? 4 : 1);
     long long start = 0;
     int uv = 0, band = 16, coop_world = 0, slot = 0, pad = 0, depth = 0;
     for (int g = 0; g < G; ++g) {
@@ -468,7 +467,7 @@ void team_layout(const mc_kp* const* kps, int G, const int* stage, const int* ti
         rk->uv_off[g] = uv;
         uv += k.W + k.H;
         rk->tile_w[g] = tile_w[g];
-        band = std::max(band, align16i((long long)k.W * (32 / tile_w[g]) * bpp));
+        band = std::max(band, mc_band_bytes(k.W, k.H, k.obs_f32, tile_w[g]));
         if (coop[g]) rk->coop_mask |= 1 << g;
         if (stage[g]) {
             rk->stage_mask |= 1 << g;
@@ -497,7 +496,7 @@ void team_layout(const mc_kp* const* kps, int G, const int* stage, const int* ti
     for (bool more = true; more;) {
         more = false;
         for (int g = 0; g < G; ++g) {
-            const int bands = kps[g]->H / (32 / tile_w[g]);
+            const int bands = (kps[g]->H * tile_w[g] + 31) / 32;
             const long long add = (long long)kps[g]->B * rk->slices[g];
             if (!coop[g] || !rk->groups[g].fast_ok || add == 0 || units + add > 888 ||
                 rk->slices[g] * 2 * team_warps > bands)

@@ -72,3 +72,12 @@ def test_records_filed_by_cost(cuda, regen):
 def test_team_images(cuda, cfg, regen):
     run(cuda, 3, 8, 54, res=(64, 64), regen=regen, cfg=cfg, obs_dtype="uint8", episode_length=4)
     run(cuda, 41, 8, 55, world=(32, 16, 32), res=(32, 32), regen=regen, cfg=cfg, obs_dtype="uint8", episode_length=4)
+
+
+@pytest.mark.parametrize("res", [(1, 1), (7, 5), (31, 33), (84, 84), (17, 64), (40, 9)])
+@pytest.mark.parametrize("cfg", [(1, 8, 4, 4, 1, 0), (1, 8, 3, 8, 4, 1), (1, 8, 2, 32, 2, 0)],
+                         ids=["per_warp", "team", "per_warp_groups"])
+def test_odd_images(cuda, res, cfg):
+    """Images that are no whole tiles, whose rows and envs start at any byte."""
+    for mode in ("uint8", "float32", "uint8_prebasis"):
+        run(cuda, 5, 6, 56, res=res, cfg=cfg, obs_dtype=mode, episode_length=4)
