@@ -1630,7 +1630,7 @@ struct FusedLayout {
     int W, H;
     int tile_w, tile_h;
     int stage_bytes;   // staging bytes per warp (one band of rows)
-    int world_bytes;   // world bytes per warp (0 when not staged)
+    int world_bytes;   // world bytes per warp (mc_world_slot; 0 when not staged)
     int warp_bytes;    // total per warp (16-aligned)
     int head_bytes;    // tables (16-aligned)
     int pad_bytes;     // allocated after the last warp's world
@@ -1645,7 +1645,7 @@ constexpr int kShadeTableBytes = 13 * 4 * 16;
 constexpr int kFastTableBytes = MC_FAST_TABLE_BYTES;
 static_assert(kFastTableBytes == kShadeTableBytes + 64, "fast tables");
 
-__host__ __device__ inline FusedLayout fused_layout(int W, int H, int wxyz, int wxz, int obs_f32, int stage,
+__host__ __device__ inline FusedLayout fused_layout(int W, int H, int slot, int wxz, int obs_f32, int stage,
                                                    int tile_w) {
     FusedLayout L;
     L.W = W;
@@ -1653,7 +1653,7 @@ __host__ __device__ inline FusedLayout fused_layout(int W, int H, int wxyz, int 
     L.tile_w = tile_w;
     L.tile_h = 32 / tile_w;
     L.stage_bytes = mc_band_bytes(W, H, obs_f32, tile_w);
-    L.world_bytes = stage ? mc_align16(wxyz) : 0;
+    L.world_bytes = stage ? slot : 0;
     L.warp_bytes = 16 + 128 + L.stage_bytes + L.world_bytes;  // 16: mbarrier, 128: packed_start table
     L.head_bytes = kFastTableBytes + mc_align16((W + H) * 4 + 13 * 3 * 4 + 16 + 13 * 3 + 3);
     // the march reads up to wx*wz bytes on either side of a staged world:
@@ -1824,11 +1824,11 @@ __device__ __forceinline__ void finish_dynamic(int32_t* flags, long long total, 
 }
 
 // Highest layer of a staged world holding a solid voxel (solid = byte >= 0,
-// sign bit clear), found by one warp; -1 for an empty world; wy - 1 when the
-// layer size is not a multiple of 16 bytes (not measured).
+// sign bit clear), found by one warp; -1 for an empty world; wy - 1 when its
+// layers are no whole aligned 16-byte chunks (not measured).
 __device__ __forceinline__ int staged_top_layer(const int8_t* world, int wx, int wy, int wz, int lane) {
     const int layer = wx * wz;
-    if (layer & 15) return wy - 1;
+    if ((layer | (int)smem_u32(world)) & 15) return wy - 1;
     const uint4* w4 = reinterpret_cast<const uint4*>(world);
     const int n16 = (layer * wy) >> 4, per_layer = layer >> 4;
     int top = -1;
@@ -1850,10 +1850,32 @@ __device__ __forceinline__ uint32_t solid_mask16(uint4 q) {
     return four(q.x) | (four(q.y) << 4) | (four(q.z) << 8) | (four(q.w) << 12);
 }
 
-// Whether staged_up_bounds can scan a world of this shape: whole 16-byte
-// chunks per row of z, at most 64 voxels a side.
+// Whether staged_up_bounds can scan a world of this shape: at most 64 voxels a side.
 __host__ __device__ __forceinline__ bool up_scan_shape(int wx, int wy, int wz) {
-    return (wz & 15) == 0 && wz <= 64 && wx <= 64 && wy <= 64;
+    return wz <= 64 && wx <= 64 && wy <= 64;
+}
+
+// Solid voxels of one row of wz bytes as a mask: 16 bytes a load when rows are
+// whole 16-byte chunks (`chunks`, uniform), else word by word, each funnelled
+// from the two aligned words it lies in (the last one reads up to 7 bytes past
+// the row; a staged world has at least one layer allocated after it).
+template <typename M>
+__device__ __forceinline__ M row_mask(const int8_t* row, int wz, bool chunks) {
+    M m = 0;
+    if (chunks) {
+        const uint4* q = reinterpret_cast<const uint4*>(row);
+        for (int k = 0; k < (wz >> 4); ++k) m |= M(solid_mask16(q[k])) << (16 * k);
+        return m;
+    }
+    const uint32_t off = smem_u32(row) & 3u;
+    const uint32_t* w = reinterpret_cast<const uint32_t*>(row - off);
+    uint32_t lo = w[0];
+    for (int k = 0; 4 * k < wz; ++k) {
+        const uint32_t hi = w[k + 1], q = __funnelshift_r(lo, hi, 8 * off);
+        m |= M(((~q & 0x80808080u) * 0x00204081u) >> 28) << (4 * k);
+        lo = hi;
+    }
+    return wz < (int)(8 * sizeof(M)) ? m & ((M(1) << wz) - 1) : m;
 }
 
 // One warp scans the rows (y >= vy, x) of a staged world (up_scan_shape;
@@ -1875,7 +1897,7 @@ struct UpPart {
 template <typename M>
 __device__ __forceinline__ UpPart<M> staged_up_part(const int8_t* world, int wx, int wy, int wz, int vx, int vy,
                                                     int vz, int lane, int w = 0, int nw = 1) {
-    const int cpr = wz >> 4;                              // 16-byte chunks per row
+    const bool chunks = ((wz | (int)smem_u32(world)) & 15) == 0;
     constexpr int kBits = 8 * sizeof(M);
     const M zpm = ~M(0) << vz;                            // z >= vz
     const M zmm = (vz + 1 < kBits) ? ((M(1) << (vz + 1)) - 1) : ~M(0);  // z <= vz
@@ -1888,13 +1910,7 @@ __device__ __forceinline__ UpPart<M> staged_up_part(const int8_t* world, int wx,
         int yp = 0, ym = 0;  // highest layer + 1 with a solid voxel at z >= vz / z <= vz
         for (int y = vy + w * G + g; y < wy; y += G * nw) {
             const int r = y * wx + x;
-            const uint4* row = reinterpret_cast<const uint4*>(world + r * wz);
-            M m = 0;
-            for (int k = 0; k < cpr; ++k) {
-                const uint4 q = in_bounds((long long)r * cpr + k, (long long)wx * wy * cpr, MC_SITE_SCAN)
-                                    ? row[k] : make_uint4(~0u, ~0u, ~0u, ~0u);
-                m |= M(solid_mask16(q)) << (16 * k);
-            }
+            const M m = in_bounds(r, (long long)wx * wy, MC_SITE_SCAN) ? row_mask<M>(world + r * wz, wz, chunks) : M(0);
             mu |= m;
             yp = (m & zpm) ? y + 1 : yp;
             ym = (m & zmm) ? y + 1 : ym;
@@ -2488,17 +2504,36 @@ __device__ __forceinline__ void team_sync(int bar, int nthreads) {
 }
 
 
-// Start the bulk copy of one world into shared memory (lane 0 issues it).
-__device__ __forceinline__ void issue_world_copy(uint32_t mbar_a, int8_t* dst, const int8_t* src, int bytes, int lane) {
+// Where the staged copy of the world at src lies in its slot: at src's offset
+// from a 16-byte boundary, so that a bulk copy can move its whole chunks.
+__device__ __forceinline__ int8_t* staged_at(int8_t* slot, const int8_t* src) { return slot + ((uintptr_t)src & 15u); }
+
+// Start the copy of one world into its slot (by one warp): the whole 16-byte
+// chunks by a bulk copy, the bytes before and after them (worlds that start or
+// end at any byte) by plain loads.  The stores precede lane 0's arrival, so
+// whoever waits on the mbarrier sees them too.
+__device__ __forceinline__ void issue_world_copy(uint32_t mbar_a, int8_t* slot, const int8_t* src, int bytes, int lane) {
+    const int off = (int)((uintptr_t)src & 15u);
+    int8_t* dst = slot + off;
+    int head = 0, body = bytes;
+    if (off | (bytes & 15)) {  // uniform
+        head = min((16 - off) & 15, bytes);
+        const int tail = (bytes - head) & 15;
+        body = bytes - head - tail;
+        if (lane < head) dst[lane] = src[lane];
+        if (lane < tail) dst[head + body + lane] = src[head + body + lane];
+        __syncwarp();
+    }
     if (lane == 0) {
         // generic-proxy reads of the previous world must precede the copy
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(mbar_a), "r"(bytes) : "memory");
-        asm volatile(
-            "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                smem_u32(dst)),
-            "l"(src), "r"(bytes), "r"(mbar_a)
-            : "memory");
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(mbar_a), "r"(body) : "memory");
+        if (body)
+            asm volatile(
+                "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                    smem_u32(dst + head)),
+                "l"(src + head), "r"(body), "r"(mbar_a)
+                : "memory");
     }
 }
 
@@ -2790,7 +2825,7 @@ __global__ void __launch_bounds__(256, MC_FUSED_MIN_BLOCKS)
     const int W = p.W, H = p.H;
     const int wxz = p.wx * p.wz;
     const int wxyz = wxz * p.wy;
-    FusedLayout L = fused_layout(W, H, wxyz, wxz, F32, STAGE, tile_w);
+    FusedLayout L = fused_layout(W, H, mc_world_slot(p), wxz, F32, STAGE, tile_w);
 
     FusedCtx cx;
     build_fast_tables(reinterpret_cast<float4*>(smem), reinterpret_cast<uint32_t*>(smem + kShadeTableBytes));
@@ -2829,11 +2864,13 @@ __global__ void __launch_bounds__(256, MC_FUSED_MIN_BLOCKS)
             if (q.bits & MC_ER_BURIED) {
                 if (part == 0) fill_env<FAM, F32>(p, q.env, q.fill_blk, cx, lane, 32);
             } else {
-                if (!stage_fits(sworld, wxyz)) {
+                if (!stage_fits(sworld, mc_world_slot(p))) {
                     no_stage = true;
                     break;
                 }
-                issue_world_copy(cx.mbar_a, sworld, world_of(p, q.env, q.bits, any_done), wxyz, lane);
+                const int8_t* src = world_of(p, q.env, q.bits, any_done);
+                issue_world_copy(cx.mbar_a, sworld, src, wxyz, lane);
+                const int8_t* world = staged_at(sworld, src);
                 EnvRender r = render_of_rec(q, p.wy);
                 if (!mbar_wait(cx.mbar_a, phase, p.wait_polls)) {
                     if (lane == 0) atomicExch(&p.flags[MC_FLAG_ERROR], MC_KERR_TMA_TIMEOUT);
@@ -2841,8 +2878,8 @@ __global__ void __launch_bounds__(256, MC_FUSED_MIN_BLOCKS)
                     break;
                 }
                 phase ^= 1u;
-                measure_staged(r, sworld, p.wx, p.wy, p.wz, lane);
-                render_fast<FAM, F32>(p, q.env, r, cx, sworld, tile_w, lane, nullptr, part, slices);
+                measure_staged(r, world, p.wx, p.wy, p.wz, lane);
+                render_fast<FAM, F32>(p, q.env, r, cx, world, tile_w, lane, nullptr, part, slices);
             }
             if (regen_env(p, q.bits, any_done) && last_slice(recs, i, slices, lane)) regen_world(p, q.env, lane, 32);
         }
@@ -2874,14 +2911,14 @@ __global__ void __launch_bounds__(256, MC_FUSED_MIN_BLOCKS)
                 fill_env<FAM, F32>(p, q.env, q.fill_blk, cx, lane, 32);
             } else {
                 const int8_t* world = world_of(p, q.env, q.bits, any_done);
-                bool staged = STAGE && !no_stage && stage_fits(sworld, wxyz);
+                bool staged = STAGE && !no_stage && stage_fits(sworld, mc_world_slot(p));
                 int ytop = p.wy - 1;
                 if (staged) {
                     issue_world_copy(cx.mbar_a, sworld, world, wxyz, lane);
                     if (mbar_wait(cx.mbar_a, phase, p.wait_polls)) {
                         phase ^= 1u;
                         EnvRender r = render_of_rec(q, p.wy);
-                        measure_staged(r, sworld, p.wx, p.wy, p.wz, lane);
+                        measure_staged(r, staged_at(sworld, world), p.wx, p.wy, p.wz, lane);
                         ytop = r.ytop;
                     } else {
                         if (lane == 0) atomicExch(&p.flags[MC_FLAG_ERROR], MC_KERR_TMA_TIMEOUT);
@@ -2889,7 +2926,7 @@ __global__ void __launch_bounds__(256, MC_FUSED_MIN_BLOCKS)
                         staged = false;
                     }
                 }
-                render_slow<FAM, F32>(p, q, ytop, cx, staged ? sworld : nullptr, world, tile_w, lane, nullptr);
+                render_slow<FAM, F32>(p, q, ytop, cx, staged ? staged_at(sworld, world) : nullptr, world, tile_w, lane, nullptr);
             }
             if (regen_env(p, q.bits, any_done)) regen_world(p, q.env, lane, 32);
         }
@@ -3101,16 +3138,20 @@ __global__ void __launch_bounds__(256, MC_TEAM_MIN_BLOCKS) k_render_team(const _
         const mc_kp& p = rk.groups[t.g];
         const int wxyz = p.wx * p.wy * p.wz;
         int8_t* world = slot_world(d, t.coop);
-        if (!stage_fits(world, wxyz)) return;
+        if (!stage_fits(world, mc_world_slot(p))) return;
         issue_world_copy((t.coop ? tmbar : cx.mbar_a) + 8 * d, world,
                          world_of(p, q.env, q.bits, (ts->any_done >> t.g) & 1), wxyz, lane);
         if (t.coop) tlive |= 1u << d;
         else wlive |= 1u << d;
     };
+    // Where the staged copy of unit t's world lies (its record q).
+    auto staged_world = [&](const Unit& t, const EnvRec& q, int d) -> const int8_t* {
+        return staged_at(slot_world(d, t.coop), world_of(rk.groups[t.g], q.env, q.bits, (ts->any_done >> t.g) & 1));
+    };
     // Wait for the copy of unit t into depth slot d.
     auto landed = [&](const Unit& t, int d) -> bool {
         const mc_kp& p = rk.groups[t.g];
-        if (!stage_fits(slot_world(d, t.coop), p.wx * p.wy * p.wz)) {
+        if (!stage_fits(slot_world(d, t.coop), mc_world_slot(p))) {
             *(volatile int*)&ts->timed_out = 1;
             return false;
         }
@@ -3173,7 +3214,7 @@ __global__ void __launch_bounds__(256, MC_TEAM_MIN_BLOCKS) k_render_team(const _
                                            t.coop ? nthr : 32);
                 } else if (!(q.bits & MC_ER_SLOW)) {
                     const bool ok = landed(t, d);
-                    const int8_t* world = slot_world(d, t.coop);
+                    const int8_t* world = staged_world(t, q, d);
                     EnvRender r = render_of_rec(q, p.wy);
                     if (t.coop && TWN > 1 && up_scan_shape(p.wx, p.wy, p.wz))  // team-uniform; the eye is in the box
                         r.ub = team_up_bounds(ok, world, p.wx, p.wy, p.wz, (int)floorf(r.c.eye_x),
@@ -3252,7 +3293,7 @@ __global__ void __launch_bounds__(256, MC_TEAM_MIN_BLOCKS) k_render_team(const _
             if (!here) {
                 // another pass's env
             } else if (q.bits & MC_ER_SLOW) {
-                const int8_t* world = slot_world(0, t.coop);
+                const int8_t* world = staged_world(t, q, 0);
                 const bool staged = may_stage && landed(t, 0);
                 const int ytop = staged ? staged_top_layer(world, p.wx, p.wy, p.wz, lane) : p.wy - 1;
                 render_slow<FAM, F32>(p, q, ytop, cx, staged ? world : nullptr,
@@ -3335,8 +3376,7 @@ static int step_plain(const mc_kp* p, cudaStream_t s) {
 }
 
 static size_t fused_smem(const mc_kp* p, const mc_fused_cfg* cfg) {
-    int wxyz = p->wx * p->wy * p->wz;
-    FusedLayout L = fused_layout(p->W, p->H, wxyz, p->wx * p->wz, p->obs_f32, cfg->stage, cfg->tile_w);
+    FusedLayout L = fused_layout(p->W, p->H, mc_world_slot(*p), p->wx * p->wz, p->obs_f32, cfg->stage, cfg->tile_w);
     return (size_t)L.head_bytes + (size_t)cfg->warps_per_cta * L.warp_bytes + (size_t)L.pad_bytes;
 }
 
@@ -3385,6 +3425,12 @@ static int launch_warp_t(const mc_kp* p, const mc_fused_cfg* cfg, int slices, lo
 template <int FAM, bool F32>
 static int launch_fused_f(const mc_kp* kp, const mc_fused_cfg* cfg, int num_sms, cudaStream_t s) {
     mc_kp p = *kp;
+    mc_fused_cfg f = *cfg;
+    cfg = &f;
+    if (!f.stage && mc_odd_world(p) && mc_world_slot(p) <= 8192 + 16) {  // as default_launch stages the others
+        f.stage = 1;
+        if (fused_smem(&p, &f) > 227 * 1024) f.stage = 0;
+    }
     p.fast_ok = mc_fast_launch(p, cfg->stage, cfg->tile_w);
     const int wpc = cfg->warps_per_cta;
     long long grid = (long long)num_sms * (cfg->ctas_per_sm > 0 ? cfg->ctas_per_sm : 1);

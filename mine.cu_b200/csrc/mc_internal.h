@@ -186,6 +186,23 @@ static inline int mc_whole_tiles(int W, int H, int obs_f32, int tile_w) {
     const int th = 32 / tile_w;
     return W % tile_w == 0 && H % th == 0 && (W * th * (obs_f32 ? 12 : 3)) % 16 == 0;
 }
+// Worlds that no single bulk copy can take: not a multiple of 16 bytes, or
+// voxels that do not start on a 16-byte boundary.  No launch shape can ask for
+// their staging, so the launches stage them whenever they fit (the chunks by a
+// bulk copy, the edges by plain loads).
+#ifdef __CUDACC__
+__host__ __device__
+#endif
+static inline int mc_odd_world(const mc_kp& k) {
+    return (((long long)k.wx * k.wy * k.wz) & 15) != 0 || (((uintptr_t)k.voxels) & 15) != 0;
+}
+// Shared-memory bytes of one staged world: 16 to spare where it starts at any byte.
+#ifdef __CUDACC__
+__host__ __device__
+#endif
+static inline int mc_world_slot(const mc_kp& k) {
+    return ((k.wx * k.wy * k.wz + 15) & ~15) + (mc_odd_world(k) ? 16 : 0);
+}
 // Shared-memory bytes of one staged band: 16 to spare where bands start at any byte.
 #ifdef __CUDACC__
 __host__ __device__

@@ -447,8 +447,8 @@ static int step_regen(const mc_kp& k) {
 
 static inline int align16i(long long x) { return (int)((x + 15) & ~15LL); }
 
-void team_layout(const mc_kp* const* kps, int G, const int* stage, const int* tile_w, const int* coop,
-                        int team_warps, int warps_per_cta, mc_ragged_kp* rk) {
+static void team_layout_of(const mc_kp* const* kps, int G, const int* stage, const int* tile_w, const int* coop,
+                           int team_warps, int warps_per_cta, mc_ragged_kp* rk) {
     *rk = mc_ragged_kp{};
     rk->ngroups = G;
     rk->team_warps = team_warps;
@@ -457,7 +457,6 @@ void team_layout(const mc_kp* const* kps, int G, const int* stage, const int* ti
     int uv = 0, band = 16, coop_world = 0, slot = 0, pad = 0, depth = 0;
     for (int g = 0; g < G; ++g) {
         const mc_kp& k = *kps[g];
-        const long long wxyz = (long long)k.wx * k.wy * k.wz;
         rk->groups[g] = k;
         rk->groups[g].fast_ok = mc_fast_launch(k, stage[g], tile_w[g]);
         rk->groups[g].regen = step_regen(k);
@@ -474,9 +473,9 @@ void team_layout(const mc_kp* const* kps, int G, const int* stage, const int* ti
             depth = std::max(depth, stage[g]);  // the launch stages every staged group at the largest depth asked
             pad = std::max(pad, align16i((long long)k.wx * k.wz));
             if (coop[g])
-                coop_world = std::max(coop_world, align16i(wxyz));
+                coop_world = std::max(coop_world, mc_world_slot(k));
             else
-                slot = std::max(slot, align16i(wxyz));
+                slot = std::max(slot, mc_world_slot(k));
         }
     }
     rk->start[G] = start;
@@ -531,6 +530,26 @@ void team_layout(const mc_kp* const* kps, int G, const int* stage, const int* ti
     rk->warp_bytes = 16 + 128 + band;
     const int after = warps_per_cta * rk->warp_bytes;
     rk->tail_bytes = after < pad ? pad - after : 0;
+}
+
+// Stages the groups whose worlds no launch shape can stage (mc_odd_world) too,
+// when one more world per team (or warp) keeps three CTAs on an SM, or the
+// CTA's shared memory at what the shape takes without them.
+void team_layout(const mc_kp* const* kps, int G, const int* stage, const int* tile_w, const int* coop,
+                        int team_warps, int warps_per_cta, mc_ragged_kp* rk) {
+    team_layout_of(kps, G, stage, tile_w, coop, team_warps, warps_per_cta, rk);
+    int all[MC_MAX_GROUPS];
+    bool more = false;
+    for (int g = 0; g < G; ++g) {
+        all[g] = !stage[g] && mc_odd_world(*kps[g]) && (long long)kps[g]->wx * kps[g]->wy * kps[g]->wz <= 227 * 1024
+                     ? 1 : stage[g];
+        more |= all[g] != stage[g];
+    }
+    if (!more) return;
+    const long long most = std::max(74LL * 1024, team_smem(*rk, warps_per_cta));
+    mc_ragged_kp with;
+    team_layout_of(kps, G, all, tile_w, coop, team_warps, warps_per_cta, &with);
+    if (team_smem(with, warps_per_cta) <= most) *rk = with;
 }
 
 long long team_smem(const mc_ragged_kp& rk, int warps_per_cta) {

@@ -81,3 +81,39 @@ def test_odd_images(cuda, res, cfg):
     """Images that are no whole tiles, whose rows and envs start at any byte."""
     for mode in ("uint8", "float32", "uint8_prebasis"):
         run(cuda, 5, 6, 56, res=res, cfg=cfg, obs_dtype=mode, episode_length=4)
+
+
+@pytest.mark.parametrize("world", [(5, 5, 5), (9, 40, 13), (7, 11, 23), (26, 33, 21), (16, 16, 17), (33, 9, 40)])
+@pytest.mark.parametrize("cfg", [None, (0, 8, 4, 8, 1, 0), (0, 8, 3, 8, 4, 1), (0, 8, 2, 8, 2, 0)],
+                         ids=["default", "per_warp", "team", "per_warp_groups"])
+def test_worlds_of_any_size(cuda, world, cfg):
+    """Worlds of no whole 16-byte chunks (every env's starts at another byte), staged by their chunks and edges."""
+    for mode in ("uint8", "uint8_minimal"):
+        run(cuda, 9, 7, 57, world=world, res=(24, 16), cfg=cfg, obs_dtype=mode, episode_length=4,
+            ground_height=min(8, world[1] // 2), regen="per_env")
+
+
+def test_voxels_at_any_byte(cuda):
+    """A voxels view that starts off a 16-byte boundary."""
+    import ctypes
+    import torch
+    B = 6
+    g = GpuEnv(cuda, B, debug=False, obs_dtype="uint8", episode_length=4)
+    base = torch.empty(B * 4096 + 32, dtype=torch.int8, device=cuda)
+    view = base[3:3 + B * 4096].view(B, 16, 16, 16)
+    g.t["voxels"] = view
+    g.st.voxels = view.data_ptr()
+    capi.check(g.L.mc_env_set_state(g.h, ctypes.byref(g.st)), "set_state")
+    g.set_fused(0, 8, 4, 4, 1, 0)
+    capi.check(g.L.mc_env_generate_world(g.h, None), "generate_world")
+    o = O.OracleEnv(batch_size=B, obs_dtype="uint8", episode_length=4, world_size=16, render_width=32, render_height=32)
+    g.reset()
+    o.reset()
+    for s in range(9):
+        _, btn, look = actions_for(B, s, 58, 0.1, True)
+        g.step(btn, look, capi.FORM_FUSED)
+        o.step(btn, look)
+        d = diff_report(g.state(), oracle_state(o))
+        assert not d, f"step {s}: {d}"
+    g.check_error()
+    g.close()
