@@ -72,7 +72,7 @@ MC_HIDDEN bool dones_possible(const mc_kp& k);
 // parameter blocks, copied into the launch's parameter block); flags and
 // actions are left to the caller.
 MC_HIDDEN void team_layout(const mc_kp* const* kps, int G, const int* stage, const int* tile_w, const int* coop,
-                           int team_warps, int warps_per_cta, mc_ragged_kp* rk);
+                           int team_warps, int warps_per_cta, int ctas_per_sm, mc_ragged_kp* rk);
 // Dynamic shared memory of that launch per CTA.
 MC_HIDDEN long long team_smem(const mc_ragged_kp& rk, int warps_per_cta);
 // MC_OK, or MC_ERR_INVALID with a message when the team launch is not possible.

@@ -445,6 +445,8 @@ static int step_regen(const mc_kp& k) {
     return k.regen_per_env ? MC_KREGEN_PER_ENV : MC_KREGEN_ALL;
 }
 
+constexpr long long kSmemPerCta = 227 * 1024;  // an SM's 228 KB hold each CTA's and 1 KB more per CTA
+
 static inline int align16i(long long x) { return (int)((x + 15) & ~15LL); }
 
 static void team_layout_of(const mc_kp* const* kps, int G, const int* stage, const int* tile_w, const int* coop,
@@ -497,7 +499,11 @@ static void team_layout_of(const mc_kp* const* kps, int G, const int* stage, con
         for (int g = 0; g < G; ++g) {
             const int bands = (kps[g]->H * tile_w[g] + 31) / 32;
             const long long add = (long long)kps[g]->B * rk->slices[g];
-            if (!coop[g] || !rk->groups[g].fast_ok || add == 0 || units + add > 888 ||
+            // (888 teams of 4 on 148 SMs; where staging a world again is cheap, up
+            // to four units a team: 1024 envs 16^3, 64x64 43.2 -> 39.9 us a step;
+            // 512 envs 32^3 would go from 48.8 to 55.3)
+            const long long most = mc_world_slot(*kps[g]) <= 8192 + 16 ? 3552 : 888;
+            if (!coop[g] || !rk->groups[g].fast_ok || add == 0 || units + add > most ||
                 rk->slices[g] * 2 * team_warps > bands)
                 continue;
             units += add;
@@ -533,20 +539,20 @@ static void team_layout_of(const mc_kp* const* kps, int G, const int* stage, con
 }
 
 // Stages the groups whose worlds no launch shape can stage (mc_odd_world) too,
-// when one more world per team (or warp) keeps three CTAs on an SM, or the
-// CTA's shared memory at what the shape takes without them.
+// when ctas_per_sm CTAs still fit an SM's shared memory with them, or the CTA
+// takes no more than without them.
 void team_layout(const mc_kp* const* kps, int G, const int* stage, const int* tile_w, const int* coop,
-                        int team_warps, int warps_per_cta, mc_ragged_kp* rk) {
+                        int team_warps, int warps_per_cta, int ctas_per_sm, mc_ragged_kp* rk) {
     team_layout_of(kps, G, stage, tile_w, coop, team_warps, warps_per_cta, rk);
     int all[MC_MAX_GROUPS];
     bool more = false;
     for (int g = 0; g < G; ++g) {
-        all[g] = !stage[g] && mc_odd_world(*kps[g]) && (long long)kps[g]->wx * kps[g]->wy * kps[g]->wz <= 227 * 1024
-                     ? 1 : stage[g];
+        const mc_kp& k = *kps[g];
+        all[g] = !stage[g] && mc_odd_world(k) && (long long)k.wx * k.wy * k.wz <= kSmemPerCta ? 1 : stage[g];
         more |= all[g] != stage[g];
     }
     if (!more) return;
-    const long long most = std::max(74LL * 1024, team_smem(*rk, warps_per_cta));
+    const long long most = std::max((kSmemPerCta + 1024) / ctas_per_sm - 1024, team_smem(*rk, warps_per_cta));
     mc_ragged_kp with;
     team_layout_of(kps, G, all, tile_w, coop, team_warps, warps_per_cta, &with);
     if (team_smem(with, warps_per_cta) <= most) *rk = with;
@@ -577,7 +583,7 @@ int team_validate(const mc_kp* const* kps, int G, const int* stage, const int* t
         }
     }
     mc_ragged_kp rk;
-    team_layout(kps, G, stage, tile_w, coop, team_warps, warps_per_cta, &rk);
+    team_layout(kps, G, stage, tile_w, coop, team_warps, warps_per_cta, ctas_per_sm, &rk);
     if (rk.ustart[G] >= (1LL << 31)) return fail(MC_ERR_INVALID, "more than 2^31 work units");
     const long long smem = team_smem(rk, warps_per_cta);
     if (smem > 227 * 1024) return fail(MC_ERR_INVALID, "team kernel shared memory %lld > 227 KB", smem);
@@ -618,15 +624,18 @@ static int validate_fused(const mc_env* e, const mc_fused_cfg* f) {
 // world staged in shared memory.  Big worlds, or big images over too few
 // envs to give every resident warp (SMs x 32) two envs: teams of 4 warps
 // render each env together from one staged copy of its world.  (16^3
-// worlds, 64x64 images: teams take 0.166 ms/step at B=4096, where one warp
-// per env takes 0.206; one warp per env takes 0.492 ms/step at B=16384,
-// where teams take 0.587.)  A shape whose shared memory does not fit falls
+// worlds, 64x64 images: teams take 85 us a step at B=4096, where one warp per
+// env takes 101; one warp per env takes 245 at B=16384, where teams take 259.)
+// Worlds above 32 KB: as many staged worlds as an SM's shared memory holds,
+// three or two CTAs with a team of 8, or one CTA with two teams of 4 or one of 8
+// (64x64 images, us a step, from global memory -> staged: 40^3 502 -> 172, 48^3
+// 647 -> 330, 56^3 439 -> 252).  A shape whose shared memory does not fit falls
 // back to the team shape (whose per-warp image band is half as tall), then
 // to one team per CTA, then to unstaged worlds.  The autotuner (minecu/autotune.py) refines the
 // shape per configuration.
 static mc_fused_cfg default_launch(const mc_env_config* cfg, const mc_kp* kp, const mc_backend* be, int num_sms) {
-    const int wxyz = cfg->world_x * cfg->world_y * cfg->world_z;
-    const bool aligned = (wxyz & 15) == 0 && !(((uintptr_t)kp->voxels) & 15);
+    const long long wxyz = (long long)cfg->world_x * cfg->world_y * cfg->world_z;
+    const bool aligned = !mc_odd_world(*kp);  // the launches stage the others by themselves
     const bool few_envs = (long long)cfg->batch_size < 2LL * num_sms * 32;
     const bool big = (cfg->render_width * cfg->render_height >= 64 * 64 && few_envs) || wxyz > 8192;
     auto team_shape = [&](mc_fused_cfg& f) {
@@ -636,6 +645,19 @@ static mc_fused_cfg default_launch(const mc_env_config* cfg, const mc_kp* kp, co
         f.tile_w = 8;
         f.team_warps = 4;
         f.coop = 1;
+        const mc_kp* kps[1] = {kp};
+        if (wxyz <= 32768 || wxyz > kSmemPerCta || !mc_fast_launch(*kp, 1, f.tile_w)) return;
+        constexpr int shapes[4][2] = {{3, 8}, {2, 8}, {1, 4}, {1, 8}};  // CTAs per SM, warps per team
+        const int staged = 1;
+        for (const auto& s : shapes) {
+            mc_ragged_kp rk;
+            team_layout_of(kps, 1, &staged, &f.tile_w, &f.coop, s[1], f.warps_per_cta, &rk);
+            if (s[0] * (team_smem(rk, f.warps_per_cta) + 1024) > kSmemPerCta + 1024) continue;
+            f.stage = aligned ? 1 : 0;
+            f.ctas_per_sm = s[0];
+            f.team_warps = s[1];
+            return;
+        }
     };
     mc_fused_cfg f;
     if (big) {
@@ -676,7 +698,7 @@ extern "C" int mc_default_fused_config(const mc_env_config* cfg, int32_t num_sms
         if (team_mode(f)) {
             const mc_kp* kps[1] = {&k};
             mc_ragged_kp rk;
-            team_layout(kps, 1, &f.stage, &f.tile_w, &f.coop, f.team_warps, f.warps_per_cta, &rk);
+            team_layout(kps, 1, &f.stage, &f.tile_w, &f.coop, f.team_warps, f.warps_per_cta, f.ctas_per_sm, &rk);
             *smem_bytes = team_smem(rk, f.warps_per_cta);
         } else {
             *smem_bytes = (int64_t)be->fused_smem_bytes(&k, &f);
@@ -827,7 +849,7 @@ static int launch_fused(mc_env* e, const mc_kp& k, cudaStream_t s, const char* w
     if (!team_mode(f)) return backend_rc(e->be->step_fused(&k, &f, e->num_sms, s), what);
     const mc_kp* kps[1] = {&k};
     mc_ragged_kp rk;
-    team_layout(kps, 1, &f.stage, &f.tile_w, &f.coop, f.team_warps, f.warps_per_cta, &rk);
+    team_layout(kps, 1, &f.stage, &f.tile_w, &f.coop, f.team_warps, f.warps_per_cta, f.ctas_per_sm, &rk);
     rk.groups[0].regen = k.regen;
     rk.flags = e->flags;
     rk.rec = e->rec;
@@ -1159,7 +1181,7 @@ extern "C" int64_t mc_env_fused_smem_bytes(const mc_env* e) {
         const mc_fused_cfg& f = e->fcfg;
         const mc_kp* kps[1] = {&e->kp};
         mc_ragged_kp rk;
-        team_layout(kps, 1, &f.stage, &f.tile_w, &f.coop, f.team_warps, f.warps_per_cta, &rk);
+        team_layout(kps, 1, &f.stage, &f.tile_w, &f.coop, f.team_warps, f.warps_per_cta, f.ctas_per_sm, &rk);
         return team_smem(rk, f.warps_per_cta);
     }
     mc_kp k = e->kp;
@@ -1244,7 +1266,7 @@ static void ragged_kps(const mc_ragged* r, std::vector<const mc_kp*>* kps) {
 static void ragged_layout(const mc_ragged* r, const mc_ragged_config* c, mc_ragged_kp* rk) {
     std::vector<const mc_kp*> kps;
     ragged_kps(r, &kps);
-    team_layout(kps.data(), (int)kps.size(), c->stage, c->tile_w, c->coop, c->team_warps, c->warps_per_cta, rk);
+    team_layout(kps.data(), (int)kps.size(), c->stage, c->tile_w, c->coop, c->team_warps, c->warps_per_cta, c->ctas_per_sm, rk);
     rk->flags = r->flags;
     rk->rec = r->rec;
 }

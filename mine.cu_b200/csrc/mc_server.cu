@@ -364,10 +364,14 @@ int run_round(mc_server* s, Slot& sl, const std::vector<Req*>& reqs, const std::
                 any_coop |= coop[g] != 0;
             }
             const int team = any_coop ? 4 : 1, cps = any_coop ? 3 : 4;
-            if (team_validate(kps.data(), G, stage, tile_w, coop, team, 8, cps) != MC_OK)
-                for (int g = 0; g < G; ++g) stage[g] = 0;  // the staged worlds do not fit together
+            // the staged worlds do not fit together: those above 32 KB give way first
+            for (const long long most : {32768LL, 0LL}) {
+                if (team_validate(kps.data(), G, stage, tile_w, coop, team, 8, cps) == MC_OK) break;
+                for (int g = 0; g < G; ++g)
+                    if ((long long)kps[g]->wx * kps[g]->wy * kps[g]->wz > most) stage[g] = 0;
+            }
             mc_ragged_kp rk;
-            team_layout(kps.data(), G, stage, tile_w, coop, team, 8, &rk);
+            team_layout(kps.data(), G, stage, tile_w, coop, team, 8, cps, &rk);
             rk.flags = s->flags;
             rk.rec = s->rec;
             rk.actions = d_act;

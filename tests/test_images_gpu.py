@@ -117,3 +117,10 @@ def test_voxels_at_any_byte(cuda):
         assert not d, f"step {s}: {d}"
     g.check_error()
     g.close()
+
+
+@pytest.mark.parametrize("world", [(40, 40, 40), (41, 39, 43), (48, 48, 48), (56, 56, 56), (64, 56, 64)])
+def test_big_worlds(cuda, world):
+    """Worlds above 32 KB, with the default launch shape (as many staged worlds as an SM holds, or none)."""
+    run(cuda, 5, 5, 59, world=world, res=(64, 48), obs_dtype="uint8", episode_length=3, regen="per_env")
+    run(cuda, 2, 4, 60, world=world, res=(31, 20), obs_dtype="uint8_minimal", episode_length=3)
