@@ -610,98 +610,122 @@ __device__ __noinline__ void march_bounds_fail(uint32_t a, SmemRange chk, int si
 }
 #endif
 
-__device__ __forceinline__ int march_packed_shared(uint32_t world, int packed, int px, int py, int pz, float& tmx,
-                                                   float& tmy, float& tmz, float tdx, float tdy, float tdz,
-                                                   SmemRange chk = SmemRange{0u, 0u}) {
+// The marches' number type: float, or binary16 for the fp16 family (held in 16
+// bits; its adds and compares keep denormals, as the half intrinsics do).
+// The axis of a step: x if tmx < tmy and tmx < tmz, else y if tmy < tmz, else
+// z (binary16 compares have no second predicate output).
+#define MC_F32_T MC_PTX_FTZ ".f32"
+#define MC_F16_T ".f16"
+#define MC_F32_AXIS                                          \
+    "setp.lt" MC_F32_T " pa|pna, %1, %2;\n\t"              \
+    "setp.lt.and" MC_F32_T " pbx|pzx, %1, %3, pa;\n\t"     \
+    "setp.lt.and" MC_F32_T " pby|pzy, %2, %3, pna;\n\t"    \
+    "or.pred pz, pzx, pzy;\n\t"
+#define MC_F16_AXIS                                          \
+    "setp.lt" MC_F16_T " pa, %1, %2;\n\t"                  \
+    "not.pred pna, pa;\n\t"                               \
+    "setp.lt.and" MC_F16_T " pbx, %1, %3, pa;\n\t"         \
+    "setp.lt.and" MC_F16_T " pby, %2, %3, pna;\n\t"        \
+    "or.pred pz, pbx, pby;\n\t"                           \
+    "not.pred pz, pz;\n\t"
+#if MC_CHECK_BOUNDS
+#define MC_MARCH_PACKED(FT, CMP, C) \
+    asm volatile( \
+        "{\n\t" \
+        ".reg .pred pa, pna, pbx, pzx, pby, pzy, pz, pq, pb1, pb2;\n\t" \
+        ".reg .b32 ra, rc;\n\t" \
+        ".reg .s32 rv;\n\t" \
+        "MC_CMARCH_LOOP:\n\t" \
+        CMP \
+        "@pbx add.s32 %4, %4, %6;\n\t" \
+        "@pby add.s32 %4, %4, %7;\n\t" \
+        "@pz add.s32 %4, %4, %8;\n\t" \
+        "shr.s32 ra, %4, 18;\n\t" \
+        "add.s32 ra, ra, %10;\n\t" \
+        "sub.u32 rc, ra, %15;\n\t" \
+        "setp.ge.u32 pb1, rc, %16;\n\t" \
+        "sub.u32 rc, ra, %17;\n\t" \
+        "setp.ge.u32 pb2, rc, %18;\n\t" \
+        "or.pred pb1, pb1, pb2;\n\t" \
+        "@pb1 mov.u32 %5, ra;\n\t" \
+        "@pb1 mov.s32 %0, -2;\n\t" \
+        "@pb1 bra MC_CMARCH_END;\n\t" \
+        "ld.shared.s8 rv, [ra];\n\t" \
+        "lop3.b32 ra, %4, rv, %9, 0xA2;\n\t" \
+        "setp.ne.b32 pq, ra, 0;\n\t" \
+        "@pq bra MC_CMARCH_DONE;\n\t" \
+        "@pbx add.rn" FT " %1, %1, %11;\n\t" \
+        "@pby add.rn" FT " %2, %2, %12;\n\t" \
+        "@pz add.rn" FT " %3, %3, %13;\n\t" \
+        "bra MC_CMARCH_LOOP;\n\t" \
+        "MC_CMARCH_DONE:\n\t" \
+        "and.b32 ra, %4, %14;\n\t" \
+        "setp.ne.b32 pq, ra, 0;\n\t" \
+        "selp.b32 %0, -1, rv, pq;\n\t" \
+        "MC_CMARCH_END:\n\t" \
+        "}" \
+        : "=&r"(b), "+" C(tmx), "+" C(tmy), "+" C(tmz), "+r"(packed), "+r"(bad) \
+        : "r"(px), "r"(py), "r"(pz), "n"(kGuard | (int)0x80000000u), "r"(world), C(tdx), C(tdy), C(tdz), \
+          "n"(kGuard), "r"(chk.lo), "r"(chk.span), "r"(dyn.lo), "r"(dyn.span) \
+        : "memory");
+#else
+// one test for both exits: a guard bit of the counts, or the sign bit clear in
+// the voxel (a block); c & (a | ~b) = lut 0xA2
+#define MC_MARCH_PACKED(FT, CMP, C) \
+    asm volatile( \
+        "{\n\t" \
+        ".reg .pred pa, pna, pbx, pzx, pby, pzy, pz, pq;\n\t" \
+        ".reg .b32 ra;\n\t" \
+        ".reg .s32 rv;\n\t" \
+        "MC_MARCH_LOOP:\n\t" \
+        CMP \
+        "@pbx add.s32 %4, %4, %5;\n\t" \
+        "@pby add.s32 %4, %4, %6;\n\t" \
+        "@pz add.s32 %4, %4, %7;\n\t" \
+        "shr.s32 ra, %4, 18;\n\t" \
+        "add.s32 ra, ra, %9;\n\t" \
+        "ld.shared.s8 rv, [ra];\n\t" \
+        "lop3.b32 ra, %4, rv, %8, 0xA2;\n\t" \
+        "setp.ne.b32 pq, ra, 0;\n\t" \
+        "@pq bra MC_MARCH_DONE;\n\t" \
+        "@pbx add.rn" FT " %1, %1, %10;\n\t" \
+        "@pby add.rn" FT " %2, %2, %11;\n\t" \
+        "@pz add.rn" FT " %3, %3, %12;\n\t" \
+        "bra MC_MARCH_LOOP;\n\t" \
+        "MC_MARCH_DONE:\n\t" \
+        "and.b32 ra, %4, %13;\n\t" \
+        "setp.ne.b32 pq, ra, 0;\n\t" \
+        "selp.b32 %0, -1, rv, pq;\n\t" \
+        "}" \
+        : "=&r"(b), "+" C(tmx), "+" C(tmy), "+" C(tmz), "+r"(packed) \
+        : "r"(px), "r"(py), "r"(pz), "n"(kGuard | (int)0x80000000u), "r"(world), C(tdx), C(tdy), C(tdz), \
+          "n"(kGuard) \
+        : "memory");
+#endif
+
+template <class T>
+__device__ __forceinline__ int march_packed_shared(uint32_t world, int& packed, int px, int py, int pz, T& tmx, T& tmy,
+                                                   T& tmz, T tdx, T tdy, T tdz, SmemRange chk = SmemRange{0u, 0u}) {
     constexpr int kGuard = (32 << 12) | (32 << 6) | 32;
     int b;
 #if MC_CHECK_BOUNDS
     const SmemRange dyn = dyn_smem_range();
     uint32_t bad = 0;
-    asm volatile(
-        "{\n\t"
-        ".reg .pred pa, pna, pbx, pzx, pby, pzy, pz, pq, pb1, pb2;\n\t"
-        ".reg .b32 ra, rc;\n\t"
-        ".reg .s32 rv;\n\t"
-        "MC_CMARCH_LOOP:\n\t"
-        "setp.lt" MC_PTX_FTZ ".f32 pa|pna, %1, %2;\n\t"
-        "setp.lt.and" MC_PTX_FTZ ".f32 pbx|pzx, %1, %3, pa;\n\t"
-        "setp.lt.and" MC_PTX_FTZ ".f32 pby|pzy, %2, %3, pna;\n\t"
-        "or.pred pz, pzx, pzy;\n\t"
-        "@pbx add.s32 %4, %4, %6;\n\t"
-        "@pby add.s32 %4, %4, %7;\n\t"
-        "@pz add.s32 %4, %4, %8;\n\t"
-        "shr.s32 ra, %4, 18;\n\t"
-        "add.s32 ra, ra, %10;\n\t"
-        "sub.u32 rc, ra, %15;\n\t"
-        "setp.ge.u32 pb1, rc, %16;\n\t"
-        "sub.u32 rc, ra, %17;\n\t"
-        "setp.ge.u32 pb2, rc, %18;\n\t"
-        "or.pred pb1, pb1, pb2;\n\t"
-        "@pb1 mov.u32 %5, ra;\n\t"
-        "@pb1 mov.s32 %0, -2;\n\t"
-        "@pb1 bra MC_CMARCH_END;\n\t"
-        "ld.shared.s8 rv, [ra];\n\t"
-        "lop3.b32 ra, %4, rv, %9, 0xA2;\n\t"
-        "setp.ne.b32 pq, ra, 0;\n\t"
-        "@pq bra MC_CMARCH_DONE;\n\t"
-        "@pbx add.rn" MC_PTX_FTZ ".f32 %1, %1, %11;\n\t"
-        "@pby add.rn" MC_PTX_FTZ ".f32 %2, %2, %12;\n\t"
-        "@pz add.rn" MC_PTX_FTZ ".f32 %3, %3, %13;\n\t"
-        "bra MC_CMARCH_LOOP;\n\t"
-        "MC_CMARCH_DONE:\n\t"
-        "and.b32 ra, %4, %14;\n\t"
-        "setp.ne.b32 pq, ra, 0;\n\t"
-        "selp.b32 %0, -1, rv, pq;\n\t"
-        "MC_CMARCH_END:\n\t"
-        "}"
-        : "=&r"(b), "+f"(tmx), "+f"(tmy), "+f"(tmz), "+r"(packed), "+r"(bad)
-        : "r"(px), "r"(py), "r"(pz), "n"(kGuard | (int)0x80000000u), "r"(world), "f"(tdx), "f"(tdy), "f"(tdz),
-          "n"(kGuard), "r"(chk.lo), "r"(chk.span), "r"(dyn.lo), "r"(dyn.span)
-        : "memory");
+#else
+    (void)chk;
+#endif
+    if constexpr (sizeof(T) == 4) {
+        MC_MARCH_PACKED(MC_F32_T, MC_F32_AXIS, "f")
+    } else {
+        MC_MARCH_PACKED(MC_F16_T, MC_F16_AXIS, "h")
+    }
+#if MC_CHECK_BOUNDS
     if (b == -2) {  // a load address outside its range: the load was skipped, the ray ends as sky
         march_bounds_fail(bad, chk, MC_SITE_MARCH_PACKED);
         b = -1;
     }
-    return b;
-#else
-    (void)chk;
-    asm volatile(
-        "{\n\t"
-        ".reg .pred pa, pna, pbx, pzx, pby, pzy, pz, pq;\n\t"
-        ".reg .b32 ra;\n\t"
-        ".reg .s32 rv;\n\t"
-        "MC_MARCH_LOOP:\n\t"
-        "setp.lt" MC_PTX_FTZ ".f32 pa|pna, %1, %2;\n\t"
-        "setp.lt.and" MC_PTX_FTZ ".f32 pbx|pzx, %1, %3, pa;\n\t"
-        "setp.lt.and" MC_PTX_FTZ ".f32 pby|pzy, %2, %3, pna;\n\t"
-        "or.pred pz, pzx, pzy;\n\t"
-        "@pbx add.s32 %4, %4, %5;\n\t"
-        "@pby add.s32 %4, %4, %6;\n\t"
-        "@pz add.s32 %4, %4, %7;\n\t"
-        "shr.s32 ra, %4, 18;\n\t"
-        "add.s32 ra, ra, %9;\n\t"
-        "ld.shared.s8 rv, [ra];\n\t"
-        // one test for both exits: a guard bit of the counts, or the sign
-        // bit clear in the voxel (a block); c & (a | ~b) = lut 0xA2
-        "lop3.b32 ra, %4, rv, %8, 0xA2;\n\t"
-        "setp.ne.b32 pq, ra, 0;\n\t"
-        "@pq bra MC_MARCH_DONE;\n\t"
-        "@pbx add.rn" MC_PTX_FTZ ".f32 %1, %1, %10;\n\t"
-        "@pby add.rn" MC_PTX_FTZ ".f32 %2, %2, %11;\n\t"
-        "@pz add.rn" MC_PTX_FTZ ".f32 %3, %3, %12;\n\t"
-        "bra MC_MARCH_LOOP;\n\t"
-        "MC_MARCH_DONE:\n\t"
-        "and.b32 ra, %4, %13;\n\t"
-        "setp.ne.b32 pq, ra, 0;\n\t"
-        "selp.b32 %0, -1, rv, pq;\n\t"
-        "}"
-        : "=&r"(b), "+f"(tmx), "+f"(tmy), "+f"(tmz), "+r"(packed)
-        : "r"(px), "r"(py), "r"(pz), "n"(kGuard | (int)0x80000000u), "r"(world), "f"(tdx), "f"(tdy), "f"(tdz),
-          "n"(kGuard)
-        : "memory");
-    return b;
 #endif
+    return b;
 }
 
 // Where a ray going up from the eye's voxel (vx, vy, vz) can still meet a
@@ -731,12 +755,13 @@ __device__ __forceinline__ int up_top(const UpBounds& b) {
 // In-box step counts of a march from the eye's voxel for ray sign
 // combination k (bit 0: x >= 0, bit 1: y >= 0, bit 2: z >= 0): the steps
 // left to each face of the box, cut for a ray going up by its quadrant's
-// bounds; a count of -1 ends the ray (as sky) at its first step.
-__device__ __forceinline__ void start_counts(int k, int vx, int vy, int vz, int wx, int wy, int wz,
+// bounds; a count of -1 ends the ray (as sky) at its first step.  ylow: the
+// lowest layer a ray may enter (0, or the ground-shortcut family's ground).
+__device__ __forceinline__ void start_counts(int k, int vx, int vy, int vz, int wx, int wy, int wz, int ylow,
                                              const UpBounds& ub, int& cx, int& cy, int& cz) {
     const bool px = k & 1, py = k & 2, pz = k & 4;
     cx = px ? wx - 1 - vx : vx;
-    cy = py ? wy - 1 - vy : vy;
+    cy = py ? wy - 1 - vy : vy - ylow;
     cz = pz ? wz - 1 - vz : vz;
     if (py) {
         const int sh = 8 * ((px ? 1 : 0) | (pz ? 2 : 0));
@@ -752,11 +777,11 @@ __device__ __forceinline__ void start_counts(int k, int vx, int vy, int vz, int 
 // y >= 0, bit 2: z >= 0): {packed index and counts, x, y and z increments}.
 // Counts from start_counts (at least -1, at most 31).
 __device__ __forceinline__ int4 packed_start(int k, int vx, int vy, int vz, int wx, int wy, int wz,
-                                             const UpBounds& ub) {
+                                             int ylow, const UpBounds& ub) {
     const int sx = (k & 1) ? 1 : -1, sy = (k & 2) ? 1 : -1, sz = (k & 4) ? 1 : -1;
     const int wxz = wx * wz, idx = vy * wxz + vx * wz + vz;
     int cx, cy, cz;
-    start_counts(k, vx, vy, vz, wx, wy, wz, ub, cx, cy, cz);
+    start_counts(k, vx, vy, vz, wx, wy, wz, ylow, ub, cx, cy, cz);
     return make_int4((idx << 18) | ((31 - cx) << 12) | ((31 - cy) << 6) | (31 - cz),
                      ((sx * wz) << 18) + (1 << 12), ((sy * wxz) << 18) + (1 << 6), (sz << 18) + 1);
 }
@@ -779,99 +804,104 @@ __device__ __forceinline__ int split_counts(int cx, int cy, int cz, int max_step
 // needs no index arithmetic.  Axis choice, predicated updates and the
 // distances left at a hit as in march_packed_shared.  Returns the block hit
 // (>= 0), or -1 when the ray left the box or ran out of steps.
-__device__ __forceinline__ int march_split_shared(uint32_t addr, int cnt, int dax, int day, int daz, float& tmx,
-                                                  float& tmy, float& tmz, float tdx, float tdy, float tdz,
-                                                  SmemRange chk = SmemRange{0u, 0u}) {
+#if MC_CHECK_BOUNDS
+#define MC_MARCH_SPLIT(FT, CMP, C) \
+    asm volatile( \
+        "{\n\t" \
+        ".reg .pred pa, pna, pbx, pzx, pby, pzy, pz, pq, pb1, pb2;\n\t" \
+        ".reg .b32 ra, rc;\n\t" \
+        ".reg .s32 rv;\n\t" \
+        "MC_CSPLIT_LOOP:\n\t" \
+        CMP \
+        "@pbx add.s32 %4, %4, %7;\n\t" \
+        "@pby add.s32 %4, %4, %8;\n\t" \
+        "@pz add.s32 %4, %4, %9;\n\t" \
+        "@pbx add.s32 %5, %5, %10;\n\t" \
+        "@pby add.s32 %5, %5, %11;\n\t" \
+        "@pz add.s32 %5, %5, %12;\n\t" \
+        "sub.u32 rc, %4, %18;\n\t" \
+        "setp.ge.u32 pb1, rc, %19;\n\t" \
+        "sub.u32 rc, %4, %20;\n\t" \
+        "setp.ge.u32 pb2, rc, %21;\n\t" \
+        "or.pred pb1, pb1, pb2;\n\t" \
+        "@pb1 mov.u32 %6, %4;\n\t" \
+        "@pb1 mov.s32 %0, -2;\n\t" \
+        "@pb1 bra MC_CSPLIT_END;\n\t" \
+        "ld.shared.s8 rv, [%4];\n\t" \
+        "lop3.b32 ra, %5, rv, %13, 0xA2;\n\t" \
+        "setp.ne.b32 pq, ra, 0;\n\t" \
+        "@pq bra MC_CSPLIT_DONE;\n\t" \
+        "@pbx add.rn" FT " %1, %1, %14;\n\t" \
+        "@pby add.rn" FT " %2, %2, %15;\n\t" \
+        "@pz add.rn" FT " %3, %3, %16;\n\t" \
+        "bra MC_CSPLIT_LOOP;\n\t" \
+        "MC_CSPLIT_DONE:\n\t" \
+        "and.b32 ra, %5, %17;\n\t" \
+        "setp.ne.b32 pq, ra, 0;\n\t" \
+        "selp.b32 %0, -1, rv, pq;\n\t" \
+        "MC_CSPLIT_END:\n\t" \
+        "}" \
+        : "=&r"(b), "+" C(tmx), "+" C(tmy), "+" C(tmz), "+r"(addr), "+r"(cnt), "+r"(bad) \
+        : "r"(dax), "r"(day), "r"(daz), "n"((1 << 7) | (1 << 21)), "n"((1 << 14) | (1 << 21)), "n"(1 | (1 << 21)), \
+          "n"(kSplitGuard | (int)0x80000000u), C(tdx), C(tdy), C(tdz), "n"(kSplitGuard), "r"(chk.lo), \
+          "r"(chk.span), "r"(dyn.lo), "r"(dyn.span) \
+        : "memory");
+#else
+#define MC_MARCH_SPLIT(FT, CMP, C) \
+    asm volatile( \
+        "{\n\t" \
+        ".reg .pred pa, pna, pbx, pzx, pby, pzy, pz, pq;\n\t" \
+        ".reg .b32 ra;\n\t" \
+        ".reg .s32 rv;\n\t" \
+        "MC_SPLIT_LOOP:\n\t" \
+        CMP \
+        "@pbx add.s32 %4, %4, %6;\n\t" \
+        "@pby add.s32 %4, %4, %7;\n\t" \
+        "@pz add.s32 %4, %4, %8;\n\t" \
+        "@pbx add.s32 %5, %5, %9;\n\t" \
+        "@pby add.s32 %5, %5, %10;\n\t" \
+        "@pz add.s32 %5, %5, %11;\n\t" \
+        "ld.shared.s8 rv, [%4];\n\t" \
+        "lop3.b32 ra, %5, rv, %12, 0xA2;\n\t" \
+        "setp.ne.b32 pq, ra, 0;\n\t" \
+        "@pq bra MC_SPLIT_DONE;\n\t" \
+        "@pbx add.rn" FT " %1, %1, %13;\n\t" \
+        "@pby add.rn" FT " %2, %2, %14;\n\t" \
+        "@pz add.rn" FT " %3, %3, %15;\n\t" \
+        "bra MC_SPLIT_LOOP;\n\t" \
+        "MC_SPLIT_DONE:\n\t" \
+        "and.b32 ra, %5, %16;\n\t" \
+        "setp.ne.b32 pq, ra, 0;\n\t" \
+        "selp.b32 %0, -1, rv, pq;\n\t" \
+        "}" \
+        : "=&r"(b), "+" C(tmx), "+" C(tmy), "+" C(tmz), "+r"(addr), "+r"(cnt) \
+        : "r"(dax), "r"(day), "r"(daz), "n"((1 << 7) | (1 << 21)), "n"((1 << 14) | (1 << 21)), "n"(1 | (1 << 21)), \
+          "n"(kSplitGuard | (int)0x80000000u), C(tdx), C(tdy), C(tdz), "n"(kSplitGuard) \
+        : "memory");
+#endif
+
+template <class T>
+__device__ __forceinline__ int march_split_shared(uint32_t addr, int& cnt, int dax, int day, int daz, T& tmx, T& tmy,
+                                                  T& tmz, T tdx, T tdy, T tdz, SmemRange chk = SmemRange{0u, 0u}) {
     int b;
 #if MC_CHECK_BOUNDS
     const SmemRange dyn = dyn_smem_range();
     uint32_t bad = 0;
-    asm volatile(
-        "{\n\t"
-        ".reg .pred pa, pna, pbx, pzx, pby, pzy, pz, pq, pb1, pb2;\n\t"
-        ".reg .b32 ra, rc;\n\t"
-        ".reg .s32 rv;\n\t"
-        "MC_CSPLIT_LOOP:\n\t"
-        "setp.lt" MC_PTX_FTZ ".f32 pa|pna, %1, %2;\n\t"
-        "setp.lt.and" MC_PTX_FTZ ".f32 pbx|pzx, %1, %3, pa;\n\t"
-        "setp.lt.and" MC_PTX_FTZ ".f32 pby|pzy, %2, %3, pna;\n\t"
-        "or.pred pz, pzx, pzy;\n\t"
-        "@pbx add.s32 %4, %4, %7;\n\t"
-        "@pby add.s32 %4, %4, %8;\n\t"
-        "@pz add.s32 %4, %4, %9;\n\t"
-        "@pbx add.s32 %5, %5, %10;\n\t"
-        "@pby add.s32 %5, %5, %11;\n\t"
-        "@pz add.s32 %5, %5, %12;\n\t"
-        "sub.u32 rc, %4, %18;\n\t"
-        "setp.ge.u32 pb1, rc, %19;\n\t"
-        "sub.u32 rc, %4, %20;\n\t"
-        "setp.ge.u32 pb2, rc, %21;\n\t"
-        "or.pred pb1, pb1, pb2;\n\t"
-        "@pb1 mov.u32 %6, %4;\n\t"
-        "@pb1 mov.s32 %0, -2;\n\t"
-        "@pb1 bra MC_CSPLIT_END;\n\t"
-        "ld.shared.s8 rv, [%4];\n\t"
-        "lop3.b32 ra, %5, rv, %13, 0xA2;\n\t"
-        "setp.ne.b32 pq, ra, 0;\n\t"
-        "@pq bra MC_CSPLIT_DONE;\n\t"
-        "@pbx add.rn" MC_PTX_FTZ ".f32 %1, %1, %14;\n\t"
-        "@pby add.rn" MC_PTX_FTZ ".f32 %2, %2, %15;\n\t"
-        "@pz add.rn" MC_PTX_FTZ ".f32 %3, %3, %16;\n\t"
-        "bra MC_CSPLIT_LOOP;\n\t"
-        "MC_CSPLIT_DONE:\n\t"
-        "and.b32 ra, %5, %17;\n\t"
-        "setp.ne.b32 pq, ra, 0;\n\t"
-        "selp.b32 %0, -1, rv, pq;\n\t"
-        "MC_CSPLIT_END:\n\t"
-        "}"
-        : "=&r"(b), "+f"(tmx), "+f"(tmy), "+f"(tmz), "+r"(addr), "+r"(cnt), "+r"(bad)
-        : "r"(dax), "r"(day), "r"(daz), "n"((1 << 7) | (1 << 21)), "n"((1 << 14) | (1 << 21)), "n"(1 | (1 << 21)),
-          "n"(kSplitGuard | (int)0x80000000u), "f"(tdx), "f"(tdy), "f"(tdz), "n"(kSplitGuard), "r"(chk.lo),
-          "r"(chk.span), "r"(dyn.lo), "r"(dyn.span)
-        : "memory");
+#else
+    (void)chk;
+#endif
+    if constexpr (sizeof(T) == 4) {
+        MC_MARCH_SPLIT(MC_F32_T, MC_F32_AXIS, "f")
+    } else {
+        MC_MARCH_SPLIT(MC_F16_T, MC_F16_AXIS, "h")
+    }
+#if MC_CHECK_BOUNDS
     if (b == -2) {
         march_bounds_fail(bad, chk, MC_SITE_MARCH_SPLIT);
         b = -1;
     }
-    return b;
-#else
-    (void)chk;
-    asm volatile(
-        "{\n\t"
-        ".reg .pred pa, pna, pbx, pzx, pby, pzy, pz, pq;\n\t"
-        ".reg .b32 ra;\n\t"
-        ".reg .s32 rv;\n\t"
-        "MC_SPLIT_LOOP:\n\t"
-        "setp.lt" MC_PTX_FTZ ".f32 pa|pna, %1, %2;\n\t"
-        "setp.lt.and" MC_PTX_FTZ ".f32 pbx|pzx, %1, %3, pa;\n\t"
-        "setp.lt.and" MC_PTX_FTZ ".f32 pby|pzy, %2, %3, pna;\n\t"
-        "or.pred pz, pzx, pzy;\n\t"
-        "@pbx add.s32 %4, %4, %6;\n\t"
-        "@pby add.s32 %4, %4, %7;\n\t"
-        "@pz add.s32 %4, %4, %8;\n\t"
-        "@pbx add.s32 %5, %5, %9;\n\t"
-        "@pby add.s32 %5, %5, %10;\n\t"
-        "@pz add.s32 %5, %5, %11;\n\t"
-        "ld.shared.s8 rv, [%4];\n\t"
-        // one test for both exits (as in march_packed_shared)
-        "lop3.b32 ra, %5, rv, %12, 0xA2;\n\t"
-        "setp.ne.b32 pq, ra, 0;\n\t"
-        "@pq bra MC_SPLIT_DONE;\n\t"
-        "@pbx add.rn" MC_PTX_FTZ ".f32 %1, %1, %13;\n\t"
-        "@pby add.rn" MC_PTX_FTZ ".f32 %2, %2, %14;\n\t"
-        "@pz add.rn" MC_PTX_FTZ ".f32 %3, %3, %15;\n\t"
-        "bra MC_SPLIT_LOOP;\n\t"
-        "MC_SPLIT_DONE:\n\t"
-        "and.b32 ra, %5, %16;\n\t"
-        "setp.ne.b32 pq, ra, 0;\n\t"
-        "selp.b32 %0, -1, rv, pq;\n\t"
-        "}"
-        : "=&r"(b), "+f"(tmx), "+f"(tmy), "+f"(tmz), "+r"(addr), "+r"(cnt)
-        : "r"(dax), "r"(day), "r"(daz), "n"((1 << 7) | (1 << 21)), "n"((1 << 14) | (1 << 21)), "n"(1 | (1 << 21)),
-          "n"(kSplitGuard | (int)0x80000000u), "f"(tdx), "f"(tdy), "f"(tdz), "n"(kSplitGuard)
-        : "memory");
-    return b;
 #endif
+    return b;
 }
 
 // March from the eye's voxel (index idx, in-box steps left cx, cy, cz) through
@@ -882,12 +912,12 @@ __device__ __forceinline__ int march_staged(uint32_t base, int idx, int cx, int 
                                            float tdx, float tdy, float tdz) {
     const SmemRange chk = staged_range(base, wx * wz, wx * wy * wz);
     if (max_steps > wx + wy + wz && wx <= 31 && wy <= 31 && wz <= 31 && wx * wy * wz < 8192) {
-        const int packed = (idx << 18) | ((31 - cx) << 12) | ((31 - max(cy, -32)) << 6) | (31 - cz);
+        int packed = (idx << 18) | ((31 - cx) << 12) | ((31 - max(cy, -32)) << 6) | (31 - cz);
         return march_packed_shared(base, packed, (dix << 18) + (1 << 12), (diy << 18) + (1 << 6), (diz << 18) + 1,
                                    tmx, tmy, tmz, tdx, tdy, tdz, chk);
     }
-    return march_split_shared(base + idx, split_counts(cx, cy, cz, max_steps, wx, wy, wz), dix, diy, diz, tmx, tmy,
-                              tmz, tdx, tdy, tdz, chk);
+    int cnt = split_counts(cx, cy, cz, max_steps, wx, wy, wz);
+    return march_split_shared(base + idx, cnt, dix, diy, diz, tmx, tmy, tmz, tdx, tdy, tdz, chk);
 }
 
 // Whether a march can run on the staged copy: V is a shared-memory source
@@ -1014,13 +1044,13 @@ __device__ __forceinline__ Hit shade_ray(const Cam& c, const Dda0& d0, float u, 
                 if (vd_safe && max_steps > wx + wy + wz && wx <= 31 && wy <= 31 && wz <= 31 &&
                            wx * wy * wz < 8192) {
                     // index and in-box counts in one register (march_packed_shared)
-                    const int packed = (idx << 18) | ((31 - cx) << 12) | ((31 - max(cy, -32)) << 6) | (31 - cz);
+                    int packed = (idx << 18) | ((31 - cx) << 12) | ((31 - max(cy, -32)) << 6) | (31 - cz);
                     b = march_packed_shared(base, packed, (dix << 18) + (1 << 12), (diy << 18) + (1 << 6),
                                             (diz << 18) + 1, tmx, tmy, tmz, tdx, tdy, tdz,
                                             staged_range(base, wxz, nvox));
                 } else {
-                    b = march_split_shared(base + idx, split_counts(cx, cy, cz, max_steps, wx, wy, wz), dix, diy,
-                                           diz, tmx, tmy, tmz, tdx, tdy, tdz, staged_range(base, wxz, nvox));
+                    int cnt = split_counts(cx, cy, cz, max_steps, wx, wy, wz);
+                    b = march_split_shared(base + idx, cnt, dix, diy, diz, tmx, tmy, tmz, tdx, tdy, tdz, staged_range(base, wxz, nvox));
                 }
                 if (b >= 0) {
                     // the axis of the last step, chosen again from the same distances
@@ -1995,16 +2025,45 @@ struct FastEnv {
     uint32_t base;      // staged world (packed) / the eye voxel's address in it (split)
     SmemRange chk;      // the staged world +- one layer (debug build)
     float vd, rcp_vd;
+    int wx, wy, wz, max_steps;  // ground-shortcut family only
 };
+
+// The ground-shortcut family's rays that leave the box sideways on their way
+// down: the reference goes on stepping while t <= the box's exit distance
+// (rounding puts the accumulated t on either side of it) and still paints the
+// ground if such a step enters it.  bx, by: the axis of the step that left the
+// box (tm not advanced for it yet); yleft: layers left above the ground; step:
+// voxels stepped.  Returns whether the ray ends in the ground, *t its distance.
+__device__ __forceinline__ bool ground_tail(const Cam& c, const FastEnv& fe, float ix, float iy, float iz, float tmx,
+                                            float tmy, float tmz, bool bx, bool by, int yleft, int step, float* t) {
+    const float lo_x = N::sub(0.0f, c.eye_x), hi_x = N::sub((float)fe.wx, c.eye_x);
+    const float lo_y = N::sub(0.0f, c.eye_y), hi_y = N::sub((float)fe.wy, c.eye_y);
+    const float lo_z = N::sub(0.0f, c.eye_z), hi_z = N::sub((float)fe.wz, c.eye_z);
+    float entry;
+    const float t_exit = aabb_exit(ix, iy, iz, lo_x, hi_x, lo_y, hi_y, lo_z, hi_z, &entry);
+    while (!(*t >= fe.vd) && !(*t > t_exit) && step < fe.max_steps) {
+        if (bx) tmx = N::add(tmx, fabsf(ix));
+        else if (by) tmy = N::add(tmy, fabsf(iy));
+        else tmz = N::add(tmz, fabsf(iz));
+        bx = tmx < tmy && tmx < tmz;
+        by = !bx && tmy < tmz;
+        *t = bx ? tmx : (by ? tmy : tmz);
+        ++step;
+        if (by && --yleft < 0) return step < fe.max_steps && !(*t >= fe.vd);
+    }
+    return false;
+}
 
 template <int FAM, bool F32, bool SPLIT, bool ODD>
 __device__ __forceinline__ void fast_band(const Cam& c, const Dda0& d0, const FastEnv& fe, int W, int H, int TW,
                                           int row0, int lane, const float* s_u, const float* s_v, const float4* s_cs,
                                           const uint32_t* s_rgbp, uint8_t* stage, uint8_t* dst) {
-    constexpr bool SHADED = FAM == MC_FAM_SHADED;
+    constexpr bool GROUND = FAM == MC_FAM_SHADED_FAST;
+    constexpr bool SHADED = FAM == MC_FAM_SHADED || GROUND;
+    constexpr bool HALF = FAM == MC_FAM_FP16;
     constexpr bool TRIG = FAM != MC_FAM_PREBASIS;
     constexpr int bpp = 3 * (F32 ? 4 : 1);
-    constexpr int m = F32 ? 0x1 : 0x3;  // sky_fused_mask of the float32 / uint8 shaded kernels
+    constexpr int m = F32 ? 0x1 : (GROUND ? MC_FASTG_SKY : 0x3);  // sky_fused_mask of the family's kernel
     const float sky0 = 0.53f, sky1 = 0.81f, sky2 = 0.92f;  // SKY_COLOR (c_sky)
     const int TH = 32 / TW;
     const int lx = lane % TW, ly = lane / TW;
@@ -2036,25 +2095,55 @@ __device__ __forceinline__ void fast_band(const Cam& c, const Dda0& d0, const Fa
             y = N::mul(y, rs);
             z = N::mul(z, rs);
         }
-        const float ix = (x != 0.0f) ? N::div(1.0f, x) : 1e30f;
-        const float iy = (y != 0.0f) ? N::div(1.0f, y) : 1e30f;
-        const float iz = (z != 0.0f) ? N::div(1.0f, z) : 1e30f;
+        constexpr float kNone = HALF ? 65504.0f : 1e30f;
+        const float ix = (x != 0.0f) ? N::div(1.0f, x) : kNone;
+        const float iy = (y != 0.0f) ? N::div(1.0f, y) : kNone;
+        const float iz = (z != 0.0f) ? N::div(1.0f, z) : kNone;
         const bool xp = x >= 0.0f, yp = y >= 0.0f, zp = z >= 0.0f;
         float tmx = N::mul(xp ? d0.nxp : d0.nxm, ix);
         float tmy = N::mul(yp ? d0.nyp : d0.nym, iy);
         float tmz = N::mul(zp ? d0.nzp : d0.nzm, iz);
-        const int4 e = fe.start[(xp ? 1 : 0) | (yp ? 2 : 0) | (zp ? 4 : 0)];
-        const int b = SPLIT ? march_split_shared(fe.base, e.x, e.y, e.z, e.w, tmx, tmy, tmz, fabsf(ix), fabsf(iy),
-                                                 fabsf(iz), fe.chk)
-                            : march_packed_shared(fe.base, e.x, e.y, e.z, e.w, tmx, tmy, tmz, fabsf(ix), fabsf(iy),
-                                                  fabsf(iz), fe.chk);
+        int4 e = fe.start[(xp ? 1 : 0) | (yp ? 2 : 0) | (zp ? 4 : 0)];
+        int b;
+        if constexpr (HALF) {
+            auto h = [](float f) { return __half_as_ushort(__float2half(f)); };
+            unsigned short hx = h(tmx), hy = h(tmy), hz = h(tmz);
+            b = SPLIT ? march_split_shared(fe.base, e.x, e.y, e.z, e.w, hx, hy, hz, h(fabsf(ix)), h(fabsf(iy)),
+                                           h(fabsf(iz)), fe.chk)
+                      : march_packed_shared(fe.base, e.x, e.y, e.z, e.w, hx, hy, hz, h(fabsf(ix)), h(fabsf(iy)),
+                                            h(fabsf(iz)), fe.chk);
+        } else {
+            b = SPLIT ? march_split_shared(fe.base, e.x, e.y, e.z, e.w, tmx, tmy, tmz, fabsf(ix), fabsf(iy), fabsf(iz),
+                                           fe.chk)
+                      : march_packed_shared(fe.base, e.x, e.y, e.z, e.w, tmx, tmy, tmz, fabsf(ix), fabsf(iy),
+                                            fabsf(iz), fe.chk);
+        }
         if (SHADED) {
             // the axis of the last step, chosen again from the same distances
             const bool bx = tmx < tmy && tmx < tmz;
             const bool by = !bx && tmy < tmz;
-            const float t = bx ? tmx : (by ? tmy : tmz);
+            float t = bx ? tmx : (by ? tmy : tmz);
+            int code = bx ? 0 : (by ? (yp ? 3 : 2) : 1);
+            if (GROUND && b < 0 && !yp) {
+                // a ray going down that left the box: into the ground (grass,
+                // from above), sideways, or out of steps (split march)
+                constexpr int kOutX = SPLIT ? 1 << 13 : 32 << 12, kOutY = SPLIT ? 1 << 20 : 32 << 6,
+                              kOutZ = SPLIT ? 1 << 6 : 32, kSpent = SPLIT ? 1 << 29 : 0;
+                if (!(e.x & kSpent)) {
+                    if (e.x & kOutY) {
+                        b = GRASS;
+                    } else if (e.x & (kOutX | kOutZ)) {
+                        const int yleft = SPLIT ? 63 - ((e.x >> 14) & 127) : 31 - ((e.x >> 6) & 63);
+                        const int s0 = fe.max_steps > fe.wx + fe.wy + fe.wz ? 0 : 256 - fe.max_steps;
+                        const int step = SPLIT ? ((e.x >> 21) & 511) - s0 : 0;
+                        if (ground_tail(c, fe, ix, iy, iz, tmx, tmy, tmz, bx, by, yleft, step, &t)) {
+                            b = GRASS;
+                            code = 2;
+                        }
+                    }
+                }
+            }
             const bool hit = b >= 0 && !(t >= fe.vd);
-            const int code = bx ? 0 : (by ? (yp ? 3 : 2) : 1);
             const float4 cs = s_cs[(b >= 0 ? b : 0) * 4 + code];
             float fog = fminf(N::div_r(t, fe.vd, fe.rcp_vd), 1.0f);
             fog = N::mul(fog, fog);
@@ -2106,11 +2195,11 @@ __device__ __forceinline__ void fast_band(const Cam& c, const Dda0& d0, const Fa
 // Start values of march_split_shared for an env whose eye is in voxel (vx,
 // vy, vz), one per sign combination k of the ray (as packed_start): {counts,
 // x, y and z address steps}; the start address is the eye voxel's.
-__device__ __forceinline__ int4 split_start(int k, int vx, int vy, int vz, int wx, int wy, int wz,
+__device__ __forceinline__ int4 split_start(int k, int vx, int vy, int vz, int wx, int wy, int wz, int ylow,
                                             const UpBounds& ub, int max_steps) {
     const int sx = (k & 1) ? 1 : -1, sy = (k & 2) ? 1 : -1, sz = (k & 4) ? 1 : -1;
     int cx, cy, cz;
-    start_counts(k, vx, vy, vz, wx, wy, wz, ub, cx, cy, cz);
+    start_counts(k, vx, vy, vz, wx, wy, wz, ylow, ub, cx, cy, cz);
     return make_int4(split_counts(cx, cy, cz, max_steps, wx, wy, wz), sx * wz, sy * wx * wz, sz);
 }
 
@@ -2119,17 +2208,18 @@ __device__ __forceinline__ int4 split_start(int k, int vx, int vy, int vz, int w
 // box within view distance), 2 split.
 template <int FAM>
 __device__ __forceinline__ int fast_kind(bool vd_safe, int max_steps, int wx, int wy, int wz) {
-    const bool packed = (FAM == MC_FAM_SHADED ? vd_safe : true) && max_steps > wx + wy + wz && wx <= 31 &&
-                        wy <= 31 && wz <= 31 && wx * wy * wz < 8192;
+    constexpr bool G = FAM == MC_FAM_SHADED_FAST;  // its rays may step on outside the box (ground_tail)
+    const bool packed = (FAM == MC_FAM_SHADED || G ? vd_safe : true) && max_steps > wx + wy + wz + (G ? 8 : 0) &&
+                        wx <= 31 && wy <= 31 && wz <= 31 && wx * wy * wz < 8192;
     return packed ? 1 : 2;
 }
 
 // The per-env start table (8 lanes write, the warp reads).
 __device__ __forceinline__ void build_fast_start(int4* sstart, int kind, const Dda0& d0, int wx, int wy, int wz,
-                                                 const UpBounds& ub, int max_steps, int lane) {
+                                                 int ylow, const UpBounds& ub, int max_steps, int lane) {
     if (lane < 8)
-        sstart[lane] = kind == 1 ? packed_start(lane, d0.vx, d0.vy, d0.vz, wx, wy, wz, ub)
-                                 : split_start(lane, d0.vx, d0.vy, d0.vz, wx, wy, wz, ub, max_steps);
+        sstart[lane] = kind == 1 ? packed_start(lane, d0.vx, d0.vy, d0.vz, wx, wy, wz, ylow, ub)
+                                 : split_start(lane, d0.vx, d0.vy, d0.vz, wx, wy, wz, ylow, ub, max_steps);
     __syncwarp();
 }
 
@@ -2237,7 +2327,7 @@ __device__ __forceinline__ void rec_facts(EnvRec& r, const mc_kp& p, bool eye_in
         skip_first = p.max_steps > 0 && !(eye_inb && eye_blk >= 0);
     }
     // the common case: the launch allows it, and the eye is inside the box with air in its voxel
-    const bool fast = p.fast_ok && skip_first && (FAM == MC_FAM_SHADED || eye_inb);
+    const bool fast = p.fast_ok && skip_first && (FAM == MC_FAM_SHADED || FAM == MC_FAM_SHADED_FAST || eye_inb);
     r.bits = (done ? MC_ER_DONE : 0) | (buried ? MC_ER_BURIED : 0) | (inside ? MC_ER_INSIDE : 0) |
              (skip_first ? MC_ER_SKIP : 0) | (!buried && !fast ? MC_ER_SLOW : 0);
 }
@@ -2728,11 +2818,6 @@ __device__ __forceinline__ void render_slow(const mc_kp& p, const EnvRec& q, int
         render_slow_from<FAM, F32>(p, q.env, r, cx, VoxGlobal{world}, tile_w, lane, band_ctr);
 }
 
-// Whether a family has the common-case loop (fast_band).
-__host__ __device__ constexpr bool fast_family(int fam) {
-    return fam == MC_FAM_SHADED || fam == MC_FAM_MINIMAL || fam == MC_FAM_PREBASIS;
-}
-
 // Row bands of slice `part` of `slices` of env e's image by one warp
 // (next_band) in the common case: the launch allows it (mc_fast_launch), the
 // world is staged, the eye is inside the box with air in its voxel.
@@ -2746,7 +2831,8 @@ __device__ __forceinline__ void render_fast(const mc_kp& p, int e, const EnvRend
     const bool vd_safe = box_within_view(r.c, p.wx, p.wy, p.wz, p.vd);
     const int fk = fast_kind<FAM>(vd_safe, p.max_steps, p.wx, p.wy, p.wz);
     const Dda0 d0 = dda0(r.c);
-    build_fast_start(cx.sstart, fk, d0, p.wx, p.wy, p.wz, r.ub, p.max_steps, lane);
+    build_fast_start(cx.sstart, fk, d0, p.wx, p.wy, p.wz, FAM == MC_FAM_SHADED_FAST ? p.gh : 0, r.ub, p.max_steps,
+                     lane);
     const uint32_t wb = smem_u32(staged);
     const int wxz = p.wx * p.wz;
     FastEnv fe;
@@ -2755,6 +2841,10 @@ __device__ __forceinline__ void render_fast(const mc_kp& p, int e, const EnvRend
     fe.chk = staged_range(wb, wxz, wxz * p.wy);
     fe.vd = p.vd;
     fe.rcp_vd = N::rcp_of(p.vd);
+    fe.wx = p.wx;
+    fe.wy = p.wy;
+    fe.wz = p.wz;
+    fe.max_steps = p.max_steps;
     const int H = p.H, nb = (H + TH - 1) / TH, b0 = part * nb / slices, nbands = (part + 1) * nb / slices - b0;
     const bool odd = p.fast_ok == 2;
     for (int b = next_band(band_ctr, -1, lane); b < nbands; b = next_band(band_ctr, b, lane)) {
@@ -2854,7 +2944,7 @@ __global__ void __launch_bounds__(256, MC_FUSED_MIN_BLOCKS)
     const EnvRec* recs = reinterpret_cast<const EnvRec*>(p.rec);
     const int first = blockIdx.x * nwarps + warp;
     const int any_done = regen_any(p);
-    if constexpr (STAGE && fast_family(FAM)) {
+    if constexpr (STAGE) {
         const int units = p.B * slices;
         int u = p.sched_dynamic ? next_unit(p, MC_FLAG_WORK, 0, total_warps, lane) : first;
         for (; u < units; u = next_unit(p, MC_FLAG_WORK, u, total_warps, lane)) {
@@ -2900,7 +2990,7 @@ __global__ void __launch_bounds__(256, MC_FUSED_MIN_BLOCKS)
     }
     // the general pass: the envs that the common path left (every env of a
     // launch that has no common path)
-    constexpr bool all = !(STAGE && fast_family(FAM));
+    constexpr bool all = !STAGE;
     const int any_slow = __shfl_sync(0xffffffffu, *(volatile int32_t*)&p.flags[MC_FLAG_ANY_SLOW], 0);
     if (all || !p.sched_dynamic || any_slow) {
         int u = p.sched_dynamic ? next_unit(p, MC_FLAG_SLOW_WORK, 0, total_warps, lane) : first;
@@ -3185,7 +3275,7 @@ __global__ void __launch_bounds__(256, MC_TEAM_MIN_BLOCKS) k_render_team(const _
         regen_world(p, e, wt * 32 + lane, nthr);
     };
 
-    if constexpr (fast_family(FAM)) {
+    {
         int k = 0;
         bool redo = false;
         if (DEPTH > 1 && ts->unit[0] < total_units) issue(locate(ts->unit[0]), 0, 0);
@@ -3265,11 +3355,9 @@ __global__ void __launch_bounds__(256, MC_TEAM_MIN_BLOCKS) k_render_team(const _
             }
         }
     }
-    // the general pass: the envs that the common path left (every env of a
-    // family that has no common path)
-    constexpr bool all = !fast_family(FAM);
+    // the general pass: the envs that the common path left
     if (claimer) {
-        ts->sunit[0] = all || *(volatile int32_t*)&rk.flags[MC_FLAG_ANY_SLOW] ? claim(MC_FLAG_SLOW_WORK) : total_units;
+        ts->sunit[0] = *(volatile int32_t*)&rk.flags[MC_FLAG_ANY_SLOW] ? claim(MC_FLAG_SLOW_WORK) : total_units;
         ts->may_stage[0] = !*(volatile int*)&ts->timed_out;
         team_unit_reset(ts, 0);
     }
@@ -3288,19 +3376,15 @@ __global__ void __launch_bounds__(256, MC_TEAM_MIN_BLOCKS) k_render_team(const _
             const EnvRec q = load_rec(recs_of(t.g), t.i);
             bits = q.bits;
             env = q.env;
-            here = t.part == 0 && (all || (q.bits & MC_ER_SLOW));
+            here = t.part == 0 && (q.bits & MC_ER_SLOW);
             use_group(t.g);
-            if (!here) {
-                // another pass's env
-            } else if (q.bits & MC_ER_SLOW) {
+            if (here) {
                 const int8_t* world = staged_world(t, q, 0);
                 const bool staged = may_stage && landed(t, 0);
                 const int ytop = staged ? staged_top_layer(world, p.wx, p.wy, p.wz, lane) : p.wy - 1;
                 render_slow<FAM, F32>(p, q, ytop, cx, staged ? world : nullptr,
                                       world_of(p, q.env, q.bits, (ts->any_done >> t.g) & 1), rk.tile_w[t.g], lane,
                                       t.coop ? &ts->band_ctr[k & 1] : nullptr);
-            } else {
-                fill_env<FAM, F32>(p, q.env, q.fill_blk, cx, t.coop ? wt * 32 + lane : lane, t.coop ? nthr : 32);
             }
         }
         if (claimer) {

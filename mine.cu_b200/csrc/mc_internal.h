@@ -213,13 +213,12 @@ static inline int mc_band_bytes(int W, int H, int obs_f32, int tile_w) {
 }
 
 // Whether a launch that stages its worlds (stage) has the images' common path
-// for this env's configuration: a family with a common-case loop, no debug
-// output, worlds within the marches' 64-voxel counts.  1: images of whole
+// for this env's configuration: no debug output, worlds within the marches' 64-voxel counts.  1: images of whole
 // tiles in 16-byte pieces; 2: any others (fast_band<ODD>).
 static inline int mc_fast_launch(const mc_kp& k, int stage, int tile_w) {
-    if (!(k.family == MC_FAM_SHADED || k.family == MC_FAM_MINIMAL || k.family == MC_FAM_PREBASIS)) return 0;
     if (!stage || k.dbg_pixel || k.max_steps <= 0 || k.wx > 64 || k.wy > 64 || k.wz > 64) return 0;
-    if (k.family == MC_FAM_SHADED && !(k.vd > 0.0f)) return 0;
+    if ((k.family == MC_FAM_SHADED || k.family == MC_FAM_SHADED_FAST) && !(k.vd > 0.0f)) return 0;
+    if (k.family == MC_FAM_SHADED_FAST && k.gh < 0) return 0;
     if (k.obs_f32 && (((uintptr_t)k.obs) & 3)) return 0;
     if (!mc_whole_tiles(k.W, k.H, k.obs_f32, tile_w)) return 2;
     return (((uintptr_t)k.obs) & 15) ? 0 : 1;

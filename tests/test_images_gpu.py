@@ -124,3 +124,20 @@ def test_big_worlds(cuda, world):
     """Worlds above 32 KB, with the default launch shape (as many staged worlds as an SM holds, or none)."""
     run(cuda, 5, 5, 59, world=world, res=(64, 48), obs_dtype="uint8", episode_length=3, regen="per_env")
     run(cuda, 2, 4, 60, world=world, res=(31, 20), obs_dtype="uint8_minimal", episode_length=3)
+
+
+@pytest.mark.parametrize("mode", ["uint8_fast", "uint8_fp16"])
+@pytest.mark.parametrize("kw", [dict(), dict(world=(32, 32, 32), res=(64, 64)), dict(world=(9, 20, 13), res=(21, 17)),
+                                dict(max_steps=20, view_distance=6.0), dict(max_steps=3, view_distance=2.5),
+                                dict(world=(24, 16, 20), ground_height=4, max_steps=61),
+                                dict(world=(6, 24, 6), res=(48, 48), ground_height=2, max_steps=37),
+                                dict(world=(16, 16, 16), ground_height=0)],
+                         ids=lambda k: "_".join(f"{a}{b}" for a, b in k.items()).replace(" ", "") or "c1")
+def test_ground_shortcut_and_fp16(cuda, mode, kw):
+    """The fast marches of the ground-shortcut and binary16 families: rays that
+    enter the ground, leave the box sideways above it, run out of steps or of
+    view."""
+    for cfg in (None, (1, 8, 3, 8, 4, 1)):
+        if cfg and (np.prod(kw.get("world", (16, 16, 16))) % 16):
+            cfg = (0,) + cfg[1:]
+        run(cuda, 14, 10, 61, obs_dtype=mode, cfg=cfg, episode_length=7, regen="per_env", **kw)
