@@ -1682,7 +1682,7 @@ __host__ __device__ inline FusedLayout fused_layout(int W, int H, int slot, int 
     L.H = H;
     L.tile_w = tile_w;
     L.tile_h = 32 / tile_w;
-    L.stage_bytes = mc_band_bytes(W, H, obs_f32, tile_w);
+    L.stage_bytes = mc_band_bytes(W, H, obs_f32, tile_w, 0);
     L.world_bytes = stage ? slot : 0;
     L.warp_bytes = 16 + 128 + L.stage_bytes + L.world_bytes;  // 16: mbarrier, 128: packed_start table
     L.head_bytes = kFastTableBytes + mc_align16((W + H) * 4 + 13 * 3 * 4 + 16 + 13 * 3 + 3);
@@ -2020,6 +2020,11 @@ __device__ __forceinline__ UpBounds staged_up_bounds(const int8_t* world, int wx
 // pixel's ray again and store nothing, and the band is staged at dst's offset
 // from a 16-byte boundary, so that all but its first and last bytes still go
 // out in 16-byte stores (`stage` has 16 bytes to spare).
+// TEAM: the team kernel stages float32 pixels two tiles at a time instead (64
+// pixels, 768 bytes, whose row pieces are whole 16-byte chunks; with ODD they go
+// straight to dst): beside 32 KB worlds, whole bands of 128-pixel rows (6 KB a
+// warp) left one CTA on an SM (4096 envs 32^3 128x128: 1151 -> 713 us a step).
+// The per-warp kernel keeps whole bands (32x32: 174 us a step, two tiles 186).
 struct FastEnv {
     const int4* start;  // per sign combination: packed (index|counts, dx, dy, dz) or split (counts, dax, day, daz)
     uint32_t base;      // staged world (packed) / the eye voxel's address in it (split)
@@ -2054,10 +2059,11 @@ __device__ __forceinline__ bool ground_tail(const Cam& c, const FastEnv& fe, flo
     return false;
 }
 
-template <int FAM, bool F32, bool SPLIT, bool ODD>
+template <int FAM, bool F32, bool SPLIT, bool ODD, bool TEAM>
 __device__ __forceinline__ void fast_band(const Cam& c, const Dda0& d0, const FastEnv& fe, int W, int H, int TW,
                                           int row0, int lane, const float* s_u, const float* s_v, const float4* s_cs,
                                           const uint32_t* s_rgbp, uint8_t* stage, uint8_t* dst) {
+    constexpr bool PAIRS = F32 && TEAM && !ODD, DIRECT = F32 && TEAM && ODD;  // how float32 pixels leave
     constexpr bool GROUND = FAM == MC_FAM_SHADED_FAST;
     constexpr bool SHADED = FAM == MC_FAM_SHADED || GROUND;
     constexpr bool HALF = FAM == MC_FAM_FP16;
@@ -2070,8 +2076,8 @@ __device__ __forceinline__ void fast_band(const Cam& c, const Dda0& d0, const Fa
     const bool in_y = !ODD || row0 + ly < H;
     const float v = s_v[ODD ? min(row0 + ly, H - 1) : row0 + ly];
     const float yraw = N::mad(v, c.uy, c.fy);
-    if (ODD) stage += (uint32_t)(uintptr_t)dst & 15u;
-    uint8_t* sp = stage + (ly * W + lx) * bpp;
+    if (ODD && !DIRECT) stage += (uint32_t)(uintptr_t)dst & 15u;
+    uint8_t* sp = DIRECT ? dst + (ly * W + lx) * bpp : stage + (ly * (PAIRS ? 2 * TW : W) + lx) * bpp;
     for (int tx0 = 0; tx0 < W; tx0 += TW, sp += TW * bpp) {
         const bool in = !ODD || (in_y && tx0 + lx < W);
         const float u = s_u[ODD ? min(tx0 + lx, W - 1) : tx0 + lx];
@@ -2172,7 +2178,21 @@ __device__ __forceinline__ void fast_band(const Cam& c, const Dda0& d0, const Fa
                 sp[2] = (uint8_t)(col >> 16);
             }
         }
+        if (PAIRS && ((tx0 & TW) || tx0 + TW == W)) {
+            // these one or two tiles' rows, 16 bytes a lane
+            const int first = tx0 & ~(2 * TW - 1), cols = tx0 + TW - first, cpr = cols * 3 / 4, n = TH * cpr;
+            const int inv = 65536 / cpr + 1;  // k / cpr for k < 48
+            __syncwarp();
+            for (int k = lane; k < n; k += 32) {
+                const int row = (k * inv) >> 16, piece = k - row * cpr;
+                *reinterpret_cast<uint4*>(dst + (row * W + first) * bpp + piece * 16) =
+                    *reinterpret_cast<const uint4*>(stage + row * 2 * TW * bpp + piece * 16);
+            }
+            __syncwarp();
+            sp = stage + (ly * 2 * TW + lx) * bpp - TW * bpp;
+        }
     }
+    if (PAIRS || DIRECT) return;
     __syncwarp();
     // copy the band (rows row0 .. row0+TH-1) out with 16-byte stores
     int bytes = W * TH * bpp;
@@ -2742,7 +2762,6 @@ __device__ __forceinline__ void render_slow_from(const mc_kp& p, int e, const En
     const float vd = p.vd;
     const long long obs_env_bytes = (long long)W * H * 3 * (F32 ? 4 : 1);
     uint8_t* oenv = (uint8_t*)p.obs + e * obs_env_bytes;
-    const bool vec_ok = ((obs_env_bytes & 15) == 0) && ((((uintptr_t)oenv) & 15) == 0);
     const bool inside = (r.bits & MC_ER_INSIDE) != 0, skip_first = (r.bits & MC_ER_SKIP) != 0;
     const MarchFacts mf = march_facts<FAM>(p, r);
     const Dda0 d0 = dda0(r.c);
@@ -2759,50 +2778,30 @@ __device__ __forceinline__ void render_slow_from(const mc_kp& p, int e, const En
             if (px < W && py < H && in_bounds(px, W, MC_SITE_TABLE)) {
                 const float u = cx.s_u[px];
                 Hit h = march_pixel<FAM, V>(rp, r.c, d0, u, v, vox, inside, skip_first, mf.sky_exit, mf.vd_safe, r.ytop);
-                const int so = ly * W + px;  // pixel within the staged band
-                if (!in_bounds((long long)(so + 1) * bpp - 1, (long long)TH * W * bpp, MC_SITE_BAND)) continue;
+                if (!in_bounds(((long long)py * W + px + 1) * bpp - 1, obs_env_bytes, MC_SITE_COPY_OUT)) continue;
+                uint8_t* o = oenv + ((long long)py * W + px) * bpp;
                 if (FAM == MC_FAM_SHADED || FAM == MC_FAM_SHADED_FAST) {
                     float rgb[3];
                     shade_rgb<F32 ? MC_COL_F32 : (FAM == MC_FAM_SHADED_FAST ? MC_COL_U8FAST : MC_COL_U8)>(
                         h, vd, cx.rcp_vd, cx.s_rgb, cx.s_sky, rgb);
                     if (F32) {
-                        float* sf = reinterpret_cast<float*>(cx.stage) + so * 3;
-                        sf[0] = rgb[0];
-                        sf[1] = rgb[1];
-                        sf[2] = rgb[2];
+#pragma unroll
+                        for (int k = 0; k < 12; ++k) o[k] = (uint8_t)(__float_as_uint(rgb[k >> 2]) >> (8 * (k & 3)));
                     } else {
-                        uint8_t* sb = cx.stage + so * 3;
-                        sb[0] = (uint8_t)to_u8(rgb[0]);
-                        sb[1] = (uint8_t)to_u8(rgb[1]);
-                        sb[2] = (uint8_t)to_u8(rgb[2]);
+                        o[0] = (uint8_t)to_u8(rgb[0]);
+                        o[1] = (uint8_t)to_u8(rgb[1]);
+                        o[2] = (uint8_t)to_u8(rgb[2]);
                     }
                 } else {
                     const uint8_t* col = (h.blk >= 0 && in_bounds(h.blk, 13, MC_SITE_TABLE)) ? cx.s_rgb8[h.blk] : cx.s_sky8;
-                    uint8_t* sb = cx.stage + so * 3;
-                    sb[0] = col[0];
-                    sb[1] = col[1];
-                    sb[2] = col[2];
+                    o[0] = col[0];
+                    o[1] = col[1];
+                    o[2] = col[2];
                 }
                 if (dbg_pixel && in_bounds(py * W + px, W * H, MC_SITE_DEBUG))
                     dbg_pixel[(long long)e * W * H + py * W + px] = dbg_code(h);
             }
         }
-        __syncwarp();
-        // copy the band (rows row0 .. row0+TH-1) out
-        const int nbytes = min(TH, H - row0) * W * bpp;
-        uint8_t* dst = oenv + (long long)row0 * W * bpp;
-        if (!in_bounds((long long)row0 * W * bpp + nbytes - 1, obs_env_bytes, MC_SITE_COPY_OUT)) {
-            __syncwarp();
-            continue;
-        }
-        if (vec_ok && (nbytes & 15) == 0 && (((long long)row0 * W * bpp) & 15) == 0) {
-            const uint4* s4 = reinterpret_cast<const uint4*>(cx.stage);
-            uint4* d4 = reinterpret_cast<uint4*>(dst);
-            for (int k = lane; k < (nbytes >> 4); k += 32) d4[k] = s4[k];
-        } else {
-            for (int k = lane; k < nbytes; k += 32) dst[k] = cx.stage[k];
-        }
-        __syncwarp();
     }
 }
 
@@ -2821,7 +2820,7 @@ __device__ __forceinline__ void render_slow(const mc_kp& p, const EnvRec& q, int
 // Row bands of slice `part` of `slices` of env e's image by one warp
 // (next_band) in the common case: the launch allows it (mc_fast_launch), the
 // world is staged, the eye is inside the box with air in its voxel.
-template <int FAM, bool F32>
+template <int FAM, bool F32, bool TEAM>
 __device__ __forceinline__ void render_fast(const mc_kp& p, int e, const EnvRender& r, const FusedCtx& cx,
                                             const int8_t* staged, int tile_w, int lane, int* band_ctr, int part,
                                             int slices) {
@@ -2852,16 +2851,16 @@ __device__ __forceinline__ void render_fast(const mc_kp& p, int e, const EnvRend
         uint8_t* dst = oenv + row0 * W * bpp;
         if (odd) {
             if (fk == 1)
-                fast_band<FAM, F32, false, true>(r.c, d0, fe, W, H, TW, row0, lane, cx.s_u, cx.s_v, cx.s_cs,
+                fast_band<FAM, F32, false, true, TEAM>(r.c, d0, fe, W, H, TW, row0, lane, cx.s_u, cx.s_v, cx.s_cs,
                                                  cx.s_rgbp, cx.stage, dst);
             else
-                fast_band<FAM, F32, true, true>(r.c, d0, fe, W, H, TW, row0, lane, cx.s_u, cx.s_v, cx.s_cs,
+                fast_band<FAM, F32, true, true, TEAM>(r.c, d0, fe, W, H, TW, row0, lane, cx.s_u, cx.s_v, cx.s_cs,
                                                 cx.s_rgbp, cx.stage, dst);
         } else if (fk == 1) {
-            fast_band<FAM, F32, false, false>(r.c, d0, fe, W, H, TW, row0, lane, cx.s_u, cx.s_v, cx.s_cs, cx.s_rgbp,
+            fast_band<FAM, F32, false, false, TEAM>(r.c, d0, fe, W, H, TW, row0, lane, cx.s_u, cx.s_v, cx.s_cs, cx.s_rgbp,
                                               cx.stage, dst);
         } else {
-            fast_band<FAM, F32, true, false>(r.c, d0, fe, W, H, TW, row0, lane, cx.s_u, cx.s_v, cx.s_cs, cx.s_rgbp,
+            fast_band<FAM, F32, true, false, TEAM>(r.c, d0, fe, W, H, TW, row0, lane, cx.s_u, cx.s_v, cx.s_cs, cx.s_rgbp,
                                              cx.stage, dst);
         }
     }
@@ -2969,7 +2968,7 @@ __global__ void __launch_bounds__(256, MC_FUSED_MIN_BLOCKS)
                 }
                 phase ^= 1u;
                 measure_staged(r, world, p.wx, p.wy, p.wz, lane);
-                render_fast<FAM, F32>(p, q.env, r, cx, world, tile_w, lane, nullptr, part, slices);
+                render_fast<FAM, F32, false>(p, q.env, r, cx, world, tile_w, lane, nullptr, part, slices);
             }
             if (regen_env(p, q.bits, any_done) && last_slice(recs, i, slices, lane)) regen_world(p, q.env, lane, 32);
         }
@@ -3313,7 +3312,7 @@ __global__ void __launch_bounds__(256, MC_TEAM_MIN_BLOCKS) k_render_team(const _
                     else if (ok)
                         measure_staged(r, world, p.wx, p.wy, p.wz, lane);
                     if (ok)
-                        render_fast<FAM, F32>(p, q.env, r, cx, world, rk.tile_w[t.g], lane,
+                        render_fast<FAM, F32, true>(p, q.env, r, cx, world, rk.tile_w[t.g], lane,
                                               t.coop ? &ts->band_ctr[k & 1] : nullptr, t.part, rk.slices[t.g]);
                 }
             }

@@ -203,11 +203,14 @@ __host__ __device__
 static inline int mc_world_slot(const mc_kp& k) {
     return ((k.wx * k.wy * k.wz + 15) & ~15) + (mc_odd_world(k) ? 16 : 0);
 }
-// Shared-memory bytes of one staged band: 16 to spare where bands start at any byte.
+// Shared-memory bytes of the pixels a warp stages: one band, with 16 to spare
+// where bands start at any byte; the team
+// kernel's float32 pixels two tiles (fast_band).
 #ifdef __CUDACC__
 __host__ __device__
 #endif
-static inline int mc_band_bytes(int W, int H, int obs_f32, int tile_w) {
+static inline int mc_band_bytes(int W, int H, int obs_f32, int tile_w, int team) {
+    if (obs_f32 && team) return 64 * 12;
     const int n = W * (32 / tile_w) * (obs_f32 ? 12 : 3);
     return ((n + 15) & ~15) + (mc_whole_tiles(W, H, obs_f32, tile_w) ? 0 : 16);
 }

@@ -468,7 +468,7 @@ static void team_layout_of(const mc_kp* const* kps, int G, const int* stage, con
         rk->uv_off[g] = uv;
         uv += k.W + k.H;
         rk->tile_w[g] = tile_w[g];
-        band = std::max(band, mc_band_bytes(k.W, k.H, k.obs_f32, tile_w[g]));
+        band = std::max(band, mc_band_bytes(k.W, k.H, k.obs_f32, tile_w[g], 1));
         if (coop[g]) rk->coop_mask |= 1 << g;
         if (stage[g]) {
             rk->stage_mask |= 1 << g;
