@@ -2896,82 +2896,42 @@ __device__ __forceinline__ bool last_slice(const EnvRec* recs, int i, int slices
 #ifndef MC_FUSED_MIN_BLOCKS
 #define MC_FUSED_MIN_BLOCKS 4
 #endif
-// One warp per env: a persistent grid whose warps claim records, fill the
-// buried envs and march the others over their world, staged in shared memory
-// (STAGE) or in global memory.  Bound by instruction issue in the march; at
-// its 64-register budget 4 CTAs of 8 warps share an SM.
-//
-// A small batch would leave most of the GPU's warps without an env: its images
-// are cut into `slices` row ranges (slice_rows), each a unit of its own that stages
-// the env's world again (a few KB from L2).
-template <int FAM, bool F32, bool STAGE>
-__global__ void __launch_bounds__(256, MC_FUSED_MIN_BLOCKS)
-    k_render_warp(const __grid_constant__ mc_kp p, int tile_w, int slices) {
-    extern __shared__ __align__(16) uint8_t smem[];
-    const int lane = threadIdx.x & 31;
-    const int warp = threadIdx.x >> 5;
-    const int nwarps = blockDim.x >> 5;
-    const int W = p.W, H = p.H;
-    const int wxz = p.wx * p.wz;
-    const int wxyz = wxz * p.wy;
-    FusedLayout L = fused_layout(W, H, mc_world_slot(p), wxz, F32, STAGE, tile_w);
-
-    FusedCtx cx;
-    build_fast_tables(reinterpret_cast<float4*>(smem), reinterpret_cast<uint32_t*>(smem + kShadeTableBytes));
+// The per-warp kernel's shared memory as one warp sees it; returns its world slot.
+__device__ __forceinline__ int8_t* warp_ctx(const mc_kp& p, const FusedLayout& L, uint8_t* smem, int warp,
+                                            FusedCtx& cx) {
     cx.s_cs = reinterpret_cast<const float4*>(smem);
     cx.s_rgbp = reinterpret_cast<const uint32_t*>(smem + kShadeTableBytes);
     float* s_u = reinterpret_cast<float*>(smem + kFastTableBytes);
-    build_uv_tables<FAM>(p, s_u, s_u + W);
     cx.s_u = s_u;
-    cx.s_v = s_u + W;
-    load_colour_tables(reinterpret_cast<uint8_t*>(s_u + W + H), cx);
+    cx.s_v = s_u + L.W;
+    colour_tables(reinterpret_cast<uint8_t*>(s_u + L.W + L.H), cx);
     uint8_t* wbase = smem + L.head_bytes + warp * L.warp_bytes;
     cx.mbar_a = smem_u32(wbase);
     cx.sstart = reinterpret_cast<int4*>(wbase + 16);
     cx.stage = wbase + 16 + 128;
-    int8_t* sworld = reinterpret_cast<int8_t*>(wbase + 16 + 128 + L.stage_bytes);
     cx.rcp_vd = N::rcp_of(p.vd);
-    if (STAGE) mbar_init_warp(cx.mbar_a, lane);
-    __syncthreads();
-    pdl_trigger();
-    pdl_wait();
+    return reinterpret_cast<int8_t*>(wbase + 16 + 128 + L.stage_bytes);
+}
 
-    uint32_t phase = 0;
-    bool no_stage = false;  // a copy timed out: this warp renders from global memory from now on
-    bool pending = false;   // ... and that copy may still land
-    const int total_warps = gridDim.x * nwarps;
+// What a warp does besides the common path, out of line after its loop (so
+// that the loop keeps its registers): from unit u on, the units of a warp
+// whose copy timed out (no_stage), then its share of the general pass.
+// state: bit 0 the mbarrier's phase, bit 1 no_stage, bit 2 that copy may still land.
+template <int FAM, bool F32, bool STAGE>
+__device__ __noinline__ void warp_rest(const mc_kp& p, int tile_w, int slices, int u, int state) {
+    extern __shared__ __align__(16) uint8_t smem[];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+    const int wxyz = p.wx * p.wy * p.wz;
+    const FusedLayout L = fused_layout(p.W, p.H, mc_world_slot(p), p.wx * p.wz, F32, STAGE, tile_w);
+    FusedCtx cx;
+    int8_t* sworld = warp_ctx(p, L, smem, warp, cx);
+    uint32_t phase = state & 1;
+    bool no_stage = state & 2, pending = state & 4;
+    const int total_warps = gridDim.x * nwarps, first = blockIdx.x * nwarps + warp;
     const EnvRec* recs = reinterpret_cast<const EnvRec*>(p.rec);
-    const int first = blockIdx.x * nwarps + warp;
     const int any_done = regen_any(p);
-    if constexpr (STAGE) {
+    if (STAGE) {
         const int units = p.B * slices;
-        int u = p.sched_dynamic ? next_unit(p, MC_FLAG_WORK, 0, total_warps, lane) : first;
-        for (; u < units; u = next_unit(p, MC_FLAG_WORK, u, total_warps, lane)) {
-            const int i = u / slices, part = u - i * slices;
-            const EnvRec q = load_rec(recs, i);
-            if (q.bits & MC_ER_SLOW) continue;
-            if (q.bits & MC_ER_BURIED) {
-                if (part == 0) fill_env<FAM, F32>(p, q.env, q.fill_blk, cx, lane, 32);
-            } else {
-                if (!stage_fits(sworld, mc_world_slot(p))) {
-                    no_stage = true;
-                    break;
-                }
-                const int8_t* src = world_of(p, q.env, q.bits, any_done);
-                issue_world_copy(cx.mbar_a, sworld, src, wxyz, lane);
-                const int8_t* world = staged_at(sworld, src);
-                EnvRender r = render_of_rec(q, p.wy);
-                if (!mbar_wait(cx.mbar_a, phase, p.wait_polls)) {
-                    if (lane == 0) atomicExch(&p.flags[MC_FLAG_ERROR], MC_KERR_TMA_TIMEOUT);
-                    no_stage = pending = true;
-                    break;
-                }
-                phase ^= 1u;
-                measure_staged(r, world, p.wx, p.wy, p.wz, lane);
-                render_fast<FAM, F32, false>(p, q.env, r, cx, world, tile_w, lane, nullptr, part, slices);
-            }
-            if (regen_env(p, q.bits, any_done) && last_slice(recs, i, slices, lane)) regen_world(p, q.env, lane, 32);
-        }
         // a copy that timed out: this unit and the rest of the warp's, from
         // global memory (a slice's warp renders the whole image: the others'
         // pixels come out the same)
@@ -2992,7 +2952,7 @@ __global__ void __launch_bounds__(256, MC_FUSED_MIN_BLOCKS)
     constexpr bool all = !STAGE;
     const int any_slow = __shfl_sync(0xffffffffu, *(volatile int32_t*)&p.flags[MC_FLAG_ANY_SLOW], 0);
     if (all || !p.sched_dynamic || any_slow) {
-        int u = p.sched_dynamic ? next_unit(p, MC_FLAG_SLOW_WORK, 0, total_warps, lane) : first;
+        u = p.sched_dynamic ? next_unit(p, MC_FLAG_SLOW_WORK, 0, total_warps, lane) : first;
         for (; u < p.B; u = next_unit(p, MC_FLAG_SLOW_WORK, u, total_warps, lane)) {
             const EnvRec q = load_rec(recs, u);
             if (!all && !(q.bits & MC_ER_SLOW)) continue;
@@ -3023,6 +2983,79 @@ __global__ void __launch_bounds__(256, MC_FUSED_MIN_BLOCKS)
     // a timed-out copy may still be in flight: let it land (bounded, with the
     // default budget) before this warp's part of shared memory can be released
     if (STAGE && pending) mbar_wait(cx.mbar_a, phase);
+}
+
+// One warp per env: a persistent grid whose warps claim records, fill the
+// buried envs and march the others over their world, staged in shared memory
+// (STAGE) or in global memory.  Bound by instruction issue in the march; at
+// its 64-register budget 4 CTAs of 8 warps share an SM.
+//
+// A small batch would leave most of the GPU's warps without an env: its images
+// are cut into `slices` row ranges (slice_rows), each a unit of its own that stages
+// the env's world again (a few KB from L2).
+template <int FAM, bool F32, bool STAGE>
+__global__ void __launch_bounds__(256, MC_FUSED_MIN_BLOCKS)
+    k_render_warp(const __grid_constant__ mc_kp p, int tile_w, int slices) {
+    extern __shared__ __align__(16) uint8_t smem[];
+    const int lane = threadIdx.x & 31;
+    const int warp = threadIdx.x >> 5;
+    const int nwarps = blockDim.x >> 5;
+    const int total_warps = gridDim.x * nwarps;
+    {
+        const FusedLayout L = fused_layout(p.W, p.H, mc_world_slot(p), p.wx * p.wz, F32, STAGE, tile_w);
+        build_fast_tables(reinterpret_cast<float4*>(smem), reinterpret_cast<uint32_t*>(smem + kShadeTableBytes));
+        float* s_u = reinterpret_cast<float*>(smem + kFastTableBytes);
+        build_uv_tables<FAM>(p, s_u, s_u + L.W);
+        FusedCtx cx;
+        load_colour_tables(reinterpret_cast<uint8_t*>(s_u + L.W + L.H), cx);
+        if (STAGE) mbar_init_warp(smem_u32(smem + L.head_bytes + warp * L.warp_bytes), lane);
+    }
+    __syncthreads();
+    pdl_trigger();
+    pdl_wait();
+
+    int u = 0, state = 0;
+    if constexpr (STAGE) {
+        const int wxyz = p.wx * p.wy * p.wz;
+        const FusedLayout L = fused_layout(p.W, p.H, mc_world_slot(p), p.wx * p.wz, F32, STAGE, tile_w);
+        FusedCtx cx;
+        int8_t* sworld = warp_ctx(p, L, smem, warp, cx);
+        const EnvRec* recs = reinterpret_cast<const EnvRec*>(p.rec);
+        const int any_done = regen_any(p);
+        const int units = p.B * slices;
+        uint32_t phase = 0;
+        u = p.sched_dynamic ? next_unit(p, MC_FLAG_WORK, 0, total_warps, lane) : blockIdx.x * nwarps + warp;
+        for (; u < units; u = next_unit(p, MC_FLAG_WORK, u, total_warps, lane)) {
+            const int i = u / slices, part = u - i * slices;
+            const EnvRec q = load_rec(recs, i);
+            if (q.bits & MC_ER_SLOW) continue;
+            if (q.bits & MC_ER_BURIED) {
+                if (part == 0) fill_env<FAM, F32>(p, q.env, q.fill_blk, cx, lane, 32);
+            } else {
+                if (!stage_fits(sworld, mc_world_slot(p))) {
+                    state = 2;
+                    break;
+                }
+                const int8_t* src = world_of(p, q.env, q.bits, any_done);
+                issue_world_copy(cx.mbar_a, sworld, src, wxyz, lane);
+                const int8_t* world = staged_at(sworld, src);
+                EnvRender r = render_of_rec(q, p.wy);
+                if (!mbar_wait(cx.mbar_a, phase, p.wait_polls)) {
+                    if (lane == 0) atomicExch(&p.flags[MC_FLAG_ERROR], MC_KERR_TMA_TIMEOUT);
+                    state = 2 | 4;
+                    break;
+                }
+                phase ^= 1u;
+                measure_staged(r, world, p.wx, p.wy, p.wz, lane);
+                render_fast<FAM, F32, false>(p, q.env, r, cx, world, tile_w, lane, nullptr, part, slices);
+            }
+            if (regen_env(p, q.bits, any_done) && last_slice(recs, i, slices, lane)) regen_world(p, q.env, lane, 32);
+        }
+        state |= phase;
+    }
+    // (a launch whose worlds are not staged has no common path)
+    const int any_slow = __shfl_sync(0xffffffffu, *(volatile int32_t*)&p.flags[MC_FLAG_ANY_SLOW], 0);
+    if (!STAGE || !p.sched_dynamic || any_slow || (state & 2)) warp_rest<FAM, F32, STAGE>(p, tile_w, slices, u, state);
     // No CTA barrier here: warps leave as soon as their last env is done.
     if (lane == 0) {
         bounds_to_flags(p.flags);
