@@ -145,6 +145,12 @@ int mc_env_step(mc_env* env, const int8_t* buttons, const float* look, int form,
 /* The discrete form step(actions) of docs/environment.md:5-17: actions
  * uint8[B] in 0..10, look step = config.look_delta. */
 int mc_env_step_discrete(mc_env* env, const uint8_t* actions, int form, void* stream);
+/* Either form of the step (actions, or buttons + look with actions NULL),
+ * with every env's done also written to dones_out, uint8[B] on the device:
+ * the fresh tensor that MineEnv.step returns (`do_reset.clone()`,
+ * minecu/__init__.py:444) without a copy after the step. */
+int mc_env_step_dones(mc_env* env, const int8_t* buttons, const float* look, const uint8_t* actions, int form,
+                      uint8_t* dones_out, void* stream);
 /* The discrete step with host buffers: the reference's step(actions) as a
  * caller with a host-side policy drives it (minecu/__init__.py:304-444; its
  * rewards and dones are then copied back to the host).  actions uint8[B]
@@ -264,6 +270,10 @@ int64_t mc_ragged_smem_bytes(const mc_ragged* r);
 int mc_ragged_step(mc_ragged* r, const int8_t* buttons, const float* look, void* stream);
 /* One step of every group: discrete actions uint8[total]. */
 int mc_ragged_step_discrete(mc_ragged* r, const uint8_t* actions, void* stream);
+/* Either form of the step of every group, with every env's done also written
+ * to dones_out, uint8[total] in group order on the device. */
+int mc_ragged_step_dones(mc_ragged* r, const int8_t* buttons, const float* look, const uint8_t* actions,
+                         uint8_t* dones_out, void* stream);
 /* The discrete step of every group with host buffers, as mc_env_step_host:
  * actions uint8[total] from pinned host memory, every env's reward
  * float32[total] and done uint8[total] (concatenated in group order) to

@@ -3570,8 +3570,19 @@ static int launch_team_t(const mc_ragged_kp* rk, int warps_per_cta, int ctas_per
     int rc;
     if (FAM == MC_FAM_SHADED && rk->groups[0].look_only)  // one group
         rc = launch_pdl(k_look, rk->ablock[G], kAgentThreads, 0, s, rk->groups[0]);
-    else
+    else if (G == 1 && rk->flags == rk->groups[0].flags) {
+        // one env's own launch: a parameter block instead of sixteen
+        mc_kp p = rk->groups[0];
+        p.rec = rk->rec;
+        p.actions = rk->actions;
+        p.buttons = rk->buttons;
+        p.look = rk->look;
+        p.res_rewards = rk->rewards_cat;
+        p.res_dones = rk->dones_cat;
+        rc = launch_pdl(k_agent<FAM>, rk->ablock[G], kAgentThreads, 0, s, p);
+    } else {
         rc = launch_pdl(k_agent_groups<FAM>, rk->ablock[G], kAgentThreads, 0, s, *rk);
+    }
     if (rc) return rc;
     const bool deep = rk->depth == 2;
     auto kern = deep ? k_render_team<FAM, F32, 2> : k_render_team<FAM, F32, 1>;

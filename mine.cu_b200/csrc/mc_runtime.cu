@@ -935,6 +935,22 @@ extern "C" int mc_env_step_discrete(mc_env* e, const uint8_t* actions, int form,
     return do_step(e, nullptr, nullptr, actions, form, (cudaStream_t)stream);
 }
 
+extern "C" int mc_env_step_dones(mc_env* e, const int8_t* buttons, const float* look, const uint8_t* actions, int form,
+                                 uint8_t* dones_out, void* stream) {
+    NvtxRange nvtx("mc_env_step");
+    if (!e) return fail(MC_ERR_INVALID, "env is NULL");
+    const size_t B = (size_t)e->cfg.batch_size;
+    if (B && !actions && (!buttons || !look)) return fail(MC_ERR_INVALID, "actions, or buttons and look, are NULL");
+    if (!actions && (((uintptr_t)look) & 3)) return fail(MC_ERR_INVALID, "look must be 4-byte aligned");
+    cudaStream_t s = (cudaStream_t)stream;
+    const bool direct = form == MC_FORM_FUSED;  // the agent kernel writes them itself
+    int rc = do_step(e, actions ? nullptr : buttons, actions ? nullptr : look, actions, form, s, nullptr,
+                     direct ? dones_out : nullptr);
+    if (rc || direct || !dones_out || !B) return rc;
+    MC_CK(cudaMemcpyAsync(dones_out, e->kp.do_reset, B, cudaMemcpyDeviceToDevice, s));
+    return MC_OK;
+}
+
 namespace {
 // rewards (float[B]) and dones (byte[B]) of the step just run, copied into
 // one block so that one buffer pair per step goes back to the host
@@ -1084,23 +1100,15 @@ static int rollout_graph(mc_env* e, const uint8_t* actions, int32_t K, float* re
             same_fcfg(g.fcfg, e->fcfg))
             hit = &g;
     if (!hit) {
-        // capture K fused steps (+ conditional regeneration and output copies)
+        // capture K fused steps, which write each step's rewards and dones out themselves
         long long B = e->cfg.batch_size;
         cudaGraph_t graph = nullptr;
         MC_CK(cudaStreamBeginCapture(e->cap_stream, cudaStreamCaptureModeThreadLocal));
         int rc = MC_OK;
         for (int k = 0; k < K && rc == MC_OK; ++k) {
-            rc = do_step(e, nullptr, nullptr, actions + (long long)k * B, MC_FORM_FUSED, e->cap_stream);
-            if (rc == MC_OK && rewards_out) {
-                cudaError_t ce = cudaMemcpyAsync(rewards_out + (long long)k * B, e->kp.rewards, B * sizeof(float),
-                                                 cudaMemcpyDeviceToDevice, e->cap_stream);
-                if (ce) rc = cuda_fail(ce, "rollout copy");
-            }
-            if (rc == MC_OK && dones_out) {
-                cudaError_t ce = cudaMemcpyAsync(dones_out + (long long)k * B, e->kp.do_reset, B,
-                                                 cudaMemcpyDeviceToDevice, e->cap_stream);
-                if (ce) rc = cuda_fail(ce, "rollout copy");
-            }
+            rc = do_step(e, nullptr, nullptr, actions + (long long)k * B, MC_FORM_FUSED, e->cap_stream,
+                         rewards_out ? rewards_out + (long long)k * B : nullptr,
+                         dones_out ? dones_out + (long long)k * B : nullptr);
         }
         cudaError_t ce = cudaStreamEndCapture(e->cap_stream, &graph);
         if (rc) {
@@ -1434,6 +1442,17 @@ extern "C" int mc_ragged_step_discrete(mc_ragged* r, const uint8_t* actions, voi
     if (!r) return fail(MC_ERR_INVALID, "ragged handle is NULL");
     if (mc_ragged_total_envs(r) > 0 && !actions) return fail(MC_ERR_INVALID, "actions is NULL");
     return ragged_do_step(r, nullptr, nullptr, actions, (cudaStream_t)stream, false);
+}
+
+extern "C" int mc_ragged_step_dones(mc_ragged* r, const int8_t* buttons, const float* look, const uint8_t* actions,
+                                    uint8_t* dones_out, void* stream) {
+    NvtxRange nvtx("mc_ragged_step");
+    if (!r) return fail(MC_ERR_INVALID, "ragged handle is NULL");
+    if (mc_ragged_total_envs(r) > 0 && !actions && (!buttons || !look))
+        return fail(MC_ERR_INVALID, "actions, or buttons and look, are NULL");
+    if (!actions && (((uintptr_t)look) & 3)) return fail(MC_ERR_INVALID, "look must be 4-byte aligned");
+    return ragged_do_step(r, actions ? nullptr : buttons, actions ? nullptr : look, actions, (cudaStream_t)stream,
+                          false, nullptr, dones_out);
 }
 
 extern "C" int mc_ragged_step_host(mc_ragged* r, const uint8_t* host_actions, float* host_rewards,

@@ -373,6 +373,8 @@ void py_render_uint8_coalesced(torch::Tensor voxels, torch::Tensor basis, torch:
 // ---------------------------------------------------------------------------
 struct Env {
     mc_env* h = nullptr;
+    int64_t batch = 0;
+    c10::Device device{c10::kCUDA, 0};
     ~Env() {
         if (h) mc_env_destroy(h);
     }
@@ -439,6 +441,8 @@ std::shared_ptr<Env> env_create(py::dict cfg, py::dict state) {
     mc_env_config c = config_of(cfg);
     mc_env_state s = state_of(state);
     ck(mc_env_create(&c, &s, &e->h), "env_create");
+    e->batch = c.batch_size;
+    e->device = c10::Device(c10::kCUDA, c10::cuda::current_device());
     return e;
 }
 
@@ -469,6 +473,38 @@ void env_step_discrete(std::shared_ptr<Env> e, torch::Tensor actions, int form) 
     ck(mc_env_step_discrete(e->h, ptr<uint8_t>(actions), form, cur_stream()), "step");
 }
 
+// t as a contiguous tensor of type dt on `dev` (t itself when it is one).
+torch::Tensor as_input(const torch::Tensor& t, c10::Device dev, at::ScalarType dt) {
+    if (t.scalar_type() == dt && t.device() == dev && t.is_contiguous()) return t;
+    return t.to(dev, dt).contiguous();
+}
+
+// MineEnv.step in one call: discrete actions, or buttons + look; returns the
+// fresh dones tensor, written by the step.
+torch::Tensor env_step_dones(const std::shared_ptr<Env>& e, const torch::Tensor& buttons,
+                             const c10::optional<torch::Tensor>& look, int form) {
+    TORCH_CHECK(e && e->h, "the env is closed");
+    const c10::cuda::CUDAGuard guard(e->device);
+    const int64_t B = e->batch;
+    torch::Tensor b, l;
+    const bool discrete = !look.has_value() || !look->defined();
+    if (discrete) {
+        b = as_input(buttons, e->device, at::kByte);
+        TORCH_CHECK_VALUE(b.numel() == B, "actions must have ", B, " entries, got ", b.numel());
+    } else {
+        b = as_input(buttons, e->device, at::kChar);
+        l = as_input(*look, e->device, at::kFloat);
+        TORCH_CHECK_VALUE(b.dim() == 2 && b.size(0) == B && b.size(1) == 8 && l.dim() == 2 && l.size(0) == B &&
+                              l.size(1) == 2,
+                          "buttons must be [", B, ", 8] and look [", B, ", 2]");
+    }
+    torch::Tensor dones = at::empty({B}, at::TensorOptions().dtype(at::kBool).device(e->device));
+    ck(mc_env_step_dones(e->h, discrete ? nullptr : ptr<int8_t>(b), discrete ? nullptr : ptr<float>(l),
+                         discrete ? ptr<uint8_t>(b) : nullptr, form, ptr<uint8_t>(dones), cur_stream()),
+       "step");
+    return dones;
+}
+
 // Host tensors of mc_env_step_host: pinned CPU memory, contiguous, n entries.
 void need_pinned(const torch::Tensor& t, const char* name, std::initializer_list<at::ScalarType> dts, int64_t n) {
     TORCH_CHECK(!t.is_cuda(), name, " must be a host (CPU) tensor");
@@ -482,6 +518,8 @@ void need_pinned(const torch::Tensor& t, const char* name, std::initializer_list
 
 void env_step_host(std::shared_ptr<Env> e, torch::Tensor actions, torch::Tensor rewards, torch::Tensor dones,
                    int64_t batch, int form) {
+    TORCH_CHECK(e && e->h, "the env is closed");
+    const c10::cuda::CUDAGuard guard(e->device);
     need_pinned(actions, "actions", {at::kByte}, batch);
     need_pinned(rewards, "rewards_out", {at::kFloat}, batch);
     need_pinned(dones, "dones_out", {at::kBool, at::kByte}, batch);
@@ -490,7 +528,11 @@ void env_step_host(std::shared_ptr<Env> e, torch::Tensor actions, torch::Tensor 
        "step_host");
 }
 
-void env_host_join(std::shared_ptr<Env> e) { ck(mc_env_host_join(e->h, cur_stream()), "host_join"); }
+void env_host_join(std::shared_ptr<Env> e) {
+    TORCH_CHECK(e && e->h, "the env is closed");
+    const c10::cuda::CUDAGuard guard(e->device);
+    ck(mc_env_host_join(e->h, cur_stream()), "host_join");
+}
 
 void obs_to_policy(torch::Tensor obs, torch::Tensor out, int64_t layout) {
     need(obs, "obs", at::kByte);
@@ -628,6 +670,31 @@ void ragged_step_discrete(std::shared_ptr<Ragged> r, torch::Tensor actions) {
     ck(mc_ragged_step_discrete(r->h, ptr<uint8_t>(actions), cur_stream()), "ragged_step");
 }
 
+// RaggedBatch.step in one call; returns every env's done in one fresh tensor.
+torch::Tensor ragged_step_dones(const std::shared_ptr<Ragged>& r, const torch::Tensor& buttons,
+                                const c10::optional<torch::Tensor>& look) {
+    const c10::Device dev = r->groups[0]->device;
+    const c10::cuda::CUDAGuard guard(dev);
+    const int64_t n = mc_ragged_total_envs(r->h);
+    torch::Tensor b, l;
+    const bool discrete = !look.has_value() || !look->defined();
+    if (discrete) {
+        b = as_input(buttons, dev, at::kByte);
+        TORCH_CHECK_VALUE(b.numel() == n, "actions must have ", n, " entries, got ", b.numel());
+    } else {
+        b = as_input(buttons, dev, at::kChar);
+        l = as_input(*look, dev, at::kFloat);
+        TORCH_CHECK_VALUE(b.dim() == 2 && b.size(0) == n && b.size(1) == 8 && l.dim() == 2 && l.size(0) == n &&
+                              l.size(1) == 2,
+                          "buttons must be [", n, ", 8] and look [", n, ", 2]");
+    }
+    torch::Tensor dones = at::empty({n}, at::TensorOptions().dtype(at::kBool).device(dev));
+    ck(mc_ragged_step_dones(r->h, discrete ? nullptr : ptr<int8_t>(b), discrete ? nullptr : ptr<float>(l),
+                            discrete ? ptr<uint8_t>(b) : nullptr, ptr<uint8_t>(dones), cur_stream()),
+       "ragged_step");
+    return dones;
+}
+
 void ragged_step_host(std::shared_ptr<Ragged> r, torch::Tensor actions, torch::Tensor rewards, torch::Tensor dones) {
     const int64_t n = mc_ragged_total_envs(r->h);
     need_pinned(actions, "actions", {at::kByte}, n);
@@ -731,6 +798,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     m.def("env_reset", &env_reset, py::arg("env"), py::arg("mask") = py::none());
     m.def("env_step", &env_step);
     m.def("env_step_discrete", &env_step_discrete);
+    m.def("env_step_dones", &env_step_dones);
     m.def("env_step_host", &env_step_host);
     m.def("env_host_join", &env_host_join);
     m.def("obs_to_policy", &obs_to_policy);
@@ -754,6 +822,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     m.def("ragged_total_envs", &ragged_total_envs);
     m.def("ragged_step", &ragged_step);
     m.def("ragged_step_discrete", &ragged_step_discrete);
+    m.def("ragged_step_dones", &ragged_step_dones);
     m.def("ragged_rollout", &ragged_rollout, py::arg("ragged"), py::arg("actions"), py::arg("prepare_only") = false);
     m.def("ragged_check_error", &ragged_check_error);
     m.def("philox_actions", &philox_actions, py::arg("out"), py::arg("env_offset"), py::arg("step0"),

@@ -297,26 +297,8 @@ class MineEnv:
              ) -> Tuple[torch.Tensor, torch.Tensor, torch.Tensor]:
         """reference minecu/__init__.py:304-444 (buttons + look), or the
         discrete form when `look` is omitted."""
-        form = FORMS[self.form]
-        with torch.cuda.device(self.device):
-            if look is None:
-                a = buttons
-                if a.dtype != torch.uint8 or a.device != self.device or not a.is_contiguous():
-                    a = a.to(device=self.device, dtype=torch.uint8).contiguous()
-                if a.numel() != self.batch_size:
-                    raise ValueError(f"actions must have {self.batch_size} entries, got {a.numel()}")
-                _C.env_step_discrete(self._env, a.reshape(self.batch_size), form)
-            else:
-                b = buttons
-                if b.dtype != torch.int8 or b.device != self.device or not b.is_contiguous():
-                    b = b.to(device=self.device, dtype=torch.int8).contiguous()
-                lk = look
-                if lk.dtype != torch.float32 or lk.device != self.device or not lk.is_contiguous():
-                    lk = lk.to(device=self.device, dtype=torch.float32).contiguous()
-                if b.shape != (self.batch_size, 8) or lk.shape != (self.batch_size, 2):
-                    raise ValueError(f"buttons must be [{self.batch_size}, 8] and look [{self.batch_size}, 2]")
-                _C.env_step(self._env, b, lk, form)
-            return self.obs_buffer, self.rewards, self.do_reset.clone()
+        dones = _C.env_step_dones(self._env, buttons, look, FORMS[self.form])
+        return self.obs_buffer, self.rewards, dones
 
     def step_host(self, actions: torch.Tensor, rewards_out: torch.Tensor, dones_out: torch.Tensor) -> torch.Tensor:
         """The discrete step for a host-side policy: actions uint8 [B] read
@@ -327,16 +309,13 @@ class MineEnv:
         a synchronisation of the current stream (e.g.
         torch.cuda.synchronize()): its actions must not be overwritten, nor
         its rewards and dones read, before then."""
-        form = FORMS[self.form]
-        with torch.cuda.device(self.device):
-            _C.env_step_host(self._env, actions, rewards_out, dones_out, self.batch_size, form)
+        _C.env_step_host(self._env, actions, rewards_out, dones_out, self.batch_size, FORMS[self.form])
         return self.obs_buffer
 
     def join_host(self) -> None:
         """Make the current stream wait for the host copies of every
         step_host call so far."""
-        with torch.cuda.device(self.device):
-            _C.env_host_join(self._env)
+        _C.env_host_join(self._env)
 
     def rollout(self, actions: torch.Tensor, rewards_out: Optional[torch.Tensor] = None,
                 dones_out: Optional[torch.Tensor] = None) -> None:

@@ -111,6 +111,7 @@ _PROTOS = {
     "mc_env_reset": (I, [P, P, P]),
     "mc_env_step": (I, [P, P, P, ctypes.c_int, P]),
     "mc_env_step_discrete": (I, [P, P, ctypes.c_int, P]),
+    "mc_env_step_dones": (I, [P, P, P, P, ctypes.c_int, P, P]),
     "mc_env_step_host": (I, [P, P, P, P, ctypes.c_int, P]),
     "mc_env_host_join": (I, [P, P]),
     "mc_env_render": (I, [P, P]),
@@ -137,6 +138,7 @@ _PROTOS = {
     "mc_ragged_smem_bytes": (ctypes.c_int64, [P]),
     "mc_ragged_step": (I, [P, P, P, P]),
     "mc_ragged_step_discrete": (I, [P, P, P]),
+    "mc_ragged_step_dones": (I, [P, P, P, P, P, P]),
     "mc_ragged_step_host": (I, [P, P, P, P, P]),
     "mc_ragged_host_join": (I, [P, P]),
     "mc_ragged_rollout": (I, [P, P, I, P]),

@@ -58,29 +58,14 @@ class RaggedBatch:
         masks = masks if masks is not None else [None] * len(self.envs)
         return [e.reset(m) for e, m in zip(self.envs, masks)]
 
-    def _u8(self, a: torch.Tensor) -> torch.Tensor:
-        if a.dtype != torch.uint8 or a.device != self.device or not a.is_contiguous():
-            a = a.to(device=self.device, dtype=torch.uint8).contiguous()
-        return a
-
     def step(self, actions: torch.Tensor, look: Optional[torch.Tensor] = None
              ) -> List[Tuple[torch.Tensor, torch.Tensor, torch.Tensor]]:
         """One step of every group.  `actions` is uint8 [total] (discrete
         actions 0..10, concatenated in group order), or int8 buttons
         [total, 8] together with float32 `look` [total, 2]."""
-        with torch.cuda.device(self.device):
-            if look is None:
-                a = self._u8(actions)
-                if a.numel() != self.total:
-                    raise ValueError(f"actions must have {self.total} entries, got {a.numel()}")
-                _C.ragged_step_discrete(self._r, a.reshape(self.total))
-            else:
-                b = actions.to(device=self.device, dtype=torch.int8).contiguous()
-                lk = look.to(device=self.device, dtype=torch.float32).contiguous()
-                if b.shape != (self.total, 8) or lk.shape != (self.total, 2):
-                    raise ValueError(f"buttons must be [{self.total}, 8] and look [{self.total}, 2]")
-                _C.ragged_step(self._r, b, lk)
-        return [(e.obs_buffer, e.rewards, e.do_reset.clone()) for e in self.envs]
+        dones = _C.ragged_step_dones(self._r, actions, look)
+        return [(e.obs_buffer, e.rewards, dones[a:b])
+                for e, a, b in zip(self.envs, self.offsets, self.offsets[1:])]
 
     def step_host(self, actions: torch.Tensor, rewards_out: torch.Tensor, dones_out: torch.Tensor
                   ) -> List[torch.Tensor]:
