@@ -75,6 +75,8 @@ MC_HIDDEN void team_layout(const mc_kp* const* kps, int G, const int* stage, con
                            int team_warps, int warps_per_cta, int ctas_per_sm, mc_ragged_kp* rk);
 // Dynamic shared memory of that launch per CTA.
 MC_HIDDEN long long team_smem(const mc_ragged_kp& rk, int warps_per_cta);
+// An env's launch shape as one group of a launch that holds many (the server's).
+MC_HIDDEN mc_fused_cfg mc_shared_launch(const mc_env* e);
 // MC_OK, or MC_ERR_INVALID with a message when the team launch is not possible.
 MC_HIDDEN int team_validate(const mc_kp* const* kps, int G, const int* stage, const int* tile_w, const int* coop,
                             int team_warps, int warps_per_cta, int ctas_per_sm);

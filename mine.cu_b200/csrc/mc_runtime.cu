@@ -629,15 +629,35 @@ static int validate_fused(const mc_env* e, const mc_fused_cfg* f) {
 // Worlds above 32 KB: as many staged worlds as an SM's shared memory holds,
 // three or two CTAs with a team of 8, or one CTA with two teams of 4 or one of 8
 // (64x64 images, us a step, from global memory -> staged: 40^3 502 -> 172, 48^3
-// 647 -> 330, 56^3 439 -> 252).  A shape whose shared memory does not fit falls
+// 647 -> 330, 56^3 439 -> 252).
+// Few tiles of 32 pixels (num_sms x 32 warps hold 4736 at a time): images are
+// cut into finer bands (wider tiles, which bands a warp can then take a few
+// tiles at a time; rays of a wide tile differ more) and bigger teams.  us a step,
+// 4-wide tiles one warp per env / as chosen: 16 envs 32x32 17.8 / 13.4 (32-wide),
+// 64 envs 19.3 / 15.4 (16-wide), 256 envs 20.4 / 17.1 (teams of 8, 16-wide), 1024 envs
+// 26.0 / 24.5 (teams of 4); 32^3 64x64, teams of 4 with 8-wide tiles / of 8 with
+// 16-wide: 64 envs 29.6 / 23.0, 1024 envs 75.1 / 69.8, but 4096 envs 196 / 231.
+// float32 images wider than 32 go to teams: a warp's band would take 6 KB.
+// `alone` false: a job of the server, whose launches hold many.  A shape whose shared memory does not fit falls
 // back to the team shape (whose per-warp image band is half as tall), then
 // to one team per CTA, then to unstaged worlds.  The autotuner (minecu/autotune.py) refines the
 // shape per configuration.
-static mc_fused_cfg default_launch(const mc_env_config* cfg, const mc_kp* kp, const mc_backend* be, int num_sms) {
+static mc_fused_cfg default_launch(const mc_env_config* cfg, const mc_kp* kp, const mc_backend* be, int num_sms,
+                                   bool alone = true) {
     const long long wxyz = (long long)cfg->world_x * cfg->world_y * cfg->world_z;
     const bool aligned = !mc_odd_world(*kp);  // the launches stage the others by themselves
     const bool few_envs = (long long)cfg->batch_size < 2LL * num_sms * 32;
-    const bool big = (cfg->render_width * cfg->render_height >= 64 * 64 && few_envs) || wxyz > 8192;
+    const int W = cfg->render_width, H = cfg->render_height;
+    const long long tiles = alone ? ((long long)cfg->batch_size * W * H + 31) / 32 : 1LL << 40;
+    const bool wide_f32 = cfg->obs_mode == MC_OBS_FLOAT32 && W > 32;
+    bool big = ((W * H >= 64 * 64 || wide_f32) && few_envs) || wxyz > 8192;
+    if (tiles > 4096 && tiles <= 65536) big = true;
+    // the widest tile up to `most` that divides the width (at least 8 of it in use otherwise)
+    auto tile = [&](int most) {
+        int t = most;
+        while (t > 8 && W % t) t /= 2;
+        return t;
+    };
     auto team_shape = [&](mc_fused_cfg& f) {
         f.warps_per_cta = 8;
         f.stage = (wxyz <= 32768 && aligned) ? 1 : 0;
@@ -645,8 +665,15 @@ static mc_fused_cfg default_launch(const mc_env_config* cfg, const mc_kp* kp, co
         f.tile_w = 8;
         f.team_warps = 4;
         f.coop = 1;
+        const bool fast = mc_fast_launch(*kp, 1, f.tile_w);  // else images are not cut into slices
+        if (fast && tiles <= (wxyz > 8192 ? 131072 : 16384)) {
+            f.tile_w = tile(tiles <= 4096 ? 32 : 16);
+            f.team_warps = 8;
+        }
         const mc_kp* kps[1] = {kp};
-        if (wxyz <= 32768 || wxyz > kSmemPerCta || !mc_fast_launch(*kp, 1, f.tile_w)) return;
+        // (an image of few pixels reads less of a big world than its staging: 535
+        // envs 48^3, 8x24 take 76 us a step and reset unstaged, 82 staged; 2657 envs 48^3, 35x10 313 and 292)
+        if (wxyz <= 32768 || wxyz > kSmemPerCta || !fast || 512LL * W * H < wxyz) return;
         constexpr int shapes[4][2] = {{3, 8}, {2, 8}, {1, 4}, {1, 8}};  // CTAs per SM, warps per team
         const int staged = 1;
         for (const auto& s : shapes) {
@@ -666,7 +693,7 @@ static mc_fused_cfg default_launch(const mc_env_config* cfg, const mc_kp* kp, co
         f.warps_per_cta = 8;
         f.stage = (wxyz <= 8192 && aligned) ? 1 : 0;
         f.ctas_per_sm = 4;
-        f.tile_w = 4;
+        f.tile_w = tiles <= 4096 && mc_fast_launch(*kp, 1, 8) ? tile(tiles <= 1024 ? 32 : 16) : 4;
         f.team_warps = 1;
         f.coop = 0;
     }
@@ -679,6 +706,8 @@ static mc_fused_cfg default_launch(const mc_env_config* cfg, const mc_kp* kp, co
 }
 
 static void default_fused(mc_env* e) { e->fcfg = default_launch(&e->cfg, &e->kp, e->be, e->num_sms); }
+
+mc_fused_cfg mc_shared_launch(const mc_env* e) { return default_launch(&e->cfg, &e->kp, e->be, e->num_sms, false); }
 
 extern "C" int mc_default_fused_config(const mc_env_config* cfg, int32_t num_sms, int32_t voxels_aligned,
                                        mc_fused_config* out, int64_t* smem_bytes) {

@@ -358,9 +358,10 @@ int run_round(mc_server* s, Slot& sl, const std::vector<Req*>& reqs, const std::
             for (int g = 0; g < G; ++g) {
                 const mc_env* e = reqs[steps[g]]->job->env;
                 kps[g] = &e->kp;
-                stage[g] = e->fcfg.stage;
-                tile_w[g] = e->fcfg.tile_w;
-                coop[g] = e->fcfg.coop;
+                const mc_fused_cfg f = mc_shared_launch(e);
+                stage[g] = f.stage;
+                tile_w[g] = f.tile_w;
+                coop[g] = f.coop;
                 any_coop |= coop[g] != 0;
             }
             const int team = any_coop ? 4 : 1, cps = any_coop ? 3 : 4;
