@@ -634,7 +634,6 @@ __device__ __noinline__ void march_bounds_fail(uint32_t a, SmemRange chk, int si
         "{\n\t" \
         ".reg .pred pa, pna, pbx, pzx, pby, pzy, pz, pq, pb1, pb2;\n\t" \
         ".reg .b32 ra, rc;\n\t" \
-        ".reg .s32 rv;\n\t" \
         "MC_CMARCH_LOOP:\n\t" \
         CMP \
         "@pbx add.s32 %4, %4, %6;\n\t" \
@@ -648,23 +647,18 @@ __device__ __noinline__ void march_bounds_fail(uint32_t a, SmemRange chk, int si
         "setp.ge.u32 pb2, rc, %18;\n\t" \
         "or.pred pb1, pb1, pb2;\n\t" \
         "@pb1 mov.u32 %5, ra;\n\t" \
-        "@pb1 mov.s32 %0, -2;\n\t" \
         "@pb1 bra MC_CMARCH_END;\n\t" \
-        "ld.shared.s8 rv, [ra];\n\t" \
-        "lop3.b32 ra, %4, rv, %9, 0xA2;\n\t" \
+        "ld.shared.s8 %0, [ra];\n\t" \
+        "lop3.b32 ra, %4, %0, %9, 0xA2;\n\t" \
         "setp.ne.b32 pq, ra, 0;\n\t" \
-        "@pq bra MC_CMARCH_DONE;\n\t" \
+        "@pq bra MC_CMARCH_END;\n\t" \
         "@pbx add.rn" FT " %1, %1, %11;\n\t" \
         "@pby add.rn" FT " %2, %2, %12;\n\t" \
         "@pz add.rn" FT " %3, %3, %13;\n\t" \
         "bra MC_CMARCH_LOOP;\n\t" \
-        "MC_CMARCH_DONE:\n\t" \
-        "and.b32 ra, %4, %14;\n\t" \
-        "setp.ne.b32 pq, ra, 0;\n\t" \
-        "selp.b32 %0, -1, rv, pq;\n\t" \
         "MC_CMARCH_END:\n\t" \
         "}" \
-        : "=&r"(b), "+" C(tmx), "+" C(tmy), "+" C(tmz), "+r"(packed), "+r"(bad) \
+        : "+r"(b), "+" C(tmx), "+" C(tmy), "+" C(tmz), "+r"(packed), "+r"(bad) \
         : "r"(px), "r"(py), "r"(pz), "n"(kGuard | (int)0x80000000u), "r"(world), C(tdx), C(tdy), C(tdz), \
           "n"(kGuard), "r"(chk.lo), "r"(chk.span), "r"(dyn.lo), "r"(dyn.span) \
         : "memory");
@@ -676,7 +670,6 @@ __device__ __noinline__ void march_bounds_fail(uint32_t a, SmemRange chk, int si
         "{\n\t" \
         ".reg .pred pa, pna, pbx, pzx, pby, pzy, pz, pq;\n\t" \
         ".reg .b32 ra;\n\t" \
-        ".reg .s32 rv;\n\t" \
         "MC_MARCH_LOOP:\n\t" \
         CMP \
         "@pbx add.s32 %4, %4, %5;\n\t" \
@@ -684,8 +677,8 @@ __device__ __noinline__ void march_bounds_fail(uint32_t a, SmemRange chk, int si
         "@pz add.s32 %4, %4, %7;\n\t" \
         "shr.s32 ra, %4, 18;\n\t" \
         "add.s32 ra, ra, %9;\n\t" \
-        "ld.shared.s8 rv, [ra];\n\t" \
-        "lop3.b32 ra, %4, rv, %8, 0xA2;\n\t" \
+        "ld.shared.s8 %0, [ra];\n\t" \
+        "lop3.b32 ra, %4, %0, %8, 0xA2;\n\t" \
         "setp.ne.b32 pq, ra, 0;\n\t" \
         "@pq bra MC_MARCH_DONE;\n\t" \
         "@pbx add.rn" FT " %1, %1, %10;\n\t" \
@@ -693,11 +686,8 @@ __device__ __noinline__ void march_bounds_fail(uint32_t a, SmemRange chk, int si
         "@pz add.rn" FT " %3, %3, %12;\n\t" \
         "bra MC_MARCH_LOOP;\n\t" \
         "MC_MARCH_DONE:\n\t" \
-        "and.b32 ra, %4, %13;\n\t" \
-        "setp.ne.b32 pq, ra, 0;\n\t" \
-        "selp.b32 %0, -1, rv, pq;\n\t" \
         "}" \
-        : "=&r"(b), "+" C(tmx), "+" C(tmy), "+" C(tmz), "+r"(packed) \
+        : "+r"(b), "+" C(tmx), "+" C(tmy), "+" C(tmz), "+r"(packed) \
         : "r"(px), "r"(py), "r"(pz), "n"(kGuard | (int)0x80000000u), "r"(world), C(tdx), C(tdy), C(tdz), \
           "n"(kGuard) \
         : "memory");
@@ -707,10 +697,10 @@ template <class T>
 __device__ __forceinline__ int march_packed_shared(uint32_t world, int& packed, int px, int py, int pz, T& tmx, T& tmy,
                                                    T& tmz, T tdx, T tdy, T tdz, SmemRange chk = SmemRange{0u, 0u}) {
     constexpr int kGuard = (32 << 12) | (32 << 6) | 32;
-    int b;
+    int b = -1;
 #if MC_CHECK_BOUNDS
     const SmemRange dyn = dyn_smem_range();
-    uint32_t bad = 0;
+    uint32_t bad = ~0u;
 #else
     (void)chk;
 #endif
@@ -720,12 +710,12 @@ __device__ __forceinline__ int march_packed_shared(uint32_t world, int& packed, 
         MC_MARCH_PACKED(MC_F16_T, MC_F16_AXIS, "h")
     }
 #if MC_CHECK_BOUNDS
-    if (b == -2) {  // a load address outside its range: the load was skipped, the ray ends as sky
+    if (bad != ~0u) {  // a load address outside its range: the load was skipped, the ray ends as sky
         march_bounds_fail(bad, chk, MC_SITE_MARCH_PACKED);
-        b = -1;
+        return -1;
     }
 #endif
-    return b;
+    return (packed & kGuard) ? -1 : b;
 }
 
 // Where a ray going up from the eye's voxel (vx, vy, vz) can still meet a
@@ -810,7 +800,6 @@ __device__ __forceinline__ int split_counts(int cx, int cy, int cz, int max_step
         "{\n\t" \
         ".reg .pred pa, pna, pbx, pzx, pby, pzy, pz, pq, pb1, pb2;\n\t" \
         ".reg .b32 ra, rc;\n\t" \
-        ".reg .s32 rv;\n\t" \
         "MC_CSPLIT_LOOP:\n\t" \
         CMP \
         "@pbx add.s32 %4, %4, %7;\n\t" \
@@ -825,23 +814,18 @@ __device__ __forceinline__ int split_counts(int cx, int cy, int cz, int max_step
         "setp.ge.u32 pb2, rc, %21;\n\t" \
         "or.pred pb1, pb1, pb2;\n\t" \
         "@pb1 mov.u32 %6, %4;\n\t" \
-        "@pb1 mov.s32 %0, -2;\n\t" \
         "@pb1 bra MC_CSPLIT_END;\n\t" \
-        "ld.shared.s8 rv, [%4];\n\t" \
-        "lop3.b32 ra, %5, rv, %13, 0xA2;\n\t" \
+        "ld.shared.s8 %0, [%4];\n\t" \
+        "lop3.b32 ra, %5, %0, %13, 0xA2;\n\t" \
         "setp.ne.b32 pq, ra, 0;\n\t" \
-        "@pq bra MC_CSPLIT_DONE;\n\t" \
+        "@pq bra MC_CSPLIT_END;\n\t" \
         "@pbx add.rn" FT " %1, %1, %14;\n\t" \
         "@pby add.rn" FT " %2, %2, %15;\n\t" \
         "@pz add.rn" FT " %3, %3, %16;\n\t" \
         "bra MC_CSPLIT_LOOP;\n\t" \
-        "MC_CSPLIT_DONE:\n\t" \
-        "and.b32 ra, %5, %17;\n\t" \
-        "setp.ne.b32 pq, ra, 0;\n\t" \
-        "selp.b32 %0, -1, rv, pq;\n\t" \
         "MC_CSPLIT_END:\n\t" \
         "}" \
-        : "=&r"(b), "+" C(tmx), "+" C(tmy), "+" C(tmz), "+r"(addr), "+r"(cnt), "+r"(bad) \
+        : "+r"(b), "+" C(tmx), "+" C(tmy), "+" C(tmz), "+r"(addr), "+r"(cnt), "+r"(bad) \
         : "r"(dax), "r"(day), "r"(daz), "n"((1 << 7) | (1 << 21)), "n"((1 << 14) | (1 << 21)), "n"(1 | (1 << 21)), \
           "n"(kSplitGuard | (int)0x80000000u), C(tdx), C(tdy), C(tdz), "n"(kSplitGuard), "r"(chk.lo), \
           "r"(chk.span), "r"(dyn.lo), "r"(dyn.span) \
@@ -852,7 +836,6 @@ __device__ __forceinline__ int split_counts(int cx, int cy, int cz, int max_step
         "{\n\t" \
         ".reg .pred pa, pna, pbx, pzx, pby, pzy, pz, pq;\n\t" \
         ".reg .b32 ra;\n\t" \
-        ".reg .s32 rv;\n\t" \
         "MC_SPLIT_LOOP:\n\t" \
         CMP \
         "@pbx add.s32 %4, %4, %6;\n\t" \
@@ -861,8 +844,8 @@ __device__ __forceinline__ int split_counts(int cx, int cy, int cz, int max_step
         "@pbx add.s32 %5, %5, %9;\n\t" \
         "@pby add.s32 %5, %5, %10;\n\t" \
         "@pz add.s32 %5, %5, %11;\n\t" \
-        "ld.shared.s8 rv, [%4];\n\t" \
-        "lop3.b32 ra, %5, rv, %12, 0xA2;\n\t" \
+        "ld.shared.s8 %0, [%4];\n\t" \
+        "lop3.b32 ra, %5, %0, %12, 0xA2;\n\t" \
         "setp.ne.b32 pq, ra, 0;\n\t" \
         "@pq bra MC_SPLIT_DONE;\n\t" \
         "@pbx add.rn" FT " %1, %1, %13;\n\t" \
@@ -870,11 +853,8 @@ __device__ __forceinline__ int split_counts(int cx, int cy, int cz, int max_step
         "@pz add.rn" FT " %3, %3, %15;\n\t" \
         "bra MC_SPLIT_LOOP;\n\t" \
         "MC_SPLIT_DONE:\n\t" \
-        "and.b32 ra, %5, %16;\n\t" \
-        "setp.ne.b32 pq, ra, 0;\n\t" \
-        "selp.b32 %0, -1, rv, pq;\n\t" \
         "}" \
-        : "=&r"(b), "+" C(tmx), "+" C(tmy), "+" C(tmz), "+r"(addr), "+r"(cnt) \
+        : "+r"(b), "+" C(tmx), "+" C(tmy), "+" C(tmz), "+r"(addr), "+r"(cnt) \
         : "r"(dax), "r"(day), "r"(daz), "n"((1 << 7) | (1 << 21)), "n"((1 << 14) | (1 << 21)), "n"(1 | (1 << 21)), \
           "n"(kSplitGuard | (int)0x80000000u), C(tdx), C(tdy), C(tdz), "n"(kSplitGuard) \
         : "memory");
@@ -883,10 +863,10 @@ __device__ __forceinline__ int split_counts(int cx, int cy, int cz, int max_step
 template <class T>
 __device__ __forceinline__ int march_split_shared(uint32_t addr, int& cnt, int dax, int day, int daz, T& tmx, T& tmy,
                                                   T& tmz, T tdx, T tdy, T tdz, SmemRange chk = SmemRange{0u, 0u}) {
-    int b;
+    int b = -1;
 #if MC_CHECK_BOUNDS
     const SmemRange dyn = dyn_smem_range();
-    uint32_t bad = 0;
+    uint32_t bad = ~0u;
 #else
     (void)chk;
 #endif
@@ -896,12 +876,12 @@ __device__ __forceinline__ int march_split_shared(uint32_t addr, int& cnt, int d
         MC_MARCH_SPLIT(MC_F16_T, MC_F16_AXIS, "h")
     }
 #if MC_CHECK_BOUNDS
-    if (b == -2) {
+    if (bad != ~0u) {
         march_bounds_fail(bad, chk, MC_SITE_MARCH_SPLIT);
-        b = -1;
+        return -1;
     }
 #endif
-    return b;
+    return (cnt & kSplitGuard) ? -1 : b;
 }
 
 // March from the eye's voxel (index idx, in-box steps left cx, cy, cz) through
@@ -2060,7 +2040,7 @@ __device__ __forceinline__ bool ground_tail(const Cam& c, const FastEnv& fe, flo
 }
 
 template <int FAM, bool F32, bool SPLIT, bool ODD, bool TEAM>
-__device__ __forceinline__ void fast_band(const Cam& c, const Dda0& d0, const FastEnv& fe, int W, int H, int TW,
+__device__ __forceinline__ void fast_band(const Cam& c, const Dda0& d0, const FastEnv& fe, int W, int H, int sh,
                                           int row0, int lane, const float* s_u, const float* s_v, const float4* s_cs,
                                           const uint32_t* s_rgbp, uint8_t* stage, uint8_t* dst) {
     constexpr bool PAIRS = F32 && TEAM && !ODD, DIRECT = F32 && TEAM && ODD;  // how float32 pixels leave
@@ -2071,8 +2051,8 @@ __device__ __forceinline__ void fast_band(const Cam& c, const Dda0& d0, const Fa
     constexpr int bpp = 3 * (F32 ? 4 : 1);
     constexpr int m = F32 ? 0x1 : (GROUND ? MC_FASTG_SKY : 0x3);  // sky_fused_mask of the family's kernel
     const float sky0 = 0.53f, sky1 = 0.81f, sky2 = 0.92f;  // SKY_COLOR (c_sky)
-    const int TH = 32 / TW;
-    const int lx = lane % TW, ly = lane / TW;
+    const int TW = 1 << sh, TH = 32 >> sh;  // sh: log2 of the tile's width
+    const int lx = lane & (TW - 1), ly = lane >> sh;
     const bool in_y = !ODD || row0 + ly < H;
     const float v = s_v[ODD ? min(row0 + ly, H - 1) : row0 + ly];
     const float yraw = N::mad(v, c.uy, c.fy);
@@ -2180,11 +2160,11 @@ __device__ __forceinline__ void fast_band(const Cam& c, const Dda0& d0, const Fa
         }
         if (PAIRS && ((tx0 & TW) || tx0 + TW == W)) {
             // these one or two tiles' rows, 16 bytes a lane
-            const int first = tx0 & ~(2 * TW - 1), cols = tx0 + TW - first, cpr = cols * 3 / 4, n = TH * cpr;
-            const int inv = 65536 / cpr + 1;  // k / cpr for k < 48
+            const int first = tx0 & ~(2 * TW - 1), cols = tx0 + TW - first, cpr = cols * 3 >> 2, n = TH * cpr;
+            const int mul = (cols >> sh) == 2 ? 43691 : 87382;  // k / cpr = (k * 4 / (3 cols)), k < 48
             __syncwarp();
             for (int k = lane; k < n; k += 32) {
-                const int row = (k * inv) >> 16, piece = k - row * cpr;
+                const int row = k * mul >> (16 + sh), piece = k - row * cpr;
                 *reinterpret_cast<uint4*>(dst + (row * W + first) * bpp + piece * 16) =
                     *reinterpret_cast<const uint4*>(stage + row * 2 * TW * bpp + piece * 16);
             }
@@ -2824,7 +2804,7 @@ template <int FAM, bool F32, bool TEAM>
 __device__ __forceinline__ void render_fast(const mc_kp& p, int e, const EnvRender& r, const FusedCtx& cx,
                                             const int8_t* staged, int tile_w, int lane, int* band_ctr, int part,
                                             int slices) {
-    const int W = p.W, TW = tile_w, TH = 32 / tile_w;
+    const int sh = __ffs(tile_w) - 1, W = p.W, TH = 32 >> sh;
     constexpr int bpp = 3 * (F32 ? 4 : 1);
     uint8_t* oenv = (uint8_t*)p.obs + e * ((long long)W * p.H * bpp);
     const bool vd_safe = box_within_view(r.c, p.wx, p.wy, p.wz, p.vd);
@@ -2844,23 +2824,23 @@ __device__ __forceinline__ void render_fast(const mc_kp& p, int e, const EnvRend
     fe.wy = p.wy;
     fe.wz = p.wz;
     fe.max_steps = p.max_steps;
-    const int H = p.H, nb = (H + TH - 1) / TH, b0 = part * nb / slices, nbands = (part + 1) * nb / slices - b0;
+    const int H = p.H, nb = (H + TH - 1) >> (5 - sh), b0 = part * nb / slices, nbands = (part + 1) * nb / slices - b0;
     const bool odd = p.fast_ok == 2;
     for (int b = next_band(band_ctr, -1, lane); b < nbands; b = next_band(band_ctr, b, lane)) {
         const int row0 = (b0 + b) * TH;
         uint8_t* dst = oenv + row0 * W * bpp;
         if (odd) {
             if (fk == 1)
-                fast_band<FAM, F32, false, true, TEAM>(r.c, d0, fe, W, H, TW, row0, lane, cx.s_u, cx.s_v, cx.s_cs,
+                fast_band<FAM, F32, false, true, TEAM>(r.c, d0, fe, W, H, sh, row0, lane, cx.s_u, cx.s_v, cx.s_cs,
                                                  cx.s_rgbp, cx.stage, dst);
             else
-                fast_band<FAM, F32, true, true, TEAM>(r.c, d0, fe, W, H, TW, row0, lane, cx.s_u, cx.s_v, cx.s_cs,
+                fast_band<FAM, F32, true, true, TEAM>(r.c, d0, fe, W, H, sh, row0, lane, cx.s_u, cx.s_v, cx.s_cs,
                                                 cx.s_rgbp, cx.stage, dst);
         } else if (fk == 1) {
-            fast_band<FAM, F32, false, false, TEAM>(r.c, d0, fe, W, H, TW, row0, lane, cx.s_u, cx.s_v, cx.s_cs, cx.s_rgbp,
+            fast_band<FAM, F32, false, false, TEAM>(r.c, d0, fe, W, H, sh, row0, lane, cx.s_u, cx.s_v, cx.s_cs, cx.s_rgbp,
                                               cx.stage, dst);
         } else {
-            fast_band<FAM, F32, true, false, TEAM>(r.c, d0, fe, W, H, TW, row0, lane, cx.s_u, cx.s_v, cx.s_cs, cx.s_rgbp,
+            fast_band<FAM, F32, true, false, TEAM>(r.c, d0, fe, W, H, sh, row0, lane, cx.s_u, cx.s_v, cx.s_cs, cx.s_rgbp,
                                              cx.stage, dst);
         }
     }
