@@ -155,14 +155,15 @@ int mc_env_step_dones(mc_env* env, const int8_t* buttons, const float* look, con
  * caller with a host-side policy drives it (minecu/__init__.py:304-444; its
  * rewards and dones are then copied back to the host).  actions uint8[B]
  * are read from host memory, rewards float32[B] and dones uint8[B] written
- * to host memory.  The copies run on the env's own upload and read-back
- * streams and overlap the device steps of the neighbouring calls: the
- * actions of call k+1 go up while step k runs, the results of step k come
- * back while step k+1 runs.  Host buffers must be pinned (cudaHostAlloc or
+ * to host memory.  Host buffers must be pinned (cudaHostAlloc or
  * cudaHostRegister) and must stay untouched until the results of the call
  * are known to be in host memory: after mc_env_host_join(env, s) on stream
- * s, once s reaches that point.  The first call allocates the env's two
- * action and two result buffers (B * 6 bytes each pair). */
+ * s, once s reaches that point.  The fused form's agent kernel reads and
+ * writes mapped buffers in place.  The plain form (and buffers that are not
+ * mapped) go through copies on the env's own upload and read-back streams,
+ * which overlap the device steps of the neighbouring calls; the first such
+ * call allocates the env's two action and two result buffers (B * 6 bytes
+ * each pair). */
 int mc_env_step_host(mc_env* env, const uint8_t* host_actions, float* host_rewards, uint8_t* host_dones, int form,
                      void* stream);
 /* Make `stream` wait, on the device, for every copy issued by the
@@ -277,8 +278,7 @@ int mc_ragged_step_dones(mc_ragged* r, const int8_t* buttons, const float* look,
 /* The discrete step of every group with host buffers, as mc_env_step_host:
  * actions uint8[total] from pinned host memory, every env's reward
  * float32[total] and done uint8[total] (concatenated in group order) to
- * pinned host memory, the copies overlapping the neighbouring steps; the
- * launch writes the results straight into the read-back buffer.  Results
+ * pinned host memory, in place where they are mapped.  Results
  * are in host memory once a stream given to mc_ragged_host_join reaches
  * that point. */
 int mc_ragged_step_host(mc_ragged* r, const uint8_t* host_actions, float* host_rewards, uint8_t* host_dones,
@@ -298,7 +298,7 @@ int mc_ragged_check_error(mc_ragged* r, void* stream);
  * launcher thread takes the oldest queued request of every job with work
  * and runs them together: resets as MineEnv.reset, steps as one launch of
  * the team kernel over the jobs (groups of up to MC_RAGGED_MAX_GROUPS), with
- * one actions upload and one rewards/dones read-back per launch.  A job's
+ * the actions read and the rewards and dones written in pinned memory.  A job's
  * requests run in submission order; each step's results equal
  * mc_env_step_discrete with the fused form on that job alone.  With
  * batching = 0 the server runs one request at a time, in arrival order, with

@@ -57,6 +57,7 @@ struct mc_env {
     cudaStream_t cap_stream;
     std::vector<RolloutGraph> graphs;
     HostIO* hio;
+    cudaEvent_t host_done;  // after the last host-buffer step that used the caller's buffers in place
     int regen_mode;  // MC_REGEN_ALL (the reference's rule) or MC_REGEN_PER_ENV
 };
 

@@ -820,6 +820,10 @@ static void hostio_close(HostIO** ph) {
 extern "C" int mc_env_destroy(mc_env* e) {
     if (!e) return MC_OK;
     hostio_close(&e->hio);
+    if (e->host_done) {
+        cudaEventSynchronize(e->host_done);  // the caller's host buffers are written until then
+        cudaEventDestroy(e->host_done);
+    }
     drop_graphs(e);
     if (e->flags) cudaFree(e->flags);
     if (e->tmpl) cudaFree(e->tmpl);
@@ -1043,6 +1047,42 @@ static int hostio_join(const HostIO* h, cudaStream_t s) {
     return MC_OK;
 }
 
+// The device's view of a caller's host buffer: non-null when it is pinned and
+// mapped, so that a kernel can read or write it itself.
+static void* device_view(const void* host) {
+    cudaPointerAttributes a{};
+    if (cudaPointerGetAttributes(&a, host) != cudaSuccess) {
+        cudaGetLastError();  // not CUDA memory: the copies take it
+        return nullptr;
+    }
+    return a.type == cudaMemoryTypeHost ? a.devicePointer : nullptr;
+}
+
+// Host buffers the agent kernel can use in place: a few bytes an env, read and
+// written by one warp instruction per 32 envs, instead of three copies on two
+// more streams with four events between them and the step (4096 envs 16^3,
+// 32x32: 55.8 -> 47.5 us a step; 64 envs 46 -> 17).
+struct HostViews {
+    const uint8_t* act;
+    float* rew;
+    uint8_t* done;
+    bool ok;
+};
+// After such a step on stream s: what a join on any stream waits for.
+static int host_mark(cudaEvent_t* ev, cudaStream_t s) {
+    if (!*ev) MC_CK(cudaEventCreateWithFlags(ev, cudaEventDisableTiming));
+    MC_CK(cudaEventRecord(*ev, s));
+    return MC_OK;
+}
+static HostViews host_views(const uint8_t* actions, float* rewards, uint8_t* dones) {
+    HostViews v{};
+    v.act = static_cast<const uint8_t*>(device_view(actions));
+    if (v.act) v.rew = static_cast<float*>(device_view(rewards));
+    if (v.rew) v.done = static_cast<uint8_t*>(device_view(dones));
+    v.ok = v.done != nullptr && !(((uintptr_t)v.rew) & 3);
+    return v;
+}
+
 extern "C" int mc_env_step_host(mc_env* e, const uint8_t* host_actions, float* host_rewards, uint8_t* host_dones,
                                 int form, void* stream) {
     NvtxRange nvtx("mc_env_step_host");
@@ -1051,10 +1091,17 @@ extern "C" int mc_env_step_host(mc_env* e, const uint8_t* host_actions, float* h
     if (B == 0) return MC_OK;
     if (!host_actions || !host_rewards || !host_dones) return fail(MC_ERR_INVALID, "host buffers are NULL");
     if (form != MC_FORM_PLAIN && form != MC_FORM_FUSED) return fail(MC_ERR_INVALID, "unknown form %d", form);
+    cudaStream_t s = (cudaStream_t)stream;
+    if (form == MC_FORM_FUSED) {
+        const HostViews v = host_views(host_actions, host_rewards, host_dones);
+        if (v.ok) {
+            const int rc = do_step(e, nullptr, nullptr, v.act, form, s, v.rew, v.done);
+            return rc ? rc : host_mark(&e->host_done, s);
+        }
+    }
     int rc = hostio_init(&e->hio, B);
     if (rc) return rc;
     HostIO* h = e->hio;
-    cudaStream_t s = (cudaStream_t)stream;
     const int i = (int)(h->calls & 1);
     rc = hostio_upload(h, i, host_actions, B, s);
     if (rc) return rc;
@@ -1078,6 +1125,7 @@ extern "C" int mc_env_step_host(mc_env* e, const uint8_t* host_actions, float* h
 
 extern "C" int mc_env_host_join(mc_env* e, void* stream) {
     if (!e) return fail(MC_ERR_INVALID, "env is NULL");
+    if (e->host_done) MC_CK(cudaStreamWaitEvent((cudaStream_t)stream, e->host_done, 0));
     return hostio_join(e->hio, (cudaStream_t)stream);
 }
 
@@ -1289,6 +1337,7 @@ struct mc_ragged {
     cudaStream_t cap_stream = nullptr;
     std::vector<RaggedGraph> graphs;
     HostIO* hio = nullptr;  // mc_ragged_step_host buffers
+    cudaEvent_t host_done = nullptr;  // after the last host-buffer step that used the caller's buffers in place
 };
 
 static long long ragged_wxyz(const mc_env* e) {
@@ -1403,6 +1452,10 @@ extern "C" int mc_ragged_create(mc_env* const* groups, int32_t ngroups, mc_ragge
 extern "C" int mc_ragged_destroy(mc_ragged* r) {
     if (!r) return MC_OK;
     hostio_close(&r->hio);
+    if (r->host_done) {
+        cudaEventSynchronize(r->host_done);
+        cudaEventDestroy(r->host_done);
+    }
     ragged_drop_graphs(r);
     if (r->flags) cudaFree(r->flags);
     if (r->rec) cudaFree(r->rec);
@@ -1491,10 +1544,15 @@ extern "C" int mc_ragged_step_host(mc_ragged* r, const uint8_t* host_actions, fl
     const long long B = mc_ragged_total_envs(r);
     if (B == 0) return MC_OK;
     if (!host_actions || !host_rewards || !host_dones) return fail(MC_ERR_INVALID, "host buffers are NULL");
+    cudaStream_t s = (cudaStream_t)stream;
+    const HostViews v = host_views(host_actions, host_rewards, host_dones);
+    if (v.ok) {
+        const int rc = ragged_do_step(r, nullptr, nullptr, v.act, s, false, v.rew, v.done);
+        return rc ? rc : host_mark(&r->host_done, s);
+    }
     int rc = hostio_init(&r->hio, B);
     if (rc) return rc;
     HostIO* h = r->hio;
-    cudaStream_t s = (cudaStream_t)stream;
     const int i = (int)(h->calls & 1);
     rc = hostio_upload(h, i, host_actions, B, s);
     if (rc) return rc;
@@ -1510,6 +1568,7 @@ extern "C" int mc_ragged_step_host(mc_ragged* r, const uint8_t* host_actions, fl
 
 extern "C" int mc_ragged_host_join(mc_ragged* r, void* stream) {
     if (!r) return fail(MC_ERR_INVALID, "ragged handle is NULL");
+    if (r->host_done) MC_CK(cudaStreamWaitEvent((cudaStream_t)stream, r->host_done, 0));
     return hostio_join(r->hio, (cudaStream_t)stream);
 }
 

@@ -9,9 +9,9 @@
 //  * the launcher takes, for every job with queued work, its oldest request
 //    (up to MC_RAGGED_MAX_GROUPS step requests of one render family per
 //    launch, oldest jobs first) and enqueues on the server stream: resets
-//    (MineEnv.reset), one upload of all step actions, one team-kernel launch
-//    over the stepping jobs (each job one group), the conditional world
-//    regenerations, one read-back of all rewards and dones, an event;
+//    (MineEnv.reset), one fused step over the stepping jobs (each job one
+//    group), whose agent kernel reads the pinned actions and writes the pinned
+//    rewards and dones in place, an event;
 //  * the completer waits for those events in launch order, hands the
 //    results to the requests and records their latency (submission to
 //    results in host memory).
@@ -19,12 +19,11 @@
 // completer its event) instead of blocking, which keeps thread wake-ups out
 // of the request latency at the cost of two busy host cores under load.
 // Up to max_inflight launches are queued on the device at once, so the host
-// work of the next launch overlaps the current one; the actions upload and
-// the results read-back run on their own streams, so they overlap the
-// neighbouring launches' kernels instead of queueing between them.  A job's requests run in
+// work of the next launch overlaps the current one.  A job's requests run in
 // submission order (one stream).  With batching = 0 the launcher takes one
-// request at a time (oldest first) and steps with the plain form: the
-// one-job-at-a-time loop the batched server is compared with.
+// request at a time (oldest first) and steps with the plain form, its actions
+// and results copied on their own streams: the one-job-at-a-time loop the
+// batched server is compared with.
 #include <cuda_runtime.h>
 #include <stdint.h>
 #include <string.h>
@@ -83,9 +82,9 @@ struct Job {
 };
 
 struct Slot {
-    cudaEvent_t ev = nullptr;     // recorded after the read-back: the launch is complete
-    cudaEvent_t ev_up = nullptr;  // actions uploaded
-    cudaEvent_t ev_k = nullptr;   // device work of the launch done
+    cudaEvent_t ev = nullptr;     // the launch is complete, its results in h_res
+    cudaEvent_t ev_up = nullptr;  // batching = 0: actions uploaded
+    cudaEvent_t ev_k = nullptr;   // batching = 0: device work of the launch done
     uint8_t* h_act = nullptr;  // pinned
     uint8_t* d_act = nullptr;
     uint8_t* h_res = nullptr;  // pinned: rewards (cap floats), then dones (cap bytes)
@@ -189,7 +188,7 @@ struct mc_server {
     bool stop = false, launcher_done = false;
     std::thread launcher, completer;
     cudaStream_t stream = nullptr, admit_stream = nullptr;
-    cudaStream_t up = nullptr, down = nullptr;  // actions uploads, results read-backs
+    cudaStream_t up = nullptr, down = nullptr;  // batching = 0: actions uploads, results read-backs
     int32_t* flags = nullptr;  // work counter of the team launches
     uint8_t* rec = nullptr;    // render records of one team launch (cap envs)
     Slot slots[kMaxSlots];
@@ -322,9 +321,11 @@ int run_batch(mc_server* s, Slot& sl, const std::vector<Req*>& reqs) {
     sl.total = off;
     if (!steps.empty()) {
         sl.step_launch = true;
-        cudaError_t ce = cudaMemcpyAsync(sl.d_act, sl.h_act, (size_t)off, cudaMemcpyHostToDevice, s->up);
-        if (ce == cudaSuccess) ce = cudaEventRecord(sl.ev_up, s->up);
-        if (ce == cudaSuccess) ce = cudaStreamWaitEvent(st, sl.ev_up, 0);
+        // a batching launch's agent kernels read the pinned actions and write
+        // the pinned results in place: no copies, no other streams
+        cudaError_t ce = s->cfg.batching ? cudaSuccess : cudaMemcpyAsync(sl.d_act, sl.h_act, (size_t)off, cudaMemcpyHostToDevice, s->up);
+        if (ce == cudaSuccess && !s->cfg.batching) ce = cudaEventRecord(sl.ev_up, s->up);
+        if (ce == cudaSuccess && !s->cfg.batching) ce = cudaStreamWaitEvent(st, sl.ev_up, 0);
         if (ce != cudaSuccess) return mc_cuda_fail(ce, "server: actions upload");
     }
     for (int rd = 0; rd < nrounds && rc == MC_OK; ++rd) {
@@ -347,9 +348,10 @@ int run_round(mc_server* s, Slot& sl, const std::vector<Req*>& reqs, const std::
     {
         const long long first = sl.offs[steps[0]];
         // rewards then dones, contiguous over the launch: one read-back
-        float* d_rew = reinterpret_cast<float*>(sl.d_res) + first;
-        uint8_t* d_done = sl.d_res + sl.total * 4 + first;
-        uint8_t* d_act = sl.d_act + first;
+        uint8_t* res = s->cfg.batching ? sl.h_res : sl.d_res;  // pinned memory is mapped
+        float* d_rew = reinterpret_cast<float*>(res) + first;
+        uint8_t* d_done = res + sl.total * 4 + first;
+        uint8_t* d_act = (s->cfg.batching ? sl.h_act : sl.d_act) + first;
         if (s->cfg.batching) {
             const int G = (int)steps.size();
             std::vector<const mc_kp*> kps(G);
@@ -395,9 +397,13 @@ int run_round(mc_server* s, Slot& sl, const std::vector<Req*>& reqs, const std::
     return rc;
 }
 
-// After the device work of a launch: its results read-back on the read-back
+// After the device work of a launch: with batching = 0 its results read-back on the read-back
 // stream, then the event the completer waits for.
 int finish_batch(mc_server* s, Slot& sl, bool readback) {
+    if (s->cfg.batching) {
+        const cudaError_t done = cudaEventRecord(sl.ev, s->stream);
+        return done == cudaSuccess ? MC_OK : mc_cuda_fail(done, "server: launch event");
+    }
     cudaError_t ce = cudaEventRecord(sl.ev_k, s->stream);
     if (ce == cudaSuccess) ce = cudaStreamWaitEvent(s->down, sl.ev_k, 0);
     if (ce == cudaSuccess && readback)

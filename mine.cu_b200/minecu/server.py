@@ -6,7 +6,7 @@ libminecu_b200.so (mc_server_*): jobs (env configurations) are admitted
 against an HBM budget and keep their worlds and agents resident on the
 device; client threads submit step/reset requests, and a native launcher
 batches the oldest request of every job with work into one team-kernel
-launch (one actions upload, one rewards/dones read-back).  Each step's
+launch, which reads the actions and writes the results in pinned memory.  Each step's
 results equal MineEnv.step on that job alone with the fused form.
 
     srv = EnvServer(hbm_budget_bytes=150e9)
