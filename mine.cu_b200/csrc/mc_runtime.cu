@@ -224,6 +224,17 @@ __global__ void k_reset_agents(float* pos, float* vel, float* yaw, float* pitch,
     og[i] = 0;
 }
 
+// update_cameras_kernel (kernels.cu:2320-2335)
+__global__ void k_cameras_rt(mc_kp p) {
+    long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= p.B) return;
+    p.cameras[i * 5 + 0] = p.positions[i * 3 + 0];
+    p.cameras[i * 5 + 1] = p.positions[i * 3 + 1];
+    p.cameras[i * 5 + 2] = p.positions[i * 3 + 2];
+    p.cameras[i * 5 + 3] = p.yaws[i];
+    p.cameras[i * 5 + 4] = p.pitches[i];
+}
+
 __global__ void k_philox(uint8_t* actions, int B, int K, int env_offset, int step0, uint64_t seed, int break_half) {
     long long n = (long long)B * K;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
@@ -900,9 +911,21 @@ static int launch_fused(mc_env* e, const mc_kp& k, cudaStream_t s, const char* w
 // come from the step's image kernels: at 4096 envs, 16^3, 64x64 a step, a
 // masked reset and the policy's input take 233 us, with the per-pixel kernel
 // 448.
+// Images so wide that a warp's band of no tile shape fits shared memory (uint8
+// rows of several thousand pixels) have no fused launch: the per-pixel kernel
+// renders them.
 static int render_obs(mc_env* e, cudaStream_t s, int regen) {
     mc_kp k = e->kp;
     if (k.B == 0) return MC_OK;
+    if (mc_env_fused_smem_bytes(e) > kSmemPerCta) {
+        if (regen != MC_KREGEN_NONE) {
+            const int rc = backend_rc(mc_launch_regen(&k, 1, s), "regen");
+            if (rc) return rc;
+        }
+        k_cameras_rt<<<blocks(k.B, 256), 256, 0, s>>>(k);
+        MC_CK(cudaGetLastError());
+        return backend_rc(e->be->render(&k, MC_FAM_SHADED, s), "render");
+    }
     k.family = MC_FAM_SHADED;
     k.look_only = 1;
     k.regen = regen;

@@ -141,3 +141,25 @@ def test_ground_shortcut_and_fp16(cuda, mode, kw):
         if cfg and (np.prod(kw.get("world", (16, 16, 16))) % 16):
             cfg = (0,) + cfg[1:]
         run(cuda, 14, 10, 61, obs_dtype=mode, cfg=cfg, episode_length=7, regen="per_env", **kw)
+
+
+@pytest.mark.parametrize("mode", ["uint8", "uint8_prebasis"])
+def test_images_too_wide_for_a_fused_launch(cuda, mode):
+    """Rows whose bands fit no launch shape's shared memory: resets and renders still work, beside plain steps."""
+    B = 2
+    kw = dict(world_x=16, world_y=16, world_z=16, render_width=20000, render_height=2, obs_dtype=mode, episode_length=2)
+    g = GpuEnv(cuda, B, debug=False, **kw)
+    o = O.OracleEnv(batch_size=B, **kw)
+    g.reset()
+    o.reset()
+    assert not diff_report(g.state(), oracle_state(o))
+    for s in range(4):
+        _, btn, look = actions_for(B, s, 62, 0.1, True)
+        g.step(btn, look, capi.FORM_PLAIN)
+        o.step(btn, look)
+        assert not diff_report(g.state(), oracle_state(o)), s
+        mask = np.array([s % 2 == 0, False])
+        g.reset(mask)
+        o.reset(mask)
+        assert not diff_report(g.state(), oracle_state(o)), s
+    g.close()
