@@ -1097,6 +1097,14 @@ static int host_mark(cudaEvent_t* ev, cudaStream_t s) {
     MC_CK(cudaEventRecord(*ev, s));
     return MC_OK;
 }
+// No host-buffer step on a stream under capture: a join after the capture
+// could not wait for an event recorded inside it.
+static int host_uncaptured(cudaStream_t s) {
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    MC_CK(cudaStreamIsCapturing(s, &cap));
+    if (cap != cudaStreamCaptureStatusNone) return fail(MC_ERR_INVALID, "a host-buffer step cannot be captured");
+    return MC_OK;
+}
 static HostViews host_views(const uint8_t* actions, float* rewards, uint8_t* dones) {
     HostViews v{};
     v.act = static_cast<const uint8_t*>(device_view(actions));
@@ -1115,14 +1123,16 @@ extern "C" int mc_env_step_host(mc_env* e, const uint8_t* host_actions, float* h
     if (!host_actions || !host_rewards || !host_dones) return fail(MC_ERR_INVALID, "host buffers are NULL");
     if (form != MC_FORM_PLAIN && form != MC_FORM_FUSED) return fail(MC_ERR_INVALID, "unknown form %d", form);
     cudaStream_t s = (cudaStream_t)stream;
+    int rc = host_uncaptured(s);
+    if (rc) return rc;
     if (form == MC_FORM_FUSED) {
         const HostViews v = host_views(host_actions, host_rewards, host_dones);
         if (v.ok) {
-            const int rc = do_step(e, nullptr, nullptr, v.act, form, s, v.rew, v.done);
+            rc = do_step(e, nullptr, nullptr, v.act, form, s, v.rew, v.done);
             return rc ? rc : host_mark(&e->host_done, s);
         }
     }
-    int rc = hostio_init(&e->hio, B);
+    rc = hostio_init(&e->hio, B);
     if (rc) return rc;
     HostIO* h = e->hio;
     const int i = (int)(h->calls & 1);
@@ -1568,12 +1578,14 @@ extern "C" int mc_ragged_step_host(mc_ragged* r, const uint8_t* host_actions, fl
     if (B == 0) return MC_OK;
     if (!host_actions || !host_rewards || !host_dones) return fail(MC_ERR_INVALID, "host buffers are NULL");
     cudaStream_t s = (cudaStream_t)stream;
+    int rc = host_uncaptured(s);
+    if (rc) return rc;
     const HostViews v = host_views(host_actions, host_rewards, host_dones);
     if (v.ok) {
-        const int rc = ragged_do_step(r, nullptr, nullptr, v.act, s, false, v.rew, v.done);
+        rc = ragged_do_step(r, nullptr, nullptr, v.act, s, false, v.rew, v.done);
         return rc ? rc : host_mark(&r->host_done, s);
     }
-    int rc = hostio_init(&r->hio, B);
+    rc = hostio_init(&r->hio, B);
     if (rc) return rc;
     HostIO* h = r->hio;
     const int i = (int)(h->calls & 1);

@@ -163,3 +163,28 @@ def test_ragged_step_host_matches_step(cuda):
             if a.dtype == torch.float32:
                 a, b = a.view(torch.int32), b.view(torch.int32)
             assert torch.equal(a, b), k
+
+
+def test_step_host_is_refused_under_capture(cuda):
+    """A stream under capture takes no host-buffer step, and later ones still run and join."""
+    import torch
+    from cuda.bindings import runtime as rt
+    B = 40
+    ref, env = _pair(cuda, "fused", batch_size=B, world_size=16, render_width=32, render_height=32, obs_dtype="uint8")
+    act = torch.full((B,), 6, dtype=torch.uint8).pin_memory()
+    rew = torch.zeros(B, dtype=torch.float32).pin_memory()
+    done = torch.zeros(B, dtype=torch.bool).pin_memory()
+    stream = torch.cuda.Stream(device=cuda)
+    torch.cuda.synchronize()
+    with torch.cuda.stream(stream):
+        assert rt.cudaStreamBeginCapture(stream.cuda_stream, rt.cudaStreamCaptureMode.cudaStreamCaptureModeThreadLocal
+                                         )[0] == rt.cudaError_t.cudaSuccess
+        with pytest.raises(RuntimeError):
+            env.step_host(act, rew, done)
+        assert rt.cudaStreamEndCapture(stream.cuda_stream)[0] == rt.cudaError_t.cudaSuccess
+    env.step_host(act, rew, done)
+    env.join_host()
+    torch.cuda.synchronize()
+    _, want, _ = ref.step(act.to(cuda))
+    assert torch.equal(rew, want.cpu())
+    assert torch.equal(env.obs_buffer, ref.obs_buffer)
