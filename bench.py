@@ -48,12 +48,13 @@ RENDER_WORKLOAD = dict(workload="render-dominated: B=4096 envs/GPU, world 32^3, 
                        obs_dtype="uint8", max_steps=64, seed=2, look_delta=0.1, break_half=True)
 METRIC = "env-steps/s at B=32K, W=16, 32x32 (fused step, CUDA graph)"
 RENDER_METRIC = "env-steps/s at B=4096, W=32, 64x64, half break actions (fused step, CUDA graph)"
-# DRAM bytes (read + written) of one launch of the workload's step kernel,
+# DRAM bytes (read + written) of one step of the workload,
 # from the ncu captures summarised in profiles/ (cold caches under ncu)
 TRAFFIC = {
-    "peak": (113.2e6 + 60.8e6, "k_step_fused, step 701, profiles/k_step_fused_peak_late_full.md"),
-    "render": (135.3e6 + 28.4e6, "k_step_team, step 301, profiles/k_step_team_B4096_w32_r64_full.md"),
-    "ragged": (70.7e6 + 15.3e6, "k_step_team, mean of its 75 launches, profiles/k_step_team_ragged_launches.md"),
+    "peak": (120.2e6 + 55.1e6, "k_agent + k_render_warp, step 701, profiles/k_render_warp_peak_late.md"),
+    "render": (135.7e6 + 26.3e6, "k_agent + k_render_team, step 301, profiles/k_render_team_B4096_w32_r64.md"),
+    "ragged": (174.6e6 + 69.0e6, "k_agent_groups + k_render_team, mean of the first 15 steps after a reset, "
+               "profiles/k_render_team_ragged_launches.md"),
 }
 
 
@@ -303,11 +304,11 @@ def run_mine(args):
     t_e2e_step = timed(e2e_loop)
     _ = float(h_rew.sum())  # the host reads the results
 
-    # the same through MineEnv.step_host: uploads and read-backs on the env's
-    # own streams, overlapping the neighbouring steps
+    # the same through MineEnv.step_host: the agent kernel reads and writes the
+    # pinned host buffers in place
     start(eager=True)
     snap = env.state_dict()
-    env.step_host(h_acts[Wm], h_rew[0], h_done[0])  # the first call allocates the host-I/O buffers
+    env.step_host(h_acts[Wm], h_rew[0], h_done[0])
     env.join_host()
     torch.cuda.synchronize()
     env.load_state_dict(snap)
@@ -404,7 +405,7 @@ def run_mine(args):
         "e2e": {"value": e2e_value, "unit": "env-steps/s", "h2d_bytes_per_step": B,
                 "d2h_bytes_per_step": B * 4 + B,
                 "path": "MineEnv.step_host per step: pinned host actions in, pinned host rewards+dones out; "
-                        "uploads and read-backs overlap the neighbouring steps",
+                        "read and written in place by the agent kernel",
                 "step_with_copies": {"value": B * K * world / t_e2e_step, "unit": "env-steps/s",
                                      "path": "MineEnv.step(actions) per step; H2D actions, D2H rewards+dones, "
                                              "one stream"}},
@@ -414,8 +415,8 @@ def run_mine(args):
                      "traffic_source": "--traffic-bytes" if args.traffic_bytes else
                      (TRAFFIC[args.workload][1] if not args.shape else None), "peak_kind": peak_kind,
                      "algorithmic_bytes_per_env_step": bytes_per_env_step,
-                     "kernel": "k_step_fused (avg over the timed region)"},
-        "gpu_launches": K,
+                     "kernel": "k_agent + k_render_warp (avg over the timed region)"},
+        "gpu_launches": 2 * K,  # agents, images
         "clocks": clk.summary(),
     }
     if f32 is not None:
@@ -581,8 +582,8 @@ def run_mine_ragged(args):
     t_e2e_step = timed(e2e_loop)
     _ = float(h_rew.sum())
 
-    # the same through RaggedBatch.step_host (uploads and read-backs overlap
-    # the neighbouring steps; the launch writes rewards and dones in batch order)
+    # the same through RaggedBatch.step_host (the agent kernel reads and
+    # writes the pinned host buffers in place, in batch order)
     batch.reset()
     for s in range(Wm):
         batch.step_host(h_acts[s], h_rew[s % K], h_done[s % K])
@@ -622,15 +623,15 @@ def run_mine_ragged(args):
         "e2e": {"value": total * K * world / t_e2e, "unit": "env-steps/s", "h2d_bytes_per_step": total,
                 "d2h_bytes_per_step": total * 5,
                 "path": "RaggedBatch.step_host per step: pinned host actions in, pinned host rewards+dones out; "
-                        "uploads and read-backs overlap the neighbouring steps",
+                        "read and written in place by the agent kernel",
                 "step_with_copies": {"value": total * K * world / t_e2e_step, "unit": "env-steps/s",
                                      "path": "RaggedBatch.step(actions); H2D actions, D2H rewards+dones per group, "
                                              "one stream"}},
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                      "traffic": TRAFFIC["ragged"][0], "traffic_source": TRAFFIC["ragged"][1], "peak_kind": peak_kind,
                      "algorithmic_bytes_per_step": bps,
-                     "kernel": "k_step_team (avg over the timed region)"},
-        "gpu_launches": K * (1 + sum(1 for e in envs if e.episode_length)),
+                     "kernel": "k_agent_groups + k_render_team (avg over the timed region)"},
+        "gpu_launches": 2 * K,  # agents, images
         "clocks": clk.summary(),
     }
     if rank == 0 and world == 1 and not args.no_cpu_baseline:
@@ -1107,7 +1108,7 @@ def run_mine_serve(args):
                 "path": "EnvServer requests: host actions in, host rewards+dones out (every request)"},
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                      "traffic": None, "peak_kind": peak_kind, "algorithmic_bytes_per_env_step": mean_bytes,
-                     "kernel": "k_step_team (served launches)"},
+                     "kernel": "k_agent_groups + k_render_team (served launches)"},
         "clocks": clk.summary(),
     }
     if rank == 0:

@@ -132,7 +132,7 @@ struct mc_fused_cfg {
     int coop;           // team kernel: 1 = a team renders each env together
 };
 
-// Several env groups stepped by one launch of the team kernel (k_step_team).
+// Several env groups stepped together (k_agent_groups, k_render_team).
 enum { MC_MAX_GROUPS = 16 };
 enum { MC_COLOUR_TABLE_BYTES = 224 };  // shared colour tables of the fused kernels (16-aligned)
 // the common-case render loop's tables (colour x shade: 13 x 4 float4; packed

@@ -304,8 +304,8 @@ class MineEnv:
         """The discrete step for a host-side policy: actions uint8 [B] read
         from pinned host memory, rewards float32 [B] and dones bool [B]
         written to pinned host memory.  Returns the (device) observation
-        buffer.  The copies overlap the device steps of the neighbouring
-        calls, so a call's host tensors stay in use until `join_host()` and
+        buffer.  The fused step reads and writes them in place (the plain
+        form copies, overlapping the neighbouring calls), so a call's host tensors stay in use until `join_host()` and
         a synchronisation of the current stream (e.g.
         torch.cuda.synchronize()): its actions must not be overwritten, nor
         its rewards and dones read, before then."""
