@@ -364,6 +364,36 @@ __device__ __forceinline__ void look_samples(Look& l, const int8_t* w, const mc_
 #pragma unroll
     for (int k = 0; k < 32; ++k) l.solid |= blk[k] >= 0 ? 1u << k : 0u;
 }
+// The samples of the envs `who` of a warp's 32, one lane per sample and four
+// envs' loads in flight; lane i gets env i's.  Called by the whole warp.
+__device__ __forceinline__ void look_together(Look& l, const int8_t* w, const mc_kp& p, unsigned who, int lane) {
+    const long long wxyz = (long long)p.wx * p.wy * p.wz;
+    while (who) {
+        int src[4], blk[4];
+        bool in[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            src[j] = __ffs(who) - 1;  // -1: none left
+            who &= who - 1u;
+            const int i = src[j] < 0 ? 0 : src[j];
+            const Sample s = interact_sample(lane, __shfl_sync(0xffffffffu, l.ex, i), __shfl_sync(0xffffffffu, l.ey, i),
+                                             __shfl_sync(0xffffffffu, l.ez, i), __shfl_sync(0xffffffffu, l.dx, i),
+                                             __shfl_sync(0xffffffffu, l.dy, i), __shfl_sync(0xffffffffu, l.dz, i),
+                                             p.wx, p.wy, p.wz);
+            const int8_t* wi = (const int8_t*)__shfl_sync(0xffffffffu, (unsigned long long)w, i);
+            in[j] = src[j] >= 0 && s.inb && in_bounds(s.idx, wxyz, MC_SITE_INTERACT);
+            blk[j] = in[j] ? wi[s.idx] : (int)AIR;
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const unsigned inb = __ballot_sync(0xffffffffu, in[j]), solid = __ballot_sync(0xffffffffu, blk[j] >= 0);
+            if (lane == src[j]) {
+                l.inb = inb;
+                l.solid = solid;
+            }
+        }
+    }
+}
 // Returns the in-env index written (-1 if none), *val the value written there.
 __device__ __forceinline__ int interact_judge(const Look& l, int8_t* w, bool brk, const mc_kp& p, float* reward,
                                               int* val) {
@@ -2332,12 +2362,22 @@ __device__ __forceinline__ void rec_facts(EnvRec& r, const mc_kp& p, bool eye_in
              (skip_first ? MC_ER_SKIP : 0) | (!buried && !fast ? MC_ER_SLOW : 0);
 }
 
+// Up to this many envs of a warp that interact share its lanes (look_together,
+// about 40 instructions an env); more take a thread each (look_samples, about
+// 750 for the warp, however few envs).  Uniform discrete actions break in 3
+// envs of 32: us a step, a thread per env -> shared lanes, 64 envs 16^3, 32x32
+// 14.8 -> 13.2, 4096 envs with host buffers 47.4 -> 45.7, 1024 envs 64x64 with
+// buttons (8 of 32) 37.9 -> 37.1; with half the actions breaking 195.0 and 195.1.
+constexpr int kLookTogether = 12;
+
 // Decode, episode rule, physics, interaction, reset, counters, camera (and
 // basis) of env e, by one thread.  Its loads come in two waves: the action and
-// state, then the eye's voxel and the interaction's samples.
+// state, then the eye's voxel and the interaction's samples.  The whole warp
+// calls it: the lanes without an env (`valid` false) bring the e of another,
+// help with the samples and write nothing.
 template <int FAM>
-__device__ __forceinline__ EnvRec agent_step(const mc_kp& p, const ActionSrc& act, long long e, float* res_rewards,
-                                             uint8_t* res_dones) {
+__device__ __forceinline__ EnvRec agent_step(const mc_kp& p, const ActionSrc& act, long long e, bool valid,
+                                             float* res_rewards, uint8_t* res_dones) {
     const long long wxyz = (long long)p.wx * p.wy * p.wz;
     int8_t btn[8];
     float l0, l1;
@@ -2370,12 +2410,18 @@ __device__ __forceinline__ EnvRec agent_step(const mc_kp& p, const ActionSrc& ac
     if (eye >= 0 && in_bounds(eye, wxyz, MC_SITE_EYE)) eye_blk = w[eye];
     float reward = 0.0f;
     int mod_idx = -1, mod_val = 0;
-    if (d.brk || d.place) {
+    const bool want = valid && (d.brk || d.place);
+    const unsigned who = __ballot_sync(0xffffffffu, want);
+    if (__popc(who) <= kLookTogether)
+        look_together(l, w, p, who, threadIdx.x & 31);
+    else if (want)
         look_samples(l, w, p);
+    if (want) {
         mod_idx = interact_judge(l, w, d.brk, p, &reward, &mod_val);
         if (mod_idx >= 0 && mod_idx == eye) eye_blk = mod_val;
     }
     rec_facts<FAM>(r, p, eye >= 0, eye_blk, done);
+    if (!valid) return r;
     store_agent(p, e, a);
     if (!p.ext_done) {
         p.step_count[e] = done ? 1 : cnt + 1;
@@ -2472,17 +2518,18 @@ __device__ __forceinline__ void file_recs(void* rec, int32_t* flags, int32_t* an
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
-// What bounds it: the latency of its dependent loads (action and state,
-// interaction samples, eye voxel), overlapped over 32 envs per warp, where
-// a warp per env repeated every instruction 32 times.
+// What bounds it: the latency of its dependent loads (action and state, then
+// interaction samples and eye voxel), overlapped over 32 envs per warp, where a
+// warp per env repeated every instruction 32 times.  Cold caches, 32768 envs
+// take 11.7 us and 4096 take 11.6, at 17% and 10% of the issue slots.
 template <int FAM>
 __global__ void __launch_bounds__(kAgentThreads) k_agent(const __grid_constant__ mc_kp p) {
     pdl_trigger();
     pdl_wait();
     const long long e = (long long)blockIdx.x * kAgentThreads + threadIdx.x;
     const bool valid = e < p.B;
-    EnvRec r{};
-    if (valid) r = agent_step<FAM>(p, ActionSrc{p.actions, p.buttons, p.look}, e, p.res_rewards, p.res_dones);
+    const EnvRec r = agent_step<FAM>(p, ActionSrc{p.actions, p.buttons, p.look}, valid ? e : p.B - 1, valid,
+                                     p.res_rewards, p.res_dones);
     file_recs(p.rec, p.flags, &p.flags[MC_FLAG_ANY_SLOW], p.B, p.compact, r, e, valid);
     if (threadIdx.x == 0) bounds_to_flags(p.flags);
 }
@@ -2531,13 +2578,10 @@ __global__ void __launch_bounds__(kAgentThreads) k_agent_groups(const __grid_con
     const mc_kp& p = rk.groups[g];
     const long long e = (long long)((int)blockIdx.x - rk.ablock[g]) * kAgentThreads + threadIdx.x, s0 = rk.start[g];
     const bool valid = e < p.B;
-    EnvRec r{};
-    if (valid) {
-        const ActionSrc act{rk.actions ? rk.actions + s0 : nullptr, rk.actions ? nullptr : rk.buttons + 8 * s0,
-                            rk.actions ? nullptr : rk.look + 2 * s0};
-        r = agent_step<FAM>(p, act, e, rk.rewards_cat ? rk.rewards_cat + s0 : nullptr,
-                            rk.dones_cat ? rk.dones_cat + s0 : nullptr);
-    }
+    const ActionSrc act{rk.actions ? rk.actions + s0 : nullptr, rk.actions ? nullptr : rk.buttons + 8 * s0,
+                        rk.actions ? nullptr : rk.look + 2 * s0};
+    const EnvRec r = agent_step<FAM>(p, act, valid ? e : p.B - 1, valid, rk.rewards_cat ? rk.rewards_cat + s0 : nullptr,
+                                     rk.dones_cat ? rk.dones_cat + s0 : nullptr);
     file_recs(reinterpret_cast<EnvRec*>(rk.rec) + s0, p.flags, &rk.flags[MC_FLAG_ANY_SLOW], p.B, p.compact, r, e, valid);
     if (threadIdx.x == 0) bounds_to_flags(p.flags);
 }

@@ -163,3 +163,27 @@ def test_images_too_wide_for_a_fused_launch(cuda, mode):
         o.reset(mask)
         assert not diff_report(g.state(), oracle_state(o)), s
     g.close()
+
+
+@pytest.mark.parametrize("B", [1, 45])
+@pytest.mark.parametrize("n", [1, 4, 5, 12, 13, 32])
+def test_interactions_per_warp(cuda, B, n):
+    """n envs of each warp break or place: up to 12 share the warp's lanes, more take a thread each."""
+    kw = dict(world_x=16, world_y=16, world_z=16, render_width=32, render_height=32, obs_dtype="uint8", episode_length=9)
+    g = GpuEnv(cuda, B, debug=False, **kw)
+    o = O.OracleEnv(batch_size=B, **kw)
+    g.reset()
+    o.reset()
+    rng = np.random.default_rng(63)
+    for s in range(14):
+        _, btn, look = actions_for(B, s, 63, 0.1, False)
+        look = (look + rng.normal(0, 0.3, look.shape)).astype(np.float32)
+        act = (np.arange(B) + 3 * s) % 32 < n
+        btn[:, 5] = act & (rng.random(B) < 0.7)
+        btn[:, 6] = act & (btn[:, 5] == 0)
+        g.step(btn, look, capi.FORM_FUSED)
+        o.step(btn, look)
+        d = diff_report(g.state(), oracle_state(o))
+        assert not d, f"step {s}: {d}"
+    g.check_error()
+    g.close()
