@@ -2520,8 +2520,9 @@ __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.lau
 
 // What bounds it: the latency of its dependent loads (action and state, then
 // interaction samples and eye voxel), overlapped over 32 envs per warp, where a
-// warp per env repeated every instruction 32 times.  Cold caches, 32768 envs
-// take 11.7 us and 4096 take 11.6, at 17% and 10% of the issue slots.
+// warp per env repeated every instruction 32 times.  Cold caches, with a thread
+// per interaction (look_samples) throughout, 32768 envs took 11.7 us and 4096
+// 11.6, at 17% and 10% of the issue slots.
 template <int FAM>
 __global__ void __launch_bounds__(kAgentThreads) k_agent(const __grid_constant__ mc_kp p) {
     pdl_trigger();
