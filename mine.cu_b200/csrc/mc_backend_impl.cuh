@@ -921,7 +921,7 @@ __device__ __forceinline__ int march_staged(uint32_t base, int idx, int cx, int 
                                            int wx, int wy, int wz, int max_steps, float& tmx, float& tmy, float& tmz,
                                            float tdx, float tdy, float tdz) {
     const SmemRange chk = staged_range(base, wx * wz, wx * wy * wz);
-    if (max_steps > wx + wy + wz && wx <= 31 && wy <= 31 && wz <= 31 && wx * wy * wz < 8192) {
+    if (max_steps > wx + wy + wz && mc_packed_world(wx, wy, wz)) {
         int packed = (idx << 18) | ((31 - cx) << 12) | ((31 - max(cy, -32)) << 6) | (31 - cz);
         return march_packed_shared(base, packed, (dix << 18) + (1 << 12), (diy << 18) + (1 << 6), (diz << 18) + 1,
                                    tmx, tmy, tmz, tdx, tdy, tdz, chk);
@@ -1051,8 +1051,7 @@ __device__ __forceinline__ Hit shade_ray(const Cam& c, const Dda0& d0, float u, 
                       cz = (sz > 0) ? wz - 1 - vz : vz;
             if (b < 0) {
                 const uint32_t base = (uint32_t)__cvta_generic_to_shared(vox.w);
-                if (vd_safe && max_steps > wx + wy + wz && wx <= 31 && wy <= 31 && wz <= 31 &&
-                           wx * wy * wz < 8192) {
+                if (vd_safe && max_steps > wx + wy + wz && mc_packed_world(wx, wy, wz)) {
                     // index and in-box counts in one register (march_packed_shared)
                     int packed = (idx << 18) | ((31 - cx) << 12) | ((31 - max(cy, -32)) << 6) | (31 - cz);
                     b = march_packed_shared(base, packed, (dix << 18) + (1 << 12), (diy << 18) + (1 << 6),
@@ -1090,7 +1089,8 @@ __device__ __forceinline__ Hit shade_ray(const Cam& c, const Dda0& d0, float u, 
         int cx = (sx > 0) ? wx - 1 - vx : vx, cy = (sy > 0) ? min(wy - 1, ytop) - vy : vy,
             cz = (sz > 0) ? wz - 1 - vz : vz;
         if (max_steps > wx + wy + wz && wx <= 31 && wy <= 31 && wz <= 31 && wx * wy * wz < 8192) {
-            // every ray leaves the box before max_steps: no step count.  The
+            // every ray leaves the box before max_steps: no step count.  (The exit
+            // test comes before the load, so the layer beyond the box need not fit.)  The
             // voxel index and the three in-box counts share one register:
             // bits 18.. the index, three 6-bit fields below it counting up
             // from 31 - (steps left) to 32, whose bit 5 marks leaving the
@@ -2240,7 +2240,7 @@ template <int FAM>
 __device__ __forceinline__ int fast_kind(bool vd_safe, int max_steps, int wx, int wy, int wz) {
     constexpr bool G = FAM == MC_FAM_SHADED_FAST;  // its rays may step on outside the box (ground_tail)
     const bool packed = (FAM == MC_FAM_SHADED || G ? vd_safe : true) && max_steps > wx + wy + wz + (G ? 8 : 0) &&
-                        wx <= 31 && wy <= 31 && wz <= 31 && wx * wy * wz < 8192;
+                        mc_packed_world(wx, wy, wz);
     return packed ? 1 : 2;
 }
 

@@ -196,6 +196,16 @@ __host__ __device__
 static inline int mc_odd_world(const mc_kp& k) {
     return (((long long)k.wx * k.wy * k.wz) & 15) != 0 || (((uintptr_t)k.voxels) & 15) != 0;
 }
+// Whether the packed march can run over a staged world: its in-box counts hold
+// 31 voxels a side, and its voxel index 14 signed bits.  The index of the step
+// that leaves the box is loaded too, up to one layer before or after the world,
+// so it is that range, -wx*wz .. wx*wz*(wy+1)-1, that has to fit.
+#ifdef __CUDACC__
+__host__ __device__
+#endif
+static inline int mc_packed_world(int wx, int wy, int wz) {
+    return wx <= 31 && wy <= 31 && wz <= 31 && wx * wz * (wy + 1) <= 8192;
+}
 // Shared-memory bytes of one staged world: 16 to spare where it starts at any byte.
 #ifdef __CUDACC__
 __host__ __device__
