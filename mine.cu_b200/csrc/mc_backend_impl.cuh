@@ -2646,11 +2646,13 @@ __device__ __forceinline__ int8_t* staged_at(int8_t* slot, const int8_t* src) { 
 // Start the copy of one world into its slot (by one warp): the whole 16-byte
 // chunks by a bulk copy, the bytes before and after them (worlds that start or
 // end at any byte) by plain loads.  The stores precede lane 0's arrival, so
-// whoever waits on the mbarrier sees them too.
+// whoever waits on the mbarrier sees them too.  All lanes are done with the
+// world that was in the slot before any of it is overwritten.
 __device__ __forceinline__ void issue_world_copy(uint32_t mbar_a, int8_t* slot, const int8_t* src, int bytes, int lane) {
     const int off = (int)((uintptr_t)src & 15u);
     int8_t* dst = slot + off;
     int head = 0, body = bytes;
+    __syncwarp();
     if (off | (bytes & 15)) {  // uniform
         head = min((16 - off) & 15, bytes);
         const int tail = (bytes - head) & 15;
@@ -2828,6 +2830,8 @@ __device__ __forceinline__ void render_slow_from(const mc_kp& p, int e, const En
             }
         }
     }
+    // the lanes' rays end at different times, and the caller may now overwrite the world (regen_world)
+    __syncwarp();
 }
 
 template <int FAM, bool F32>
