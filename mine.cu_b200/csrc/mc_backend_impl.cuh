@@ -3121,8 +3121,9 @@ struct TeamShared {
     unsigned unit[4];      // claimed units, unit k's number at k & 3
     int band_ctr[2];       // next row band of the cooperative env of unit k & 1
     unsigned long long mbar[2];
-    int timed_out;         // a wait for a copy ran out: no further copies, render from global memory
-    int may_stage[2];      // general pass: whether unit k & 1 may be staged
+    int timed_out[2];      // a wait for the copy of unit k ran out, at k & 1: no further copies, render from
+                           // global memory (read after unit k's barrier: by then only unit k + 1's warps write,
+                           // to the other one, and once it is set nobody stages again)
     unsigned sunit[2];     // general pass: claimed units, alternating slots
     int any_done;          // bit g: every world of group g is to be regenerated
     int last;              // the team rendered its env's last slice
@@ -3239,7 +3240,7 @@ __global__ void __launch_bounds__(256, MC_TEAM_MIN_BLOCKS) k_render_team(const _
     pdl_wait();
     if (claimer) {
         for (int k = 0; k < DEPTH; ++k) ts->unit[k] = claim(MC_FLAG_WORK);
-        ts->timed_out = 0;
+        ts->timed_out[0] = ts->timed_out[1] = 0;
         int any = 0;
         for (int g = 0; g < G; ++g)
             if (rk.groups[g].regen == MC_KREGEN_ALL && *(volatile int32_t*)&rk.groups[g].flags[MC_FLAG_ANY_DONE])
@@ -3299,17 +3300,17 @@ __global__ void __launch_bounds__(256, MC_TEAM_MIN_BLOCKS) k_render_team(const _
     auto staged_world = [&](const Unit& t, const EnvRec& q, int d) -> const int8_t* {
         return staged_at(slot_world(d, t.coop), world_of(rk.groups[t.g], q.env, q.bits, (ts->any_done >> t.g) & 1));
     };
-    // Wait for the copy of unit t into depth slot d.
-    auto landed = [&](const Unit& t, int d) -> bool {
+    // Wait for the copy of unit t, the team's k-th, into depth slot d.
+    auto landed = [&](const Unit& t, int d, int k) -> bool {
         const mc_kp& p = rk.groups[t.g];
         if (!stage_fits(slot_world(d, t.coop), mc_world_slot(p))) {
-            *(volatile int*)&ts->timed_out = 1;
+            *(volatile int*)&ts->timed_out[k & 1] = 1;
             return false;
         }
         uint32_t& ph = t.coop ? tphase : wphase;
         if (!mbar_wait((t.coop ? tmbar : cx.mbar_a) + 8 * d, (ph >> d) & 1u, p.wait_polls)) {
             if (lane == 0) atomicExch(&p.flags[MC_FLAG_ERROR], MC_KERR_TMA_TIMEOUT);
-            *(volatile int*)&ts->timed_out = 1;
+            *(volatile int*)&ts->timed_out[k & 1] = 1;
             return false;
         }
         ph ^= 1u << d;
@@ -3336,9 +3337,9 @@ __global__ void __launch_bounds__(256, MC_TEAM_MIN_BLOCKS) k_render_team(const _
         regen_world(p, e, wt * 32 + lane, nthr);
     };
 
+    bool redo = false;  // the same for the whole team
     {
         int k = 0;
-        bool redo = false;
         if (DEPTH > 1 && ts->unit[0] < total_units) issue(locate(ts->unit[0]), 0, 0);
         for (;; ++k) {
             const int d = DEPTH > 1 ? (k & 1) : 0;  // world slot and mbarrier of this unit
@@ -3364,7 +3365,7 @@ __global__ void __launch_bounds__(256, MC_TEAM_MIN_BLOCKS) k_render_team(const _
                         fill_env<FAM, F32>(p, q.env, q.fill_blk, cx, t.coop ? wt * 32 + lane : lane,
                                            t.coop ? nthr : 32);
                 } else if (!(q.bits & MC_ER_SLOW)) {
-                    const bool ok = landed(t, d);
+                    const bool ok = landed(t, d, k);
                     const int8_t* world = staged_world(t, q, d);
                     EnvRender r = render_of_rec(q, p.wy);
                     if (t.coop && TWN > 1 && up_scan_shape(p.wx, p.wy, p.wz))  // team-uniform; the eye is in the box
@@ -3380,7 +3381,7 @@ __global__ void __launch_bounds__(256, MC_TEAM_MIN_BLOCKS) k_render_team(const _
             }
             if (claimer) ts->unit[(k + DEPTH) & 3] = claim(MC_FLAG_WORK);
             team_sync(bar, nthr);
-            if (*(volatile int*)&ts->timed_out) {  // set before the barrier: the same for the whole team
+            if (*(volatile int*)&ts->timed_out[k & 1]) {
                 redo = true;
                 break;
             }
@@ -3419,16 +3420,16 @@ __global__ void __launch_bounds__(256, MC_TEAM_MIN_BLOCKS) k_render_team(const _
     // the general pass: the envs that the common path left
     if (claimer) {
         ts->sunit[0] = *(volatile int32_t*)&rk.flags[MC_FLAG_ANY_SLOW] ? claim(MC_FLAG_SLOW_WORK) : total_units;
-        ts->may_stage[0] = !*(volatile int*)&ts->timed_out;
         team_unit_reset(ts, 0);
     }
     team_sync(bar, nthr);
+    bool stage_ok = !redo;  // the same for the whole team
     for (int k = 0;; ++k) {
         const unsigned u = ts->sunit[k & 1];
         if (u >= total_units) break;
         const Unit t = locate(u);
         const mc_kp& p = rk.groups[t.g];
-        const bool may_stage = ((rk.stage_mask >> t.g) & 1) && ts->may_stage[k & 1];  // team-uniform
+        const bool may_stage = ((rk.stage_mask >> t.g) & 1) && stage_ok;
         if (may_stage && t.part == 0) issue(t, 0, MC_ER_SLOW);
         if (claimer) team_unit_reset(ts, (k + 1) & 1);
         int bits = 0, env = 0;
@@ -3441,18 +3442,16 @@ __global__ void __launch_bounds__(256, MC_TEAM_MIN_BLOCKS) k_render_team(const _
             use_group(t.g);
             if (here) {
                 const int8_t* world = staged_world(t, q, 0);
-                const bool staged = may_stage && landed(t, 0);
+                const bool staged = may_stage && landed(t, 0, k);
                 const int ytop = staged ? staged_top_layer(world, p.wx, p.wy, p.wz, lane) : p.wy - 1;
                 render_slow<FAM, F32>(p, q, ytop, cx, staged ? world : nullptr,
                                       world_of(p, q.env, q.bits, (ts->any_done >> t.g) & 1), rk.tile_w[t.g], lane,
                                       t.coop ? &ts->band_ctr[k & 1] : nullptr);
             }
         }
-        if (claimer) {
-            ts->sunit[(k + 1) & 1] = claim(MC_FLAG_SLOW_WORK);
-            ts->may_stage[(k + 1) & 1] = !*(volatile int*)&ts->timed_out;
-        }
+        if (claimer) ts->sunit[(k + 1) & 1] = claim(MC_FLAG_SLOW_WORK);
         team_sync(bar, nthr);
+        stage_ok &= !*(volatile int*)&ts->timed_out[k & 1];
         if (here) regen(t, bits, env, false);
     }
     // timed-out copies may still be in flight: let them land (bounded) before
