@@ -3541,6 +3541,18 @@ static int launch_pdl(void (*kern)(P...), long long grid, int threads, size_t sm
     return (int)cudaLaunchKernelEx(&lc, kern, std::forward<A>(args)...);
 }
 
+// A kernel's dynamic shared memory above 48 KB has to be allowed on each device.
+template <class K>
+static int allow_smem(mc_once_per_device& limit, K kern, size_t smem) {
+    if (smem <= 48 * 1024) return 0;
+    int dev = -1;
+    const cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return (int)e;
+    return limit(dev, [&] {
+        return (int)cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+    });
+}
+
 // Row ranges each image of the per-warp kernel is cut into: up to two units
 // per warp of the grid.  Measured at 16^3, 32x32 images, in units per warp
 // (4736 warps): 4096 envs 64.6 us a step at 0.9, 54.9 at 1.7, 61.8 at 3.5 (a
@@ -3556,12 +3568,9 @@ template <int FAM, bool F32, bool STAGE>
 static int launch_warp_t(const mc_kp* p, const mc_fused_cfg* cfg, int slices, long long grid, cudaStream_t s) {
     auto kern = k_render_warp<FAM, F32, STAGE>;
     const size_t smem = fused_smem(p, cfg);
-    static size_t attr_set = 0;  // per instantiation
-    if (smem > 48 * 1024 && smem > attr_set) {
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return (int)e;
-        attr_set = smem;
-    }
+    static mc_once_per_device limit;  // per instantiation
+    const int rc = allow_smem(limit, kern, smem);
+    if (rc) return rc;
     return launch_pdl(kern, grid, 32 * cfg->warps_per_cta, smem, s, *p, cfg->tile_w, slices);
 }
 
@@ -3615,12 +3624,9 @@ static int launch_team_t(const mc_ragged_kp* rk, int warps_per_cta, int ctas_per
     const bool deep = rk->depth == 2;
     auto kern = deep ? k_render_team<FAM, F32, 2> : k_render_team<FAM, F32, 1>;
     size_t smem = (size_t)rk->warps_off + (size_t)warps_per_cta * rk->warp_bytes + (size_t)rk->tail_bytes;
-    static size_t attr_set[2] = {0, 0};  // per kernel of this instantiation
-    if (smem > 48 * 1024 && smem > attr_set[deep]) {
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return (int)e;
-        attr_set[deep] = smem;
-    }
+    static mc_once_per_device limit[2];  // per kernel of this instantiation
+    rc = allow_smem(limit[deep], kern, smem);
+    if (rc) return rc;
     const int teams_per_cta = warps_per_cta / rk->team_warps;
     long long ctas_needed = (rk->ustart[rk->ngroups] + teams_per_cta - 1) / teams_per_cta;
     long long grid = (long long)num_sms * (ctas_per_sm > 0 ? ctas_per_sm : 1);

@@ -4,6 +4,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
+
 // Render families: one per reference render kernel.
 enum {
     MC_FAM_SHADED = 0,       // render_kernel / render_kernel_uint8 (kernels.cu:87-470)
@@ -236,6 +238,20 @@ static inline int mc_fast_launch(const mc_kp& k, int stage, int tile_w) {
     if (!mc_whole_tiles(k.W, k.H, k.obs_f32, tile_w)) return 2;
     return (((uintptr_t)k.obs) & 15) ? 0 : 1;
 }
+
+// A setting that a device keeps (a kernel's shared-memory limit): `set` runs
+// until it has succeeded once for each device; threads may run it twice.
+struct mc_once_per_device {
+    std::atomic<unsigned long long> done{0};  // bit d: device d has it
+    template <class Set>
+    int operator()(int device, Set set) {
+        const unsigned long long bit = device >= 0 && device < 64 ? 1ull << device : 0ull;
+        if (done.load(std::memory_order_acquire) & bit) return 0;
+        const int rc = set();
+        if (rc == 0) done.fetch_or(bit, std::memory_order_release);
+        return rc;
+    }
+};
 
 // One numerics back end (ref_fast or ieee).
 struct mc_backend {
