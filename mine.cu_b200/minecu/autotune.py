@@ -39,7 +39,7 @@ import torch
 
 from minecu import MineEnv, _C
 
-TILE_WIDTHS = (4, 8, 16)
+TILE_WIDTHS = (4, 8, 16, 32)
 MAX_SMEM = 227 * 1024
 
 
@@ -115,6 +115,13 @@ def env_candidates() -> List[Tuple[int, int, int, int, int, int]]:
     return per_warp + teams
 
 
+def _with_current(current: dict, candidates: Iterable[Tuple[int, ...]]) -> List[Tuple[int, ...]]:
+    """The shape the env has now, then the other candidates: tuning never ends
+    with a shape slower than the one it found."""
+    now = tuple(int(current[k]) for k in ("stage", "warps_per_cta", "ctas_per_sm", "tile_w", "team_warps", "coop"))
+    return [now] + [c for c in candidates if tuple(c) != now]
+
+
 def tune_env(env: MineEnv, steps: int = 40, warm_steps: int = 50, seed: int = 1, use_cache: bool = True,
              candidates: Optional[Iterable[Tuple[int, ...]]] = None, verbose: bool = False) -> dict:
     """Choose (stage, warps_per_cta, ctas_per_sm, tile_w, team_warps, coop)
@@ -135,7 +142,7 @@ def tune_env(env: MineEnv, steps: int = 40, warm_steps: int = 50, seed: int = 1,
         snap = env.state_dict()
         window = acts[warm_steps:]
         if candidates is None:
-            candidates = env_candidates()
+            candidates = _with_current(env.launch_config(), env_candidates())
         results: List[Tuple[float, tuple]] = []
         for cfg in candidates:
             try:
