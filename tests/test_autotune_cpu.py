@@ -74,3 +74,9 @@ def test_tuning_never_ends_slower_than_the_shape_it_found(clock, B):
 def test_the_tuner_tries_every_tile_width_the_defaults_use(B):
     tiles = {c[3] for c in autotune.env_candidates()}
     assert _default_shape(B)[3] in tiles
+
+
+def test_no_two_candidates_are_the_same_launch():
+    """With one warp per env a staging depth of 2 is one of 1."""
+    launches = [c if c[5] or c[4] > 1 else (min(c[0], 1),) + tuple(c[1:]) for c in autotune.env_candidates()]
+    assert len(set(launches)) == len(launches)
