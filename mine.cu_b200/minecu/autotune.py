@@ -24,11 +24,14 @@ For a `RaggedBatch` ``tile_w``, ``stage`` and ``coop`` are chosen per group.  Ev
 trial restores the same snapshot of the env state, replays the same K-step
 action window through a CUDA graph and is timed with CUDA events, so trials
 see identical work; the winner is set on the env and cached in a JSON file
-keyed by device name and workload signature (``$MINECU_TUNE_CACHE`` or
+keyed by device name, kernels (a hash of the library: shapes tuned for other
+kernels are measured again) and workload signature (``$MINECU_TUNE_CACHE`` or
 ``~/.cache/minecu_b200/autotune.json``).
 """
 from __future__ import annotations
 
+import functools
+import hashlib
 import json
 import os
 import time
@@ -36,7 +39,7 @@ from typing import Dict, Iterable, List, Optional, Sequence, Tuple
 
 import torch
 
-from minecu import MineEnv, _C
+from minecu import MineEnv, _C, capi
 
 TILE_WIDTHS = (4, 8, 16, 32)
 MAX_SMEM = 227 * 1024
@@ -78,6 +81,16 @@ def env_signature(e: MineEnv) -> str:
 
 def _device_key(dev: torch.device) -> str:
     return torch.cuda.get_device_name(dev).replace(" ", "_")
+
+
+@functools.lru_cache(maxsize=None)
+def _library_hash(path: str) -> str:
+    with open(path, "rb") as f:
+        return hashlib.sha256(f.read()).hexdigest()[:16]
+
+
+def _cache_key(kind: str, dev: torch.device, signature: str) -> str:
+    return f"{kind}|{_device_key(dev)}|{_library_hash(capi.LIB_PATH)}|{signature}"
 
 
 def _time_window(run, restore, reps: int = 2) -> float:
@@ -126,7 +139,7 @@ def tune_env(env: MineEnv, steps: int = 40, warm_steps: int = 50, seed: int = 1,
     """Choose (stage, warps_per_cta, ctas_per_sm, tile_w, team_warps, coop)
     for `env`'s fused step, set it on the env and return {"config": ...,
     "ms_per_step": ...}.  The env's state is restored afterwards."""
-    key = f"env|{_device_key(env.device)}|{env_signature(env)}"
+    key = _cache_key("env", env.device, env_signature(env))
     if use_cache:
         hit = _load_cache().get(key)
         if hit:
@@ -167,7 +180,7 @@ def tune_env(env: MineEnv, steps: int = 40, warm_steps: int = 50, seed: int = 1,
 # a RaggedBatch
 # ---------------------------------------------------------------------------
 def _ragged_key(batch) -> str:
-    return "ragged|" + _device_key(batch.device) + "|" + "+".join(env_signature(e) for e in batch.envs)
+    return _cache_key("ragged", batch.device, "+".join(env_signature(e) for e in batch.envs))
 
 
 def tune_ragged(batch, steps: int = 30, warm_steps: int = 50, seed: int = 3, use_cache: bool = True,

@@ -80,3 +80,23 @@ def test_no_two_candidates_are_the_same_launch():
     """With one warp per env a staging depth of 2 is one of 1."""
     launches = [c if c[5] or c[4] > 1 else (min(c[0], 1),) + tuple(c[1:]) for c in autotune.env_candidates()]
     assert len(set(launches)) == len(launches)
+
+
+def test_shapes_tuned_for_other_kernels_are_measured_again(clock, monkeypatch, tmp_path):
+    slow, quick = (0, 8, 4, 4, 1, 0), (1, 8, 3, 8, 4, 1)
+    libs = []
+    for k in range(2):
+        libs.append(tmp_path / f"lib{k}.so")
+        libs[k].write_bytes(b"kernels %d" % k)
+    cands = [slow, quick]
+    monkeypatch.setattr(capi, "LIB_PATH", str(libs[0]))
+    clock["env"] = env = FakeEnv(slow, lambda s: 1.0 if s == slow else 2.0)
+    assert tuple(autotune.tune_env(env, steps=2, warm_steps=1, candidates=cands)["config"]) == slow
+    clock["env"] = env = FakeEnv(slow, lambda s: 1.0 if s == quick else 2.0)
+    assert tuple(autotune.tune_env(env, steps=2, warm_steps=1, candidates=cands)["config"]) == slow  # remembered
+    monkeypatch.setattr(capi, "LIB_PATH", str(libs[1]))  # other kernels
+    assert tuple(autotune.tune_env(env, steps=2, warm_steps=1, candidates=cands)["config"]) == quick
+    batch = type("Batch", (), dict(device="cpu", envs=[env]))()
+    other = autotune._ragged_key(batch)
+    monkeypatch.setattr(capi, "LIB_PATH", str(libs[0]))
+    assert autotune._ragged_key(batch) != other
