@@ -53,6 +53,7 @@ struct mc_env {
     int32_t* flags;
     int8_t* tmpl;
     uint8_t* rec;      // render records of the fused form (MC_REC_BYTES per env)
+    bool rec_borrowed; // rec is the server's
     uint8_t* scratch;  // plain-form decode buffers
     cudaStream_t cap_stream;
     std::vector<RolloutGraph> graphs;
@@ -61,6 +62,10 @@ struct mc_env {
     int regen_mode;  // MC_REGEN_ALL (the reference's rule) or MC_REGEN_PER_ENV
 };
 
+// mc_env_create with render records that the caller owns (NULL: the env's own),
+// and other ones later.  Launches that share records run on one stream.
+MC_HIDDEN int mc_env_create_with_rec(const mc_env_config* cfg, const mc_env_state* state, uint8_t* rec, mc_env** out);
+MC_HIDDEN void mc_env_borrow_rec(mc_env* e, uint8_t* rec);
 // Record a formatted message for mc_last_error() and return `code`.
 MC_HIDDEN int mc_fail(int code, const char* fmt, ...);
 // MC_ERR_CUDA with the CUDA error string.

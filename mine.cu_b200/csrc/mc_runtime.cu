@@ -753,7 +753,16 @@ static void drop_graphs(mc_env* e) {
     e->graphs.clear();
 }
 
+void mc_env_borrow_rec(mc_env* e, uint8_t* rec) {  // e has never had records of its own
+    e->rec = rec;
+    e->kp.rec = rec;
+}
+
 extern "C" int mc_env_create(const mc_env_config* cfg, const mc_env_state* state, mc_env** out) {
+    return mc_env_create_with_rec(cfg, state, nullptr, out);
+}
+
+int mc_env_create_with_rec(const mc_env_config* cfg, const mc_env_state* state, uint8_t* rec, mc_env** out) {
     if (!out) return fail(MC_ERR_INVALID, "out is NULL");
     *out = nullptr;
     int rc = check_config(cfg);
@@ -777,7 +786,9 @@ extern "C" int mc_env_create(const mc_env_config* cfg, const mc_env_state* state
     if (ce == cudaSuccess) ce = cudaMalloc(&e->flags, MC_FLAG_WORDS * sizeof(int32_t));
     if (ce == cudaSuccess) ce = cudaMemset(e->flags, 0, MC_FLAG_WORDS * sizeof(int32_t));
     if (ce == cudaSuccess) ce = cudaMalloc(&e->tmpl, (size_t)((wxyz + 15) & ~15LL));
-    if (ce == cudaSuccess) ce = cudaMalloc(&e->rec, (size_t)cfg->batch_size * MC_REC_BYTES + 16);
+    e->rec = rec;
+    e->rec_borrowed = rec != nullptr;
+    if (ce == cudaSuccess && !rec) ce = cudaMalloc(&e->rec, (size_t)cfg->batch_size * MC_REC_BYTES + 16);
     if (ce == cudaSuccess) ce = cudaStreamCreateWithFlags(&e->cap_stream, cudaStreamNonBlocking);
     if (ce == cudaSuccess) {
         // the template world: generate + tree + house on one env
@@ -838,7 +849,7 @@ extern "C" int mc_env_destroy(mc_env* e) {
     drop_graphs(e);
     if (e->flags) cudaFree(e->flags);
     if (e->tmpl) cudaFree(e->tmpl);
-    if (e->rec) cudaFree(e->rec);
+    if (e->rec && !e->rec_borrowed) cudaFree(e->rec);
     if (e->scratch) cudaFree(e->scratch);
     if (e->cap_stream) cudaStreamDestroy(e->cap_stream);
     delete e;

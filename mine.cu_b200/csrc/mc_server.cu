@@ -190,7 +190,7 @@ struct mc_server {
     cudaStream_t stream = nullptr, admit_stream = nullptr;
     cudaStream_t up = nullptr, down = nullptr;  // batching = 0: actions uploads, results read-backs
     int32_t* flags = nullptr;  // work counter of the team launches
-    uint8_t* rec = nullptr;    // render records of one team launch (cap envs)
+    uint8_t* rec = nullptr;    // render records of the launches on `stream` (cap envs)
     Slot slots[kMaxSlots];
     int nslots = 0;
     std::deque<int> flight;  // busy slots in launch order
@@ -742,13 +742,24 @@ extern "C" int mc_server_admit(mc_server* s, const mc_env_config* cfg, int32_t* 
     st.basis = L.basis == (size_t)-1 ? nullptr : reinterpret_cast<float*>(b + L.basis);
     st.obs = b + L.obs;
     st.rewards = reinterpret_cast<float*>(b + L.rewards);
+    // A job has no render records of its own beside the bytes it is charged for:
+    // its launches on the server's stream use the server's, and the reset here,
+    // on another stream, passing ones.
+    void* rec = nullptr;
+    ce = cudaMallocAsync(&rec, (size_t)cfg->batch_size * MC_REC_BYTES + 16, s->admit_stream);
     mc_env* env = nullptr;
-    int rc = mc_env_create(cfg, &st, &env);
+    int rc = ce == cudaSuccess ? mc_env_create_with_rec(cfg, &st, static_cast<uint8_t*>(rec), &env)
+                               : mc_cuda_fail(ce, "mc_server_admit: allocation");
     if (rc == MC_OK) rc = mc_env_generate_world(env, s->admit_stream);
     if (rc == MC_OK) rc = mc_env_reset(env, nullptr, s->admit_stream);
     if (rc == MC_OK) {
         ce = cudaStreamSynchronize(s->admit_stream);
         if (ce != cudaSuccess) rc = mc_cuda_fail(ce, "mc_server_admit: world generation");
+    }
+    if (rec) {
+        if (env) mc_env_borrow_rec(env, s->rec);
+        cudaFreeAsync(rec, s->admit_stream);
+        cudaStreamSynchronize(s->admit_stream);  // returns what is not in use to the device
     }
     if (rc != MC_OK) {
         if (env) mc_env_destroy(env);
