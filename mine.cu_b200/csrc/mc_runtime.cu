@@ -1212,6 +1212,19 @@ static bool same_fcfg(const mc_fused_cfg& a, const mc_fused_cfg& b) {
            a.tile_w == b.tile_w && a.team_warps == b.team_warps && a.coop == b.coop;
 }
 
+// Whether the env's kernels may write an output at p themselves: this device's
+// memory (or managed), aligned.  Copies take any byte, another device's memory
+// too, and turn the rest away.
+static bool kernel_writes(const mc_env* e, const void* p, unsigned align) {
+    cudaPointerAttributes a{};
+    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    const bool here = (a.type == cudaMemoryTypeDevice && a.device == e->device) || a.type == cudaMemoryTypeManaged;
+    return here && ((uintptr_t)p) % align == 0;
+}
+
 static int rollout_graph(mc_env* e, const uint8_t* actions, int32_t K, float* rewards_out, uint8_t* dones_out,
                          RolloutGraph** out) {
     *out = nullptr;
@@ -1226,10 +1239,19 @@ static int rollout_graph(mc_env* e, const uint8_t* actions, int32_t K, float* re
         cudaGraph_t graph = nullptr;
         MC_CK(cudaStreamBeginCapture(e->cap_stream, cudaStreamCaptureModeThreadLocal));
         int rc = MC_OK;
+        const bool rew_direct = rewards_out && kernel_writes(e, rewards_out, 4);
+        const bool done_direct = dones_out && kernel_writes(e, dones_out, 1);
         for (int k = 0; k < K && rc == MC_OK; ++k) {
+            float* rew = rewards_out ? rewards_out + (long long)k * B : nullptr;
+            uint8_t* done = dones_out ? dones_out + (long long)k * B : nullptr;
             rc = do_step(e, nullptr, nullptr, actions + (long long)k * B, MC_FORM_FUSED, e->cap_stream,
-                         rewards_out ? rewards_out + (long long)k * B : nullptr,
-                         dones_out ? dones_out + (long long)k * B : nullptr);
+                         rew_direct ? rew : nullptr, done_direct ? done : nullptr);
+            cudaError_t ce = cudaSuccess;
+            if (rc == MC_OK && rew && !rew_direct)
+                ce = cudaMemcpyAsync(rew, e->kp.rewards, B * sizeof(float), cudaMemcpyDeviceToDevice, e->cap_stream);
+            if (rc == MC_OK && ce == cudaSuccess && done && !done_direct)
+                ce = cudaMemcpyAsync(done, e->kp.do_reset, B, cudaMemcpyDeviceToDevice, e->cap_stream);
+            if (ce != cudaSuccess) rc = cuda_fail(ce, "rollout copy");
         }
         cudaError_t ce = cudaStreamEndCapture(e->cap_stream, &graph);
         if (rc) {
