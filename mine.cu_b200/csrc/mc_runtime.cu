@@ -710,7 +710,10 @@ static mc_fused_cfg default_launch(const mc_env_config* cfg, const mc_kp* kp, co
     }
     const std::string saved = mc_last_error();  // probing shapes must not replace the caller's message
     if (!big && validate_fused_kp(cfg, kp, be, &f) != MC_OK) team_shape(f);  // e.g. wide float32 images
-    if (validate_fused_kp(cfg, kp, be, &f) != MC_OK) f.warps_per_cta = 4;    // one team per CTA
+    if (validate_fused_kp(cfg, kp, be, &f) != MC_OK) {  // one team per CTA
+        f.warps_per_cta = 4;
+        f.team_warps = std::min(f.team_warps, 4);
+    }
     if (validate_fused_kp(cfg, kp, be, &f) != MC_OK) f.stage = 0;  // e.g. a world too big for a team's copy
     mc_set_error(MC_OK, saved.c_str());
     return f;
