@@ -2639,6 +2639,21 @@ __device__ __forceinline__ void team_sync(int bar, int nthreads) {
 }
 
 
+// The same barrier, with the team's answer to whether any of its threads says v.
+__device__ __forceinline__ bool team_any(int bar, int nthreads, bool v) {
+    if (nthreads == 32) return __any_sync(0xffffffffu, v);
+    int any;
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t"
+        "setp.ne.s32 p, %3, 0;\n\t"
+        "barrier.cta.red.or.pred q, %1, %2, p;\n\t"
+        "selp.s32 %0, 1, 0, q;\n\t}"
+        : "=r"(any)
+        : "r"(bar), "r"(nthreads), "r"((int)v)
+        : "memory");
+    return any;
+}
+
 // Where the staged copy of the world at src lies in its slot: at src's offset
 // from a 16-byte boundary, so that a bulk copy can move its whole chunks.
 __device__ __forceinline__ int8_t* staged_at(int8_t* slot, const int8_t* src) { return slot + ((uintptr_t)src & 15u); }
@@ -3121,9 +3136,6 @@ struct TeamShared {
     unsigned unit[4];      // claimed units, unit k's number at k & 3
     int band_ctr[2];       // next row band of the cooperative env of unit k & 1
     unsigned long long mbar[2];
-    int timed_out[2];      // a wait for the copy of unit k ran out, at k & 1: no further copies, render from
-                           // global memory (read after unit k's barrier: by then only unit k + 1's warps write,
-                           // to the other one, and once it is set nobody stages again)
     unsigned sunit[2];     // general pass: claimed units, alternating slots
     int any_done;          // bit g: every world of group g is to be regenerated
     int last;              // the team rendered its env's last slice
@@ -3240,7 +3252,6 @@ __global__ void __launch_bounds__(256, MC_TEAM_MIN_BLOCKS) k_render_team(const _
     pdl_wait();
     if (claimer) {
         for (int k = 0; k < DEPTH; ++k) ts->unit[k] = claim(MC_FLAG_WORK);
-        ts->timed_out[0] = ts->timed_out[1] = 0;
         int any = 0;
         for (int g = 0; g < G; ++g)
             if (rk.groups[g].regen == MC_KREGEN_ALL && *(volatile int32_t*)&rk.groups[g].flags[MC_FLAG_ANY_DONE])
@@ -3300,17 +3311,14 @@ __global__ void __launch_bounds__(256, MC_TEAM_MIN_BLOCKS) k_render_team(const _
     auto staged_world = [&](const Unit& t, const EnvRec& q, int d) -> const int8_t* {
         return staged_at(slot_world(d, t.coop), world_of(rk.groups[t.g], q.env, q.bits, (ts->any_done >> t.g) & 1));
     };
-    // Wait for the copy of unit t, the team's k-th, into depth slot d.
-    auto landed = [&](const Unit& t, int d, int k) -> bool {
+    // Wait for the copy of unit t into depth slot d; false: no further copies,
+    // render from global memory (team_any tells the team).
+    auto landed = [&](const Unit& t, int d) -> bool {
         const mc_kp& p = rk.groups[t.g];
-        if (!stage_fits(slot_world(d, t.coop), mc_world_slot(p))) {
-            *(volatile int*)&ts->timed_out[k & 1] = 1;
-            return false;
-        }
+        if (!stage_fits(slot_world(d, t.coop), mc_world_slot(p))) return false;
         uint32_t& ph = t.coop ? tphase : wphase;
         if (!mbar_wait((t.coop ? tmbar : cx.mbar_a) + 8 * d, (ph >> d) & 1u, p.wait_polls)) {
             if (lane == 0) atomicExch(&p.flags[MC_FLAG_ERROR], MC_KERR_TMA_TIMEOUT);
-            *(volatile int*)&ts->timed_out[k & 1] = 1;
             return false;
         }
         ph ^= 1u << d;
@@ -3355,6 +3363,7 @@ __global__ void __launch_bounds__(256, MC_TEAM_MIN_BLOCKS) k_render_team(const _
             if (claimer) team_unit_reset(ts, (k + 1) & 1);
             const mc_kp& p = rk.groups[t.g];
             int bits = MC_ER_SLOW, env = 0;
+            bool timed_out = false;
             if (t.mine) {
                 const EnvRec q = load_rec(recs_of(t.g), t.i);
                 bits = q.bits;
@@ -3365,7 +3374,8 @@ __global__ void __launch_bounds__(256, MC_TEAM_MIN_BLOCKS) k_render_team(const _
                         fill_env<FAM, F32>(p, q.env, q.fill_blk, cx, t.coop ? wt * 32 + lane : lane,
                                            t.coop ? nthr : 32);
                 } else if (!(q.bits & MC_ER_SLOW)) {
-                    const bool ok = landed(t, d, k);
+                    const bool ok = landed(t, d);
+                    timed_out = !ok;
                     const int8_t* world = staged_world(t, q, d);
                     EnvRender r = render_of_rec(q, p.wy);
                     if (t.coop && TWN > 1 && up_scan_shape(p.wx, p.wy, p.wz))  // team-uniform; the eye is in the box
@@ -3380,8 +3390,7 @@ __global__ void __launch_bounds__(256, MC_TEAM_MIN_BLOCKS) k_render_team(const _
                 }
             }
             if (claimer) ts->unit[(k + DEPTH) & 3] = claim(MC_FLAG_WORK);
-            team_sync(bar, nthr);
-            if (*(volatile int*)&ts->timed_out[k & 1]) {
+            if (team_any(bar, nthr, timed_out)) {
                 redo = true;
                 break;
             }
@@ -3433,6 +3442,7 @@ __global__ void __launch_bounds__(256, MC_TEAM_MIN_BLOCKS) k_render_team(const _
         if (may_stage && t.part == 0) issue(t, 0, MC_ER_SLOW);
         if (claimer) team_unit_reset(ts, (k + 1) & 1);
         int bits = 0, env = 0;
+        bool timed_out = false;
         bool here = false;  // this unit's env is rendered in this pass (the first slice's unit renders all of it)
         if (t.mine) {
             const EnvRec q = load_rec(recs_of(t.g), t.i);
@@ -3442,7 +3452,8 @@ __global__ void __launch_bounds__(256, MC_TEAM_MIN_BLOCKS) k_render_team(const _
             use_group(t.g);
             if (here) {
                 const int8_t* world = staged_world(t, q, 0);
-                const bool staged = may_stage && landed(t, 0, k);
+                const bool staged = may_stage && landed(t, 0);
+                timed_out = may_stage && !staged;
                 const int ytop = staged ? staged_top_layer(world, p.wx, p.wy, p.wz, lane) : p.wy - 1;
                 render_slow<FAM, F32>(p, q, ytop, cx, staged ? world : nullptr,
                                       world_of(p, q.env, q.bits, (ts->any_done >> t.g) & 1), rk.tile_w[t.g], lane,
@@ -3450,8 +3461,7 @@ __global__ void __launch_bounds__(256, MC_TEAM_MIN_BLOCKS) k_render_team(const _
             }
         }
         if (claimer) ts->sunit[(k + 1) & 1] = claim(MC_FLAG_SLOW_WORK);
-        team_sync(bar, nthr);
-        stage_ok &= !*(volatile int*)&ts->timed_out[k & 1];
+        stage_ok &= !team_any(bar, nthr, timed_out);
         if (here) regen(t, bits, env, false);
     }
     // timed-out copies may still be in flight: let them land (bounded) before
