@@ -1686,13 +1686,13 @@ constexpr int kFastTableBytes = MC_FAST_TABLE_BYTES;
 static_assert(kFastTableBytes == kShadeTableBytes + 64, "fast tables");
 
 __host__ __device__ inline FusedLayout fused_layout(int W, int H, int slot, int wxz, int obs_f32, int stage,
-                                                   int tile_w) {
+                                                   int tile_w, int fast) {
     FusedLayout L;
     L.W = W;
     L.H = H;
     L.tile_w = tile_w;
     L.tile_h = 32 / tile_w;
-    L.stage_bytes = mc_band_bytes(W, H, obs_f32, tile_w, 0);
+    L.stage_bytes = mc_band_bytes(W, obs_f32, tile_w, 0, fast);
     L.world_bytes = stage ? slot : 0;
     L.warp_bytes = 16 + 128 + L.stage_bytes + L.world_bytes;  // 16: mbarrier, 128: packed_start table
     L.head_bytes = kFastTableBytes + mc_align16((W + H) * 4 + 13 * 3 * 4 + 16 + 13 * 3 + 3);
@@ -2966,7 +2966,7 @@ __device__ __noinline__ void warp_rest(const mc_kp& p, int tile_w, int slices, i
     extern __shared__ __align__(16) uint8_t smem[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
     const int wxyz = p.wx * p.wy * p.wz;
-    const FusedLayout L = fused_layout(p.W, p.H, mc_world_slot(p), p.wx * p.wz, F32, STAGE, tile_w);
+    const FusedLayout L = fused_layout(p.W, p.H, mc_world_slot(p), p.wx * p.wz, F32, STAGE, tile_w, p.fast_ok);
     FusedCtx cx;
     int8_t* sworld = warp_ctx(p, L, smem, warp, cx);
     uint32_t phase = state & 1;
@@ -3046,7 +3046,7 @@ __global__ void __launch_bounds__(256, MC_FUSED_MIN_BLOCKS)
     const int nwarps = blockDim.x >> 5;
     const int total_warps = gridDim.x * nwarps;
     {
-        const FusedLayout L = fused_layout(p.W, p.H, mc_world_slot(p), p.wx * p.wz, F32, STAGE, tile_w);
+        const FusedLayout L = fused_layout(p.W, p.H, mc_world_slot(p), p.wx * p.wz, F32, STAGE, tile_w, p.fast_ok);
         build_fast_tables(reinterpret_cast<float4*>(smem), reinterpret_cast<uint32_t*>(smem + kShadeTableBytes));
         float* s_u = reinterpret_cast<float*>(smem + kFastTableBytes);
         build_uv_tables<FAM>(p, s_u, s_u + L.W);
@@ -3061,7 +3061,7 @@ __global__ void __launch_bounds__(256, MC_FUSED_MIN_BLOCKS)
     int u = 0, state = 0;
     if constexpr (STAGE) {
         const int wxyz = p.wx * p.wy * p.wz;
-        const FusedLayout L = fused_layout(p.W, p.H, mc_world_slot(p), p.wx * p.wz, F32, STAGE, tile_w);
+        const FusedLayout L = fused_layout(p.W, p.H, mc_world_slot(p), p.wx * p.wz, F32, STAGE, tile_w, p.fast_ok);
         FusedCtx cx;
         int8_t* sworld = warp_ctx(p, L, smem, warp, cx);
         const EnvRec* recs = reinterpret_cast<const EnvRec*>(p.rec);
@@ -3529,10 +3529,18 @@ static int step_plain(const mc_kp* p, cudaStream_t s) {
     return render_launch(p, p->family, s);
 }
 
-static size_t fused_smem(const mc_kp* p, const mc_fused_cfg* cfg) {
-    FusedLayout L = fused_layout(p->W, p->H, mc_world_slot(*p), p->wx * p->wz, p->obs_f32, cfg->stage, cfg->tile_w);
-    return (size_t)L.head_bytes + (size_t)cfg->warps_per_cta * L.warp_bytes + (size_t)L.pad_bytes;
+static size_t warp_smem(const mc_kp& p, const mc_fused_cfg& cfg, int fast) {
+    FusedLayout L = fused_layout(p.W, p.H, mc_world_slot(p), p.wx * p.wz, p.obs_f32, cfg.stage, cfg.tile_w, fast);
+    return (size_t)L.head_bytes + (size_t)cfg.warps_per_cta * L.warp_bytes + (size_t)L.pad_bytes;
 }
+
+// The per-warp kernel's common path in this shape (mc_fast_launch, 0 where it does not fit).
+static int warp_fast(const mc_kp& p, const mc_fused_cfg& cfg) {
+    const int fast = mc_fast_launch(p, cfg.stage, cfg.tile_w);
+    return warp_smem(p, cfg, fast) > 227 * 1024 ? 0 : fast;
+}
+
+static size_t fused_smem(const mc_kp* p, const mc_fused_cfg* cfg) { return warp_smem(*p, *cfg, warp_fast(*p, *cfg)); }
 
 // A launch whose kernel waits for its predecessor itself (pdl_wait), so that
 // its own set-up overlaps the predecessor's end.
@@ -3577,7 +3585,7 @@ static int slices_of(long long B, int bands, long long warps) {
 template <int FAM, bool F32, bool STAGE>
 static int launch_warp_t(const mc_kp* p, const mc_fused_cfg* cfg, int slices, long long grid, cudaStream_t s) {
     auto kern = k_render_warp<FAM, F32, STAGE>;
-    const size_t smem = fused_smem(p, cfg);
+    const size_t smem = warp_smem(*p, *cfg, p->fast_ok);
     static mc_once_per_device limit;  // per instantiation
     const int rc = allow_smem(limit, kern, smem);
     if (rc) return rc;
@@ -3594,7 +3602,7 @@ static int launch_fused_f(const mc_kp* kp, const mc_fused_cfg* cfg, int num_sms,
         f.stage = 1;
         if (fused_smem(&p, &f) > 227 * 1024) f.stage = 0;
     }
-    p.fast_ok = mc_fast_launch(p, cfg->stage, cfg->tile_w);
+    p.fast_ok = warp_fast(p, f);
     const int wpc = cfg->warps_per_cta;
     long long grid = (long long)num_sms * (cfg->ctas_per_sm > 0 ? cfg->ctas_per_sm : 1);
     const int slices = p.fast_ok && p.sched_dynamic ? slices_of(p.B, (p.H * cfg->tile_w + 31) / 32, grid * wpc) : 1;

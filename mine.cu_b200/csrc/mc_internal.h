@@ -215,16 +215,18 @@ __host__ __device__
 static inline int mc_world_slot(const mc_kp& k) {
     return ((k.wx * k.wy * k.wz + 15) & ~15) + (mc_odd_world(k) ? 16 : 0);
 }
-// Shared-memory bytes of the pixels a warp stages: one band, with 16 to spare
-// where bands start at any byte; the team
-// kernel's float32 pixels two tiles (fast_band).
+// Shared-memory bytes of the pixels a warp stages on the images' common path
+// (fast: mc_fast_launch): one band, with 16 to spare where bands start at any
+// byte; the team kernel's float32 pixels two tiles (fast_band).  A launch that
+// does not fit with these goes without the common path (fast 0), so that no
+// image is too wide for a launch because of them.
 #ifdef __CUDACC__
 __host__ __device__
 #endif
-static inline int mc_band_bytes(int W, int H, int obs_f32, int tile_w, int team) {
-    if (obs_f32 && team) return 64 * 12;
-    const int n = W * (32 / tile_w) * (obs_f32 ? 12 : 3);
-    return ((n + 15) & ~15) + (mc_whole_tiles(W, H, obs_f32, tile_w) ? 0 : 16);
+static inline int mc_band_bytes(int W, int obs_f32, int tile_w, int team, int fast) {
+    const int n = (W * (32 / tile_w) * (obs_f32 ? 12 : 3) + 15) & ~15;
+    if (obs_f32 && team) return fast == 1 || n > 64 * 12 ? 64 * 12 : n;
+    return n + (fast == 2 ? 16 : 0);
 }
 
 // Whether a launch that stages its worlds (stage) has the images' common path

@@ -460,8 +460,9 @@ constexpr long long kSmemPerCta = 227 * 1024;  // an SM's 228 KB hold each CTA's
 
 static inline int align16i(long long x) { return (int)((x + 15) & ~15LL); }
 
-static void team_layout_of(const mc_kp* const* kps, int G, const int* stage, const int* tile_w, const int* coop,
-                           int team_warps, int warps_per_cta, mc_ragged_kp* rk) {
+// common: whether the images may take their common path (mc_fast_launch).
+static void team_layout_as(const mc_kp* const* kps, int G, const int* stage, const int* tile_w, const int* coop,
+                           int team_warps, int warps_per_cta, bool common, mc_ragged_kp* rk) {
     *rk = mc_ragged_kp{};
     rk->ngroups = G;
     rk->team_warps = team_warps;
@@ -471,7 +472,8 @@ static void team_layout_of(const mc_kp* const* kps, int G, const int* stage, con
     for (int g = 0; g < G; ++g) {
         const mc_kp& k = *kps[g];
         rk->groups[g] = k;
-        rk->groups[g].fast_ok = mc_fast_launch(k, stage[g], tile_w[g]);
+        const int fast = common ? mc_fast_launch(k, stage[g], tile_w[g]) : 0;
+        rk->groups[g].fast_ok = fast;
         rk->groups[g].regen = step_regen(k);
         rk->slices[g] = 1;
         rk->start[g] = start;
@@ -479,7 +481,7 @@ static void team_layout_of(const mc_kp* const* kps, int G, const int* stage, con
         rk->uv_off[g] = uv;
         uv += k.W + k.H;
         rk->tile_w[g] = tile_w[g];
-        band = std::max(band, mc_band_bytes(k.W, k.H, k.obs_f32, tile_w[g], 1));
+        band = std::max(band, mc_band_bytes(k.W, k.obs_f32, tile_w[g], 1, fast));
         if (coop[g]) rk->coop_mask |= 1 << g;
         if (stage[g]) {
             rk->stage_mask |= 1 << g;
@@ -547,6 +549,13 @@ static void team_layout_of(const mc_kp* const* kps, int G, const int* stage, con
     rk->warp_bytes = 16 + 128 + band;
     const int after = warps_per_cta * rk->warp_bytes;
     rk->tail_bytes = after < pad ? pad - after : 0;
+}
+
+static void team_layout_of(const mc_kp* const* kps, int G, const int* stage, const int* tile_w, const int* coop,
+                           int team_warps, int warps_per_cta, mc_ragged_kp* rk) {
+    team_layout_as(kps, G, stage, tile_w, coop, team_warps, warps_per_cta, true, rk);
+    if (team_smem(*rk, warps_per_cta) > kSmemPerCta)
+        team_layout_as(kps, G, stage, tile_w, coop, team_warps, warps_per_cta, false, rk);
 }
 
 // Stages the groups whose worlds no launch shape can stage (mc_odd_world) too,

@@ -24,3 +24,18 @@ def test_wide_images_of_few_envs_have_a_shape(mode, world):
                 rc, f, smem = default_shape(B, W, H, world, mode)
                 assert rc == capi.MC_OK, (B, W, H, capi.last_error())
                 assert smem <= 227 * 1024 and f.warps_per_cta % f.team_warps == 0
+
+
+@pytest.mark.parametrize("world", [(16, 16, 16), (32, 32, 32), (9, 13, 11)], ids=lambda w: "x".join(map(str, w)))
+@pytest.mark.parametrize("mode", ["uint8", "uint8_minimal"])
+def test_the_widest_images_of_a_plain_band_have_a_shape(mode, world):
+    """The bytes to spare of images that start at any byte take no width away."""
+    for W in range(4400, 4432):
+        for H in (1, 3):
+            head = 224 + 13 * 4 * 16 + 64 + (W + H) * 4 + 15 & ~15
+            band = W * 4 * 3 + 15 & ~15  # 8-wide tiles: four rows
+            if head + 256 + 4 * (16 + 128 + band) > 227 * 1024:
+                continue  # one unstaged team of 4 warps does not fit
+            for B in (1, 64, 4096):
+                rc, f, smem = default_shape(B, W, H, world, mode)
+                assert rc == capi.MC_OK and smem <= 227 * 1024, (B, W, H, capi.last_error())
