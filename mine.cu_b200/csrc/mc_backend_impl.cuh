@@ -2465,6 +2465,40 @@ __device__ __forceinline__ const int8_t* world_of(const mc_kp& p, int e, int bit
                                                    : p.voxels + e * (long long)p.wx * p.wy * p.wz;
 }
 
+// The record of env e, its agent at x, y, z, from its state alone (no step's):
+// reset and get_obs, and the images of a launch that has no records (p.rec NULL:
+// the stateless step).
+template <int FAM>
+__device__ __forceinline__ EnvRec look_rec(const mc_kp& p, long long e, float x, float y, float z, float yaw, float pitch,
+                                           bool done, int any_done) {
+    EnvRec r;
+    r.env = (int)e;
+    r.ex = x;
+    r.ey = N::add(y, 1.6f);
+    r.ez = z;
+    rec_trig<FAM>(r, yaw, pitch);
+    const long long wxyz = (long long)p.wx * p.wy * p.wz;
+    const int eye = eye_index(r, p);
+    int eye_blk = AIR;
+    if (eye >= 0 && in_bounds(eye, wxyz, MC_SITE_EYE)) eye_blk = world_of(p, (int)e, done ? MC_ER_DONE : 0, any_done)[eye];
+    rec_facts<FAM>(r, p, eye >= 0, eye_blk, done);
+    return r;
+}
+template <int FAM>
+__device__ __noinline__ void look_rec_out(const mc_kp& p, int i, EnvRec& r) {
+    const long long e = i;
+    r = look_rec<FAM>(p, e, p.positions[e * 3 + 0], p.positions[e * 3 + 1], p.positions[e * 3 + 2], p.yaws[e],
+                      p.pitches[e], false, 0);
+}
+// The record of the launch's i-th unit.
+template <int FAM>
+__device__ __forceinline__ EnvRec rec_of(const mc_kp& p, int i) {
+    if (p.rec) return load_rec(p.rec, i);
+    EnvRec r;
+    look_rec_out<FAM>(p, i, r);
+    return r;
+}
+
 constexpr int kAgentThreads = MC_AGENT_THREADS;
 
 // File the block's records (called by all its threads): record e at e, or,
@@ -2484,7 +2518,7 @@ __device__ __forceinline__ void file_recs(void* rec, int32_t* flags, int32_t* an
     const unsigned done = __ballot_sync(0xffffffffu, step && valid && (r.bits & MC_ER_DONE));
     if (done && lane == 0) atomicOr(&flags[MC_FLAG_ANY_DONE], 1);
     if (!compact) {
-        if (valid) store_rec(rec, e, r);
+        if (valid && rec) store_rec(rec, e, r);
         return;
     }
     const unsigned mm = __ballot_sync(0xffffffffu, march), mb = __ballot_sync(0xffffffffu, fill);
@@ -2554,16 +2588,7 @@ __global__ void __launch_bounds__(kAgentThreads) k_look(const __grid_constant__ 
         p.cameras[e * 5 + 2] = z;
         p.cameras[e * 5 + 3] = yaw;
         p.cameras[e * 5 + 4] = pitch;
-        r.env = (int)e;
-        r.ex = x;
-        r.ey = N::add(y, 1.6f);
-        r.ez = z;
-        rec_trig<MC_FAM_SHADED>(r, yaw, pitch);
-        const long long wxyz = (long long)p.wx * p.wy * p.wz;
-        const int eye = eye_index(r, p);
-        int eye_blk = AIR;
-        if (eye >= 0 && in_bounds(eye, wxyz, MC_SITE_EYE)) eye_blk = world_of(p, (int)e, done ? MC_ER_DONE : 0, any_done)[eye];
-        rec_facts<MC_FAM_SHADED>(r, p, eye >= 0, eye_blk, done);
+        r = look_rec<MC_FAM_SHADED>(p, e, x, y, z, yaw, pitch, done, any_done);
     }
     file_recs(p.rec, p.flags, &p.flags[MC_FLAG_ANY_SLOW], p.B, p.compact, r, e, valid, false);
     if (threadIdx.x == 0) bounds_to_flags(p.flags);
@@ -2981,7 +3006,7 @@ __device__ __noinline__ void warp_rest(const mc_kp& p, int tile_w, int slices, i
         // pixels come out the same)
         for (; no_stage && u < units; u = next_unit(p, MC_FLAG_WORK, u, total_warps, lane)) {
             const int i = u / slices, part = u - i * slices;
-            const EnvRec q = load_rec(recs, i);
+            const EnvRec q = rec_of<FAM>(p, i);
             if (q.bits & MC_ER_SLOW) continue;
             if (!(q.bits & MC_ER_BURIED))
                 render_slow<FAM, F32>(p, q, p.wy - 1, cx, nullptr, world_of(p, q.env, q.bits, any_done), tile_w, lane,
@@ -2998,7 +3023,7 @@ __device__ __noinline__ void warp_rest(const mc_kp& p, int tile_w, int slices, i
     if (all || !p.sched_dynamic || any_slow) {
         u = p.sched_dynamic ? next_unit(p, MC_FLAG_SLOW_WORK, 0, total_warps, lane) : first;
         for (; u < p.B; u = next_unit(p, MC_FLAG_SLOW_WORK, u, total_warps, lane)) {
-            const EnvRec q = load_rec(recs, u);
+            const EnvRec q = rec_of<FAM>(p, u);
             if (!all && !(q.bits & MC_ER_SLOW)) continue;
             if (q.bits & MC_ER_BURIED) {
                 fill_env<FAM, F32>(p, q.env, q.fill_blk, cx, lane, 32);
@@ -3071,7 +3096,7 @@ __global__ void __launch_bounds__(256, MC_FUSED_MIN_BLOCKS)
         u = p.sched_dynamic ? next_unit(p, MC_FLAG_WORK, 0, total_warps, lane) : blockIdx.x * nwarps + warp;
         for (; u < units; u = next_unit(p, MC_FLAG_WORK, u, total_warps, lane)) {
             const int i = u / slices, part = u - i * slices;
-            const EnvRec q = load_rec(recs, i);
+            const EnvRec q = rec_of<FAM>(p, i);
             if (q.bits & MC_ER_SLOW) continue;
             if (q.bits & MC_ER_BURIED) {
                 if (part == 0) fill_env<FAM, F32>(p, q.env, q.fill_blk, cx, lane, 32);

@@ -1888,11 +1888,9 @@ extern "C" int mc_step_stateless(const mc_env_config* cfg, const mc_env_state* s
         f.tile_w = 4;
         f.team_warps = 1;
         f.coop = 0;
-        // the render records live for this call only (stream-ordered, so calls on other streams have their own)
-        MC_CK(cudaMallocAsync(&k.rec, (size_t)k.B * MC_REC_BYTES, (cudaStream_t)stream));
-        rc = backend_rc(be->step_fused(&k, &f, sms, (cudaStream_t)stream), "step_fused");
-        MC_CK(cudaFreeAsync(k.rec, (cudaStream_t)stream));
-        return rc;
+        // no render records (k.rec NULL): the images read the state the agents left,
+        // so the call allocates nothing and calls on other streams share nothing
+        return backend_rc(be->step_fused(&k, &f, sms, (cudaStream_t)stream), "step_fused");
     }
     return fail(MC_ERR_INVALID, "unknown form %d", form);
 }

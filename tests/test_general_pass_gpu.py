@@ -95,3 +95,43 @@ def test_worlds_regenerated_by_the_general_pass(cuda, regen, cfg):
         assert not d, f"step {s}: {d}"
     g.check_error()
     g.close()
+
+
+def test_the_stateless_fused_step_allocates_nothing(cuda):
+    """Under capture it leaves kernels only, and its graph can be instantiated
+    more than once at a time, as one with allocations cannot."""
+    import torch
+    from cuda.bindings import runtime as rt
+
+    def ok(r):
+        assert r[0] == rt.cudaError_t.cudaSuccess, r[0]
+        return r[1] if len(r) == 2 else r[1:]
+
+    n = 300
+    envs = [GpuEnv(cuda, n, obs_dtype="uint8", numerics="ieee", debug=False) for _ in range(2)]
+    want, g = envs
+    for e in envs:
+        e.reset()
+        e.t["do_reset"].zero_()
+    _, btn, look = actions_for(n, 0, 83, 0.1, True)
+    _stateless(g, btn, look, capi.FORM_FUSED)  # first use
+    _stateless(want, btn, look, capi.FORM_FUSED)
+    s = torch.cuda.Stream(device=cuda)
+    torch.cuda.synchronize()
+    ok(rt.cudaStreamBeginCapture(s.cuda_stream, rt.cudaStreamCaptureMode.cudaStreamCaptureModeThreadLocal) + (None,))
+    rc = g.L.mc_step_stateless(ctypes.byref(g.cfg), ctypes.byref(g.st), g.buttons.data_ptr(), g.look.data_ptr(), None,
+                               capi.FORM_FUSED, s.cuda_stream)
+    graph = ok(rt.cudaStreamEndCapture(s.cuda_stream))
+    capi.check(rc, "captured step")
+    execs = [ok(rt.cudaGraphInstantiate(graph, 0)) for _ in range(2)]
+    for x in execs:
+        ok(rt.cudaGraphLaunch(x, s.cuda_stream) + (None,))
+        _stateless(want, btn, look, capi.FORM_FUSED)
+    torch.cuda.synchronize()
+    d = diff_report(g.state(), want.state())
+    assert not d, d
+    for x in execs:
+        ok(rt.cudaGraphExecDestroy(x) + (None,))
+    ok(rt.cudaGraphDestroy(graph) + (None,))
+    for e in envs:
+        e.close()
