@@ -2985,7 +2985,8 @@ __device__ __forceinline__ int8_t* warp_ctx(const mc_kp& p, const FusedLayout& L
 // What a warp does besides the common path, out of line after its loop (so
 // that the loop keeps its registers): from unit u on, the units of a warp
 // whose copy timed out (no_stage), then its share of the general pass.
-// state: bit 0 the mbarrier's phase, bit 1 no_stage, bit 2 that copy may still land.
+// state: bit 0 the mbarrier's phase, bit 1 no_stage, bit 2 that copy may still
+// land, bit 3 a unit was left to the general pass.
 template <int FAM, bool F32, bool STAGE>
 __device__ __noinline__ void warp_rest(const mc_kp& p, int tile_w, int slices, int u, int state) {
     extern __shared__ __align__(16) uint8_t smem[];
@@ -2995,7 +2996,7 @@ __device__ __noinline__ void warp_rest(const mc_kp& p, int tile_w, int slices, i
     FusedCtx cx;
     int8_t* sworld = warp_ctx(p, L, smem, warp, cx);
     uint32_t phase = state & 1;
-    bool no_stage = state & 2, pending = state & 4;
+    bool no_stage = state & 2, pending = state & 4, slow = state & 8;
     const int total_warps = gridDim.x * nwarps, first = blockIdx.x * nwarps + warp;
     const EnvRec* recs = reinterpret_cast<const EnvRec*>(p.rec);
     const int any_done = regen_any(p);
@@ -3007,7 +3008,10 @@ __device__ __noinline__ void warp_rest(const mc_kp& p, int tile_w, int slices, i
         for (; no_stage && u < units; u = next_unit(p, MC_FLAG_WORK, u, total_warps, lane)) {
             const int i = u / slices, part = u - i * slices;
             const EnvRec q = rec_of<FAM>(p, i);
-            if (q.bits & MC_ER_SLOW) continue;
+            if (q.bits & MC_ER_SLOW) {
+                slow = true;
+                continue;
+            }
             if (!(q.bits & MC_ER_BURIED))
                 render_slow<FAM, F32>(p, q, p.wy - 1, cx, nullptr, world_of(p, q.env, q.bits, any_done), tile_w, lane,
                                       nullptr);
@@ -3020,10 +3024,13 @@ __device__ __noinline__ void warp_rest(const mc_kp& p, int tile_w, int slices, i
     // launch that has no common path)
     constexpr bool all = !STAGE;
     const int any_slow = __shfl_sync(0xffffffffu, *(volatile int32_t*)&p.flags[MC_FLAG_ANY_SLOW], 0);
-    if (all || !p.sched_dynamic || any_slow) {
+    if (all || (p.sched_dynamic ? any_slow != 0 : slow)) {
+        // (claimed: the envs; in turn: this warp's units again, whose first slices draw the whole image)
+        const int per = p.sched_dynamic ? 1 : slices, units = p.B * per;
         u = p.sched_dynamic ? next_unit(p, MC_FLAG_SLOW_WORK, 0, total_warps, lane) : first;
-        for (; u < p.B; u = next_unit(p, MC_FLAG_SLOW_WORK, u, total_warps, lane)) {
-            const EnvRec q = rec_of<FAM>(p, u);
+        for (; u < units; u = next_unit(p, MC_FLAG_SLOW_WORK, u, total_warps, lane)) {
+            if (u % per) continue;
+            const EnvRec q = rec_of<FAM>(p, u / per);
             if (!all && !(q.bits & MC_ER_SLOW)) continue;
             if (q.bits & MC_ER_BURIED) {
                 fill_env<FAM, F32>(p, q.env, q.fill_blk, cx, lane, 32);
@@ -3097,7 +3104,10 @@ __global__ void __launch_bounds__(256, MC_FUSED_MIN_BLOCKS)
         for (; u < units; u = next_unit(p, MC_FLAG_WORK, u, total_warps, lane)) {
             const int i = u / slices, part = u - i * slices;
             const EnvRec q = rec_of<FAM>(p, i);
-            if (q.bits & MC_ER_SLOW) continue;
+            if (q.bits & MC_ER_SLOW) {
+                phase |= 2u;
+                continue;
+            }
             if (q.bits & MC_ER_BURIED) {
                 if (part == 0) fill_env<FAM, F32>(p, q.env, q.fill_blk, cx, lane, 32);
             } else {
@@ -3109,7 +3119,7 @@ __global__ void __launch_bounds__(256, MC_FUSED_MIN_BLOCKS)
                 issue_world_copy(cx.mbar_a, sworld, src, wxyz, lane);
                 const int8_t* world = staged_at(sworld, src);
                 EnvRender r = render_of_rec(q, p.wy);
-                if (!mbar_wait(cx.mbar_a, phase, p.wait_polls)) {
+                if (!mbar_wait(cx.mbar_a, phase & 1u, p.wait_polls)) {
                     if (lane == 0) atomicExch(&p.flags[MC_FLAG_ERROR], MC_KERR_TMA_TIMEOUT);
                     state = 2 | 4;
                     break;
@@ -3120,11 +3130,11 @@ __global__ void __launch_bounds__(256, MC_FUSED_MIN_BLOCKS)
             }
             if (regen_env(p, q.bits, any_done) && last_slice(recs, i, slices, lane)) regen_world(p, q.env, lane, 32);
         }
-        state |= phase;
+        state |= (phase & 1u) | (phase & 2u) << 2;
     }
     // (a launch whose worlds are not staged has no common path)
     const int any_slow = __shfl_sync(0xffffffffu, *(volatile int32_t*)&p.flags[MC_FLAG_ANY_SLOW], 0);
-    if (!STAGE || !p.sched_dynamic || any_slow || (state & 2)) warp_rest<FAM, F32, STAGE>(p, tile_w, slices, u, state);
+    if (!STAGE || (p.sched_dynamic ? any_slow != 0 : (state & 8) != 0) || (state & 2)) warp_rest<FAM, F32, STAGE>(p, tile_w, slices, u, state);
     // No CTA barrier here: warps leave as soon as their last env is done.
     if (lane == 0) {
         bounds_to_flags(p.flags);
@@ -3630,9 +3640,13 @@ static int launch_fused_f(const mc_kp* kp, const mc_fused_cfg* cfg, int num_sms,
     p.fast_ok = warp_fast(p, f);
     const int wpc = cfg->warps_per_cta;
     long long grid = (long long)num_sms * (cfg->ctas_per_sm > 0 ? cfg->ctas_per_sm : 1);
-    const int slices = p.fast_ok && p.sched_dynamic ? slices_of(p.B, (p.H * cfg->tile_w + 31) / 32, grid * wpc) : 1;
+    const int slices = p.fast_ok ? slices_of(p.B, (p.H * cfg->tile_w + 31) / 32, grid * wpc) : 1;
     const long long units = (long long)p.B * slices;
     p.compact = p.sched_dynamic && units > grid * wpc;
+    // static striding: four waves of CTAs, so that warps whose envs are cheap make
+    // room (the stateless step, us: 32768 envs 16^3, 32x32 203 in one wave, 194 in
+    // two, 190 in four, 204 in six; 4096 envs 45 in each)
+    if (!p.sched_dynamic) grid *= 4;
     grid = std::max(1LL, std::min(grid, (units + wpc - 1) / wpc));
     int rc;
     if (FAM == MC_FAM_SHADED && p.look_only)

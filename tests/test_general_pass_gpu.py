@@ -42,21 +42,23 @@ def _stateless(g, btn, look, form, dec=None):
 @pytest.mark.parametrize("mode", ["uint8", "float32", "uint8_minimal", "uint8_prebasis", "uint8_prebasis_full",
                                   "uint8_fp16", "uint8_fast"])
 @pytest.mark.parametrize("kw", [ABOVE, dict()], ids=["above", "inside"])
-def test_stateless_fused_step_equals_the_plain_one(cuda, mode, kw):
+@pytest.mark.parametrize("n, res", [(B, 8), (300, 32), (5, 33)])  # several envs a warp; images in slices
+def test_stateless_fused_step_equals_the_plain_one(cuda, mode, kw, n, res):
     import torch
-    envs = [GpuEnv(cuda, B, render_width=8, render_height=8, obs_dtype=mode, numerics="ieee", debug=False,
+    envs = [GpuEnv(cuda, n, render_width=res, render_height=res, obs_dtype=mode, numerics="ieee", debug=False,
                    episode_length=5, **kw) for _ in range(2)]
     plain, fused = envs
-    dec, keep = _decode(B, cuda)
+    dec, keep = _decode(n, cuda)
     rng = np.random.default_rng(81)
     for g in envs:
         g.reset()
         g.t["pitches"].fill_(-1.4)  # down, into the world
+        g.t["positions"][::3, 1] -= 4.0  # some lower than the others
         torch.cuda.synchronize()
     for s in range(6):
-        _, btn, look = actions_for(B, s, 81, 0.1, True)
-        btn[:, 6] = rng.random(B) < 0.1
-        done = rng.random(B) < 0.1
+        _, btn, look = actions_for(n, s, 81, 0.1, True)
+        btn[:, 6] = rng.random(n) < 0.1
+        done = rng.random(n) < 0.1
         for g in envs:
             if mode != "uint8_prebasis_full":
                 g.t["do_reset"].copy_(torch.from_numpy(done))
