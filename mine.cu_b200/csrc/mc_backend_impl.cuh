@@ -3396,6 +3396,11 @@ __global__ void __launch_bounds__(256, MC_TEAM_MIN_BLOCKS) k_render_team(const _
         regen_world(p, e, wt * 32 + lane, nthr);
     };
 
+    // The end of the team's unit k: the next claim, the unit's barrier, and whether a warp's wait ran out.
+    auto end_unit = [&](int k, bool timed_out) -> bool {
+        if (claimer) ts->unit[(k + DEPTH) & 3] = claim(MC_FLAG_WORK);
+        return team_any(bar, nthr, timed_out);
+    };
     bool redo = false;  // the same for the whole team
     {
         int k = 0;
@@ -3414,7 +3419,6 @@ __global__ void __launch_bounds__(256, MC_TEAM_MIN_BLOCKS) k_render_team(const _
             if (claimer) team_unit_reset(ts, (k + 1) & 1);
             const mc_kp& p = rk.groups[t.g];
             int bits = MC_ER_SLOW, env = 0;
-            bool timed_out = false;
             if (t.mine) {
                 const EnvRec q = load_rec(recs_of(t.g), t.i);
                 bits = q.bits;
@@ -3426,7 +3430,6 @@ __global__ void __launch_bounds__(256, MC_TEAM_MIN_BLOCKS) k_render_team(const _
                                            t.coop ? nthr : 32);
                 } else if (!(q.bits & MC_ER_SLOW)) {
                     const bool ok = landed(t, d);
-                    timed_out = !ok;
                     const int8_t* world = staged_world(t, q, d);
                     EnvRender r = render_of_rec(q, p.wy);
                     if (t.coop && TWN > 1 && up_scan_shape(p.wx, p.wy, p.wz))  // team-uniform; the eye is in the box
@@ -3435,16 +3438,16 @@ __global__ void __launch_bounds__(256, MC_TEAM_MIN_BLOCKS) k_render_team(const _
                                               bar);
                     else if (ok)
                         measure_staged(r, world, p.wx, p.wy, p.wz, lane);
-                    if (ok)
-                        render_fast<FAM, F32, true>(p, q.env, r, cx, world, rk.tile_w[t.g], lane,
+                    if (!ok) {
+                        redo = end_unit(k, true);
+                        break;
+                    }
+                    render_fast<FAM, F32, true>(p, q.env, r, cx, world, rk.tile_w[t.g], lane,
                                               t.coop ? &ts->band_ctr[k & 1] : nullptr, t.part, rk.slices[t.g]);
                 }
             }
-            if (claimer) ts->unit[(k + DEPTH) & 3] = claim(MC_FLAG_WORK);
-            if (team_any(bar, nthr, timed_out)) {
-                redo = true;
-                break;
-            }
+            redo = end_unit(k, false);
+            if (redo) break;
             if (!(bits & MC_ER_SLOW)) regen(t, bits, env, true);
         }
         // a copy timed out: this unit again and the rest of the team's, from global memory
