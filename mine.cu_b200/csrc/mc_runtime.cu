@@ -657,6 +657,12 @@ static int validate_fused(const mc_env* e, const mc_fused_cfg* f) {
 // 64 envs 19.3 / 15.4 (16-wide), 256 envs 20.4 / 17.1 (teams of 8, 16-wide), 1024 envs
 // 26.0 / 24.5 (teams of 4); 32^3 64x64, teams of 4 with 8-wide tiles / of 8 with
 // 16-wide: 64 envs 29.6 / 23.0, 1024 envs 75.1 / 69.8, but 4096 envs 196 / 231.
+// Enough envs to go round need no bigger teams, however few tiles each has, and
+// an image of two tiles has no work for one.  us a step: 16^3 8x8, one warp per
+// env / a team: 4096 envs 22.8 / 40.9, 8192 envs 30.1 / 70.7; 16x16, 2048 envs
+// 23.7 / 21.3, 4096 envs 31.3 / 30.8, 8192 envs 34.6 / 48.6.  32^3, teams of 4 / of 8:
+// 8x8 256 envs 18.8 / 17.0, 1024 envs 25.1 / 28.4, 8192 envs 88 / 136; 32x32 256 envs
+// 25.3 / 24.0, 1024 envs 38.0 / 39.0, 4096 envs 89.7 / 112.
 // float32 images wider than 32 go to teams: a warp's band would take 6 KB.
 // `alone` false: a job of the server, whose launches hold many.  A shape whose shared memory does not fit falls
 // back to the team shape (whose per-warp image band is half as tall), then
@@ -671,7 +677,8 @@ static mc_fused_cfg default_launch(const mc_env_config* cfg, const mc_kp* kp, co
     const long long tiles = alone ? ((long long)cfg->batch_size * W * H + 31) / 32 : 1LL << 40;
     const bool wide_f32 = cfg->obs_mode == MC_OBS_FLOAT32 && W > 32;
     bool big = ((W * H >= 64 * 64 || wide_f32) && few_envs) || wxyz > 8192;
-    if (tiles > 4096 && tiles <= 65536) big = true;
+    const long long B = cfg->batch_size;
+    if (tiles > 4096 && tiles <= 65536 && B <= 2048 && W * H >= 128) big = true;
     // the widest tile up to `most` that divides the width (at least 8 of it in use otherwise)
     auto tile = [&](int most) {
         int t = most;
@@ -686,7 +693,7 @@ static mc_fused_cfg default_launch(const mc_env_config* cfg, const mc_kp* kp, co
         f.team_warps = 4;
         f.coop = 1;
         const bool fast = mc_fast_launch(*kp, 1, f.tile_w);  // else images are not cut into slices
-        if (fast && tiles <= (wxyz > 8192 ? 131072 : 16384)) {
+        if (fast && tiles <= (wxyz > 8192 ? 131072 : 16384) && (B <= 512 || (B <= 1024 && W * H >= 64 * 64))) {
             f.tile_w = tile(tiles <= 4096 ? 32 : 16);
             f.team_warps = 8;
         }
@@ -713,7 +720,7 @@ static mc_fused_cfg default_launch(const mc_env_config* cfg, const mc_kp* kp, co
         f.warps_per_cta = 8;
         f.stage = (wxyz <= 8192 && aligned) ? 1 : 0;
         f.ctas_per_sm = 4;
-        f.tile_w = tiles <= 4096 && mc_fast_launch(*kp, 1, 8) ? tile(tiles <= 1024 ? 32 : 16) : 4;
+        f.tile_w = tiles <= 4096 && W * H >= 256 && mc_fast_launch(*kp, 1, 8) ? tile(tiles <= 1024 ? 32 : 16) : 4;
         f.team_warps = 1;
         f.coop = 0;
     }
