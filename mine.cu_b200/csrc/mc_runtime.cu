@@ -662,7 +662,8 @@ static int validate_fused(const mc_env* e, const mc_fused_cfg* f) {
 // env / a team: 4096 envs 22.8 / 40.9, 8192 envs 30.1 / 70.7; 16x16, 2048 envs
 // 23.7 / 21.3, 4096 envs 31.3 / 30.8, 8192 envs 34.6 / 48.6.  32^3, teams of 4 / of 8:
 // 8x8 256 envs 18.8 / 17.0, 1024 envs 25.1 / 28.4, 8192 envs 88 / 136; 32x32 256 envs
-// 25.3 / 24.0, 1024 envs 38.0 / 39.0, 4096 envs 89.7 / 112.
+// 25.3 / 24.0, 1024 envs 38.0 / 39.0, 4096 envs 89.7 / 112.  Worlds above 32 KB have
+// few teams anyway: 1024 envs 48^3 32x32 96.1 / 71.1, 64^3 (from global memory) 247 / 209.
 // float32 images wider than 32 go to teams: a warp's band would take 6 KB.
 // `alone` false: a job of the server, whose launches hold many.  A shape whose shared memory does not fit falls
 // back to the team shape (whose per-warp image band is half as tall), then
@@ -693,7 +694,8 @@ static mc_fused_cfg default_launch(const mc_env_config* cfg, const mc_kp* kp, co
         f.team_warps = 4;
         f.coop = 1;
         const bool fast = mc_fast_launch(*kp, 1, f.tile_w);  // else images are not cut into slices
-        if (fast && tiles <= (wxyz > 8192 ? 131072 : 16384) && (B <= 512 || (B <= 1024 && W * H >= 64 * 64))) {
+        const bool few = B <= 512 || (B <= 1024 && W * H >= 64 * 64) || (wxyz > 32768 && W * H >= 1024);
+        if (fast && few && tiles <= (wxyz > 8192 ? 131072 : 16384)) {
             f.tile_w = tile(tiles <= 4096 ? 32 : 16);
             f.team_warps = 8;
         }

@@ -38,3 +38,11 @@ def test_teams_over_big_worlds(B, image, team):
 @pytest.mark.parametrize("B", [1, 64, 256, 1024, 2048])
 def test_images_of_two_tiles_have_no_team(B):
     assert shape(B, 8, 16).coop == 0
+
+
+@pytest.mark.parametrize("B, image, world, tile", [(1024, 32, 48, 16), (4096, 32, 48, 16), (1024, 32, 64, 16),
+                                                   (1024, 8, 64, 8)])
+def test_worlds_above_32_kb_take_wide_tiles_by_the_tiles(B, image, world, tile):
+    f = shape(B, image, world)
+    assert f.coop == 1 and f.tile_w == tile
+    assert world != 64 or f.team_warps == (8 if tile == 16 else 4)
