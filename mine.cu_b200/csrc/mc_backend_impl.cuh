@@ -3174,6 +3174,9 @@ __global__ void __launch_bounds__(256, MC_FUSED_MIN_BLOCKS)
 // Units are ordered by decreasing per-env cost across groups, so the most
 // expensive envs are claimed first and do not straggle at the end.
 //
+// DEPTH 0: a launch without the images' common path (no group has it): the
+// general pass alone, buried envs too.  (Passing every unit over in the common
+// path's loop first cost 8192 envs 48^3 8x8 627 us a step instead of 375.)
 // DEPTH 1: one world buffer per team (or warp); the unit's copy starts when
 // its record is read.  DEPTH 2: two buffers; unit k+1's record is read and its
 // copy started before unit k is rendered, so it overlaps that render (one
@@ -3260,6 +3263,8 @@ __device__ __forceinline__ UpBounds team_up_bounds(bool have, const int8_t* worl
 #endif
 template <int FAM, bool F32, int DEPTH>
 __global__ void __launch_bounds__(256, MC_TEAM_MIN_BLOCKS) k_render_team(const __grid_constant__ mc_ragged_kp rk) {
+    constexpr bool COMMON = DEPTH > 0;
+    constexpr int SLOTS = DEPTH > 1 ? DEPTH : 1;
     extern __shared__ __align__(16) uint8_t smem[];
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
@@ -3288,7 +3293,7 @@ __global__ void __launch_bounds__(256, MC_TEAM_MIN_BLOCKS) k_render_team(const _
     cx.stage = wbase + 16 + 128;
     const bool claimer = (wt == 0 && lane == 0);
     if (lane == 0) {
-        for (int d = 0; d < DEPTH; ++d) {
+        for (int d = 0; d < SLOTS; ++d) {
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(cx.mbar_a + 8 * d) : "memory");
             if (wt == 0) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(tmbar + 8 * d) : "memory");
         }
@@ -3402,7 +3407,7 @@ __global__ void __launch_bounds__(256, MC_TEAM_MIN_BLOCKS) k_render_team(const _
         return team_any(bar, nthr, timed_out);
     };
     bool redo = false;  // the same for the whole team
-    {
+    if constexpr (COMMON) {
         int k = 0;
         if (DEPTH > 1 && ts->unit[0] < total_units) issue(locate(ts->unit[0]), 0, 0);
         for (;; ++k) {
@@ -3481,8 +3486,9 @@ __global__ void __launch_bounds__(256, MC_TEAM_MIN_BLOCKS) k_render_team(const _
         }
     }
     // the general pass: the envs that the common path left
+    constexpr int kGeneral = COMMON ? MC_ER_SLOW : MC_ER_SLOW | MC_ER_BURIED;
     if (claimer) {
-        ts->sunit[0] = *(volatile int32_t*)&rk.flags[MC_FLAG_ANY_SLOW] ? claim(MC_FLAG_SLOW_WORK) : total_units;
+        ts->sunit[0] = !COMMON || *(volatile int32_t*)&rk.flags[MC_FLAG_ANY_SLOW] ? claim(MC_FLAG_SLOW_WORK) : total_units;
         team_unit_reset(ts, 0);
     }
     team_sync(bar, nthr);
@@ -3502,9 +3508,11 @@ __global__ void __launch_bounds__(256, MC_TEAM_MIN_BLOCKS) k_render_team(const _
             const EnvRec q = load_rec(recs_of(t.g), t.i);
             bits = q.bits;
             env = q.env;
-            here = t.part == 0 && (q.bits & MC_ER_SLOW);
+            here = t.part == 0 && (q.bits & kGeneral);
             use_group(t.g);
-            if (here) {
+            if (!COMMON && (q.bits & MC_ER_BURIED)) {
+                fill_env<FAM, F32>(p, q.env, q.fill_blk, cx, t.coop ? wt * 32 + lane : lane, t.coop ? nthr : 32);
+            } else if (here) {
                 const int8_t* world = staged_world(t, q, 0);
                 const bool staged = may_stage && landed(t, 0);
                 timed_out = may_stage && !staged;
@@ -3520,7 +3528,7 @@ __global__ void __launch_bounds__(256, MC_TEAM_MIN_BLOCKS) k_render_team(const _
     }
     // timed-out copies may still be in flight: let them land (bounded) before
     // this warp's part of shared memory can be released
-    for (int d = 0; d < DEPTH; ++d) {
+    for (int d = 0; d < SLOTS; ++d) {
         if ((tlive >> d) & 1u) mbar_wait(tmbar + 8 * d, (tphase >> d) & 1u);
         if ((wlive >> d) & 1u) mbar_wait(cx.mbar_a + 8 * d, (wphase >> d) & 1u);
     }
@@ -3697,11 +3705,13 @@ static int launch_team_t(const mc_ragged_kp* rk, int warps_per_cta, int ctas_per
         rc = launch_pdl(k_agent_groups<FAM>, rk->ablock[G], kAgentThreads, 0, s, *rk);
     }
     if (rc) return rc;
-    const bool deep = rk->depth == 2;
-    auto kern = deep ? k_render_team<FAM, F32, 2> : k_render_team<FAM, F32, 1>;
+    bool common = false;
+    for (int g = 0; g < G; ++g) common |= rk->groups[g].fast_ok != 0;
+    const int which = !common ? 0 : (rk->depth == 2 ? 2 : 1);
+    auto kern = which == 0 ? k_render_team<FAM, F32, 0> : (which == 2 ? k_render_team<FAM, F32, 2> : k_render_team<FAM, F32, 1>);
     size_t smem = (size_t)rk->warps_off + (size_t)warps_per_cta * rk->warp_bytes + (size_t)rk->tail_bytes;
-    static mc_once_per_device limit[2];  // per kernel of this instantiation
-    rc = allow_smem(limit[deep], kern, smem);
+    static mc_once_per_device limit[3];  // per kernel of this instantiation
+    rc = allow_smem(limit[which], kern, smem);
     if (rc) return rc;
     const int teams_per_cta = warps_per_cta / rk->team_warps;
     long long ctas_needed = (rk->ustart[rk->ngroups] + teams_per_cta - 1) / teams_per_cta;
