@@ -2451,6 +2451,9 @@ __device__ __forceinline__ EnvRec agent_step(const mc_kp& p, const ActionSrc& ac
 // after its image, with no pass over all worlds and no kernel of its own.
 // Which worlds (p.regen): none, all of them when any env of the group is done
 // (MC_KREGEN_ALL; the agent kernel has settled that), or the done envs' own.
+// Launches without the common path leave it to a kernel after them (their
+// worlds are big beside their images: 1024 envs 80^3 8x8 of which one in 30 is
+// done, 170 us a step, 116 with a kernel of its own).
 __device__ __forceinline__ int regen_any(const mc_kp& p) {
     return p.regen == MC_KREGEN_ALL
                ? __shfl_sync(0xffffffffu, *(volatile int32_t*)&p.flags[MC_FLAG_ANY_DONE], 0) : 0;
@@ -3155,7 +3158,10 @@ __global__ void __launch_bounds__(256, MC_FUSED_MIN_BLOCKS)
     if (lane == 0) {
         bounds_to_flags(p.flags);
         // every claim of this warp has returned (the last one >= B)
-        if (p.sched_dynamic) finish_dynamic(p.flags, total_warps, [&] { p.flags[MC_FLAG_ANY_DONE] = 0; });
+        if (p.sched_dynamic)
+            finish_dynamic(p.flags, total_warps, [&] {
+                if (p.regen != MC_KREGEN_NONE) p.flags[MC_FLAG_ANY_DONE] = 0;
+            });
     }
 }
 
@@ -3537,7 +3543,8 @@ __global__ void __launch_bounds__(256, MC_TEAM_MIN_BLOCKS) k_render_team(const _
     }
     if (claimer)
         finish_dynamic(rk.flags, total_teams, [&] {
-            for (int g = 0; g < G; ++g) rk.groups[g].flags[MC_FLAG_ANY_DONE] = 0;
+            for (int g = 0; g < G; ++g)
+                if (rk.groups[g].regen != MC_KREGEN_NONE) rk.groups[g].flags[MC_FLAG_ANY_DONE] = 0;
         });
 }
 
@@ -3602,6 +3609,16 @@ static int warp_fast(const mc_kp& p, const mc_fused_cfg& cfg) {
     return warp_smem(p, cfg, fast) > 227 * 1024 ? 0 : fast;
 }
 
+// The shape as it is launched: small worlds that no shape can ask to stage are staged where they fit.
+static mc_fused_cfg warp_stage(const mc_kp& p, const mc_fused_cfg& cfg) {
+    mc_fused_cfg f = cfg;
+    if (!f.stage && mc_odd_world(p) && mc_world_slot(p) <= 8192 + 16) {  // as default_launch stages the others
+        f.stage = 1;
+        if (warp_smem(p, f, warp_fast(p, f)) > 227 * 1024) f.stage = 0;
+    }
+    return f;
+}
+
 static size_t fused_smem(const mc_kp* p, const mc_fused_cfg* cfg) { return warp_smem(*p, *cfg, warp_fast(*p, *cfg)); }
 
 // A launch whose kernel waits for its predecessor itself (pdl_wait), so that
@@ -3658,12 +3675,8 @@ static int launch_warp_t(const mc_kp* p, const mc_fused_cfg* cfg, int slices, lo
 template <int FAM, bool F32>
 static int launch_fused_f(const mc_kp* kp, const mc_fused_cfg* cfg, int num_sms, cudaStream_t s) {
     mc_kp p = *kp;
-    mc_fused_cfg f = *cfg;
+    mc_fused_cfg f = warp_stage(p, *cfg);
     cfg = &f;
-    if (!f.stage && mc_odd_world(p) && mc_world_slot(p) <= 8192 + 16) {  // as default_launch stages the others
-        f.stage = 1;
-        if (fused_smem(&p, &f) > 227 * 1024) f.stage = 0;
-    }
     p.fast_ok = warp_fast(p, f);
     const int wpc = cfg->warps_per_cta;
     long long grid = (long long)num_sms * (cfg->ctas_per_sm > 0 ? cfg->ctas_per_sm : 1);
@@ -3735,6 +3748,9 @@ static int step_team(const mc_ragged_kp* rk, int family, int obs_f32, int warps_
         default: return (int)cudaErrorInvalidValue;
     }
 }
+
+// Whether the per-warp launch of this shape has the images' common path.
+static int fused_common(const mc_kp* p, const mc_fused_cfg* cfg) { return warp_fast(*p, warp_stage(*p, *cfg)) != 0; }
 
 static int step_fused(const mc_kp* p, const mc_fused_cfg* cfg, int num_sms, cudaStream_t s) {
     if (p->B == 0) return 0;

@@ -81,6 +81,10 @@ MC_HIDDEN void team_layout(const mc_kp* const* kps, int G, const int* stage, con
                            int team_warps, int warps_per_cta, int ctas_per_sm, mc_ragged_kp* rk);
 // Dynamic shared memory of that launch per CTA.
 MC_HIDDEN long long team_smem(const mc_ragged_kp& rk, int warps_per_cta);
+// A step of the laid-out groups, and the regeneration of those whose worlds its
+// images do not regenerate.  Returns a cudaError_t.
+MC_HIDDEN int step_team_regen(const mc_backend* be, const mc_ragged_kp* rk, int warps_per_cta, int ctas_per_sm,
+                              int num_sms, cudaStream_t s);
 // An env's launch shape as one group of a launch that holds many (the server's).
 MC_HIDDEN mc_fused_cfg mc_shared_launch(const mc_env* e);
 // MC_OK, or MC_ERR_INVALID with a message when the team launch is not possible.

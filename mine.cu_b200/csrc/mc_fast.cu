@@ -19,6 +19,7 @@ static const mc_backend g_backend = {
     interact_launch,
     coalesced_launch,
     fused_smem,
+    fused_common,
     step_team,
     bounds_report,
     bounds_selftest,

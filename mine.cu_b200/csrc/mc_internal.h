@@ -114,7 +114,8 @@ struct mc_kp {
     void* rec;    // fused form: the agent kernel's render records, MC_REC_BYTES each
     int fast_ok;  // fused form: the launch has the images' common path (set per launch)
     int compact;  // fused form: records filed marching envs first (set per launch)
-    int regen;    // fused form: MC_KREGEN_*, worlds the launch's images regenerate (set per launch)
+    int regen;    // fused form: MC_KREGEN_*, worlds the launch's images regenerate (set per launch; none
+                  // where a kernel after it does)
     int fresh;    // ... and show regenerated (a reset; a step's images show the worlds before it)
     int look_only;  // fused form: images without a step (reset, get_obs)
 };
@@ -270,6 +271,8 @@ struct mc_backend {
     int (*render_coalesced)(const int8_t* vox_yxzb, const float* basis, uint8_t* out, int B, int ws,
                             int W, int H, int max_steps, cudaStream_t s);
     size_t (*fused_smem_bytes)(const mc_kp* p, const mc_fused_cfg* cfg);
+    // whether the per-warp launch of this shape has the images' common path
+    int (*fused_common)(const mc_kp* p, const mc_fused_cfg* cfg);
     // the team kernel over rk's groups: grid = SMs x ctas_per_sm (at most one unit per team)
     int (*step_team)(const mc_ragged_kp* rk, int family, int obs_f32, int warps_per_cta, int ctas_per_sm,
                      int num_sms, cudaStream_t s);

@@ -474,7 +474,8 @@ static void team_layout_as(const mc_kp* const* kps, int G, const int* stage, con
         rk->groups[g] = k;
         const int fast = common ? mc_fast_launch(k, stage[g], tile_w[g]) : 0;
         rk->groups[g].fast_ok = fast;
-        rk->groups[g].regen = step_regen(k);
+        // (step_team_regen takes the groups without a common path)
+        rk->groups[g].regen = fast ? step_regen(k) : (int)MC_KREGEN_NONE;
         rk->slices[g] = 1;
         rk->start[g] = start;
         start += k.B;
@@ -608,6 +609,17 @@ int team_validate(const mc_kp* const* kps, int G, const int* stage, const int* t
     const long long smem = team_smem(rk, warps_per_cta);
     if (smem > 227 * 1024) return fail(MC_ERR_INVALID, "team kernel shared memory %lld > 227 KB", smem);
     return MC_OK;
+}
+
+int step_team_regen(const mc_backend* be, const mc_ragged_kp* rk, int warps_per_cta, int ctas_per_sm, int num_sms,
+                    cudaStream_t s) {
+    const mc_kp& k0 = rk->groups[0];
+    int rc = be->step_team(rk, k0.family, k0.obs_f32, warps_per_cta, ctas_per_sm, num_sms, s);
+    for (int g = 0; g < rk->ngroups && !rc; ++g) {
+        const mc_kp& k = rk->groups[g];
+        if (k.B && !k.fast_ok && step_regen(k) != MC_KREGEN_NONE) rc = mc_launch_regen(&k, 1, s);
+    }
+    return rc;
 }
 
 static bool team_mode(const mc_fused_cfg& f) { return f.team_warps > 1 || f.coop; }
@@ -918,23 +930,41 @@ extern "C" int mc_env_generate_world(mc_env* e, void* stream) {
     return backend_rc(mc_launch_regen(&e->kp, 0, (cudaStream_t)stream), "regen");
 }
 
+// Whether the fused launch of this env's shape over k has the images' common
+// path (*rk: its layout, when a team launch).
+static bool launch_common(const mc_env* e, const mc_kp& k, mc_ragged_kp* rk) {
+    const mc_fused_cfg& f = e->fcfg;
+    if (!team_mode(f)) return e->be->fused_common(&k, &f) != 0;
+    const mc_kp* kps[1] = {&k};
+    team_layout(kps, 1, &f.stage, &f.tile_w, &f.coop, f.team_warps, f.warps_per_cta, f.ctas_per_sm, rk);
+    return rk->groups[0].fast_ok != 0;
+}
+
 // One launch of the fused form over the env's batch: k holds what differs
 // from e->kp (actions, result buffers, regeneration, family).
 static int launch_fused(mc_env* e, const mc_kp& k, cudaStream_t s, const char* what) {
     const mc_fused_cfg& f = e->fcfg;
-    if (!team_mode(f)) return backend_rc(e->be->step_fused(&k, &f, e->num_sms, s), what);
-    const mc_kp* kps[1] = {&k};
     mc_ragged_kp rk;
-    team_layout(kps, 1, &f.stage, &f.tile_w, &f.coop, f.team_warps, f.warps_per_cta, f.ctas_per_sm, &rk);
-    rk.groups[0].regen = k.regen;
-    rk.flags = e->flags;
-    rk.rec = e->rec;
-    rk.rewards_cat = k.res_rewards;
-    rk.dones_cat = k.res_dones;
-    rk.actions = k.actions;
-    rk.buttons = k.buttons;
-    rk.look = k.look;
-    return backend_rc(e->be->step_team(&rk, k.family, k.obs_f32, f.warps_per_cta, f.ctas_per_sm, e->num_sms, s), what);
+    // regenerated by a kernel of its own (unless the images show the worlds regenerated)
+    const bool after = !launch_common(e, k, &rk) && k.regen != MC_KREGEN_NONE && !k.fresh;
+    int rc;
+    if (!team_mode(f)) {
+        mc_kp p = k;
+        if (after) p.regen = MC_KREGEN_NONE;
+        rc = e->be->step_fused(&p, &f, e->num_sms, s);
+    } else {
+        rk.groups[0].regen = after ? (int)MC_KREGEN_NONE : k.regen;
+        rk.flags = e->flags;
+        rk.rec = e->rec;
+        rk.rewards_cat = k.res_rewards;
+        rk.dones_cat = k.res_dones;
+        rk.actions = k.actions;
+        rk.buttons = k.buttons;
+        rk.look = k.look;
+        rc = e->be->step_team(&rk, k.family, k.obs_f32, f.warps_per_cta, f.ctas_per_sm, e->num_sms, s);
+    }
+    if (rc || !after) return backend_rc(rc, what);
+    return backend_rc(mc_launch_regen(&k, 1, s), "regen");
 }
 
 // Cameras and images without a step; regen: the worlds regenerated first.
@@ -1593,9 +1623,7 @@ static int ragged_do_step(mc_ragged* r, const int8_t* buttons, const float* look
     rk.actions = actions;
     rk.buttons = buttons;
     rk.look = look;
-    return backend_rc(r->be->step_team(&rk, r->family, r->obs_f32, r->cfg.warps_per_cta, r->cfg.ctas_per_sm,
-                                       r->num_sms, s),
-                      "step_team");
+    return backend_rc(step_team_regen(r->be, &rk, r->cfg.warps_per_cta, r->cfg.ctas_per_sm, r->num_sms, s), "step_team");
 }
 
 extern "C" int mc_ragged_step(mc_ragged* r, const int8_t* buttons, const float* look, void* stream) {

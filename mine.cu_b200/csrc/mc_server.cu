@@ -380,8 +380,7 @@ int run_round(mc_server* s, Slot& sl, const std::vector<Req*>& reqs, const std::
             rk.actions = d_act;
             rk.rewards_cat = d_rew;
             rk.dones_cat = d_done;
-            const mc_kp& k0 = *kps[0];
-            rc = s->be->step_team(&rk, k0.family, k0.obs_f32, 8, cps, s->num_sms, st);
+            rc = step_team_regen(s->be, &rk, 8, cps, s->num_sms, st);
             if (rc) return mc_cuda_fail((cudaError_t)rc, "server: step launch");
         } else {
             Req* r = reqs[steps[0]];
