@@ -3661,6 +3661,10 @@ static int slices_of(long long B, int bands, long long warps) {
     return n;
 }
 
+static int warp_slices(const mc_kp& p, const mc_fused_cfg& f, int num_sms) {
+    return slices_of(p.B, (p.H * f.tile_w + 31) / 32, (long long)num_sms * std::max(f.ctas_per_sm, 1) * f.warps_per_cta);
+}
+
 template <int FAM, bool F32, bool STAGE>
 static int launch_warp_t(const mc_kp* p, const mc_fused_cfg* cfg, int slices, long long grid, cudaStream_t s) {
     auto kern = k_render_warp<FAM, F32, STAGE>;
@@ -3680,7 +3684,7 @@ static int launch_fused_f(const mc_kp* kp, const mc_fused_cfg* cfg, int num_sms,
     p.fast_ok = warp_fast(p, f);
     const int wpc = cfg->warps_per_cta;
     long long grid = (long long)num_sms * (cfg->ctas_per_sm > 0 ? cfg->ctas_per_sm : 1);
-    const int slices = p.fast_ok ? slices_of(p.B, (p.H * cfg->tile_w + 31) / 32, grid * wpc) : 1;
+    const int slices = p.fast_ok ? warp_slices(p, f, num_sms) : 1;
     const long long units = (long long)p.B * slices;
     p.compact = p.sched_dynamic && units > grid * wpc;
     // static striding: four waves of CTAs, so that warps whose envs are cheap make
@@ -3749,8 +3753,10 @@ static int step_team(const mc_ragged_kp* rk, int family, int obs_f32, int warps_
     }
 }
 
-// Whether the per-warp launch of this shape has the images' common path.
-static int fused_common(const mc_kp* p, const mc_fused_cfg* cfg) { return warp_fast(*p, warp_stage(*p, *cfg)) != 0; }
+static int fused_common(const mc_kp* p, const mc_fused_cfg* cfg, int num_sms) {
+    const mc_fused_cfg f = warp_stage(*p, *cfg);
+    return warp_fast(*p, f) ? warp_slices(*p, f, num_sms) : 0;
+}
 
 static int step_fused(const mc_kp* p, const mc_fused_cfg* cfg, int num_sms, cudaStream_t s) {
     if (p->B == 0) return 0;

@@ -59,6 +59,7 @@ struct mc_env {
     std::vector<RolloutGraph> graphs;
     HostIO* hio;
     cudaEvent_t host_done;  // after the last host-buffer step that used the caller's buffers in place
+    int images[2] = {-1, -1};  // whether get_obs, reset render through the image kernels (-1: not settled)
     int regen_mode;  // MC_REGEN_ALL (the reference's rule) or MC_REGEN_PER_ENV
 };
 

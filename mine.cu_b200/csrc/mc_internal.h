@@ -271,8 +271,8 @@ struct mc_backend {
     int (*render_coalesced)(const int8_t* vox_yxzb, const float* basis, uint8_t* out, int B, int ws,
                             int W, int H, int max_steps, cudaStream_t s);
     size_t (*fused_smem_bytes)(const mc_kp* p, const mc_fused_cfg* cfg);
-    // whether the per-warp launch of this shape has the images' common path
-    int (*fused_common)(const mc_kp* p, const mc_fused_cfg* cfg);
+    // units of the per-warp launch of this shape per env where it has the images' common path, else 0
+    int (*fused_common)(const mc_kp* p, const mc_fused_cfg* cfg, int num_sms);
     // the team kernel over rk's groups: grid = SMs x ctas_per_sm (at most one unit per team)
     int (*step_team)(const mc_ragged_kp* rk, int family, int obs_f32, int warps_per_cta, int ctas_per_sm,
                      int num_sms, cudaStream_t s);

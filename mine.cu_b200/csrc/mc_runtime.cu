@@ -904,6 +904,7 @@ extern "C" int mc_env_set_state(mc_env* e, const mc_env_state* s) {
     e->kp.wait_polls = polls;
     e->kp.regen_per_env = e->regen_mode == MC_REGEN_PER_ENV;
     e->kp.sched_dynamic = 1;
+    e->images[0] = e->images[1] = -1;
     drop_graphs(e);
     return MC_OK;
 }
@@ -930,14 +931,19 @@ extern "C" int mc_env_generate_world(mc_env* e, void* stream) {
     return backend_rc(mc_launch_regen(&e->kp, 0, (cudaStream_t)stream), "regen");
 }
 
-// Whether the fused launch of this env's shape over k has the images' common
-// path (*rk: its layout, when a team launch).
-static bool launch_common(const mc_env* e, const mc_kp& k, mc_ragged_kp* rk) {
+// Warps that work on the images at a time in the fused launch of this env's
+// shape over k, 0 where it has no common path (*rk: its layout, when a team launch).
+static long long launch_common(const mc_env* e, const mc_kp& k, mc_ragged_kp* rk) {
     const mc_fused_cfg& f = e->fcfg;
-    if (!team_mode(f)) return e->be->fused_common(&k, &f) != 0;
-    const mc_kp* kps[1] = {&k};
-    team_layout(kps, 1, &f.stage, &f.tile_w, &f.coop, f.team_warps, f.warps_per_cta, f.ctas_per_sm, rk);
-    return rk->groups[0].fast_ok != 0;
+    long long warps;
+    if (!team_mode(f)) {
+        warps = (long long)k.B * e->be->fused_common(&k, &f, e->num_sms);
+    } else {
+        const mc_kp* kps[1] = {&k};
+        team_layout(kps, 1, &f.stage, &f.tile_w, &f.coop, f.team_warps, f.warps_per_cta, f.ctas_per_sm, rk);
+        warps = rk->groups[0].fast_ok ? rk->ustart[1] * f.team_warps : 0;
+    }
+    return std::min(warps, (long long)e->num_sms * f.ctas_per_sm * f.warps_per_cta);
 }
 
 // One launch of the fused form over the env's batch: k holds what differs
@@ -967,19 +973,44 @@ static int launch_fused(mc_env* e, const mc_kp& k, cudaStream_t s, const char* w
     return backend_rc(mc_launch_regen(&k, 1, s), "regen");
 }
 
+// Whether reset() or get_obs() renders through the step's image kernels, with
+// `warps` (launch_common) at work; else by the per-pixel kernel after the
+// regeneration, a thread a ray over the worlds in global memory.  Launches
+// without the common path march like that one, with fewer rays in flight.  With
+// it, many warps or short queues are quicker: us, per-pixel / image kernels, get_obs:
+// 1024 envs 16^3 64x64 86 / 37, 64 envs 32^3 128x96 (2048 warps, 12 tiles each) 55 / 36,
+// 64 envs 16^3 84x84 (1024 warps, 14 tiles each) 19 / 27 but 32^3 37 / 32, one env 32^3
+// 200x120 (16 warps) 19 / 52; 8192 envs 32^3 8x8 (two tiles each) 60 / 82; reset
+// (whose images regenerate the worlds too): 64 envs 16^3 200x120 65 / 63, one env 28
+// / 68; one env 80^3 200x120 45 / 676, but 64 envs 48^3 8x8 (worlds that could be staged,
+// marched from global memory for their few rays) 43 / 31.
+static bool obs_by_images(const mc_env* e, long long warps, bool reset) {
+    const mc_fused_cfg& f = e->fcfg;
+    const int tw = f.tile_w, th = 32 / tw, W = e->cfg.render_width, H = e->cfg.render_height;
+    const long long B = e->cfg.batch_size, tiles = B * ((W + tw - 1) / tw) * ((H + th - 1) / th);
+    const long long wxyz = (long long)e->cfg.world_x * e->cfg.world_y * e->cfg.world_z;
+    if (!warps) return reset && wxyz > 32768 && wxyz <= kSmemPerCta && 512LL * W * H < wxyz && !e->kp.dbg_pixel;
+    if (!reset && W * H < 128 && B > 1024) return false;
+    return tiles <= 4 * warps || warps >= (reset ? 512 : (wxyz >= 32768 ? 1024 : 2048));
+}
+
 // Cameras and images without a step; regen: the worlds regenerated first.
 // MineEnv._render always uses the shaded kernel: float32 for "float32",
-// render_uint8 for every uint8 mode (minecu/__init__.py:455-464).  The images
-// come from the step's image kernels: at 4096 envs, 16^3, 64x64 a step, a
-// masked reset and the policy's input take 233 us, with the per-pixel kernel
-// 448.
+// render_uint8 for every uint8 mode (minecu/__init__.py:455-464).  At 4096 envs,
+// 16^3, 64x64 a step, a masked reset and the policy's input take 233 us through
+// the image kernels, with the per-pixel kernel 448.
 // Images so wide that a warp's band of no tile shape fits shared memory (uint8
-// rows of several thousand pixels) have no fused launch: the per-pixel kernel
-// renders them.
+// rows of several thousand pixels) have no fused launch either.
 static int render_obs(mc_env* e, cudaStream_t s, int regen) {
     mc_kp k = e->kp;
     if (k.B == 0) return MC_OK;
-    if (mc_env_fused_smem_bytes(e) > kSmemPerCta) {
+    k.family = MC_FAM_SHADED;
+    const bool reset = regen != MC_KREGEN_NONE;
+    if (e->images[reset] < 0) {  // settled once for this shape and state
+        mc_ragged_kp rk;
+        e->images[reset] = obs_by_images(e, launch_common(e, k, &rk), reset) && mc_env_fused_smem_bytes(e) <= kSmemPerCta;
+    }
+    if (!e->images[reset]) {
         if (regen != MC_KREGEN_NONE) {
             const int rc = backend_rc(mc_launch_regen(&k, 1, s), "regen");
             if (rc) return rc;
@@ -988,7 +1019,6 @@ static int render_obs(mc_env* e, cudaStream_t s, int regen) {
         MC_CK(cudaGetLastError());
         return backend_rc(e->be->render(&k, MC_FAM_SHADED, s), "render");
     }
-    k.family = MC_FAM_SHADED;
     k.look_only = 1;
     k.regen = regen;
     k.fresh = 1;
@@ -1363,6 +1393,7 @@ extern "C" int mc_env_set_fused_config(mc_env* e, const mc_fused_config* c) {
     int rc = validate_fused(e, &f);
     if (rc) return rc;
     e->fcfg = f;
+    e->images[0] = e->images[1] = -1;
     return MC_OK;
 }
 
