@@ -734,7 +734,8 @@ static mc_fused_cfg default_launch(const mc_env_config* cfg, const mc_kp* kp, co
         f.warps_per_cta = 8;
         f.stage = (wxyz <= 8192 && aligned) ? 1 : 0;
         f.ctas_per_sm = 4;
-        f.tile_w = tiles <= 4096 && W * H >= 256 && mc_fast_launch(*kp, 1, 8) ? tile(tiles <= 1024 ? 32 : 16) : 4;
+        const bool wide = tiles <= 400 || (tiles <= 4096 && W * H >= 256);  // (256 envs 8x8, 512 tiles: 15.8 us wide, 15.4)
+        f.tile_w = wide && mc_fast_launch(*kp, 1, 8) ? tile(tiles <= 1024 ? 32 : 16) : 4;
         f.team_warps = 1;
         f.coop = 0;
     }
