@@ -2667,21 +2667,6 @@ __device__ __forceinline__ void team_sync(int bar, int nthreads) {
 }
 
 
-// The same barrier, with the team's answer to whether any of its threads says v.
-__device__ __forceinline__ bool team_any(int bar, int nthreads, bool v) {
-    if (nthreads == 32) return __any_sync(0xffffffffu, v);
-    int any;
-    asm volatile(
-        "{\n\t.reg .pred p, q;\n\t"
-        "setp.ne.s32 p, %3, 0;\n\t"
-        "barrier.cta.red.or.pred q, %1, %2, p;\n\t"
-        "selp.s32 %0, 1, 0, q;\n\t}"
-        : "=r"(any)
-        : "r"(bar), "r"(nthreads), "r"((int)v)
-        : "memory");
-    return any;
-}
-
 // Where the staged copy of the world at src lies in its slot: at src's offset
 // from a 16-byte boundary, so that a bulk copy can move its whole chunks.
 __device__ __forceinline__ int8_t* staged_at(int8_t* slot, const int8_t* src) { return slot + ((uintptr_t)src & 15u); }
@@ -3197,6 +3182,9 @@ struct TeamShared {
     int band_ctr[2];       // next row band of the cooperative env of unit k & 1
     unsigned long long mbar[2];
     unsigned sunit[2];     // general pass: claimed units, alternating slots
+    int lost;              // the unit (the team's k-th; kGeneralUnit + k in the general pass) whose wait for a copy
+                           // ran out: no further copies, render from global memory.  A warp compares it with
+                           // its own unit, so what warps ahead of it write there does not count yet.
     int any_done;          // bit g: every world of group g is to be regenerated
     int last;              // the team rendered its env's last slice
     int pad;
@@ -3205,6 +3193,7 @@ struct TeamShared {
     unsigned long long ump[2], umm[2];
 };
 static_assert(sizeof(TeamShared) <= MC_TEAM_HEAD_BYTES, "team head");
+constexpr int kGeneralUnit = 1 << 30;
 
 __device__ __forceinline__ void team_unit_reset(TeamShared* ts, int d) {
     ts->band_ctr[d] = 0;
@@ -3313,6 +3302,7 @@ __global__ void __launch_bounds__(256, MC_TEAM_MIN_BLOCKS) k_render_team(const _
     pdl_trigger();
     pdl_wait();
     if (claimer) {
+        ts->lost = 0x7fffffff;
         for (int k = 0; k < DEPTH; ++k) ts->unit[k] = claim(MC_FLAG_WORK);
         int any = 0;
         for (int g = 0; g < G; ++g)
@@ -3373,14 +3363,17 @@ __global__ void __launch_bounds__(256, MC_TEAM_MIN_BLOCKS) k_render_team(const _
     auto staged_world = [&](const Unit& t, const EnvRec& q, int d) -> const int8_t* {
         return staged_at(slot_world(d, t.coop), world_of(rk.groups[t.g], q.env, q.bits, (ts->any_done >> t.g) & 1));
     };
-    // Wait for the copy of unit t into depth slot d; false: no further copies,
-    // render from global memory (team_any tells the team).
-    auto landed = [&](const Unit& t, int d) -> bool {
+    // Wait for the copy of unit t, the team's number n, into depth slot d.
+    auto landed = [&](const Unit& t, int d, int n) -> bool {
         const mc_kp& p = rk.groups[t.g];
-        if (!stage_fits(slot_world(d, t.coop), mc_world_slot(p))) return false;
+        if (!stage_fits(slot_world(d, t.coop), mc_world_slot(p))) {
+            *(volatile int*)&ts->lost = n;
+            return false;
+        }
         uint32_t& ph = t.coop ? tphase : wphase;
         if (!mbar_wait((t.coop ? tmbar : cx.mbar_a) + 8 * d, (ph >> d) & 1u, p.wait_polls)) {
             if (lane == 0) atomicExch(&p.flags[MC_FLAG_ERROR], MC_KERR_TMA_TIMEOUT);
+            *(volatile int*)&ts->lost = n;
             return false;
         }
         ph ^= 1u << d;
@@ -3407,14 +3400,9 @@ __global__ void __launch_bounds__(256, MC_TEAM_MIN_BLOCKS) k_render_team(const _
         regen_world(p, e, wt * 32 + lane, nthr);
     };
 
-    // The end of the team's unit k: the next claim, the unit's barrier, and whether a warp's wait ran out.
-    auto end_unit = [&](int k, bool timed_out) -> bool {
-        if (claimer) ts->unit[(k + DEPTH) & 3] = claim(MC_FLAG_WORK);
-        return team_any(bar, nthr, timed_out);
-    };
-    bool redo = false;  // the same for the whole team
     if constexpr (COMMON) {
         int k = 0;
+        bool redo = false;
         if (DEPTH > 1 && ts->unit[0] < total_units) issue(locate(ts->unit[0]), 0, 0);
         for (;; ++k) {
             const int d = DEPTH > 1 ? (k & 1) : 0;  // world slot and mbarrier of this unit
@@ -3440,7 +3428,7 @@ __global__ void __launch_bounds__(256, MC_TEAM_MIN_BLOCKS) k_render_team(const _
                         fill_env<FAM, F32>(p, q.env, q.fill_blk, cx, t.coop ? wt * 32 + lane : lane,
                                            t.coop ? nthr : 32);
                 } else if (!(q.bits & MC_ER_SLOW)) {
-                    const bool ok = landed(t, d);
+                    const bool ok = landed(t, d, k);
                     const int8_t* world = staged_world(t, q, d);
                     EnvRender r = render_of_rec(q, p.wy);
                     if (t.coop && TWN > 1 && up_scan_shape(p.wx, p.wy, p.wz))  // team-uniform; the eye is in the box
@@ -3449,16 +3437,17 @@ __global__ void __launch_bounds__(256, MC_TEAM_MIN_BLOCKS) k_render_team(const _
                                               bar);
                     else if (ok)
                         measure_staged(r, world, p.wx, p.wy, p.wz, lane);
-                    if (!ok) {
-                        redo = end_unit(k, true);
-                        break;
-                    }
-                    render_fast<FAM, F32, true>(p, q.env, r, cx, world, rk.tile_w[t.g], lane,
-                                              t.coop ? &ts->band_ctr[k & 1] : nullptr, t.part, rk.slices[t.g]);
+                    if (ok)
+                        render_fast<FAM, F32, true>(p, q.env, r, cx, world, rk.tile_w[t.g], lane,
+                                                    t.coop ? &ts->band_ctr[k & 1] : nullptr, t.part, rk.slices[t.g]);
                 }
             }
-            redo = end_unit(k, false);
-            if (redo) break;
+            if (claimer) ts->unit[(k + DEPTH) & 3] = claim(MC_FLAG_WORK);
+            team_sync(bar, nthr);
+            if (*(volatile int*)&ts->lost <= k) {  // the same for the whole team
+                redo = true;
+                break;
+            }
             if (!(bits & MC_ER_SLOW)) regen(t, bits, env, true);
         }
         // a copy timed out: this unit again and the rest of the team's, from global memory
@@ -3498,17 +3487,15 @@ __global__ void __launch_bounds__(256, MC_TEAM_MIN_BLOCKS) k_render_team(const _
         team_unit_reset(ts, 0);
     }
     team_sync(bar, nthr);
-    bool stage_ok = !redo;  // the same for the whole team
     for (int k = 0;; ++k) {
         const unsigned u = ts->sunit[k & 1];
         if (u >= total_units) break;
         const Unit t = locate(u);
         const mc_kp& p = rk.groups[t.g];
-        const bool may_stage = ((rk.stage_mask >> t.g) & 1) && stage_ok;
+        const bool may_stage = ((rk.stage_mask >> t.g) & 1) && *(volatile int*)&ts->lost >= kGeneralUnit + k;
         if (may_stage && t.part == 0) issue(t, 0, MC_ER_SLOW);
         if (claimer) team_unit_reset(ts, (k + 1) & 1);
         int bits = 0, env = 0;
-        bool timed_out = false;
         bool here = false;  // this unit's env is rendered in this pass (the first slice's unit renders all of it)
         if (t.mine) {
             const EnvRec q = load_rec(recs_of(t.g), t.i);
@@ -3520,8 +3507,7 @@ __global__ void __launch_bounds__(256, MC_TEAM_MIN_BLOCKS) k_render_team(const _
                 fill_env<FAM, F32>(p, q.env, q.fill_blk, cx, t.coop ? wt * 32 + lane : lane, t.coop ? nthr : 32);
             } else if (here) {
                 const int8_t* world = staged_world(t, q, 0);
-                const bool staged = may_stage && landed(t, 0);
-                timed_out = may_stage && !staged;
+                const bool staged = may_stage && landed(t, 0, kGeneralUnit + k);
                 const int ytop = staged ? staged_top_layer(world, p.wx, p.wy, p.wz, lane) : p.wy - 1;
                 render_slow<FAM, F32>(p, q, ytop, cx, staged ? world : nullptr,
                                       world_of(p, q.env, q.bits, (ts->any_done >> t.g) & 1), rk.tile_w[t.g], lane,
@@ -3529,7 +3515,7 @@ __global__ void __launch_bounds__(256, MC_TEAM_MIN_BLOCKS) k_render_team(const _
             }
         }
         if (claimer) ts->sunit[(k + 1) & 1] = claim(MC_FLAG_SLOW_WORK);
-        stage_ok &= !team_any(bar, nthr, timed_out);
+        team_sync(bar, nthr);
         if (here) regen(t, bits, env, false);
     }
     // timed-out copies may still be in flight: let them land (bounded) before
