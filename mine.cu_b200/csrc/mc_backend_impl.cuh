@@ -2928,7 +2928,7 @@ __device__ __forceinline__ void render_fast(const mc_kp& p, int e, const EnvRend
 // each funnelled from the two of the template it lies across, and the bytes
 // before and after them.  (A byte a thread left a warp's 4680-byte world at 147
 // rounds of a load and a store: a reset of 64 envs 9x40x13 took 42 us.)
-__device__ __noinline__ void regen_odd(int8_t* d, const int8_t* t, int n, int t0, int nt) {
+__device__ __forceinline__ void regen_odd(int8_t* d, const int8_t* t, int n, int t0, int nt) {
     const int head = min((int)(-(uint32_t)(uintptr_t)d & 3u), n), words = (n - head) >> 2, tail = (n - head) & 3;
     if (t0 < head) d[t0] = t[t0];
     if (t0 < tail) d[n - tail + t0] = t[n - tail + t0];
