@@ -53,7 +53,7 @@ RENDER_METRIC = "env-steps/s at B=4096, W=32, 64x64, half break actions (fused s
 TRAFFIC = {
     "peak": (120.2e6 + 55.1e6, "k_agent + k_render_warp, step 701, profiles/k_render_warp_peak_late.md"),
     "render": (135.7e6 + 26.3e6, "k_agent + k_render_team, step 301, profiles/k_render_team_B4096_w32_r64.md"),
-    "ragged": (174.6e6 + 69.0e6, "k_agent_groups + k_render_team, mean of the first 15 steps after a reset, "
+    "ragged": (160.1e6 + 67.5e6, "k_agent_groups + k_render_team, mean of steps 5..54 (the timed window), "
                "profiles/k_render_team_ragged_launches.md"),
 }
 

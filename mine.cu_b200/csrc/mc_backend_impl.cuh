@@ -2033,7 +2033,7 @@ __device__ __forceinline__ UpBounds staged_up_bounds(const int8_t* world, int wx
 // TEAM: the team kernel stages float32 pixels two tiles at a time instead (64
 // pixels, 768 bytes, whose row pieces are whole 16-byte chunks; with ODD they go
 // straight to dst): beside 32 KB worlds, whole bands of 128-pixel rows (6 KB a
-// warp) left one CTA on an SM (4096 envs 32^3 128x128: 1151 -> 713 us a step).
+// warp) left one CTA on an SM (4096 envs 32^3 128x128: 1151 -> 710 us a step).
 // The per-warp kernel keeps whole bands (32x32: 174 us a step, two tiles 186).
 struct FastEnv {
     const int4* start;  // per sign combination: packed (index|counts, dx, dy, dz) or split (counts, dax, day, daz)
@@ -3173,10 +3173,10 @@ __global__ void __launch_bounds__(256, MC_FUSED_MIN_BLOCKS)
 // copy started before unit k is rendered, so it overlaps that render (one
 // claim further ahead, twice the shared memory).
 //
-// A warp whose wait for a copy runs out records the timeout, never reads a
-// staged world again and renders its bands from global memory; in the shared
-// scan it stands in for its share of the layers with bounds that cut
-// nothing, so the others' results stay exact.
+// A warp whose wait for a copy runs out records the timeout; in the shared scan
+// it stands in for its share of the layers with bounds that cut nothing, so
+// the others' results stay exact.  After the unit's barrier its whole team draws
+// that unit again and the rest of its units from global memory.
 struct TeamShared {
     unsigned unit[4];      // claimed units, unit k's number at k & 3
     int band_ctr[2];       // next row band of the cooperative env of unit k & 1

@@ -41,10 +41,8 @@ enum {
     MC_SITE_MARCH_PACKED = 5,  // PTX packed march: load address vs the staged world +- one layer
     MC_SITE_MARCH_SPLIT = 6,   // PTX split march: the same
     MC_SITE_MARCH_SMEM = 7,    // PTX marches: load address vs the CTA's dynamic shared memory
-    MC_SITE_BAND = 8,          // a pixel's bytes in the shared-memory band
     MC_SITE_COPY_OUT = 9,      // a band's bytes in the env's observation
     MC_SITE_DEBUG = 10,        // per-pixel debug code
-    MC_SITE_PATCH = 11,        // the interaction's voxel patched into the staged world
     MC_SITE_TABLE = 12,        // u/v tables, colour tables
     MC_SITE_STAGE = 13,        // a bulk copy's destination vs the CTA's dynamic shared memory
     MC_SITE_SCAN = 14,         // a staged world's rows read by the up-bounds scan
@@ -111,7 +109,8 @@ struct mc_kp {
     // written here, in env order (the host-buffer step's read-back buffer)
     float* res_rewards;
     uint8_t* res_dones;
-    void* rec;    // fused form: the agent kernel's render records, MC_REC_BYTES each
+    void* rec;    // fused form: the agent kernel's render records, MC_REC_BYTES each (NULL: the images
+                  // settle them from the state, the stateless step)
     int fast_ok;  // fused form: the launch has the images' common path (set per launch)
     int compact;  // fused form: records filed marching envs first (set per launch)
     int regen;    // fused form: MC_KREGEN_*, worlds the launch's images regenerate (set per launch; none

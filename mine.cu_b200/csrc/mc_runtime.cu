@@ -532,7 +532,11 @@ static void team_layout_as(const mc_kp* const* kps, int G, const int* stage, con
         const long long B = kps[g]->B;
         rk->ustart[v + 1] = rk->ustart[v] + (coop[g] ? B * rk->slices[g] : (B + team_warps - 1) / team_warps);
     }
-    for (int g = 0; g < G; ++g) rk->groups[g].compact = rk->ustart[G] > 512;  // more units than a grid's teams
+    // records filed by cost, where most teams get several units (us a step, in order
+    // / by cost: 16^3 64x64 200 envs 21.2 / 21.7, 400 envs (1600 units) 24.4 / 23.4, 3000 envs
+    // 68.4 / 66.0; 32^3 64x64 400 envs 41.0 / 41.4, 1500 envs 89.5 / 90.0, 3000 envs 151.0 / 150.0)
+    const bool compact = rk->ustart[G] > 512;
+    for (int g = 0; g < G; ++g) rk->groups[g].compact = compact;
     rk->slot_bytes = slot;
     rk->tables_off = MC_COLOUR_TABLE_BYTES + MC_FAST_TABLE_BYTES;
     rk->teams_off = rk->tables_off + align16i((long long)uv * 4);

@@ -340,7 +340,7 @@ int run_batch(mc_server* s, Slot& sl, const std::vector<Req*>& reqs) {
 }
 
 // One round's step requests (at most one per job, one render family) as one
-// team launch plus the conditional regenerations.
+// team launch, whose images regenerate most worlds (step_team_regen).
 int run_round(mc_server* s, Slot& sl, const std::vector<Req*>& reqs, const std::vector<size_t>& steps,
               cudaStream_t st) {
     int rc = MC_OK;
@@ -367,7 +367,13 @@ int run_round(mc_server* s, Slot& sl, const std::vector<Req*>& reqs, const std::
                 any_coop |= coop[g] != 0;
             }
             const int team = any_coop ? 4 : 1, cps = any_coop ? 3 : 4;
-            // the staged worlds do not fit together: those above 32 KB give way first
+            // The staged worlds do not fit together: those above 32 KB give way first.
+            // (While they fit they are staged, although a launch with a 40^3 job then has
+            // one CTA an SM instead of three, for its other jobs too: us a round, staged /
+            // from global memory, 4 jobs of 2048 envs 16^3 32x32 with one of 256 envs 40^3
+            // 64x64 203 / 347, 4 of 4096 with one of 16 228 / 334, 2 of 1024 envs 32^3 64x64 with
+            // one of 256 266 / 453, 6 of 1024 envs 16^3 64x64 with one of 8 283 / 379; one 40^3
+            // job alone 195 / 357.)
             for (const long long most : {32768LL, 0LL}) {
                 if (team_validate(kps.data(), G, stage, tile_w, coop, team, 8, cps) == MC_OK) break;
                 for (int g = 0; g < G; ++g)
