@@ -2934,7 +2934,7 @@ __device__ __forceinline__ void regen_odd(int8_t* d, const int8_t* t, int n, int
     if (t0 < tail) d[n - tail + t0] = t[n - tail + t0];
     const uint32_t* s4 = reinterpret_cast<const uint32_t*>(t);
     uint32_t* d4 = reinterpret_cast<uint32_t*>(d + head);
-#pragma unroll 4
+#pragma unroll 1
     for (int k = t0; k < words; k += nt)
         d4[k] = __funnelshift_r(__ldg(s4 + k), head ? __ldg(s4 + k + 1) : 0u, 8 * head);
 }
