@@ -2939,7 +2939,11 @@ __device__ __forceinline__ void regen_odd(int8_t* d, const int8_t* t, int n, int
         d4[k] = __funnelshift_r(__ldg(s4 + k), head ? __ldg(s4 + k + 1) : 0u, 8 * head);
 }
 
-// The template's bytes over env e's world, by nt threads.
+// The template's bytes over env e's world, by nt threads.  WORDS: worlds of no whole
+// 16 bytes by regen_odd (the per-warp kernel); the team kernel's four or eight
+// warps take them a byte a thread, since the words cost its other launches 1% (six
+// ragged groups 240.7 -> 242.9 us a step).
+template <bool WORDS>
 __device__ __forceinline__ void regen_world(const mc_kp& p, int e, int t, int nt) {
     const int wxyz = p.wx * p.wy * p.wz;
     int8_t* d = p.voxels + e * (long long)wxyz;
@@ -2950,7 +2954,10 @@ __device__ __forceinline__ void regen_world(const mc_kp& p, int e, int t, int nt
         const uint4* t4 = reinterpret_cast<const uint4*>(p.world_template);
         for (int k = t; k < (wxyz >> 4); k += nt) d4[k] = __ldg(t4 + k);
     } else {
-        regen_odd(d, p.world_template, wxyz, t, nt);
+        if (WORDS)
+            regen_odd(d, p.world_template, wxyz, t, nt);
+        else
+            for (int k = t; k < wxyz; k += nt) d[k] = p.world_template[k];
     }
 }
 // Whether this warp is the last of its env's slices to get here (all of them
@@ -3021,7 +3028,7 @@ __device__ __noinline__ void warp_rest(const mc_kp& p, int tile_w, int slices, i
                                       nullptr);
             else if (part == 0)
                 fill_env<FAM, F32>(p, q.env, q.fill_blk, cx, lane, 32);
-            if (regen_env(p, q.bits, any_done) && last_slice(recs, i, slices, lane)) regen_world(p, q.env, lane, 32);
+            if (regen_env(p, q.bits, any_done) && last_slice(recs, i, slices, lane)) regen_world<true>(p, q.env, lane, 32);
         }
     }
     // the general pass: the envs that the common path left (every env of a
@@ -3057,7 +3064,7 @@ __device__ __noinline__ void warp_rest(const mc_kp& p, int tile_w, int slices, i
                 }
                 render_slow<FAM, F32>(p, q, ytop, cx, staged ? staged_at(sworld, world) : nullptr, world, tile_w, lane, nullptr);
             }
-            if (regen_env(p, q.bits, any_done)) regen_world(p, q.env, lane, 32);
+            if (regen_env(p, q.bits, any_done)) regen_world<true>(p, q.env, lane, 32);
         }
     }
     // a timed-out copy may still be in flight: let it land (bounded, with the
@@ -3132,7 +3139,7 @@ __global__ void __launch_bounds__(256, MC_FUSED_MIN_BLOCKS)
                 measure_staged(r, world, p.wx, p.wy, p.wz, lane);
                 render_fast<FAM, F32, false>(p, q.env, r, cx, world, tile_w, lane, nullptr, part, slices);
             }
-            if (regen_env(p, q.bits, any_done) && last_slice(recs, i, slices, lane)) regen_world(p, q.env, lane, 32);
+            if (regen_env(p, q.bits, any_done) && last_slice(recs, i, slices, lane)) regen_world<true>(p, q.env, lane, 32);
         }
         state |= (phase & 1u) | (phase & 2u) << 2;
     }
@@ -3386,7 +3393,7 @@ __global__ void __launch_bounds__(256, MC_TEAM_MIN_BLOCKS) k_render_team(const _
         if (!t.mine || !regen_env(rk.groups[t.g], bits, (ts->any_done >> t.g) & 1)) return;
         const mc_kp& p = rk.groups[t.g];
         if (!t.coop) {
-            regen_world(p, e, lane, 32);
+            regen_world<false>(p, e, lane, 32);
             return;
         }
         if (sliced && rk.slices[t.g] > 1) {  // team-uniform
@@ -3397,7 +3404,7 @@ __global__ void __launch_bounds__(256, MC_TEAM_MIN_BLOCKS) k_render_team(const _
             team_sync(bar, nthr);
             if (!ts->last) return;
         }
-        regen_world(p, e, wt * 32 + lane, nthr);
+        regen_world<false>(p, e, wt * 32 + lane, nthr);
     };
 
     if constexpr (COMMON) {
