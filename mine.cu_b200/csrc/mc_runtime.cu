@@ -988,13 +988,16 @@ static int launch_fused(mc_env* e, const mc_kp& k, cudaStream_t s, const char* w
 // 200x120 (16 warps) 19 / 52; 8192 envs 32^3 8x8 (two tiles each) 60 / 82; reset
 // (whose images regenerate the worlds too): 64 envs 16^3 200x120 65 / 63, one env 28
 // / 68; one env 80^3 200x120 45 / 676, but 64 envs 48^3 8x8 (worlds that could be staged,
-// marched from global memory for their few rays) 43 / 31.
+// marched from global memory for their few rays) 43 / 31, 1024 envs 64^3 64x64 392 / 306
+// and 128x16x128 341 / 309 (80^3 457 / 583).
 static bool obs_by_images(const mc_env* e, long long warps, bool reset) {
     const mc_fused_cfg& f = e->fcfg;
     const int tw = f.tile_w, th = 32 / tw, W = e->cfg.render_width, H = e->cfg.render_height;
     const long long B = e->cfg.batch_size, tiles = B * ((W + tw - 1) / tw) * ((H + th - 1) / th);
     const long long wxyz = (long long)e->cfg.world_x * e->cfg.world_y * e->cfg.world_z;
-    if (!warps) return reset && wxyz > 32768 && wxyz <= kSmemPerCta && 512LL * W * H < wxyz && !e->kp.dbg_pixel;
+    if (!warps)
+        return reset && wxyz > 32768 && !e->kp.dbg_pixel &&
+               ((wxyz <= kSmemPerCta && 512LL * W * H < wxyz) || (wxyz <= 262144 && B * W * H >= 1LL << 22));
     if (!reset && W * H < 128 && B > 1024) return false;
     return tiles <= 4 * warps || warps >= (reset ? 512 : (wxyz >= 32768 ? 1024 : 2048));
 }

@@ -48,7 +48,8 @@ def _walk(g, o, B, seed, steps=3):
                                            (1, (9, 40, 13), (120, 64)), (64, (16, 16, 16), (64, 64)),
                                            (40, (16, 16, 16), (84, 84)), (3, (48, 48, 48), (8, 8)),
                                            (2, (70, 16, 66), (24, 20)), (2, (64, 64, 64), (32, 32)),
-                                           (1100, (16, 16, 16), (8, 8))])
+                                           (1100, (16, 16, 16), (8, 8)),
+                                           (180, (66, 24, 60), (160, 152))])
 def test_images_of_both_routes(cuda, mode, B, world, res):
     g, o = _pair(cuda, B, world, res, obs_dtype=mode)
     _walk(g, o, B, 121)
