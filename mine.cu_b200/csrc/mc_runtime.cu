@@ -140,6 +140,20 @@ __global__ void k_place_house(int8_t* vox, int B, int wx, int wy, int wz, int hx
         for (int dz = 0; dz < D; ++dz) house_set(w, wx, wy, wz, hx, hz, gh, H, dx, dz, BRICK);
 }
 
+// n bytes of the template t (4-byte aligned, allocated to a multiple of 16) to a
+// world d that starts at any byte, by the block: the world's aligned words, each
+// funnelled from the two of the template it lies across, and the bytes beside them.
+__device__ __forceinline__ void copy_odd(int8_t* d, const int8_t* t, int n) {
+    const int t0 = threadIdx.x, nt = blockDim.x;
+    const int head = min((int)(-(uint32_t)(uintptr_t)d & 3u), n), words = (n - head) >> 2, tail = (n - head) & 3;
+    if (t0 < head) d[t0] = t[t0];
+    if (t0 < tail) d[n - tail + t0] = t[n - tail + t0];
+    const uint32_t* s4 = reinterpret_cast<const uint32_t*>(t);
+    uint32_t* d4 = reinterpret_cast<uint32_t*>(d + head);
+    for (int k = t0; k < words; k += nt)
+        d4[k] = __funnelshift_r(__ldg(s4 + k), head ? __ldg(s4 + k + 1) : 0u, 8 * head);
+}
+
 // Regenerate every world from the template (generate + tree + house give the
 // same bytes for every env, so one generated world is broadcast).  With
 // `conditional`, nothing is written unless flags[ANY_DONE] is set.  The last
@@ -165,8 +179,7 @@ __global__ void k_regen(int8_t* vox, const int8_t* tmpl, int B, int wxyz, int32_
             }
         } else {
             for (long long b = blockIdx.x; b < B; b += gridDim.x) {
-                int8_t* d = vox + b * (long long)wxyz;
-                for (int k = threadIdx.x; k < wxyz; k += blockDim.x) d[k] = tmpl[k];
+                copy_odd(vox + b * (long long)wxyz, tmpl, wxyz);
             }
         }
     }
@@ -279,8 +292,7 @@ __global__ void k_regen_masked(int8_t* vox, const int8_t* tmpl, const uint8_t* d
             const uint4* t4 = reinterpret_cast<const uint4*>(tmpl);
             for (int k = threadIdx.x; k < (wxyz >> 4); k += blockDim.x) d4[k] = __ldg(t4 + k);
         } else {
-            int8_t* d = vox + b * (long long)wxyz;
-            for (int k = threadIdx.x; k < wxyz; k += blockDim.x) d[k] = tmpl[k];
+            copy_odd(vox + b * (long long)wxyz, tmpl, wxyz);
         }
     }
 }
@@ -460,6 +472,11 @@ constexpr long long kSmemPerCta = 227 * 1024;  // an SM's 228 KB hold each CTA's
 
 static inline int align16i(long long x) { return (int)((x + 15) & ~15LL); }
 
+// Whether a kernel after a team launch's step regenerates the worlds of group k
+// (laid out), not its teams: without the common path (big worlds beside their
+// images), and worlds of no whole 16 bytes, which the team kernel has no words for.
+static bool regen_after_team(const mc_kp& k) { return !k.fast_ok || mc_odd_world(k); }
+
 // common: whether the images may take their common path (mc_fast_launch).
 static void team_layout_as(const mc_kp* const* kps, int G, const int* stage, const int* tile_w, const int* coop,
                            int team_warps, int warps_per_cta, bool common, mc_ragged_kp* rk) {
@@ -474,8 +491,7 @@ static void team_layout_as(const mc_kp* const* kps, int G, const int* stage, con
         rk->groups[g] = k;
         const int fast = common ? mc_fast_launch(k, stage[g], tile_w[g]) : 0;
         rk->groups[g].fast_ok = fast;
-        // (step_team_regen takes the groups without a common path)
-        rk->groups[g].regen = fast ? step_regen(k) : (int)MC_KREGEN_NONE;
+        rk->groups[g].regen = regen_after_team(rk->groups[g]) ? (int)MC_KREGEN_NONE : step_regen(k);
         rk->slices[g] = 1;
         rk->start[g] = start;
         start += k.B;
@@ -621,7 +637,7 @@ int step_team_regen(const mc_backend* be, const mc_ragged_kp* rk, int warps_per_
     int rc = be->step_team(rk, k0.family, k0.obs_f32, warps_per_cta, ctas_per_sm, num_sms, s);
     for (int g = 0; g < rk->ngroups && !rc; ++g) {
         const mc_kp& k = rk->groups[g];
-        if (k.B && !k.fast_ok && step_regen(k) != MC_KREGEN_NONE) rc = mc_launch_regen(&k, 1, s);
+        if (k.B && regen_after_team(k) && step_regen(k) != MC_KREGEN_NONE) rc = mc_launch_regen(&k, 1, s);
     }
     return rc;
 }
@@ -957,7 +973,8 @@ static int launch_fused(mc_env* e, const mc_kp& k, cudaStream_t s, const char* w
     const mc_fused_cfg& f = e->fcfg;
     mc_ragged_kp rk;
     // regenerated by a kernel of its own (unless the images show the worlds regenerated)
-    const bool after = !launch_common(e, k, &rk) && k.regen != MC_KREGEN_NONE && !k.fresh;
+    const bool common = launch_common(e, k, &rk) != 0;
+    const bool after = k.regen != MC_KREGEN_NONE && !k.fresh && (team_mode(f) ? regen_after_team(rk.groups[0]) : !common);
     int rc;
     if (!team_mode(f)) {
         mc_kp p = k;
