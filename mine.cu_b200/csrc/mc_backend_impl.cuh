@@ -2453,7 +2453,8 @@ __device__ __forceinline__ EnvRec agent_step(const mc_kp& p, const ActionSrc& ac
 // (MC_KREGEN_ALL; the agent kernel has settled that), or the done envs' own.
 // Launches without the common path leave it to a kernel after them (their
 // worlds are big beside their images: 1024 envs 80^3 8x8 of which one in 30 is
-// done, 170 us a step, 116 with a kernel of its own).
+// done, 170 us a step, 116 with a kernel of its own), and so do team launches
+// over worlds of no whole 16 bytes (6153 envs 25x22x39 119.9 -> 81.9).
 __device__ __forceinline__ int regen_any(const mc_kp& p) {
     return p.regen == MC_KREGEN_ALL
                ? __shfl_sync(0xffffffffu, *(volatile int32_t*)&p.flags[MC_FLAG_ANY_DONE], 0) : 0;
@@ -2940,9 +2941,10 @@ __device__ __forceinline__ void regen_odd(int8_t* d, const int8_t* t, int n, int
 }
 
 // The template's bytes over env e's world, by nt threads.  WORDS: worlds of no whole
-// 16 bytes by regen_odd (the per-warp kernel); the team kernel's four or eight
-// warps take them a byte a thread, since the words cost its other launches 1% (six
-// ragged groups 240.7 -> 242.9 us a step).
+// 16 bytes by regen_odd (the per-warp kernel); the team kernel, which has them in
+// resets only (a kernel after its steps regenerates them), takes a byte a thread,
+// since the words' code cost its other launches 1% (six ragged groups 240.7 -> 242.9
+// us a step).
 template <bool WORDS>
 __device__ __forceinline__ void regen_world(const mc_kp& p, int e, int t, int nt) {
     const int wxyz = p.wx * p.wy * p.wz;
