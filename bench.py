@@ -7,7 +7,7 @@ limit; synthetic discrete actions uniform over the 11 actions from a seeded
 Philox4x32-10 stream (seed 1; counter = (global env, step)).
 
 Metric: env-steps/s (B x steps x GPUs / time), higher is better.
-  value  the fused step (one persistent kernel per step) of K steps captured
+  value  the fused step (agents, then images) of K steps captured
          in a CUDA graph, actions resident in HBM, timed with CUDA events on
          the launching stream, max over ranks.
   e2e    MineEnv.step(actions) through the public API, every step copying
