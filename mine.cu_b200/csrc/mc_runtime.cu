@@ -475,7 +475,11 @@ static inline int align16i(long long x) { return (int)((x + 15) & ~15LL); }
 // Whether a kernel after a team launch's step regenerates the worlds of group k
 // (laid out), not its teams: without the common path (big worlds beside their
 // images), and worlds of no whole 16 bytes, which the team kernel has no words for.
-static bool regen_after_team(const mc_kp& k) { return !k.fast_ok || mc_odd_world(k); }
+// The kernel costs each step 2.4 us, so not for the few envs of which seldom one is
+// done (2 envs 41x23x42 47x60, one in 60: 20.6 us a step with it, 18.2 without; 188
+// envs 15x29x45 9x48, one in 120: 23.5, 27.1).
+constexpr int kRegenKernelEnvs = 48;  // with more
+static bool regen_after_team(const mc_kp& k) { return (!k.fast_ok || mc_odd_world(k)) && k.B > kRegenKernelEnvs; }
 
 // common: whether the images may take their common path (mc_fast_launch).
 static void team_layout_as(const mc_kp* const* kps, int G, const int* stage, const int* tile_w, const int* coop,
@@ -974,7 +978,7 @@ static int launch_fused(mc_env* e, const mc_kp& k, cudaStream_t s, const char* w
     mc_ragged_kp rk;
     // regenerated by a kernel of its own (unless the images show the worlds regenerated)
     const bool common = launch_common(e, k, &rk) != 0;
-    const bool after = k.regen != MC_KREGEN_NONE && !k.fresh && (team_mode(f) ? regen_after_team(rk.groups[0]) : !common);
+    const bool after = k.regen != MC_KREGEN_NONE && !k.fresh && (team_mode(f) ? regen_after_team(rk.groups[0]) : !common && k.B > kRegenKernelEnvs);
     int rc;
     if (!team_mode(f)) {
         mc_kp p = k;

@@ -10,11 +10,13 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("regen", ["all", "per_env"])
 @pytest.mark.parametrize("world, res, cfg", [((70, 16, 66), (24, 20), None), ((64, 64, 64), (16, 16), None),
+                                             ((25, 22, 39), (24, 24), None),
                                              ((16, 16, 16), (32, 32), (0, 8, 4, 4, 1, 0)),
                                              ((32, 32, 32), (32, 32), (0, 8, 3, 8, 4, 1))])
 def test_worlds_regenerated_after_the_images(cuda, regen, world, res, cfg):
     T.run(cuda, 7, 9, 111, world=world, res=res, regen=regen, cfg=cfg, obs_dtype="uint8", episode_length=3)
-    T.run(cuda, 40, 7, 112, world=world, res=(8, 8), regen=regen, cfg=cfg, obs_dtype="uint8_minimal", episode_length=4)
+    for B in (48, 49, 70):  # by the images, and by the kernel after them
+        T.run(cuda, B, 5, 112, world=world, res=(8, 8), regen=regen, cfg=cfg, obs_dtype="uint8_minimal", episode_length=4)
 
 
 @pytest.mark.parametrize("regen", ["all", "per_env"])
@@ -22,7 +24,7 @@ def test_groups_with_and_without_a_common_path(cuda, regen):
     import torch
     from minecu import MineEnv, _C
     from minecu.ragged import RaggedBatch
-    groups = [(33, (16, 16, 16), 32, 4), (5, (70, 16, 70), 24, 3), (9, (64, 64, 64), 16, 5), (21, (8, 8, 8), 16, None)]
+    groups = [(33, (16, 16, 16), 32, 4), (53, (70, 16, 70), 24, 3), (60, (25, 22, 39), 24, 4), (9, (64, 64, 64), 16, 5), (21, (8, 8, 8), 16, None)]
 
     def make():
         return [MineEnv(batch_size=b, world_x=w[0], world_y=w[1], world_z=w[2], render_width=r, render_height=r,
