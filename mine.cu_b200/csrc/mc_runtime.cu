@@ -477,9 +477,14 @@ static inline int align16i(long long x) { return (int)((x + 15) & ~15LL); }
 // images), and worlds of no whole 16 bytes, which the team kernel has no words for.
 // The kernel costs each step 2.4 us, so not for the few envs of which seldom one is
 // done (2 envs 41x23x42 47x60, one in 60: 20.6 us a step with it, 18.2 without; 188
-// envs 15x29x45 9x48, one in 120: 23.5, 27.1).
+// envs 15x29x45 9x48, one in 120: 23.5, 27.1), nor for odd worlds of up to 2 KB, a
+// dozen bytes a thread (148 envs 22x6x11 64x64 67.1 us with it, 64.3 without; 745 envs
+// 26x10x11 16x16 20.6, 22.4).
 constexpr int kRegenKernelEnvs = 48;  // with more
-static bool regen_after_team(const mc_kp& k) { return (!k.fast_ok || mc_odd_world(k)) && k.B > kRegenKernelEnvs; }
+static bool regen_after_team(const mc_kp& k) {
+    const bool odd = mc_odd_world(k) && (long long)k.wx * k.wy * k.wz > 2048;
+    return (!k.fast_ok || odd) && k.B > kRegenKernelEnvs;
+}
 
 // common: whether the images may take their common path (mc_fast_launch).
 static void team_layout_as(const mc_kp* const* kps, int G, const int* stage, const int* tile_w, const int* coop,
